@@ -40,6 +40,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -251,6 +252,25 @@ struct PairView {
     uint32_t dead;
 };
 
+// Groups of length-1 candidates that are the same function of the state on
+// every output the run compares (CUDA semantics, per dead-flags mask): one
+// member stands for all of them in the join's table and in every survivor
+// record, and k_emit_all gives each passing record's rules member by member.
+// At mask 0xFF the 600,000 targets that change no live output each match 779
+// candidates that change none either (CMP, CPX and CPY with any operand, the
+// flag instructions); they fall into 8 records instead, and the full length-2
+// enumeration at that mask, which is bound by the records it verifies, takes
+// 21.4 ms instead of 441 (0.74 ns of it per record before, 482 M of them).
+struct CandGroups {
+    uint16_t mult[kNumInsns];    // members of the group that candidate c stands for (0: another stands for c)
+    uint16_t first[kNumInsns];   // index of its first member in `member`
+    uint16_t member[kNumInsns];  // candidate indices, group by group
+};
+
+__device__ __forceinline__ uint32_t surv_weight(uint32_t code, const uint16_t* mult) {
+    return mult && !(code & kSurvLen2) ? mult[code & 0x7FFFFFu] : 1u;
+}
+
 // Pair sources: survivors of the enumeration pipeline, or explicit CSR pairs.
 struct SurvSource {
     const Surv* surv;
@@ -258,6 +278,7 @@ struct SurvSource {
     uint32_t tlen;
     uint32_t run_dead;
     int go;
+    const uint16_t* mult;   // CandGroups::mult of the run's mask, or null: every record is one pair
     __device__ void load(uint64_t p, uint16_t* st, uint16_t* sc, int& tn, int& cn, uint32_t& dead,
                          int lane) const {
         Surv s = surv[p];
@@ -276,6 +297,8 @@ struct SurvSource {
     __device__ bool probed(uint64_t p) const { return (surv[p].c & kSurvProbed) != 0; }
     // Pairs with the same id share their target (the probe reuses its outputs).
     __device__ uint64_t target_id(uint64_t p) const { return surv[p].t; }
+    // Pairs that record p stands for.
+    __device__ uint32_t weight(uint64_t p) const { return surv_weight(surv[p].c, mult); }
 };
 
 struct CsrSource {
@@ -295,6 +318,7 @@ struct CsrSource {
     }
     __device__ bool probed(uint64_t) const { return false; }
     __device__ uint64_t target_id(uint64_t) const { return kNoTarget; }
+    __device__ uint32_t weight(uint64_t) const { return 1u; }
 };
 
 // Decode parameters of one cone sweep.  State index bits: A (8, if in the
@@ -1051,7 +1075,8 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
                                                   const uint8_t* __restrict__ cmeta, const uint64_t* __restrict__ skeys,
                                                   const uint16_t* __restrict__ sidx, uint32_t nsorted, uint32_t dead,
                                                   uint32_t stages, Surv* __restrict__ surv, uint64_t cap,
-                                                  Counters* __restrict__ cnt, uint32_t probe) {
+                                                  Counters* __restrict__ cnt, uint32_t probe,
+                                                  const uint16_t* __restrict__ mult) {
     __shared__ uint64_t s_key[kNumInsns];
     __shared__ uint64_t s_tprobe[PROBE ? kWarpsPerBlock : 1][2][32];   // target outputs on the probe states
     __shared__ uint16_t s_idx[kNumInsns];
@@ -1156,9 +1181,10 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
                 bool pass = false;
                 uint32_t code = c;
                 if (!GO) {
-                    nqc += lane == 0;
+                    const uint32_t m1 = mult[c];   // candidates this one stands for
+                    nqc += lane == 0 ? m1 : 0u;
                     const bool mid = !(stages & M6502_CHECK_MID) || lo_eq == kFull;
-                    if (mid) { nmid += lane == 0; pass = true; }
+                    if (mid) { nmid += lane == 0 ? m1 : 0u; pass = true; }
                     if (PROBE && pass && probe) {
                         if (!tp_ready) {
                             tp_sw = __reduce_or_sync(kFull, lane < (int)tlen ? (uint32_t)c_sweep[ins & 0xFFu] : 0u);
@@ -1188,7 +1214,7 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
                                 }
                                 differ = __any_sync(kFull, ((tout ^ pack(ps)) & m) != 0);
                             }
-                            if (differ) { pass = false; nprobe_rej += lane == 0; }
+                            if (differ) { pass = false; nprobe_rej += lane == 0 ? m1 : 0u; }
                             else code |= kSurvProbed;
                         }
                     }
@@ -1455,7 +1481,7 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
             const uint32_t sw = sw_t | sw_c;   // swept extra registers
             const bool prep = a.sweep == M6502_SWEEP_REFERENCE && __popc(sw) >= 3;
             if (!probe_pair(pv, sw_t, sw_c, prep, tid, p, tc, lane)) {
-                if (lane == 0) { a.fail[p] = 1u; probe_rej++; }
+                if (lane == 0) { a.fail[p] = 1u; probe_rej += src.weight(p); }
                 __syncwarp();
                 continue;
             }
@@ -1577,7 +1603,7 @@ __global__ void __launch_bounds__(256) k_probe_pairs(Src src, const unsigned lon
             __syncwarp();
         }
         if (!pass) {
-            if (lane == 0) { a.fail[p] = 1u; probe_rej++; }
+            if (lane == 0) { a.fail[p] = 1u; probe_rej += src.weight(p); }
         } else {
             if (lane == 0) s_pass[w][npass] = (uint32_t)p;
             __syncwarp();
@@ -1632,41 +1658,62 @@ __device__ __forceinline__ unsigned long long algo_ops(const uint16_t* t, uint32
     return (1ull << bits) * (unsigned long long)(10 * (tn + cn) + 3);
 }
 
-// CUDA semantics: every passing survivor is a rule; its target is ids[t], or
-// tbase + t (the pass-local index made global) without ids.
+// CUDA semantics: every pair of a passing record is a rule; its target is
+// ids[t], or tbase + t (the pass-local index made global) without ids.  The
+// rules of a record that stands for several candidates are written by the
+// whole warp, one member per lane.
 __global__ void k_emit_all(const Surv* __restrict__ surv, const unsigned long long* n_ptr, uint64_t n_cap,
                            const uint32_t* __restrict__ fail, const uint64_t* __restrict__ ids, uint64_t tbase,
                            uint32_t run_dead, m6502_rule* __restrict__ rules, uint64_t rcap,
                            unsigned long long* rule_ctr, Counters* cnt, int check_exh,
-                           const uint16_t* __restrict__ targets, uint32_t tlen, uint32_t sweep_mode) {
+                           const uint16_t* __restrict__ targets, uint32_t tlen, uint32_t sweep_mode,
+                           const CandGroups* __restrict__ groups) {
     const uint64_t n = min((uint64_t)*n_ptr, n_cap);
     const int lane = threadIdx.x & 31;
+    const uint16_t* mult = groups ? groups->mult : nullptr;
     unsigned long long npass = 0, algo = 0, nund = 0;
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t p = base + threadIdx.x;
         bool pass = p < n && (!check_exh || fail[p] == 0);
-        nund += (p < n && check_exh && fail[p] == 3u) ? 1u : 0u;   // left undecided: counted, not a rule
+        const Surv s = p < n ? surv[p] : Surv{0, 0};
+        const uint32_t w = p < n ? surv_weight(s.c, mult) : 0u;
+        nund += (p < n && check_exh && fail[p] == 3u) ? w : 0u;   // left undecided: counted, not a rule
         m6502_rule r;
         memset(&r, 0, sizeof r);
+        const uint32_t idx = s.c & 0x7FFFFFu;
         if (pass) {
-            Surv s = surv[p];
-            uint32_t idx = s.c & 0x7FFFFFu;
             r.target = ids ? ids[s.t] : tbase + s.t;
             r.dead_flags = (uint8_t)run_dead;
             if (s.c & kSurvLen2) { r.cand_len = 2; r.cand[0] = c_tab[idx / kNumInsns]; r.cand[1] = c_tab[idx % kNumInsns]; }
             else { r.cand_len = 1; r.cand[0] = c_tab[idx]; }
-            npass++;
-            if (check_exh) algo += algo_ops(targets + (uint64_t)s.t * tlen, tlen, r.cand, r.cand_len, sweep_mode);
+            npass += w;
+            if (check_exh) algo += w * algo_ops(targets + (uint64_t)s.t * tlen, tlen, r.cand, r.cand_len, sweep_mode);
         }
-        unsigned vote = __ballot_sync(kFull, pass);
-        if (vote) {
-            int leader = __ffs(vote) - 1;
-            unsigned long long b = 0;
-            if (lane == leader) b = atomicAdd(rule_ctr, (unsigned long long)__popc(vote));
-            b = __shfl_sync(kFull, b, leader);
-            if (pass) {
-                unsigned long long idx = b + __popc(vote & ((1u << lane) - 1u));
-                if (idx < rcap) rules[idx] = r;
+        const unsigned vote = __ballot_sync(kFull, pass);
+        if (!vote) continue;
+        uint32_t at = pass ? w : 0u;   // inclusive running count of the warp's rules
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(kFull, at, o);
+            at += lane >= o ? x : 0u;
+        }
+        unsigned long long b = 0;
+        if (lane == 31) b = atomicAdd(rule_ctr, (unsigned long long)at);
+        b = __shfl_sync(kFull, b, 31);
+        if (rcap == 0) continue;       // counted only
+        const unsigned long long mine = b + at - (pass ? w : 0u);
+        if (pass && w == 1 && mine < rcap) rules[mine] = r;
+        for (unsigned many = __ballot_sync(kFull, pass && w > 1); many; many &= many - 1) {
+            const int l = __ffs(many) - 1;
+            const uint32_t mw = __shfl_sync(kFull, w, l), c = __shfl_sync(kFull, idx, l);
+            const unsigned long long m0 = __shfl_sync(kFull, mine, l);
+            m6502_rule q;
+            memset(&q, 0, sizeof q);
+            q.target = __shfl_sync(kFull, (unsigned long long)r.target, l);
+            q.dead_flags = (uint8_t)run_dead;
+            q.cand_len = 1;
+            for (uint32_t j = lane; j < mw; j += 32) {
+                q.cand[0] = c_tab[groups->member[groups->first[c] + j]];
+                if (m0 + j < rcap) rules[m0 + j] = q;
             }
         }
     }
@@ -2050,10 +2097,12 @@ struct m6502_ctx {
     std::vector<uint64_t> h_cfp8;     // QC-vector outputs [8][2863] (host copy)
     DevBuf cfp1cm;                    // candidate-major fingerprints [2863][32]
     std::vector<uint8_t> h_cmeta;
+    std::vector<uint16_t> h_tab;      // instructions, CUDA order (host copy)
     DevBuf go_keys, go_keys2, go_ord, go_round, go_sort_tmp;   // Go-order verification rounds
     DevBuf jitems;                                             // chunks of long length-2 equal ranges
     DevBuf order;                                              // k_probe_pairs: the pairs it passed on
-    DevBuf join_keys[256], join_idx[256];
+    DevBuf join_keys[2][256], join_idx[2][256];   // by semantics and dead-flags mask
+    DevBuf join_groups[256];                      // CandGroups of the CUDA-semantics tables
     struct Cand2Table {            // sorted (key, index) of all length-2 sequences for one mask
         uint32_t dead = 0xFFFFFFFFu;
         DevBuf keys, idx;
@@ -2061,7 +2110,7 @@ struct m6502_ctx {
     } cand2[4];                    // least recently used mask is rebuilt
     uint64_t cand2_clock = 0;
     DevBuf c2_keys_in, c2_idx_in, c2_sort_tmp;
-    uint32_t join_n[256] = {};
+    uint32_t join_n[2][256] = {};
     DevBuf st_tins, st_toffs, st_tout, st_tbytes, st_chains, st_entries, st_vidx, st_proven, st_cnt, st_pidx,
         st_mex, st_probs, st_traj, st_row;
     DevBuf st_keys, st_keys2, st_vals2, st_rep, st_ord, st_verdict, st_vlist, st_vpos, st_sort_tmp, st_vphase,
@@ -2132,21 +2181,28 @@ int launch_exh(m6502_ctx* ctx, const SurvSource& src, const unsigned long long* 
     return M6502_OK;
 }
 
+const uint16_t* join_mult(const m6502_ctx* ctx, uint32_t dead) {
+    const CandGroups* g = (const CandGroups*)ctx->join_groups[dead].p;
+    return g ? g->mult : nullptr;
+}
+
 // The length-1 QuickCheck join under CUDA semantics, with the probe of its
 // MidCheck survivors when `probe` (1 + the sweep mode) is set.
 int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt, uint32_t dead, uint32_t stages,
                  uint64_t scap, Counters* cnt, uint32_t probe) {
     const uint32_t jgrid = (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 8, (nt + kWarpsPerBlock - 1) / kWarpsPerBlock);
-    const uint64_t* jk = (const uint64_t*)ctx->join_keys[dead].p;
-    const uint16_t* ji = (const uint16_t*)ctx->join_idx[dead].p;
+    const uint64_t* jk = (const uint64_t*)ctx->join_keys[0][dead].p;
+    const uint16_t* ji = (const uint16_t*)ctx->join_idx[0][dead].p;
+    const uint32_t jn = ctx->join_n[0][dead];
+    const uint16_t* mult = join_mult(ctx, dead);
     if (probe)
         k_qc_join<false, true><<<jgrid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, (uint64_t*)ctx->cfp1cm.p,
-                                                                 (uint8_t*)ctx->cmeta1.p, jk, ji, ctx->join_n[dead],
-                                                                 dead, stages, (Surv*)ctx->surv.p, scap, cnt, probe);
+                                                                 (uint8_t*)ctx->cmeta1.p, jk, ji, jn, dead, stages,
+                                                                 (Surv*)ctx->surv.p, scap, cnt, probe, mult);
     else
         k_qc_join<false, false><<<jgrid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, (uint64_t*)ctx->cfp1cm.p,
-                                                                  (uint8_t*)ctx->cmeta1.p, jk, ji, ctx->join_n[dead],
-                                                                  dead, stages, (Surv*)ctx->surv.p, scap, cnt, 0u);
+                                                                  (uint8_t*)ctx->cmeta1.p, jk, ji, jn, dead, stages,
+                                                                  (Surv*)ctx->surv.p, scap, cnt, 0u, mult);
     CKL("k_qc_join");
     return M6502_OK;
 }
@@ -2236,6 +2292,7 @@ int init_ctx(m6502_ctx* ctx) {
     TRY(ensure(ctx, ctx->cfp1cm, sizeof(uint64_t) * 32 * kNumInsns));
     CK(cudaMemcpyAsync(ctx->cfp1cm.p, h.data(), h.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
     ctx->h_cmeta = meta;
+    ctx->h_tab.assign(tab, tab + kNumInsns);
     CK(cudaMemcpyAsync(ctx->cfp1.p, tr.data(), tr.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->cmeta1.p, meta.data(), meta.size(), cudaMemcpyHostToDevice, ctx->stream));
     TRY(ensure(ctx, ctx->cnt, sizeof(Counters)));
@@ -2244,14 +2301,40 @@ int init_ctx(m6502_ctx* ctx) {
     return M6502_OK;
 }
 
+// The group of a length-1 candidate under a dead-flags mask (see CandGroups),
+// or -1 when it is alone in its group.  An instruction that writes only dead
+// flags is the identity on every compared output; two of them stand for each
+// other when the pairs they form also sweep the same registers (op_reads) and
+// pass the same byte filter.  Then the verdict of (target, candidate) is the
+// same for both: the same outputs, cones, domain and values.
+int cand_group(uint32_t op, uint32_t dead) {
+    uint16_t dep[NUM_LOCS];
+    const uint32_t written = op_deps(op, dep);
+    for (uint32_t l = 0; l < NUM_LOCS; l++)
+        if ((written & LB(l)) && !(flag_bit(l) & dead)) return -1;   // a live output changes
+    return (int)(sweep_locs_of_reads(op_reads(op)) << 4 | bytes_cuda(op));
+}
+
 // Sorted (QuickCheck key, candidate) table of the non-pruned length-1
-// candidates for one dead-flags mask, built once per mask.
-int join_table(m6502_ctx* ctx, uint32_t dead) {
-    if (ctx->join_n[dead]) return M6502_OK;
+// candidates for one dead-flags mask, built once per mask.  CUDA semantics:
+// one entry per group of candidates; Go semantics: every candidate (its
+// passes and ranks tell the members of a group apart).
+int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
+    if (ctx->join_n[go][dead]) return M6502_OK;
     const uint64_t loose = cmp_mask(dead);
     std::vector<std::pair<uint64_t, uint16_t>> v;
+    CandGroups gr;
+    std::memset(&gr, 0, sizeof gr);
+    std::vector<std::vector<uint16_t>> groups;   // members; a lone candidate is a group of its own
+    std::map<int, size_t> group_of;
     for (int c = 0; c < kNumInsns; c++) {
         if (ctx->h_cmeta[c] & 0x10) continue;
+        const int g = go ? -1 : cand_group(ctx->h_tab[c] & 0xFFu, dead);
+        if (g >= 0) {
+            const auto at = group_of.emplace(g, groups.size());
+            if (!at.second) { groups[at.first->second].push_back((uint16_t)c); continue; }
+        }
+        groups.push_back({(uint16_t)c});
         uint64_t x = 0;
         for (int q = 0; q < 8; q++) x ^= key_term(ctx->h_cfp8[(size_t)q * kNumInsns + c] & loose, q);
         const uint64_t key = key_final(x);
@@ -2261,11 +2344,21 @@ int join_table(m6502_ctx* ctx, uint32_t dead) {
     std::vector<uint64_t> keys(v.size());
     std::vector<uint16_t> idx(v.size());
     for (size_t i = 0; i < v.size(); i++) { keys[i] = v[i].first; idx[i] = v[i].second; }
-    TRY(ensure(ctx, ctx->join_keys[dead], keys.size() * 8));
-    TRY(ensure(ctx, ctx->join_idx[dead], idx.size() * 2));
-    CK(cudaMemcpy(ctx->join_keys[dead].p, keys.data(), keys.size() * 8, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->join_idx[dead].p, idx.data(), idx.size() * 2, cudaMemcpyHostToDevice));
-    ctx->join_n[dead] = (uint32_t)v.size();
+    TRY(ensure(ctx, ctx->join_keys[go][dead], keys.size() * 8));
+    TRY(ensure(ctx, ctx->join_idx[go][dead], idx.size() * 2));
+    CK(cudaMemcpy(ctx->join_keys[go][dead].p, keys.data(), keys.size() * 8, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(ctx->join_idx[go][dead].p, idx.data(), idx.size() * 2, cudaMemcpyHostToDevice));
+    if (!go) {
+        uint16_t at = 0;
+        for (const auto& e : groups) {
+            gr.mult[e[0]] = (uint16_t)e.size();
+            gr.first[e[0]] = at;
+            for (uint16_t c : e) gr.member[at++] = c;
+        }
+        TRY(ensure(ctx, ctx->join_groups[dead], sizeof gr));
+        CK(cudaMemcpy(ctx->join_groups[dead].p, &gr, sizeof gr, cudaMemcpyHostToDevice));
+    }
+    ctx->join_n[go][dead] = (uint32_t)v.size();
     return M6502_OK;
 }
 
@@ -2332,7 +2425,10 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
     const bool exh = (stages & M6502_CHECK_EXH) != 0;
     const bool rounds = go && exh;   // Go semantics: verify in Go order, stop at the first pass
     const bool phase2 = cfg.max_cand_len >= 2;
-    if (!scan) TRY(join_table(ctx, dead));
+    if (!scan) TRY(join_table(ctx, dead, go));
+    // the scan's survivors are single candidates; the join's may stand for a group
+    const CandGroups* groups = scan || go ? nullptr : (const CandGroups*)ctx->join_groups[dead].p;
+    const uint16_t* mult = groups ? groups->mult : nullptr;
     for (int attempt = 0; attempt < 6; attempt++) {
         // Every buffer the pass uses is allocated here, so that the launches
         // below can be recorded as one CUDA graph and replayed.
@@ -2376,13 +2472,14 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         uint32_t qgrid = (uint32_t)std::min<uint64_t>(ctx->qc_blocks, (nt + kQcTile - 1) / kQcTile);
         if (!scan) {
             uint32_t jgrid = (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 8, (nt + kWarpsPerBlock - 1) / kWarpsPerBlock);
-            const uint64_t* jk = (const uint64_t*)ctx->join_keys[dead].p;
-            const uint16_t* ji = (const uint16_t*)ctx->join_idx[dead].p;
+            const uint64_t* jk = (const uint64_t*)ctx->join_keys[1][dead].p;
+            const uint16_t* ji = (const uint16_t*)ctx->join_idx[1][dead].p;
             if (go)
                 k_qc_join<true><<<jgrid, 256, 0, ctx->stream>>>(d_targets, tlen,
                                                                 (uint32_t)nt, (uint64_t*)ctx->cfp1cm.p,
-                                                                (uint8_t*)ctx->cmeta1.p, jk, ji, ctx->join_n[dead],
-                                                                dead, stages, (Surv*)ctx->surv.p, scap, cnt, 0u);
+                                                                (uint8_t*)ctx->cmeta1.p, jk, ji, ctx->join_n[1][dead],
+                                                                dead, stages, (Surv*)ctx->surv.p, scap, cnt, 0u,
+                                                                nullptr);
             else
                 TRY(launch_join1(ctx, d_targets, tlen, nt, dead, stages, scap, cnt,
                                  (ctx->tune.join_probe && exh) ? 1u + cfg.sweep : 0u));
@@ -2398,7 +2495,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
                                                          (Surv*)ctx->surv.p, scap, cnt);
         CKL("k_qc1");
         CK(rec(ctx->sev[2]));
-        SurvSource src{(const Surv*)ctx->surv.p, d_targets, tlen, dead, go ? 1 : 0};
+        SurvSource src{(const Surv*)ctx->surv.p, d_targets, tlen, dead, go ? 1 : 0, mult};
         ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, cfg.sweep, cfg.exh_mode == M6502_EXH_BRUTE};
         // Go-order verification rounds over the survivors in ctx->surv; on
         // return `best` holds the first passing candidate per target and pass.
@@ -2421,7 +2518,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
             k_go_ord<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const uint64_t*)ctx->go_keys2.p, &cnt->surv, scap,
                                                             (uint32_t*)ctx->go_ord.p, cnt);
             CKL("k_go_ord");
-            SurvSource rs{(const Surv*)ctx->go_round.p, d_targets, tlen, dead, 1};
+            SurvSource rs{(const Surv*)ctx->go_round.p, d_targets, tlen, dead, 1, nullptr};
             for (uint64_t lo = 0, blk = 64; lo < bound; lo += blk, blk = std::min<uint64_t>(blk * 2, 1ull << 22)) {
                 const uint64_t hi = std::min<uint64_t>(lo + blk, 0xFFFFFFFFull);
                 CK(cudaMemsetAsync(&cnt->round_n, 0, sizeof(unsigned long long), ctx->stream));
@@ -2465,7 +2562,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
                 k_emit_all<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const Surv*)ctx->surv.p, &cnt->surv, scap,
                                                                   (const uint32_t*)ctx->fail.p, d_ids, 0, dead,
                                                                   (m6502_rule*)ctx->rules.p, rlim, &cnt->rules, cnt,
-                                                                  exh ? 1 : 0, d_targets, tlen, cfg.sweep);
+                                                                  exh ? 1 : 0, d_targets, tlen, cfg.sweep, groups);
                 CKL("k_emit_all");
             }
             return M6502_OK;
@@ -2531,7 +2628,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
                 (uint64_t)(uintptr_t)ctx->go_keys.p, (uint64_t)(uintptr_t)ctx->go_keys2.p,
                 (uint64_t)(uintptr_t)ctx->go_ord.p, (uint64_t)(uintptr_t)ctx->go_round.p,
                 (uint64_t)(uintptr_t)ctx->go_sort_tmp.p, ctx->go_sort_tmp.bytes, (uint64_t)(uintptr_t)ctx->jitems.p,
-                (uint64_t)(uintptr_t)ctx->join_keys[dead].p, c2 ? (uint64_t)(uintptr_t)c2->keys.p : 0,
+                (uint64_t)(uintptr_t)ctx->join_keys[go][dead].p, c2 ? (uint64_t)(uintptr_t)c2->keys.p : 0,
                 c2e ? (uint64_t)(uintptr_t)c2e->keys.p : 0, ctx->tune.exh_minb, ctx->tune.ticket_batch,
                 ctx->tune.chunk_log2, ctx->tune.join_probe};
             m6502_ctx::PassGraph* pg = nullptr;
@@ -2595,7 +2692,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
             st->pairs += nt * ((uint64_t)kNumInsns + (phase2 ? (uint64_t)kNumInsns * kNumInsns : 0u));
             st->qc_hits += hc.qc;
             st->mid_hits += hc.mid;
-            st->exh_checked += !exh ? 0 : rounds ? hc.round_checked : hc.surv + hc.surv1 + hc.join_probe_rej;
+            st->exh_checked += !exh ? 0 : rounds ? hc.round_checked : hc.mid;
             st->exh_passed += hc.exh_pass;
             st->rules += hc.rules;
             st->exh_states += hc.states;
@@ -2653,7 +2750,8 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
         TRY(ensure(ctx, ctx->tfp, pmax * 32 * sizeof(uint64_t)));
         TRY(ensure(ctx, ctx->tmeta, pmax));
     }
-    if (!scan) TRY(join_table(ctx, dead));
+    if (!scan) TRY(join_table(ctx, dead, false));
+    const CandGroups* groups = scan ? nullptr : (const CandGroups*)ctx->join_groups[dead].p;
     TRY(ensure(ctx, ctx->cnt_slots, npass * sizeof(Counters)));
     Counters* slots = (Counters*)ctx->cnt_slots.p;
     for (int attempt = 0; attempt < 6; attempt++) {
@@ -2697,7 +2795,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                                      (ctx->tune.join_probe && exh) ? 1u + cfg.sweep : 0u));
                 }
                 CK(rec(ev[2]));
-                SurvSource src{(const Surv*)ctx->surv.p, d_t, tlen, dead, 0};
+                SurvSource src{(const Surv*)ctx->surv.p, d_t, tlen, dead, 0, groups ? groups->mult : nullptr};
                 ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, cfg.sweep,
                            cfg.exh_mode == M6502_EXH_BRUTE};
                 if (exh) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea, true));
@@ -2708,7 +2806,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                                                                   (const uint32_t*)ctx->fail.p, nullptr, b, dead,
                                                                   (m6502_rule*)ctx->rules.p, count_only ? 0 : rcap,
                                                                   &slots[0].rules, cnt, exh ? 1 : 0, d_t, tlen,
-                                                                  cfg.sweep);
+                                                                  cfg.sweep, groups);
                 CKL("k_emit_all");
                 CK(rec(ev[5]));
             }
@@ -2723,7 +2821,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 (uint64_t)(uintptr_t)ctx->fail.p, (uint64_t)(uintptr_t)ctx->items.p, (uint64_t)(uintptr_t)ctx->order.p,
                 (uint64_t)(uintptr_t)ctx->rules.p, (uint64_t)(uintptr_t)ctx->cnt_slots.p,
                 (uint64_t)(uintptr_t)ctx->tfp.p, (uint64_t)(uintptr_t)ctx->tmeta.p,
-                (uint64_t)(uintptr_t)ctx->join_keys[dead].p, ctx->tune.exh_minb, ctx->tune.ticket_batch,
+                (uint64_t)(uintptr_t)ctx->join_keys[0][dead].p, ctx->tune.exh_minb, ctx->tune.ticket_batch,
                 ctx->tune.chunk_log2, ctx->tune.join_probe};
             if (!(ctx->graph.exec && ctx->graph.key == key)) {
                 if (ctx->graph.exec) { cudaGraphExecDestroy(ctx->graph.exec); ctx->graph.exec = nullptr; }
@@ -2791,7 +2889,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 st->pairs += nt * (uint64_t)kNumInsns;
                 st->qc_hits += c.qc;
                 st->mid_hits += c.mid;
-                st->exh_checked += exh ? c.surv + c.join_probe_rej : 0;   // the join's probe is part of the check
+                st->exh_checked += exh ? c.mid : 0;   // every MidCheck survivor, the join's probe included
                 st->exh_passed += c.exh_pass;
                 st->exh_states += c.states;
                 st->exh_items += c.items;
@@ -2998,8 +3096,11 @@ void m6502_destroy(m6502_ctx* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (int i = 0; i < 256; i++) {
-        if (ctx->join_keys[i].p) cudaFree(ctx->join_keys[i].p);
-        if (ctx->join_idx[i].p) cudaFree(ctx->join_idx[i].p);
+        for (int g = 0; g < 2; g++) {
+            if (ctx->join_keys[g][i].p) cudaFree(ctx->join_keys[g][i].p);
+            if (ctx->join_idx[g][i].p) cudaFree(ctx->join_idx[g][i].p);
+        }
+        if (ctx->join_groups[i].p) cudaFree(ctx->join_groups[i].p);
     }
     DevBuf* bufs[] = {&ctx->cfp1cm, &ctx->cfp1, &ctx->cmeta1, &ctx->targets, &ctx->ids, &ctx->tfp, &ctx->tmeta,
                       &ctx->surv, &ctx->fail, &ctx->items, &ctx->rules, &ctx->cnt, &ctx->best,

@@ -416,6 +416,7 @@ struct StokeSource {
     }
     __device__ bool probed(uint64_t) const { return false; }
     __device__ uint64_t target_id(uint64_t) const { return kNoTarget; }   // candidates may be empty
+    __device__ uint32_t weight(uint64_t) const { return 1u; }
 };
 
 // Over the vec_ok entries sorted by key (one CTA, chunks of 1,024): rep[i] =
