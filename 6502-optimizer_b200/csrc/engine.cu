@@ -4,11 +4,10 @@
 // length-1 candidates queues every pass and syncs once at the end):
 //
 //   k_check_ops     every opcode of the targets, once per search.
-//   k_qc_join       (default) warp per target, lane v runs the target on
-//                   test vector v; the 8 masked QC outputs are hashed and
-//                   looked up in the candidates' sorted key table (shared
-//                   memory, bucket directory); only the equal range is
-//                   checked, on all 32 vectors (QuickCheck + MidCheck).
+//   k_qc_join       (default) lane per target: its 8 masked QC outputs are
+//                   hashed and looked up among the candidates' distinct
+//                   outputs (keys and bucket directory in shared memory);
+//                   only a match runs the 24 MidCheck vectors.
 //   k_fingerprint + k_qc1  (M6502_QC_SCAN) 32 packed output states per
 //                   target, then a tile of 64 targets x all 2,863
 //                   candidates per CTA with one masked 64-bit compare per
@@ -37,12 +36,14 @@
 #include <algorithm>
 #include <cctype>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "internal.h"
@@ -65,7 +66,6 @@ constexpr uint64_t kMaxItemsPerCone = 1ull << 16;   // larger cones get larger i
 // more; they get the verdict "undecided" instead of an endless sweep.
 constexpr uint32_t kMaxConeBits = 34;
 constexpr unsigned kTicketBatch = 4;           // pairs a warp takes per ticket atomic
-constexpr int kJoinBatch = 4;                  // candidate rows a join warp loads before using them
 constexpr int kDirBits = 12;                   // key-bucket directory of the length-1 join (4,096 buckets)
 constexpr int kMaxAsyncPasses = 64;            // passes of one search queued without a host round trip
 
@@ -97,6 +97,7 @@ const uint8_t kRepValues[32] = {
 };
 
 __constant__ uint64_t c_vec[32];             // packed test vectors
+__constant__ uint32_t c_vec4[8][8];           // the same, vectors 4 g .. 4 g + 3 one per byte of each field (A X Y P S M S0 S1)
 __constant__ uint16_t c_dep[NUM_OPS][NUM_LOCS];
 __constant__ uint16_t c_wr[NUM_OPS];          // written locations per opcode
 __constant__ uint16_t c_sweep[NUM_OPS];       // swept locations implied by opReads
@@ -178,6 +179,42 @@ __host__ __device__ __forceinline__ uint64_t key_term(uint64_t masked_out, int v
 }
 __host__ __device__ __forceinline__ uint64_t key_final(uint64_t x) { return key_mix(x ^ 0x6502ull); }
 
+// Key of the length-1 join: a hash of the 8 QuickCheck outputs as 16 packed
+// words (fields A X Y P S M S0 S1 of vectors 0-3, then of vectors 4-7, one
+// vector per byte; P masked), one 32 x 32 + 64 bit multiply-add per word.
+__host__ __device__ __forceinline__ uint64_t join_key(const uint32_t (&w)[16]) {
+    constexpr uint32_t kMul[16] = {0x9E3779B1u, 0x85EBCA77u, 0xC2B2AE3Du, 0x27D4EB2Fu, 0x165667B1u, 0xD3A2646Du,
+                                   0xFD7046C5u, 0xB55A4F09u, 0x8DA6B343u, 0xD8163841u, 0xCB1AB31Fu, 0xA2C2A7D5u,
+                                   0x91E10DA5u, 0xE7037ED1u, 0xF4914F6Du, 0xAF251AF3u};
+    uint64_t h = 0x6502;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int i = 0; i < 16; i++) h += (uint64_t)w[i] * kMul[i];
+    h ^= h >> 29;
+    h *= 0xFF51AFD7ED558CCDull;
+    return h ^ (h >> 32);
+}
+
+// The length-1 join's table for one dead-flags mask.  The non-pruned
+// candidates fall into classes of equal QuickCheck outputs (1,883 at mask
+// 0x00) and those into subclasses of equal MidCheck outputs (2,032): a class
+// is an entry, by ascending key (two entries may share one), and a target's
+// outputs are compared once per class and subclass, not once per candidate
+// (runs of up to 43 compare operands share a class).  `key` and `dir`, a
+// directory of the keys' top bits, are copied into shared memory; the rest
+// is read for the targets that match (15 %).
+struct alignas(16) JoinTable {
+    uint64_t key[kNumInsns + 1];
+    uint16_t dir[(1u << kDirBits) + 8];    // first entry whose key's top kDirBits bits are >= b
+    uint16_t sub[kNumInsns + 1];           // subclasses of entry u: sub[u] .. sub[u + 1]
+    uint16_t start[kNumInsns + 1];         // candidates of subclass j: cand[start[j] .. start[j + 1])
+    uint16_t cand[kNumInsns + 1];          // index | byte size << 12
+    uint16_t weight[kNumInsns + 1][2];     // pairs (CandGroups) of entry u's candidates of 1 byte, of at most 2
+};
+constexpr size_t kJoinShared = offsetof(JoinTable, sub);
+static_assert(kJoinShared % 16 == 0 && kNumInsns < (1 << 12), "copied in 16-byte words; 12-bit indices");
+
 // Warp-collective key of the outputs held by lanes 0..7 (lane v: vector v).
 __device__ __forceinline__ uint64_t warp_key(uint64_t tv, uint64_t mask, int lane) {
     uint64_t h = lane < 8 ? key_term(tv & mask, lane) : 0ull;
@@ -214,9 +251,6 @@ struct Surv {
     uint32_t c;
 };
 constexpr uint32_t kSurvLen2 = 1u << 23, kSurvMasked = 1u << 24;
-// The join already ran the random-state probe on this pair and found no
-// difference (k_exhaustive skips its own probe).
-constexpr uint32_t kSurvProbed = 1u << 31;
 // target_id of a pair source whose pairs do not share targets.
 constexpr uint64_t kNoTarget = ~0ull;
 __host__ __device__ __forceinline__ uint32_t fd_pack(uint32_t fd) { return (fd & 0x0Fu) | ((fd >> 2) & 0x30u); }
@@ -225,12 +259,12 @@ struct Counters {
     unsigned long long qc, mid, surv, exh_ticket, items, item_ticket, rules, exh_pass, states, algo, probe_rejects;
     unsigned long long round_n, max_ord;   // Go-order verification rounds
     unsigned long long join_items;         // chunks of long length-2 equal ranges
-    unsigned long long join_probe_rej;     // MidCheck survivors the join's probe rejected
     unsigned long long undecided;          // pairs left undecided (a cone beyond the sweep cap)
     unsigned long long round_checked, round_items;   // Go-order rounds: pairs and work items, summed
     unsigned long long surv1, items1;      // phase-1 survivors and work items (length-2 phase runs after)
     unsigned long long surv_need, items_need;   // largest survivor / work-item counts seen, for the
                                                 // overflow check after the pass
+    unsigned long long join_ticket;        // k_qc_join: claimed chunks of targets
     unsigned long long probe_ticket, probe_pass;   // k_probe_pairs: claimed pairs, pairs it passed on
 };
 
@@ -294,7 +328,6 @@ struct SurvSource {
         }
         dead = go ? ((s.c & kSurvMasked) ? run_dead : 0u) : run_dead;
     }
-    __device__ bool probed(uint64_t p) const { return (surv[p].c & kSurvProbed) != 0; }
     // Pairs with the same id share their target (the probe reuses its outputs).
     __device__ uint64_t target_id(uint64_t p) const { return surv[p].t; }
     // Pairs that record p stands for.
@@ -316,7 +349,6 @@ struct CsrSource {
         if (lane < cn) sc[lane] = c_ins[c0 + lane];
         dead = dead_;
     }
-    __device__ bool probed(uint64_t) const { return false; }
     __device__ uint64_t target_id(uint64_t) const { return kNoTarget; }
     __device__ uint32_t weight(uint64_t) const { return 1u; }
 };
@@ -1058,190 +1090,175 @@ __global__ void __launch_bounds__(256) k_qc1(const uint64_t* __restrict__ tfp, c
     }
 }
 
-// QC (+ MidCheck) of targets x all length-1 candidates as an exact join:
-// the non-pruned candidates sorted by the hash of their 8 masked QuickCheck
-// outputs (skeys/sidx, built per dead-flags mask) sit in shared memory with
-// a directory of key buckets; a warp takes one target, finds its own key's
-// equal range and checks only those candidates -- a superset of those
-// QuickCheck passes.
-// Lane v checks vector v from the candidate-major fingerprints (cfp_cm,
-// 256 contiguous bytes per candidate).  Same survivors as k_qc1.
-// PROBE: the random-state probe of MidCheck survivors runs here (CUDA
-// semantics only; a separate instantiation, so that the join without it
-// keeps its registers).
-template <bool GO, bool PROBE = false>
-__global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__ targets, uint32_t tlen,
-                                                  uint32_t nt, const uint64_t* __restrict__ cfp_cm,
-                                                  const uint8_t* __restrict__ cmeta, const uint64_t* __restrict__ skeys,
-                                                  const uint16_t* __restrict__ sidx, uint32_t nsorted, uint32_t dead,
+// QC (+ MidCheck) of targets x all length-1 candidates as an exact join
+// through the mask's JoinTable.  A warp takes `chunk` (1..32) consecutive
+// targets in two phases:
+//   - a lane per target runs it on the 8 QuickCheck vectors (two packed words
+//     of four states), hashes the outputs, finds the key's entry and checks
+//     the outputs against it (cfp4: 256 packed bytes per candidate), then
+//     runs it on the 24 MidCheck vectors and finds its subclass;
+//   - the candidates of all its targets, numbered through, go round the lanes
+//     and are appended as survivors.
+// Same survivors as k_qc1.  Bound by integer issue: a warp per target with a
+// lane per vector spent 400 warp instructions per target, most of them on
+// dispatch, hashing and ballots for 32 states of two instructions; here those
+// are paid once for 32 targets with four states per register.  Lanes whose
+// targets differ in opcode diverge, which the enumeration's order makes rare
+// and the packed words cheap.
+// 1.9 M length-2 targets (every fourth), mask 0x00: 945 -> 138 us; 60 M warp
+// instructions, latency bound now (38 % of issue slots).
+template <bool GO>
+__global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__ targets, uint32_t tlen, uint32_t nt,
+                                                  uint32_t chunk, const uint4* __restrict__ cfp4,
+                                                  const JoinTable* __restrict__ table, uint32_t dead,
                                                   uint32_t stages, Surv* __restrict__ surv, uint64_t cap,
-                                                  Counters* __restrict__ cnt, uint32_t probe,
-                                                  const uint16_t* __restrict__ mult) {
-    __shared__ uint64_t s_key[kNumInsns];
-    __shared__ uint64_t s_tprobe[PROBE ? kWarpsPerBlock : 1][2][32];   // target outputs on the probe states
-    __shared__ uint16_t s_idx[kNumInsns];
-    __shared__ uint8_t s_meta[kNumInsns];
-    __shared__ uint16_t s_dir[(1u << kDirBits) + 1];
+                                                  Counters* __restrict__ cnt, const uint16_t* __restrict__ mult) {
+    __shared__ alignas(16) uint8_t s_raw[kJoinShared];
+    const JoinTable& s_tab = *reinterpret_cast<const JoinTable*>(s_raw);   // key and dir only
     __shared__ Surv s_stage[kWarpsPerBlock][kStage];
-    Surv* stage = s_stage[threadIdx.x >> 5];
-    int nstage = 0;
-    for (uint32_t i = threadIdx.x; i < nsorted; i += blockDim.x) {
-        s_key[i] = skeys[i];
-        s_idx[i] = sidx[i];
-    }
-    for (uint32_t i = threadIdx.x; i < (uint32_t)kNumInsns; i += blockDim.x) s_meta[i] = cmeta[i];
-    __syncthreads();
-    // Bucket directory over the keys' top kDirBits bits: s_dir[b] is the
-    // first index whose key lies in bucket b or above.  Index i fills the
-    // buckets above its predecessor's, up to its own.
-    for (uint32_t i = threadIdx.x; i <= nsorted; i += blockDim.x) {
-        const uint32_t b0 = i == 0 ? 0u : (uint32_t)(s_key[i - 1] >> (64 - kDirBits)) + 1u;
-        const uint32_t b1 = i == nsorted ? (1u << kDirBits) : (uint32_t)(s_key[i] >> (64 - kDirBits));
-        for (uint32_t b = b0; b <= b1; b++) s_dir[b] = (uint16_t)i;
-    }
+    for (uint32_t i = threadIdx.x; i < kJoinShared / 16; i += blockDim.x)
+        reinterpret_cast<uint4*>(s_raw)[i] = reinterpret_cast<const uint4*>(table)[i];
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint64_t loose = cmp_mask(dead), exact = cmp_mask(0);
-    const uint64_t vin = c_vec[lane];   // lane v's test vector, read once
-    unsigned long long nqc = 0, nmid = 0, nprobe_rej = 0;
-    const uint32_t stride = gridDim.x * kWarpsPerBlock;
-    uint32_t t = blockIdx.x * kWarpsPerBlock + w;
-    // Lane i holds instruction i of the warp's target (tlen <= 32); the next
-    // target's are loaded while this one is processed.
-    uint32_t ins_next = (t < nt && lane < (int)tlen) ? targets[(uint64_t)t * tlen + lane] : 0u;
-    for (; t < nt; t += stride) {
-        const uint32_t ins = ins_next;
-        const uint64_t tnext = (uint64_t)t + stride;
-        ins_next = (tnext < nt && lane < (int)tlen) ? targets[tnext * tlen + lane] : 0u;
-        // The target's outputs, computed here rather than stored: lane v runs
-        // it on vector v (its instructions are warp-uniform shuffles).
-        St st = unpack(vin);
-        for (uint32_t i = 0; i < tlen; i++) exec(st, __shfl_sync(kFull, ins, (int)i));
-        const uint32_t tb = __reduce_add_sync(
-            kFull, lane < (int)tlen ? (GO ? bytes_go(ins & 0xFFu) : bytes_cuda(ins & 0xFFu)) : 0u);
-        const uint64_t tv = fp_of(st);   // lane v holds the target's output on vector v
-        const uint64_t key = warp_key(tv, loose, lane);
-        // The equal range within the key's bucket: one compare per lane when
-        // the bucket holds at most 32 keys, else a search inside it.
-        const uint32_t bkt = (uint32_t)(key >> (64 - kDirBits));
-        uint32_t lo = s_dir[bkt], end;
-        const uint32_t bhi = s_dir[bkt + 1];
-        if (bhi - lo <= 32) {
-            const uint32_t i = lo + (uint32_t)lane;
-            const uint64_t k = i < bhi ? s_key[i] : ~0ull;
-            const unsigned below = __ballot_sync(kFull, i < bhi && k < key);
-            const unsigned same = __ballot_sync(kFull, i < bhi && k == key);
-            lo += (uint32_t)__popc(below);
-            end = lo + (uint32_t)__popc(same);
-        } else {
-            lo += warp_lower_bound(s_key + lo, bhi - lo, key, lane);
-            end = lo;
-            while (end < bhi && s_key[end] == key) end++;
-        }
-        if (lo == end) continue;
-        // Random-state probe of the MidCheck survivors (CUDA semantics, before
-        // ExhaustiveCheck; `probe` = 1 + the sweep mode, 0 = off).  Lane l
-        // takes domain states l and l + 32 drawn from this target's salt.  The
-        // target's outputs on them are computed once, on the first survivor,
-        // over the target's own domain (A, carry and the registers it reads)
-        // and reused by every candidate that reads no other register; a
-        // candidate that widens the domain runs the target again on the wider
-        // states.  A difference rejects the pair, as ExhaustiveCheck would
-        // (the states lie in its domain); under the reduced sweep, pairs
-        // reading three or more extra registers are left to k_exhaustive.
-        bool tp_ready = false;
-        uint32_t tp_sw = 0;
-        const uint64_t salt = (uint64_t)t * 0xD1B54A32D192ED03ull + 0x632BE59BD9B4E019ull;
-        for (uint32_t i0 = lo; i0 < end; i0 += kJoinBatch) {
-            // The rows of up to kJoinBatch candidates are loaded before any is
-            // used, so their latencies overlap.
-            uint64_t row[kJoinBatch];
-            uint32_t cidx[kJoinBatch];
-            bool keep[kJoinBatch];
+    Surv* stage = s_stage[w];
+    int nstage = 0;
+    const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;   // compared bits of a packed P word
+    unsigned long long nqc = 0, nmid = 0;
+    // Chunks come from a ticket, claimed one ahead: their hits are uneven, and
+    // a fixed stride left some SMs with half the work of others.
+    unsigned long long next = 0;
+    if (lane == 0) next = atomicAdd(&cnt->join_ticket, 1ull);
+    for (;;) {
+        const uint64_t base = __shfl_sync(kFull, next, 0) * chunk;
+        if (base >= nt) break;
+        if (lane == 0) next = atomicAdd(&cnt->join_ticket, 1ull);
+        // -- a lane per target --
+        const bool have = (uint32_t)lane < chunk && base + lane < nt;
+        const uint16_t* tp = targets + (base + (have ? lane : 0)) * tlen;
+        uint32_t ins01 = tp[0], ins2 = 0;   // its instructions: two in the first word, the third in the second
+        if (tlen > 1) ins01 |= (uint32_t)tp[1] << 16;
+        if (tlen > 2) ins2 = tp[2];
+        uint32_t tb = 0, lo = 0, n = 0, tp0, tp1;   // tp: P after the QuickCheck vectors
+        // Its outputs on vectors 8 r .. 8 r + 7 against candidate c's.
+        auto run = [&](St (&v)[2], int r) {
 #pragma unroll
-            for (int j = 0; j < kJoinBatch; j++) {
-                keep[j] = false; row[j] = 0; cidx[j] = 0;
-                if (i0 + j < end) {
-                    const uint32_t c = s_idx[i0 + j];
-                    const uint32_t cm = s_meta[c];
-                    const uint32_t cb = GO ? ((cm >> 2) & 3u) : (cm & 3u);
-                    cidx[j] = c;
-                    keep[j] = !((cm & 0x10u) || cb >= tb);   // pruned or not shorter (uniform)
-                    if (keep[j]) row[j] = cfp_cm[(uint64_t)c * 32 + lane];   // one coalesced 256-byte row
+            for (int g = 0; g < 2; g++)
+                v[g] = St{c_vec4[2 * r + g][0], c_vec4[2 * r + g][1], c_vec4[2 * r + g][2], c_vec4[2 * r + g][3],
+                          c_vec4[2 * r + g][4], c_vec4[2 * r + g][5], c_vec4[2 * r + g][6], c_vec4[2 * r + g][7]};
+            for (uint32_t i = 0; i < tlen; i++) exec_x4n(v, i == 0 ? ins01 & 0xFFFFu : i == 1 ? ins01 >> 16 : ins2);
+        };
+        auto differ = [&](const St (&v)[2], int r, uint32_t c) -> uint32_t {
+            const uint4* row = cfp4 + (size_t)c * 16 + r * 4;
+            uint32_t d = 0;
+#pragma unroll
+            for (int g = 0; g < 2; g++) {
+                const uint4 q0 = __ldg(row + 2 * g), q1 = __ldg(row + 2 * g + 1);
+                d |= (v[g].a ^ q0.x) | (v[g].x ^ q0.y) | (v[g].y ^ q0.z) | ((v[g].p ^ q0.w) & pm) | (v[g].s ^ q1.x) |
+                     (v[g].m ^ q1.y) | (v[g].s0 ^ q1.z) | (v[g].s1 ^ q1.w);
+            }
+            return d;
+        };
+        {
+            St v[2];
+            run(v, 0);
+            for (uint32_t i = 0; i < tlen; i++) {
+                const uint32_t op = (i == 0 ? ins01 : i == 1 ? ins01 >> 16 : ins2) & 0xFFu;
+                tb += GO ? bytes_go(op) : bytes_cuda(op);
+            }
+            const uint32_t words[16] = {v[0].a, v[0].x, v[0].y, v[0].p & pm, v[0].s, v[0].m, v[0].s0, v[0].s1,
+                                        v[1].a, v[1].x, v[1].y, v[1].p & pm, v[1].s, v[1].m, v[1].s0, v[1].s1};
+            tp0 = v[0].p;
+            tp1 = v[1].p;
+            const uint64_t key = join_key(words);
+            const uint32_t b = (uint32_t)(key >> (64 - kDirBits));
+            uint32_t j0 = 0, j1 = 0;   // subclasses of the entry that matches
+            for (uint32_t u = s_tab.dir[b], e = s_tab.dir[b + 1]; have && u < e; u++) {
+                if (s_tab.key[u] != key) continue;
+                const uint32_t j = table->sub[u];
+                if (differ(v, 0, table->cand[table->start[j]] & 0xFFFu)) continue;
+                j0 = j;
+                j1 = table->sub[u + 1];
+                if (!GO && tb > 1) nqc += table->weight[u][tb > 2];
+                break;
+            }
+            if (GO || !(stages & M6502_CHECK_MID)) {   // every candidate of the entry
+                lo = table->start[j0];
+                n = table->start[j1] - lo;
+            } else if (tb <= 1) {
+                j1 = j0;                               // nothing is shorter
+            }
+            if (!GO && (stages & M6502_CHECK_MID)) {   // the subclass with the target's outputs, if any
+                for (; j0 < j1; j0++) {
+                    const uint32_t c = table->cand[table->start[j0]] & 0xFFFu;
+                    bool equal = true;
+                    for (int r = 1; r < 4 && equal; r++) {
+                        run(v, r);
+                        equal = differ(v, r, c) == 0;
+                    }
+                    if (!equal) continue;
+                    lo = table->start[j0];
+                    n = table->start[j0 + 1] - lo;
+                    break;
                 }
             }
+        }
+        uint32_t upto = n;   // hits of this lane's and the lanes below
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(kFull, upto, o);
+            upto += lane >= o ? x : 0u;
+        }
+        const uint32_t total = __shfl_sync(kFull, upto, 31);
+        // -- a lane per hit --
+        for (uint32_t h0 = 0; h0 < total; h0 += 32) {
+            const uint32_t h = h0 + (uint32_t)lane;
+            uint32_t own = 0;   // lanes whose hits end at or before h
 #pragma unroll
-            for (int j = 0; j < kJoinBatch; j++) {
-                if (!keep[j]) continue;
-                const uint32_t c = cidx[j];
-                const uint64_t x = tv ^ row[j];
-                const unsigned lo_eq = __ballot_sync(kFull, (x & loose) == 0);
-                const unsigned ex_eq = __ballot_sync(kFull, (x & exact) == 0);
-                if ((lo_eq & 0xFFu) != 0xFFu) continue;          // QuickCheck fails
-                bool pass = false;
-                uint32_t code = c;
-                if (!GO) {
-                    const uint32_t m1 = mult[c];   // candidates this one stands for
-                    nqc += lane == 0 ? m1 : 0u;
-                    const bool mid = !(stages & M6502_CHECK_MID) || lo_eq == kFull;
-                    if (mid) { nmid += lane == 0 ? m1 : 0u; pass = true; }
-                    if (PROBE && pass && probe) {
-                        if (!tp_ready) {
-                            tp_sw = __reduce_or_sync(kFull, lane < (int)tlen ? (uint32_t)c_sweep[ins & 0xFFu] : 0u);
-                            for (int r = 0; r < 2; r++) {
-                                St ts = probe_state(tp_sw | LB(L_A) | LB(L_C), false, probe_z(salt, lane + 32 * r));
-                                for (uint32_t i = 0; i < tlen; i++) exec(ts, __shfl_sync(kFull, ins, (int)i));
-                                s_tprobe[w][r][lane] = pack(ts);
-                            }
-                            tp_ready = true;
-                        }
-                        const uint32_t cins = c_tab[c];
-                        const uint32_t swc = c_sweep[cins & 0xFFu], swu = tp_sw | swc;
-                        if (probe != 1u + M6502_SWEEP_REFERENCE || __popc(swu) < 3) {
-                            const bool same = (swc & ~tp_sw) == 0;   // uniform
-                            const uint64_t m = cmp_mask(dead);
-                            bool differ = false;
-                            for (int r = 0; r < 2 && !differ; r++) {
-                                const St in = probe_state(swu | LB(L_A) | LB(L_C), false, probe_z(salt, lane + 32 * r));
-                                uint64_t tout = s_tprobe[w][r][lane];
-                                St ps = in;
-                                // one exec site: the target (when the domain widened), then the candidate
-                                for (int i = same ? (int)tlen : 0; i <= (int)tlen; i++) {
-                                    uint32_t insn = cins;
-                                    if (i < (int)tlen) insn = __shfl_sync(kFull, ins, i);
-                                    else { if (!same) tout = pack(ps); ps = in; }
-                                    exec(ps, insn);
-                                }
-                                differ = __any_sync(kFull, ((tout ^ pack(ps)) & m) != 0);
-                            }
-                            if (differ) { pass = false; nprobe_rej += lane == 0 ? m1 : 0u; }
-                            else code |= kSurvProbed;
-                        }
-                    }
-                } else if ((ex_eq & 0xFFu) == 0xFFu) {           // processTask: unmasked QC passes
-                    nqc += lane == 0; nmid += lane == 0; pass = true;
-                } else if (dead) {                               // processTaskMasked, FlagDiff != 0
-                    uint32_t fd = lane < 8 ? ((uint32_t)(x >> 24) & kPMask) : 0u;
-                    fd = __reduce_or_sync(kFull, fd);
+            for (uint32_t o = 16; o; o >>= 1) {
+                const uint32_t x = __shfl_sync(kFull, upto, (int)(own + o - 1));
+                own += x <= h ? o : 0u;
+            }
+            own = min(own, 31u);
+            const uint32_t end = __shfl_sync(kFull, upto, (int)own), cnt_o = __shfl_sync(kFull, n, (int)own);
+            const uint32_t lo_o = __shfl_sync(kFull, lo, (int)own), tb_o = __shfl_sync(kFull, tb, (int)own);
+            bool pass = h < total;
+            uint32_t c = 0;
+            if (pass) {
+                c = table->cand[lo_o + (h - (end - cnt_o))];
+                pass = (c >> 12) < tb_o;   // not shorter in bytes: not a candidate
+                c &= 0xFFFu;
+            }
+            uint32_t code = c;
+            if (GO) {
+                // FlagDiff over the QC vectors: zero when the unmasked QuickCheck
+                // passes too (processTask), else the masked pass (processTaskMasked).
+                const uint32_t p0 = __shfl_sync(kFull, tp0, (int)own), p1 = __shfl_sync(kFull, tp1, (int)own);
+                if (pass) {
+                    const uint32_t* row = reinterpret_cast<const uint32_t*>(cfp4) + (size_t)c * 64;
+                    uint32_t fd = ((p0 ^ __ldg(row + 3)) | (p1 ^ __ldg(row + 11))) & (kPMask * kB1);
+                    fd |= fd >> 16;
+                    fd = (fd | (fd >> 8)) & 0xFFu;
                     if (fd) {
-                        nqc += lane == 0; nmid += lane == 0; pass = true;
+                        pass = dead != 0;
                         code = c | kSurvMasked | (fd_pack(fd) << 25);
                     }
                 }
-                stage_push(pass && lane == 0, Surv{t, code}, stage, nstage, surv, cap, &cnt->surv, lane);
+                nqc += pass;
+                nmid += pass;
+            } else if (pass) {
+                nmid += mult[c];
             }
+            const uint32_t t = (uint32_t)base + own;
+            stage_push(pass, Surv{t, code}, stage, nstage, surv, cap, &cnt->surv, lane);
         }
     }
     stage_flush(stage, nstage, surv, cap, &cnt->surv, lane);
     for (int o = 16; o; o >>= 1) {
         nqc += __shfl_down_sync(kFull, nqc, o);
         nmid += __shfl_down_sync(kFull, nmid, o);
-        nprobe_rej += __shfl_down_sync(kFull, nprobe_rej, o);
     }
     if (lane == 0) {
         if (nqc) atomicAdd(&cnt->qc, nqc);
         if (nmid) atomicAdd(&cnt->mid, nmid);
-        if (nprobe_rej) atomicAdd(&cnt->join_probe_rej, nprobe_rej);
     }
 }
 
@@ -1472,7 +1489,7 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
         pv.t = s_t[w]; pv.c = s_c[w];
         src.load(p, s_t[w], s_c[w], pv.tn, pv.cn, pv.dead, lane);
         const uint64_t tid = src.target_id(p);
-        const bool probed = a.order != nullptr || src.probed(p);
+        const bool probed = a.order != nullptr;
         __syncwarp();
         if (!probed) {
             uint32_t sw_t = 0, sw_c = 0;
@@ -1555,8 +1572,7 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
 // a lean persistent kernel (many resident warps) runs probe_pair on each
 // surviving pair, marks the pairs it rejects (fail = 1) and appends the
 // others to `order`, 32 at a time per warp so that the passed pairs of one
-// target stay together; k_exhaustive then sweeps only those.  Pairs the
-// join already probed are passed on unprobed.
+// target stay together; k_exhaustive then sweeps only those. 
 template <class Src>
 __global__ void __launch_bounds__(256) k_probe_pairs(Src src, const unsigned long long* n_pairs_ptr, uint64_t n_cap,
                                                      ExhArgs a, uint32_t* __restrict__ order) {
@@ -1588,8 +1604,8 @@ __global__ void __launch_bounds__(256) k_probe_pairs(Src src, const unsigned lon
         }
         const unsigned long long p = next++;
         if (p >= n) break;
-        bool pass = true;
-        if (!src.probed(p)) {
+        bool pass;
+        {
             PairView pv;
             pv.t = s_t[w]; pv.c = s_c[w];
             src.load(p, s_t[w], s_c[w], pv.tn, pv.cn, pv.dead, lane);
@@ -2093,15 +2109,14 @@ struct m6502_ctx {
     DevBuf cfp1, cmeta1, targets, ids, tfp, tmeta, surv, fail, items, rules, cnt, best, pins, poffs,
         cins, coffs, pout, pfd, enum_count;
     std::vector<m6502_rule> staging;
-    std::vector<uint64_t> h_cfp0;     // vector-0 outputs of the length-1 candidates (host copy)
-    std::vector<uint64_t> h_cfp8;     // QC-vector outputs [8][2863] (host copy)
-    DevBuf cfp1cm;                    // candidate-major fingerprints [2863][32]
+    DevBuf cfp4;                      // packed outputs of the length-1 candidates: [2863][8 groups of 4 vectors][8 fields]
+    std::vector<uint32_t> h_cfp4;     // host copy
     std::vector<uint8_t> h_cmeta;
     std::vector<uint16_t> h_tab;      // instructions, CUDA order (host copy)
     DevBuf go_keys, go_keys2, go_ord, go_round, go_sort_tmp;   // Go-order verification rounds
     DevBuf jitems;                                             // chunks of long length-2 equal ranges
     DevBuf order;                                              // k_probe_pairs: the pairs it passed on
-    DevBuf join_keys[2][256], join_idx[2][256];   // by semantics and dead-flags mask
+    DevBuf join_tab[2][256];                      // JoinTable by semantics and dead-flags mask
     DevBuf join_groups[256];                      // CandGroups of the CUDA-semantics tables
     struct Cand2Table {            // sorted (key, index) of all length-2 sequences for one mask
         uint32_t dead = 0xFFFFFFFFu;
@@ -2110,7 +2125,6 @@ struct m6502_ctx {
     } cand2[4];                    // least recently used mask is rebuilt
     uint64_t cand2_clock = 0;
     DevBuf c2_keys_in, c2_idx_in, c2_sort_tmp;
-    uint32_t join_n[2][256] = {};
     DevBuf st_tins, st_toffs, st_tout, st_tbytes, st_chains, st_entries, st_vidx, st_proven, st_cnt, st_pidx,
         st_mex, st_probs, st_traj, st_row;
     DevBuf st_keys, st_keys2, st_vals2, st_rep, st_ord, st_verdict, st_vlist, st_vpos, st_sort_tmp, st_vphase,
@@ -2186,23 +2200,22 @@ const uint16_t* join_mult(const m6502_ctx* ctx, uint32_t dead) {
     return g ? g->mult : nullptr;
 }
 
-// The length-1 QuickCheck join under CUDA semantics, with the probe of its
-// MidCheck survivors when `probe` (1 + the sweep mode) is set.
+// The length-1 QuickCheck join.  A warp takes as many targets as fill the
+// resident warps, up to a lane each: small searches spread over all SMs.
 int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt, uint32_t dead, uint32_t stages,
-                 uint64_t scap, Counters* cnt, uint32_t probe) {
-    const uint32_t jgrid = (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 8, (nt + kWarpsPerBlock - 1) / kWarpsPerBlock);
-    const uint64_t* jk = (const uint64_t*)ctx->join_keys[0][dead].p;
-    const uint16_t* ji = (const uint16_t*)ctx->join_idx[0][dead].p;
-    const uint32_t jn = ctx->join_n[0][dead];
-    const uint16_t* mult = join_mult(ctx, dead);
-    if (probe)
-        k_qc_join<false, true><<<jgrid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, (uint64_t*)ctx->cfp1cm.p,
-                                                                 (uint8_t*)ctx->cmeta1.p, jk, ji, jn, dead, stages,
-                                                                 (Surv*)ctx->surv.p, scap, cnt, probe, mult);
+                 uint64_t scap, Counters* cnt, bool go) {
+    const uint64_t warps = (uint64_t)ctx->sms * 4 * kWarpsPerBlock;   // 4 resident blocks per SM
+    const uint32_t chunk = (uint32_t)std::min<uint64_t>(32, (nt + warps - 1) / warps);
+    const uint64_t blocks = (nt + (uint64_t)chunk * kWarpsPerBlock - 1) / ((uint64_t)chunk * kWarpsPerBlock);
+    const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->sms * 4, blocks));
+    const JoinTable* tab = (const JoinTable*)ctx->join_tab[go][dead].p;
+    const uint4* cfp4 = (const uint4*)ctx->cfp4.p;
+    if (go)
+        k_qc_join<true><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages,
+                                                       (Surv*)ctx->surv.p, scap, cnt, nullptr);
     else
-        k_qc_join<false, false><<<jgrid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, (uint64_t*)ctx->cfp1cm.p,
-                                                                  (uint8_t*)ctx->cmeta1.p, jk, ji, jn, dead, stages,
-                                                                  (Surv*)ctx->surv.p, scap, cnt, 0u, mult);
+        k_qc_join<false><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages,
+                                                        (Surv*)ctx->surv.p, scap, cnt, join_mult(ctx, dead));
     CKL("k_qc_join");
     return M6502_OK;
 }
@@ -2215,6 +2228,13 @@ int launch_items(m6502_ctx* ctx, const SurvSource& src, ExhArgs ea) {
     k_exh_items<SurvSource><<<ctx->exh_item_blocks, 256, 0, ctx->stream>>>(src, ea);
     CKL("k_exh_items");
     return M6502_OK;
+}
+
+// Field f (byte f of a packed state) of four states, one per byte.
+uint32_t pack4(const uint64_t* states, int f) {
+    uint32_t w = 0;
+    for (int k = 0; k < 4; k++) w |= (uint32_t)((states[k] >> (8 * f)) & 0xFFu) << (8 * k);
+    return w;
 }
 
 int init_ctx(m6502_ctx* ctx) {
@@ -2236,7 +2256,11 @@ int init_ctx(m6502_ctx* ctx) {
     host_tables(tab, gotab, gorank);
     uint32_t rep[32];
     for (int i = 0; i < 32; i++) rep[i] = kRepValues[i];
+    uint32_t vec4[8][8];
+    for (int g = 0; g < 8; g++)
+        for (int f = 0; f < 8; f++) vec4[g][f] = pack4(vec + 4 * g, f);
     CK(cudaMemcpyToSymbol(c_vec, vec, sizeof vec));
+    CK(cudaMemcpyToSymbol(c_vec4, vec4, sizeof vec4));
     CK(cudaMemcpyToSymbol(c_dep, dep, sizeof dep));
     CK(cudaMemcpyToSymbol(c_wr, wr, sizeof wr));
     CK(cudaMemcpyToSymbol(c_sweep, sw, sizeof sw));
@@ -2287,10 +2311,13 @@ int init_ctx(m6502_ctx* ctx) {
         uint16_t one = tab[c];
         meta[c] = (uint8_t)(bytes_cuda(op) | (bytes_go(op) << 2) | (should_prune(&one, 1) ? 0x10 : 0));
     }
-    ctx->h_cfp0.assign(tr.begin(), tr.begin() + kNumInsns);
-    ctx->h_cfp8.assign(tr.begin(), tr.begin() + 8 * (size_t)kNumInsns);
-    TRY(ensure(ctx, ctx->cfp1cm, sizeof(uint64_t) * 32 * kNumInsns));
-    CK(cudaMemcpyAsync(ctx->cfp1cm.p, h.data(), h.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
+    ctx->h_cfp4.resize((size_t)kNumInsns * 64);
+    for (int c = 0; c < kNumInsns; c++)
+        for (int g = 0; g < 8; g++)
+            for (int f = 0; f < 8; f++) ctx->h_cfp4[(size_t)c * 64 + 8 * g + f] = pack4(&h[(size_t)c * 32 + 4 * g], f);
+    TRY(ensure(ctx, ctx->cfp4, ctx->h_cfp4.size() * sizeof(uint32_t)));
+    CK(cudaMemcpyAsync(ctx->cfp4.p, ctx->h_cfp4.data(), ctx->h_cfp4.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                       ctx->stream));
     ctx->h_cmeta = meta;
     ctx->h_tab.assign(tab, tab + kNumInsns);
     CK(cudaMemcpyAsync(ctx->cfp1.p, tr.data(), tr.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
@@ -2320,9 +2347,14 @@ int cand_group(uint32_t op, uint32_t dead) {
 // one entry per group of candidates; Go semantics: every candidate (its
 // passes and ranks tell the members of a group apart).
 int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
-    if (ctx->join_n[go][dead]) return M6502_OK;
-    const uint64_t loose = cmp_mask(dead);
-    std::vector<std::pair<uint64_t, uint16_t>> v;
+    if (ctx->join_tab[go][dead].p) return M6502_OK;
+    const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;
+    struct Entry {
+        uint64_t key;
+        std::vector<uint32_t> words;
+        uint16_t cand;
+    };
+    std::vector<Entry> v;
     CandGroups gr;
     std::memset(&gr, 0, sizeof gr);
     std::vector<std::vector<uint16_t>> groups;   // members; a lone candidate is a group of its own
@@ -2335,19 +2367,36 @@ int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
             if (!at.second) { groups[at.first->second].push_back((uint16_t)c); continue; }
         }
         groups.push_back({(uint16_t)c});
-        uint64_t x = 0;
-        for (int q = 0; q < 8; q++) x ^= key_term(ctx->h_cfp8[(size_t)q * kNumInsns + c] & loose, q);
-        const uint64_t key = key_final(x);
-        v.emplace_back(key, (uint16_t)c);
+        std::vector<uint32_t> words(ctx->h_cfp4.begin() + (long)c * 64, ctx->h_cfp4.begin() + (long)(c + 1) * 64);
+        for (int g = 0; g < 8; g++) words[8 * g + 3] &= pm;
+        uint32_t qc[16];
+        std::copy(words.begin(), words.begin() + 16, qc);
+        v.push_back({join_key(qc), std::move(words), (uint16_t)c});
     }
-    std::sort(v.begin(), v.end());
-    std::vector<uint64_t> keys(v.size());
-    std::vector<uint16_t> idx(v.size());
-    for (size_t i = 0; i < v.size(); i++) { keys[i] = v[i].first; idx[i] = v[i].second; }
-    TRY(ensure(ctx, ctx->join_keys[go][dead], keys.size() * 8));
-    TRY(ensure(ctx, ctx->join_idx[go][dead], idx.size() * 2));
-    CK(cudaMemcpy(ctx->join_keys[go][dead].p, keys.data(), keys.size() * 8, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->join_idx[go][dead].p, idx.data(), idx.size() * 2, cudaMemcpyHostToDevice));
+    std::sort(v.begin(), v.end(), [](const Entry& a, const Entry& b) {
+        return std::tie(a.key, a.words, a.cand) < std::tie(b.key, b.words, b.cand);
+    });
+    std::vector<JoinTable> tab(1);
+    JoinTable& t = tab[0];
+    std::memset(&t, 0, sizeof t);
+    uint32_t nu = 0, nj = 0, bucket = 0;
+    for (size_t i = 0; i < v.size(); i++) {
+        const Entry& e = v[i];
+        const uint32_t op = ctx->h_tab[e.cand] & 0xFFu, bytes = go ? bytes_go(op) : bytes_cuda(op);
+        const bool entry = i == 0 || e.key != v[i - 1].key ||
+                           !std::equal(e.words.begin(), e.words.begin() + 16, v[i - 1].words.begin());
+        if (entry) {
+            t.key[nu] = e.key;
+            t.sub[nu] = (uint16_t)nj;
+            for (const uint32_t b = (uint32_t)(e.key >> (64 - kDirBits)); bucket <= b; bucket++) t.dir[bucket] = (uint16_t)nu;
+            nu++;
+        }
+        if (entry || e.words != v[i - 1].words) t.start[nj++] = (uint16_t)i;
+        t.cand[i] = (uint16_t)(e.cand | bytes << 12);
+    }
+    t.sub[nu] = (uint16_t)nj;
+    t.start[nj] = (uint16_t)v.size();
+    for (; bucket <= (1u << kDirBits); bucket++) t.dir[bucket] = (uint16_t)nu;
     if (!go) {
         uint16_t at = 0;
         for (const auto& e : groups) {
@@ -2355,10 +2404,14 @@ int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
             gr.first[e[0]] = at;
             for (uint16_t c : e) gr.member[at++] = c;
         }
+        for (uint32_t u = 0; u < nu; u++)
+            for (uint32_t i = t.start[t.sub[u]]; i < t.start[t.sub[u + 1]]; i++)
+                for (uint32_t b = t.cand[i] >> 12; b <= 2; b++) t.weight[u][b - 1] += gr.mult[t.cand[i] & 0xFFFu];
         TRY(ensure(ctx, ctx->join_groups[dead], sizeof gr));
         CK(cudaMemcpy(ctx->join_groups[dead].p, &gr, sizeof gr, cudaMemcpyHostToDevice));
     }
-    ctx->join_n[go][dead] = (uint32_t)v.size();
+    TRY(ensure(ctx, ctx->join_tab[go][dead], sizeof t));
+    CK(cudaMemcpy(ctx->join_tab[go][dead].p, &t, sizeof t, cudaMemcpyHostToDevice));
     return M6502_OK;
 }
 
@@ -2471,18 +2524,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         CK(rec(ctx->sev[1]));
         uint32_t qgrid = (uint32_t)std::min<uint64_t>(ctx->qc_blocks, (nt + kQcTile - 1) / kQcTile);
         if (!scan) {
-            uint32_t jgrid = (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 8, (nt + kWarpsPerBlock - 1) / kWarpsPerBlock);
-            const uint64_t* jk = (const uint64_t*)ctx->join_keys[1][dead].p;
-            const uint16_t* ji = (const uint16_t*)ctx->join_idx[1][dead].p;
-            if (go)
-                k_qc_join<true><<<jgrid, 256, 0, ctx->stream>>>(d_targets, tlen,
-                                                                (uint32_t)nt, (uint64_t*)ctx->cfp1cm.p,
-                                                                (uint8_t*)ctx->cmeta1.p, jk, ji, ctx->join_n[1][dead],
-                                                                dead, stages, (Surv*)ctx->surv.p, scap, cnt, 0u,
-                                                                nullptr);
-            else
-                TRY(launch_join1(ctx, d_targets, tlen, nt, dead, stages, scap, cnt,
-                                 (ctx->tune.join_probe && exh) ? 1u + cfg.sweep : 0u));
+            TRY(launch_join1(ctx, d_targets, tlen, nt, dead, stages, scap, cnt, go));
         } else if (go)
             k_qc1<true><<<qgrid, 256, 0, ctx->stream>>>((uint64_t*)ctx->tfp.p, (uint8_t*)ctx->tmeta.p,
                                                         (uint32_t)nt, (uint64_t*)ctx->cfp1.p,
@@ -2628,9 +2670,9 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
                 (uint64_t)(uintptr_t)ctx->go_keys.p, (uint64_t)(uintptr_t)ctx->go_keys2.p,
                 (uint64_t)(uintptr_t)ctx->go_ord.p, (uint64_t)(uintptr_t)ctx->go_round.p,
                 (uint64_t)(uintptr_t)ctx->go_sort_tmp.p, ctx->go_sort_tmp.bytes, (uint64_t)(uintptr_t)ctx->jitems.p,
-                (uint64_t)(uintptr_t)ctx->join_keys[go][dead].p, c2 ? (uint64_t)(uintptr_t)c2->keys.p : 0,
+                (uint64_t)(uintptr_t)ctx->join_tab[go][dead].p, c2 ? (uint64_t)(uintptr_t)c2->keys.p : 0,
                 c2e ? (uint64_t)(uintptr_t)c2e->keys.p : 0, ctx->tune.exh_minb, ctx->tune.ticket_batch,
-                ctx->tune.chunk_log2, ctx->tune.join_probe};
+                ctx->tune.chunk_log2};
             m6502_ctx::PassGraph* pg = nullptr;
             for (m6502_ctx::PassGraph& g : ctx->pass_graphs)
                 if (g.exec && g.key == key) pg = &g;
@@ -2698,7 +2740,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
             st->exh_states += hc.states;
             st->exh_items += rounds ? hc.round_items : hc.items + hc.items1;
             st->exh_algo_ops += hc.algo;
-            st->exh_probe_rejects += hc.probe_rejects + hc.join_probe_rej;
+            st->exh_probe_rejects += hc.probe_rejects;
             st->exh_undecided += hc.undecided;
             float ms[5];
             for (int i = 0; i < 5; i++) cudaEventElapsedTime(&ms[i], ctx->sev[i], ctx->sev[i + 1]);
@@ -2791,8 +2833,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                                                                  (Surv*)ctx->surv.p, scap, cnt);
                     CKL("k_qc1");
                 } else {
-                    TRY(launch_join1(ctx, d_t, tlen, nt, dead, stages, scap, cnt,
-                                     (ctx->tune.join_probe && exh) ? 1u + cfg.sweep : 0u));
+                    TRY(launch_join1(ctx, d_t, tlen, nt, dead, stages, scap, cnt, false));
                 }
                 CK(rec(ev[2]));
                 SurvSource src{(const Surv*)ctx->surv.p, d_t, tlen, dead, 0, groups ? groups->mult : nullptr};
@@ -2821,8 +2862,8 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 (uint64_t)(uintptr_t)ctx->fail.p, (uint64_t)(uintptr_t)ctx->items.p, (uint64_t)(uintptr_t)ctx->order.p,
                 (uint64_t)(uintptr_t)ctx->rules.p, (uint64_t)(uintptr_t)ctx->cnt_slots.p,
                 (uint64_t)(uintptr_t)ctx->tfp.p, (uint64_t)(uintptr_t)ctx->tmeta.p,
-                (uint64_t)(uintptr_t)ctx->join_keys[0][dead].p, ctx->tune.exh_minb, ctx->tune.ticket_batch,
-                ctx->tune.chunk_log2, ctx->tune.join_probe};
+                (uint64_t)(uintptr_t)ctx->join_tab[0][dead].p, ctx->tune.exh_minb, ctx->tune.ticket_batch,
+                ctx->tune.chunk_log2};
             if (!(ctx->graph.exec && ctx->graph.key == key)) {
                 if (ctx->graph.exec) { cudaGraphExecDestroy(ctx->graph.exec); ctx->graph.exec = nullptr; }
                 // Record; if recording or instantiation fails, this context stops
@@ -2894,7 +2935,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 st->exh_states += c.states;
                 st->exh_items += c.items;
                 st->exh_algo_ops += c.algo;
-                st->exh_probe_rejects += c.probe_rejects + c.join_probe_rej;
+                st->exh_probe_rejects += c.probe_rejects;
                 st->exh_undecided += c.undecided;
                 float ms[5];
                 for (int i = 0; i < 5; i++) cudaEventElapsedTime(&ms[i], ctx->aev[6 * p + i], ctx->aev[6 * p + i + 1]);
@@ -3096,13 +3137,11 @@ void m6502_destroy(m6502_ctx* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (int i = 0; i < 256; i++) {
-        for (int g = 0; g < 2; g++) {
-            if (ctx->join_keys[g][i].p) cudaFree(ctx->join_keys[g][i].p);
-            if (ctx->join_idx[g][i].p) cudaFree(ctx->join_idx[g][i].p);
-        }
+        for (int g = 0; g < 2; g++)
+            if (ctx->join_tab[g][i].p) cudaFree(ctx->join_tab[g][i].p);
         if (ctx->join_groups[i].p) cudaFree(ctx->join_groups[i].p);
     }
-    DevBuf* bufs[] = {&ctx->cfp1cm, &ctx->cfp1, &ctx->cmeta1, &ctx->targets, &ctx->ids, &ctx->tfp, &ctx->tmeta,
+    DevBuf* bufs[] = {&ctx->cfp4, &ctx->cfp1, &ctx->cmeta1, &ctx->targets, &ctx->ids, &ctx->tfp, &ctx->tmeta,
                       &ctx->surv, &ctx->fail, &ctx->items, &ctx->rules, &ctx->cnt, &ctx->best,
                       &ctx->pins, &ctx->poffs, &ctx->cins, &ctx->coffs, &ctx->pout, &ctx->pfd,
                       &ctx->enum_count, &ctx->st_tins, &ctx->st_toffs, &ctx->st_tout, &ctx->st_tbytes,
@@ -3444,14 +3483,14 @@ int m6502_autotune(m6502_ctx* ctx, const char* cache_path, uint32_t flags, m6502
         return M6502_OK;
     };
     m6502_tune best = ctx->tune;
-    best.exh_minb = 4; best.ticket_batch = 4; best.chunk_log2 = 11; best.join_probe = 1;
+    best.exh_minb = 4; best.ticket_batch = 4; best.chunk_log2 = 11; best.join_probe = 1;   // join_probe: no effect
     double best_ms = 0;
     int rc = measure(best, &best_ms);
     // Coordinate descent: each knob in turn over its candidates, the others held.
-    const uint32_t probe_v[] = {0, 1}, minb_v[] = {2, 3, 4}, tb_v[] = {2, 4, 8, 16}, ck_v[] = {10, 11, 12, 13};
+    const uint32_t minb_v[] = {2, 3, 4}, tb_v[] = {2, 4, 8, 16}, ck_v[] = {10, 11, 12, 13};
     using Field = uint32_t m6502_tune::*;
     struct Knob { Field f; const uint32_t* v; int n; };
-    const Knob knobs[] = {{&m6502_tune::join_probe, probe_v, 2}, {&m6502_tune::exh_minb, minb_v, 3},
+    const Knob knobs[] = {{&m6502_tune::exh_minb, minb_v, 3},
                           {&m6502_tune::ticket_batch, tb_v, 4}, {&m6502_tune::chunk_log2, ck_v, 4}};
     for (const Knob& k : knobs) {
         if (rc != M6502_OK) break;

@@ -321,6 +321,20 @@ M6502_HD void exec_x4(St& s, uint32_t insn) {
     }
 }
 
+// The same instruction on N packed words of states (4 N states) with one
+// dispatch.
+template <int N>
+M6502_HD void exec_x4n(St (&v)[N], uint32_t insn) {
+    const uint32_t immw = (insn >> 8) * kB1;
+    (void)immw;
+    switch (insn & 0xFFu) {
+#define M6502_CASE_X4N(op, ...) case op: { for (int k_ = 0; k_ < N; k_++) { St& s = v[k_]; __VA_ARGS__; } } break;
+        M6502_OPCODES_X4(M6502_CASE_X4N)
+#undef M6502_CASE_X4N
+    default: break;
+    }
+}
+
 // ---- Four states per register through per-opcode descriptors ----
 //
 // exec_x4d runs an instruction from a small descriptor instead of one case

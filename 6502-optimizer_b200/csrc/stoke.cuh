@@ -414,7 +414,6 @@ struct StokeSource {
         if (lane < cn) sc[lane] = e.ins[lane];
         dead = dead_;
     }
-    __device__ bool probed(uint64_t) const { return false; }
     __device__ uint64_t target_id(uint64_t) const { return kNoTarget; }   // candidates may be empty
     __device__ uint32_t weight(uint64_t) const { return 1u; }
 };

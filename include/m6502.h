@@ -156,9 +156,9 @@ typedef struct m6502_tune {
                                64 registers per thread) */
     uint32_t ticket_batch;  /* 1..32: pairs an exhaustive warp claims per ticket */
     uint32_t chunk_log2;    /* 9..16: states per work item of a large cone, log2 */
-    uint32_t join_probe;    /* 0 or 1: the random-state probe of MidCheck survivors runs
-                               inside the QuickCheck join (CUDA semantics, length-1
-                               candidates) instead of in the exhaustive kernel */
+    uint32_t join_probe;    /* 0 or 1, without effect: the random-state probe of MidCheck
+                               survivors always runs in a kernel of its own (inside the
+                               QuickCheck join it doubled the full length-2 search) */
     uint32_t reserved[4];
 } m6502_tune;               /* 32 bytes */
 
@@ -171,8 +171,8 @@ int m6502_tune_set(m6502_ctx *ctx, const m6502_tune *t);
 enum { M6502_TUNE_FORCE = 1 /* tune even when a cache for this device exists */ };
 /* Picks the knobs for this device by timing them on the device (full
  * length-2 enumeration, CUDA semantics, full sweep, mask 0x00: coordinate
- * descent over join_probe, exh_minb, ticket_batch and chunk_log2, median of
- * three timed runs each, about a second), sets them on ctx and writes them to
+ * descent over exh_minb, ticket_batch and chunk_log2, median of three timed
+ * runs each, about a second), sets them on ctx and writes them to
  * `cache_path` (NULL: $M6502_TUNE_CACHE, else $XDG_CACHE_HOME/m6502/ or
  * ~/.cache/m6502/, one file per device name and SM count).  Without
  * M6502_TUNE_FORCE a readable cache for the device is used instead of
