@@ -12,9 +12,10 @@
 //                   target, then a tile of 64 targets x all 2,863
 //                   candidates per CTA with one masked 64-bit compare per
 //                   pair; the same survivors as the join.
-//   k_probe_pairs   persistent, lean; 128 random states of every surviving
-//                   pair's sweep domain (four per lane, packed); rejects are
-//                   marked, the rest listed for k_exhaustive.
+//   k_expand        matching targets x their candidates -> survivors; those
+//                   that differ on the line states are rejected here.
+//   k_small         lane per pair; decides the pairs whose outputs depend on
+//                   at most nine input bits, lists the rest for k_exhaustive.
 //   k_exhaustive    persistent; a warp takes one listed pair from a device
 //                   ticket, derives the pair's swept input space (reference
 //                   rule) and the input cone of every output location, and
@@ -98,6 +99,7 @@ const uint8_t kRepValues[32] = {
 
 __constant__ uint64_t c_vec[32];             // packed test vectors
 __constant__ uint32_t c_vec4[8][8];           // the same, vectors 4 g .. 4 g + 3 one per byte of each field (A X Y P S M S0 S1)
+__constant__ uint32_t c_line[64][8];         // the 256 line states (see k_expand), four per word, by field
 __constant__ uint16_t c_dep[NUM_OPS][NUM_LOCS];
 __constant__ uint16_t c_wr[NUM_OPS];          // written locations per opcode
 __constant__ uint16_t c_sweep[NUM_OPS];       // swept locations implied by opReads
@@ -243,6 +245,8 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const uint64_t* __restrict_
     return lo + (uint32_t)__popc(__ballot_sync(kFull, i < hi && keys[i] < key));
 }
 
+constexpr int kVerifyCounters = 5;   // exh_ticket .. small_left of Counters
+
 // Survivor record: target (index within the pass) and candidate code:
 // bits 0..22 candidate index, bit 23 length-2 candidate, bit 24 Go masked
 // pass, bits 25..30 FlagDiff (P bits 0-3, 6-7 compressed to 6 bits).
@@ -256,7 +260,10 @@ constexpr uint64_t kNoTarget = ~0ull;
 __host__ __device__ __forceinline__ uint32_t fd_pack(uint32_t fd) { return (fd & 0x0Fu) | ((fd >> 2) & 0x30u); }
 
 struct Counters {
-    unsigned long long qc, mid, surv, exh_ticket, items, item_ticket, rules, exh_pass, states, algo, probe_rejects;
+    unsigned long long qc, mid;
+    // reset together for every verification (surv: for every phase)
+    unsigned long long surv, exh_ticket, items, item_ticket, small_ticket, small_left;
+    unsigned long long rules, exh_pass, states, algo, probe_rejects;
     unsigned long long round_n, max_ord;   // Go-order verification rounds
     unsigned long long join_items;         // chunks of long length-2 equal ranges
     unsigned long long undecided;          // pairs left undecided (a cone beyond the sweep cap)
@@ -264,8 +271,7 @@ struct Counters {
     unsigned long long surv1, items1;      // phase-1 survivors and work items (length-2 phase runs after)
     unsigned long long surv_need, items_need;   // largest survivor / work-item counts seen, for the
                                                 // overflow check after the pass
-    unsigned long long join_ticket;        // k_qc_join: claimed chunks of targets
-    unsigned long long probe_ticket, probe_pass;   // k_probe_pairs: claimed pairs, pairs it passed on
+    unsigned long long join_ticket, matches;   // k_qc_join: claimed chunks of targets, matching targets
 };
 
 struct Item {   // one chunk of a large cone sweep
@@ -307,6 +313,7 @@ __device__ __forceinline__ uint32_t surv_weight(uint32_t code, const uint16_t* m
 
 // Pair sources: survivors of the enumeration pipeline, or explicit CSR pairs.
 struct SurvSource {
+    static constexpr int kMaxT = 3, kMaxC = 2;   // longest target and candidate
     const Surv* surv;
     const uint16_t* targets;
     uint32_t tlen;
@@ -328,6 +335,17 @@ struct SurvSource {
         }
         dead = go ? ((s.c & kSurvMasked) ? run_dead : 0u) : run_dead;
     }
+    // Pair p into a lane's column of the staging array (instruction i at st[i * ld]).
+    __device__ void load_lane(uint64_t p, uint16_t* st, uint16_t* sc, int ld, int& tn, int& cn, uint32_t& dead) const {
+        const Surv s = surv[p];
+        tn = (int)tlen;
+        for (int i = 0; i < tn; i++) st[i * ld] = targets[(uint64_t)s.t * tlen + i];
+        const uint32_t idx = s.c & 0x7FFFFFu;
+        cn = (s.c & kSurvLen2) ? 2 : 1;
+        sc[0] = c_tab[cn == 2 ? idx / kNumInsns : idx];
+        if (cn == 2) sc[ld] = c_tab[idx % kNumInsns];
+        dead = go && !(s.c & kSurvMasked) ? 0u : run_dead;
+    }
     // Pairs with the same id share their target (the probe reuses its outputs).
     __device__ uint64_t target_id(uint64_t p) const { return surv[p].t; }
     // Pairs that record p stands for.
@@ -335,6 +353,7 @@ struct SurvSource {
 };
 
 struct CsrSource {
+    static constexpr int kMaxT = kMaxSeq, kMaxC = kMaxSeq;
     const uint16_t* t_ins;
     const uint32_t* t_off;
     const uint16_t* c_ins;
@@ -347,6 +366,14 @@ struct CsrSource {
         cn = (int)(c_off[p + 1] - c0);
         if (lane < tn) st[lane] = t_ins[t0 + lane];
         if (lane < cn) sc[lane] = c_ins[c0 + lane];
+        dead = dead_;
+    }
+    __device__ void load_lane(uint64_t p, uint16_t* st, uint16_t* sc, int ld, int& tn, int& cn, uint32_t& dead) const {
+        const uint32_t t0 = t_off[p], c0 = c_off[p];
+        tn = (int)(t_off[p + 1] - t0);
+        cn = (int)(c_off[p + 1] - c0);
+        for (int i = 0; i < tn; i++) st[i * ld] = t_ins[t0 + i];
+        for (int i = 0; i < cn; i++) sc[i * ld] = c_ins[c0 + i];
         dead = dead_;
     }
     __device__ uint64_t target_id(uint64_t) const { return kNoTarget; }
@@ -434,24 +461,6 @@ __device__ __forceinline__ uint32_t state_diff_in(const PairView& pv, const OutM
 __device__ __forceinline__ uint32_t state_diff(const PairView& pv, const Fields& f, const OutMask& m, uint64_t s) {
     return state_diff_in(pv, m, decode_state(f, s));
 }
-
-// Target and candidate on two states per lane: one loop over target then
-// candidate (a single inlined copy of the opcode switch per call site keeps
-// the code, and instruction-cache misses, small) and one dispatch per
-// instruction for both states (exec2).  The inputs are decoded again for the
-// candidate instead of being kept live.
-__device__ __forceinline__ uint32_t state_diff2(const PairView& pv, const Fields& f, const OutMask& m, uint64_t sa,
-                                                uint64_t sb) {
-    St c0 = decode_state(f, sa), c1 = decode_state(f, sb), t0 = c0, t1 = c1;
-    const int n = pv.tn + pv.cn;
-    for (int i = 0; i < n; i++) {
-        if (i == pv.tn) { t0 = c0; t1 = c1; c0 = decode_state(f, sa); c1 = decode_state(f, sb); }
-        exec2(c0, c1, i < pv.tn ? pv.t[i] : pv.c[i - pv.tn]);
-    }
-    if (pv.cn == 0) { t0 = c0; t1 = c1; c0 = decode_state(f, sa); c1 = decode_state(f, sb); }
-    return out_diff(t0, c0, m) | out_diff(t1, c1, m);
-}
-
 
 // One uniformly random state of a pair's whole sweep domain, from 64 random
 // bits: every swept register takes its own byte of z (its representative
@@ -605,20 +614,12 @@ __device__ __forceinline__ St decode_x4(const Fields& f, uint64_t s) {
     return o;
 }
 
-// DESC: run the instructions through their descriptors (exec_x4d, a
-// 12-way class switch) instead of the per-opcode switch (exec_x4).  The
-// descriptors pay off where the warps of an SM hop between different pairs
-// (fewer branch targets to fetch); long sweeps of one pair prefer the
-// specialised cases.
-template <bool DESC>
 __device__ __forceinline__ uint32_t state_diff_x4(const PairView& pv, const Fields& f, const OutMask& m4, uint64_t s) {
     St c = decode_x4(f, s), t = c;
     const int n = pv.tn + pv.cn;
     for (int i = 0; i < n; i++) {
         if (i == pv.tn) { t = c; c = decode_x4(f, s); }
-        const uint32_t insn = i < pv.tn ? pv.t[i] : pv.c[i - pv.tn];
-        if (DESC) exec_x4d(c, insn, desc_x4(insn));
-        else exec_x4(c, insn);
+        exec_x4(c, i < pv.tn ? pv.t[i] : pv.c[i - pv.tn]);
     }
     if (pv.cn == 0) { t = c; c = decode_x4(f, s); }
     return out_diff(t, c, m4);
@@ -629,10 +630,10 @@ __device__ __forceinline__ uint32_t state_diff_x4(const PairView& pv, const Fiel
 // becomes nonzero (another item of the same pair failed) the sweep ends
 // early; its result is then irrelevant.
 // PER_LANE = 4: four consecutive states per lane packed one per byte
-// (exec_x4: one dispatch, byte-parallel arithmetic); 2: two states per lane
-// and dispatch; 1: one.  The packed path needs 4-aligned ranges and a
-// lowest field of at least 2 bits, and falls back to one state per lane.
-template <int PER_LANE, bool DESC = false>
+// (exec_x4: one dispatch, byte-parallel arithmetic); 1: one.  The packed path
+// needs 4-aligned ranges and a lowest field of at least 2 bits, and falls
+// back to one state per lane.
+template <int PER_LANE>
 __device__ __forceinline__ bool sweep_states(const PairView& pv, const Fields& f, uint64_t om, uint64_t s0,
                                              uint64_t s1, const volatile uint32_t* stop, unsigned long long* nstates,
                                              int lane) {
@@ -644,24 +645,84 @@ __device__ __forceinline__ bool sweep_states(const PairView& pv, const Fields& f
     }
     uint64_t iter = 0;
     constexpr uint64_t kStep = 32 * PER_LANE;
-    for (uint64_t b = s0; b < s1; b += kStep, iter++) {   // lane: states b + lane (+ 32)
-        const uint64_t sa = b + (uint64_t)lane;
+    for (uint64_t b = s0; b < s1; b += kStep, iter++) {
+        const uint64_t s = b + PER_LANE * (uint64_t)lane;
         uint32_t d = 0;
-        if (PER_LANE == 4) {
-            const uint64_t s4 = b + 4 * (uint64_t)lane;
-            d = s4 < s1 ? state_diff_x4<DESC>(pv, f, m, s4) : 0u;
-        } else if (PER_LANE == 2) {
-            const uint64_t sb = sa + 32;   // past the end: evaluate a state in range again
-            d = sa < s1 ? state_diff2(pv, f, m, sa, sb < s1 ? sb : sa) : 0u;
-        } else {
-            d = sa < s1 ? state_diff(pv, f, m, sa) : 0u;
-        }
+        if (s < s1) d = PER_LANE == 4 ? state_diff_x4(pv, f, m, s) : state_diff(pv, f, m, s);
         if (__any_sync(kFull, d != 0)) {
             if (lane == 0) *nstates += min((b - s0) + kStep, s1 - s0);
             return false;
         }
         if ((iter & (255 / PER_LANE)) == (255 / PER_LANE) && stop) {
             uint32_t sv = lane == 0 ? *stop : 0u;   // one read, broadcast: keeps the warp uniform
+            if (__shfl_sync(kFull, sv, 0)) break;
+        }
+    }
+    if (lane == 0) *nstates += s1 - s0;
+    return true;
+}
+__device__ __noinline__ bool sweep_general(const PairView& pv, uint32_t cone, uint32_t swept, bool rep, uint64_t om,
+                                           uint64_t s0, uint64_t s1, const volatile uint32_t* stop,
+                                           unsigned long long* nstates, int lane) {
+    return sweep_states<4>(pv, make_fields(cone, swept, rep), om, s0, s1, stop, nstates, lane);
+}
+
+// The same sweep by rows of 256 states when the cone's lowest field is a
+// whole register (A, or any register under the full sweep) and the range is
+// made of rows.  Lane l holds values 4 l .. 4 l + 3 and 4 l + 128 .. of that
+// register in two packed words for good; a row sets the other fields, the
+// same in every lane, and runs both words with one dispatch per instruction.
+// The general sweep decodes 8 fields with 64-bit shifts for every word and
+// sequence: 300 warp instructions per word, against 85 here (the work items
+// of the full length-2 enumeration: 0.60 -> 0.28 ms).
+__device__ __forceinline__ bool sweep_cone(const PairView& pv, uint32_t cone, uint32_t swept, bool rep, uint64_t om,
+                                           uint64_t s0, uint64_t s1, const volatile uint32_t* stop,
+                                           unsigned long long* nstates, int lane) {
+    const uint32_t regs = cone & ~LB(L_C);
+    const uint32_t low = (cone & LB(L_A)) ? LB(L_A) : (regs & (0u - regs));   // A first, then X Y S M S0 S1
+    if (low == 0 || (rep && low != LB(L_A)) || ((s0 | s1) & 255))
+        return sweep_general(pv, cone, swept, rep, om, s0, s1, stop, nstates, lane);
+    const uint32_t high = cone & ~low, bs = (swept & LB(L_S)) ? 0u : 0xFDu;   // S outside the cone: its first value
+    const uint32_t v0 = 4u * (uint32_t)lane * kB1 + 0x03020100u, v1 = v0 + 0x80808080u;
+    OutMask m = out_mask(om);
+    m.a *= kB1; m.x *= kB1; m.y *= kB1; m.p *= kB1; m.s *= kB1; m.m *= kB1; m.s0 *= kB1; m.s1 *= kB1;
+    const uint32_t r1 = (uint32_t)(s1 >> 8);
+    for (uint32_t row = (uint32_t)(s0 >> 8); row < r1; row++) {
+        uint32_t bits = row;
+        auto field = [&](uint32_t l, uint32_t fixed) -> uint32_t {   // the row's value of a location, in every byte
+            if (!(high & LB(l))) return fixed * kB1;
+            const uint32_t w = rep ? 5u : 8u, x = bits & ((1u << w) - 1u);
+            bits >>= w;
+            return (rep ? c_rep[x] : x) * kB1;
+        };
+        St in;
+        in.a = 0;
+        in.x = field(L_X, 0); in.y = field(L_Y, 0); in.s = field(L_S, bs); in.m = field(L_M, 0);
+        in.s0 = field(L_S0, 0); in.s1 = field(L_S1, 0);
+        in.p = (high & LB(L_C)) ? (bits & 1u) * kB1 : 0u;
+        St t[2], c[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint32_t v = k ? v1 : v0;
+            c[k] = in;
+            if (low == LB(L_A)) c[k].a = v;
+            else if (low == LB(L_X)) c[k].x = v;
+            else if (low == LB(L_Y)) c[k].y = v;
+            else if (low == LB(L_S)) c[k].s = v;
+            else if (low == LB(L_M)) c[k].m = v;
+            else if (low == LB(L_S0)) c[k].s0 = v;
+            else c[k].s1 = v;
+            t[k] = c[k];
+        }
+        for (int i = 0; i < pv.tn; i++) exec_x4n(t, pv.t[i]);
+        for (int i = 0; i < pv.cn; i++) exec_x4n(c, pv.c[i]);
+        const uint32_t d = out_diff(t[0], c[0], m) | out_diff(t[1], c[1], m);
+        if (__any_sync(kFull, d != 0)) {
+            if (lane == 0) *nstates += ((uint64_t)row << 8) + 256 - s0;
+            return false;
+        }
+        if ((row & 31) == 31 && stop) {
+            const uint32_t sv = lane == 0 ? *stop : 0u;   // one read, broadcast: keeps the warp uniform
             if (__shfl_sync(kFull, sv, 0)) break;
         }
     }
@@ -795,19 +856,6 @@ __device__ __forceinline__ uint32_t compose_s(uint32_t D, const uint16_t* seq, i
     return D;
 }
 
-__device__ __forceinline__ Flow dataflow_s(const PairView& pv, int lane, const uint16_t (*dep_tab)[NUM_LOCS]) {
-    Flow fl;
-    uint32_t wt = 0, wc = 0, sw = 0;
-    uint32_t id = (lane < NUM_LOCS) ? (1u << lane) : 0u;
-    uint32_t dt = compose_s(id, pv.t, pv.tn, lane, wt, sw, dep_tab);
-    uint32_t dc = compose_s(id, pv.c, pv.cn, lane, wc, sw, dep_tab);
-    fl.k = __popc(sw);
-    fl.swept = sw | LB(L_A) | LB(L_C);
-    fl.written = wt | wc;
-    fl.cone = (dt | dc) & fl.swept;
-    return fl;
-}
-
 // The same composition with the target's half kept in the warp's cache:
 // pairs of one target (consecutive survivors) compose only their candidate.
 // The two halves are independent: each starts from the identity.
@@ -890,8 +938,8 @@ struct ExhArgs {
     uint32_t defer_bits;         // > 0: pairs with a cone above 2^defer_bits states get fail = 4 (deferred)
     uint32_t ticket_batch;       // pairs a warp claims per ticket atomic (0 = kTicketBatch)
     uint32_t chunk_log2;         // states per work item, at least (0 = kChunk)
-    const uint32_t* order;       // non-null: ticket q sweeps pair order[q] (the pairs k_probe_pairs
-                                 // passed on, already probed); null: ticket q is pair q
+    const uint32_t* order;       // non-null: ticket q sweeps pair order[q] (the pairs k_small left);
+                                 // null: ticket q is pair q
 };
 
 // ---------------------------------------------------------------------------
@@ -1092,14 +1140,13 @@ __global__ void __launch_bounds__(256) k_qc1(const uint64_t* __restrict__ tfp, c
 
 // QC (+ MidCheck) of targets x all length-1 candidates as an exact join
 // through the mask's JoinTable.  A warp takes `chunk` (1..32) consecutive
-// targets in two phases:
-//   - a lane per target runs it on the 8 QuickCheck vectors (two packed words
-//     of four states), hashes the outputs, finds the key's entry and checks
-//     the outputs against it (cfp4: 256 packed bytes per candidate), then
-//     runs it on the 24 MidCheck vectors and finds its subclass;
-//   - the candidates of all its targets, numbered through, go round the lanes
-//     and are appended as survivors.
-// Same survivors as k_qc1.  Bound by integer issue: a warp per target with a
+// targets, a lane each: it runs its target on the 8 QuickCheck vectors (two
+// packed words of four states), hashes the outputs, finds the key's entry
+// and checks the outputs against it (cfp4: 256 packed bytes per candidate),
+// then runs it on the 24 MidCheck vectors and finds its subclass.  A match is
+// written as {target, first candidate in JoinTable::cand | count << 16};
+// k_expand turns matches into the survivors that k_qc1 finds.
+// Bound by integer issue: a warp per target with a
 // lane per vector spent 400 warp instructions per target, most of them on
 // dispatch, hashing and ballots for 32 states of two instructions; here those
 // are paid once for 32 targets with four states per register.  Lanes whose
@@ -1111,8 +1158,8 @@ template <bool GO>
 __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__ targets, uint32_t tlen, uint32_t nt,
                                                   uint32_t chunk, const uint4* __restrict__ cfp4,
                                                   const JoinTable* __restrict__ table, uint32_t dead,
-                                                  uint32_t stages, Surv* __restrict__ surv, uint64_t cap,
-                                                  Counters* __restrict__ cnt, const uint16_t* __restrict__ mult) {
+                                                  uint32_t stages, Surv* __restrict__ match,
+                                                  Counters* __restrict__ cnt) {
     __shared__ alignas(16) uint8_t s_raw[kJoinShared];
     const JoinTable& s_tab = *reinterpret_cast<const JoinTable*>(s_raw);   // key and dir only
     __shared__ Surv s_stage[kWarpsPerBlock][kStage];
@@ -1123,7 +1170,7 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
     Surv* stage = s_stage[w];
     int nstage = 0;
     const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;   // compared bits of a packed P word
-    unsigned long long nqc = 0, nmid = 0;
+    unsigned long long nqc = 0;
     // Chunks come from a ticket, claimed one ahead: their hits are uneven, and
     // a fixed stride left some SMs with half the work of others.
     unsigned long long next = 0;
@@ -1132,13 +1179,12 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
         const uint64_t base = __shfl_sync(kFull, next, 0) * chunk;
         if (base >= nt) break;
         if (lane == 0) next = atomicAdd(&cnt->join_ticket, 1ull);
-        // -- a lane per target --
         const bool have = (uint32_t)lane < chunk && base + lane < nt;
         const uint16_t* tp = targets + (base + (have ? lane : 0)) * tlen;
         uint32_t ins01 = tp[0], ins2 = 0;   // its instructions: two in the first word, the third in the second
         if (tlen > 1) ins01 |= (uint32_t)tp[1] << 16;
         if (tlen > 2) ins2 = tp[2];
-        uint32_t tb = 0, lo = 0, n = 0, tp0, tp1;   // tp: P after the QuickCheck vectors
+        uint32_t tb = 0, lo = 0, n = 0;
         // Its outputs on vectors 8 r .. 8 r + 7 against candidate c's.
         auto run = [&](St (&v)[2], int r) {
 #pragma unroll
@@ -1167,8 +1213,6 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
             }
             const uint32_t words[16] = {v[0].a, v[0].x, v[0].y, v[0].p & pm, v[0].s, v[0].m, v[0].s0, v[0].s1,
                                         v[1].a, v[1].x, v[1].y, v[1].p & pm, v[1].s, v[1].m, v[1].s0, v[1].s1};
-            tp0 = v[0].p;
-            tp1 = v[1].p;
             const uint64_t key = join_key(words);
             const uint32_t b = (uint32_t)(key >> (64 - kDirBits));
             uint32_t j0 = 0, j1 = 0;   // subclasses of the entry that matches
@@ -1202,24 +1246,151 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
                 }
             }
         }
-        uint32_t upto = n;   // hits of this lane's and the lanes below
+        stage_push(n > 0, Surv{(uint32_t)base + (uint32_t)lane, lo | n << 16}, stage, nstage, match, nt, &cnt->matches, lane);
+    }
+    stage_flush(stage, nstage, match, nt, &cnt->matches, lane);
+    for (int o = 16; o; o >>= 1) nqc += __shfl_down_sync(kFull, nqc, o);
+    if (lane == 0 && nqc) atomicAdd(&cnt->qc, nqc);
+}
+
+// ---- Matches to survivors ----
+//
+// A target that passes MidCheck with a run of compare operands (CMP #k for
+// the k that no test vector tells apart) matches up to 43 candidates of which
+// one is right, and a random state of the sweep domain tells two of them
+// apart with a chance of a few in 256.  The line states do so for all of them
+// at once: 256 states in which A and every register that the target reads
+// take each value once (c_line: a permutation per register), the carry both
+// values, and the others the sweep's fixed ones.  They lie in the sweep
+// domain of every pair whose candidate reads no other register, so a pair
+// whose outputs differ there is rejected, as ExhaustiveCheck would.  The
+// outputs are compared by a 32-bit hash of the compared fields: the target's
+// is computed once for all its candidates, the candidates' are tabulated per
+// set of swept registers (k_line_hash, 64 x 2,863 per mask).  Unequal hashes
+// come from unequal outputs only; equal ones are left to ExhaustiveCheck.
+// Not filtered: pairs whose candidate reads a register the target does not,
+// and pairs swept over representative values (three or more extra registers
+// under the reduced sweep).
+
+// Bits 0..5 of a register set: X, Y, S, M, S0, S1 (the swept locations less A and carry).
+__host__ __device__ __forceinline__ uint32_t extra_bits(uint32_t swept) { return (swept >> 1) & 0x3Fu; }
+
+// Hash of the outputs of a sequence on the line states of register set
+// `regs`: the sum of a term per packed word, of which this call adds words
+// 2 sub, 2 sub + 1, then every 2 << g further on (2^g lanes share a
+// sequence); run(v) executes it on two words.
+template <class Run>
+__device__ __forceinline__ uint32_t line_hash(uint32_t regs, uint32_t pm, const Run& run, uint32_t sub = 0, int g = 0) {
+    auto mask = [&](uint32_t l) { return (regs & LB(l)) ? 0xFFFFFFFFu : 0u; };
+    const uint32_t mx = mask(L_X), my = mask(L_Y), ms = mask(L_S), mm = mask(L_M), m0 = mask(L_S0), m1 = mask(L_S1);
+    const uint32_t bs = ms ? 0u : 0xFDu * kB1;
+    uint32_t h = 0;
+    for (uint32_t j = 2 * sub; j < 64; j += 2u << g) {
+        St v[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint32_t* w = c_line[j + k];
+            v[k] = St{w[0], w[1] & mx, w[2] & my, w[3], (w[4] & ms) | bs, w[5] & mm, w[6] & m0, w[7] & m1};
+        }
+        run(v);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const St& s = v[k];
+            uint32_t x = (j + k) * 0x2C1B3C6Du + s.a * 0x9E3779B1u + s.x * 0x85EBCA77u + s.y * 0xC2B2AE3Du +
+                         (s.p & pm) * 0x27D4EB2Fu + s.s * 0x165667B1u + s.m * 0xD3A2646Du + s.s0 * 0xFD7046C5u +
+                         s.s1 * 0xB55A4F09u;
+            x = (x ^ (x >> 15)) * 0x2C1B3C6Du;
+            h += x ^ (x >> 13);
+        }
+    }
+    return h;
+}
+
+// Thread per (register set, candidate): the candidates' hashes for one mask.
+__global__ void __launch_bounds__(256) k_line_hash(uint32_t dead, uint32_t* __restrict__ out) {
+    const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 64u * kNumInsns; i += gridDim.x * blockDim.x) {
+        const uint32_t insn = c_tab[i % kNumInsns];
+        out[i] = line_hash((i / kNumInsns) << 1, pm, [&](St (&v)[2]) { exec_x4n(v, insn); });
+    }
+}
+
+// A lane per match, or 2^g lanes while the matches alone do not fill the
+// chip; a static stride, since each costs about the same.  FILTER computes
+// the target's line hash; then the candidates of the warp's matches, numbered
+// through, go round the lanes, and those that are shorter and not rejected
+// are appended as survivors.
+// The filter leaves 1.1 of the 5.4 M MidCheck survivors of the full length-2
+// enumeration (mask 0x00); the random probe it replaces (128 states, a warp
+// per pair) left 1.36 M in 2.42 ms.  Here, candidates and survivors included:
+// 0.48 ms.
+template <bool GO, bool FILTER>
+__global__ void __launch_bounds__(256, 4) k_expand(const Surv* __restrict__ match, const uint16_t* __restrict__ targets,
+                                                 uint32_t tlen, const uint4* __restrict__ cfp4,
+                                                 const JoinTable* __restrict__ table, uint32_t dead, uint32_t sweep,
+                                                 const uint16_t* __restrict__ mult, const uint32_t* __restrict__ lines,
+                                                 Surv* __restrict__ surv, uint64_t cap, Counters* __restrict__ cnt) {
+    __shared__ Surv s_stage[kWarpsPerBlock][kStage];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    Surv* stage = s_stage[w];
+    int nstage = 0;
+    const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;   // compared bits of a packed P word
+    unsigned long long nqc = 0, nmid = 0, nrej = 0;
+    const uint32_t nmatch = (uint32_t)cnt->matches;
+    int g = 4;   // lanes per match, log2
+    for (uint64_t warps = (uint64_t)gridDim.x * kWarpsPerBlock * 2; g > 0 && nmatch > warps; g--) warps <<= 1;
+    const uint32_t sub = (uint32_t)lane & ((1u << g) - 1u), per = 32u >> g;
+    for (uint64_t base = ((uint64_t)blockIdx.x * kWarpsPerBlock + w) * per; base < nmatch;
+         base += (uint64_t)gridDim.x * kWarpsPerBlock * per) {
+        const uint64_t mi = base + (uint32_t)(lane >> g);
+        const bool have = mi < nmatch && sub == 0;   // the lane that stands for the match
+        const Surv m = match[mi < nmatch ? mi : base];
+        const uint16_t* tp = targets + (uint64_t)m.t * tlen;
+        uint32_t ins01 = tp[0], ins2 = 0;
+        if (tlen > 1) ins01 |= (uint32_t)tp[1] << 16;
+        if (tlen > 2) ins2 = tp[2];
+        const uint32_t lo = m.c & 0xFFFFu, n = have ? m.c >> 16 : 0u;
+        auto run = [&](St (&v)[2]) {
+            for (uint32_t i = 0; i < tlen; i++) exec_x4n(v, i == 0 ? ins01 & 0xFFFFu : i == 1 ? ins01 >> 16 : ins2);
+        };
+        uint32_t tb = 0, regs = 0;
+        for (uint32_t i = 0; i < tlen; i++) {
+            const uint32_t op = (i == 0 ? ins01 : i == 1 ? ins01 >> 16 : ins2) & 0xFFu;
+            tb += GO ? bytes_go(op) : bytes_cuda(op);
+            regs |= c_sweep[op];
+        }
+        uint32_t hash = 0, tp0 = 0, tp1 = 0;   // tp: P after the QuickCheck vectors (Go semantics)
+        bool filter = FILTER && !(sweep == M6502_SWEEP_REFERENCE && __popc(regs) >= 3);
+        if (FILTER) {
+            hash = line_hash(regs, pm, run, sub, g);
+            for (int o = 0; o < g; o++) hash += __shfl_xor_sync(kFull, hash, 1 << o);
+        } else if (GO) {
+            St v[2];
+#pragma unroll
+            for (int g = 0; g < 2; g++)
+                v[g] = St{c_vec4[g][0], c_vec4[g][1], c_vec4[g][2], c_vec4[g][3],
+                          c_vec4[g][4], c_vec4[g][5], c_vec4[g][6], c_vec4[g][7]};
+            run(v);
+            tp0 = v[0].p;
+            tp1 = v[1].p;
+        }
+        uint32_t upto = n;   // candidates of this lane's match and the lanes' below
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t x = __shfl_up_sync(kFull, upto, o);
             upto += lane >= o ? x : 0u;
         }
         const uint32_t total = __shfl_sync(kFull, upto, 31);
-        // -- a lane per hit --
         for (uint32_t h0 = 0; h0 < total; h0 += 32) {
             const uint32_t h = h0 + (uint32_t)lane;
-            uint32_t own = 0;   // lanes whose hits end at or before h
+            uint32_t own = 0;   // lanes whose candidates end at or before h
 #pragma unroll
             for (uint32_t o = 16; o; o >>= 1) {
                 const uint32_t x = __shfl_sync(kFull, upto, (int)(own + o - 1));
                 own += x <= h ? o : 0u;
             }
-            own = min(own, 31u);
             const uint32_t end = __shfl_sync(kFull, upto, (int)own), cnt_o = __shfl_sync(kFull, n, (int)own);
             const uint32_t lo_o = __shfl_sync(kFull, lo, (int)own), tb_o = __shfl_sync(kFull, tb, (int)own);
+            const uint32_t t = __shfl_sync(kFull, m.t, (int)own);
             bool pass = h < total;
             uint32_t c = 0;
             if (pass) {
@@ -1244,10 +1415,19 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
                 }
                 nqc += pass;
                 nmid += pass;
-            } else if (pass) {
-                nmid += mult[c];
+            } else {
+                const uint32_t weight = pass ? mult[c] : 0u;   // pairs this record stands for
+                nmid += weight;
+                if (FILTER) {
+                    const uint32_t hash_o = __shfl_sync(kFull, hash, (int)own), regs_o = __shfl_sync(kFull, regs, (int)own);
+                    const bool filter_o = __shfl_sync(kFull, (int)filter, (int)own) != 0;
+                    if (pass && filter_o && !(c_sweep[c_tab[c] & 0xFFu] & ~regs_o) &&
+                        lines[extra_bits(regs_o) * kNumInsns + c] != hash_o) {
+                        pass = false;
+                        nrej += weight;
+                    }
+                }
             }
-            const uint32_t t = (uint32_t)base + own;
             stage_push(pass, Surv{t, code}, stage, nstage, surv, cap, &cnt->surv, lane);
         }
     }
@@ -1255,10 +1435,12 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
     for (int o = 16; o; o >>= 1) {
         nqc += __shfl_down_sync(kFull, nqc, o);
         nmid += __shfl_down_sync(kFull, nmid, o);
+        nrej += __shfl_down_sync(kFull, nrej, o);
     }
     if (lane == 0) {
         if (nqc) atomicAdd(&cnt->qc, nqc);
         if (nmid) atomicAdd(&cnt->mid, nmid);
+        if (nrej) atomicAdd(&cnt->probe_rejects, nrej);
     }
 }
 
@@ -1489,9 +1671,8 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
         pv.t = s_t[w]; pv.c = s_c[w];
         src.load(p, s_t[w], s_c[w], pv.tn, pv.cn, pv.dead, lane);
         const uint64_t tid = src.target_id(p);
-        const bool probed = a.order != nullptr;
         __syncwarp();
-        if (!probed) {
+        {
             uint32_t sw_t = 0, sw_c = 0;
             for (int i = 0; i < pv.tn; i++) sw_t |= c_sweep[pv.t[i] & 0xFFu];
             for (int i = 0; i < pv.cn; i++) sw_c |= c_sweep[pv.c[i] & 0xFFu];
@@ -1532,10 +1713,9 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
             if (a.brute) { o = 0; bits = brute_bits; cone = fl.swept; mask = cmp_mask(pv.dead); }
             else next_group(lg, rem, lane, o, bits, cone, mask);
             rem &= ~(1u << o);
-            Fields f = make_fields(cone, fl.swept, rep);
             const uint64_t total = 1ull << bits;
             const uint64_t end = total <= kSmallSweep ? total : kProbe;
-            ok = sweep_states<4, true>(pv, f, mask, 0, end, nullptr, &nstates, lane);
+            ok = sweep_cone(pv, cone, fl.swept, rep, mask, 0, end, nullptr, &nstates, lane);
             if (ok && end < total) big |= 1u << o;
         }
         if (ok && big) {
@@ -1568,74 +1748,121 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
     if (lane == 0 && probe_rej) atomicAdd(&a.cnt->probe_rejects, probe_rej);
 }
 
-// The random-state probe of every pair on its own, ahead of k_exhaustive:
-// a lean persistent kernel (many resident warps) runs probe_pair on each
-// surviving pair, marks the pairs it rejects (fail = 1) and appends the
-// others to `order`, 32 at a time per warp so that the passed pairs of one
-// target stay together; k_exhaustive then sweeps only those. 
+// ExhaustiveCheck of the pairs whose compared outputs depend on at most nine
+// bits of the swept input, a lane per pair, ahead of k_exhaustive.
+//
+// The union U of the cones of all compared outputs comes from walking the
+// sequences backwards (a set of locations in, the set it depends on out).
+// With at most 9 bits, U is one swept register or none, and the carry or
+// not: the lane runs target and candidate on every value of it, eight states
+// (two packed words) at a time, inputs outside U at the first value of their
+// range, and compares every output.  That is exact: U contains each output's
+// cone, and the states lie in the sweep domain.  Of the pairs of the full
+// length-2 enumeration that the line filter leaves, 99.6 % are decided here;
+// the others are listed for k_exhaustive, in which a warp spends about 1,500
+// instructions per pair (cone analysis by shuffles, ticket, staging) on 64
+// packed words of states.  The line at 9 bits: a lane takes 64 dispatches per
+// instruction for 512 states; one more register would make it 16,384.
+// Several lanes share a pair (a warp while that fills the chip, else four:
+// lanes whose candidates differ in opcode diverge).  The same enumeration:
+// 0.56 ms for 1.1 M pairs; k_exhaustive took 2.63 ms for 1.36 M.
+constexpr int kSmallLanesLog2 = 2;   // lanes per pair once the pairs alone fill the chip: 2^2
+__device__ __forceinline__ uint32_t backward(uint32_t locs, uint32_t op, const uint16_t (*dep)[16]) {
+    const uint32_t wr = c_wr[op];
+    uint32_t r = locs & ~wr;
+    for (uint32_t o = locs & wr; o; o &= o - 1) r |= dep[op][__ffs(o) - 1];
+    return r;
+}
+
 template <class Src>
-__global__ void __launch_bounds__(256) k_probe_pairs(Src src, const unsigned long long* n_pairs_ptr, uint64_t n_cap,
-                                                     ExhArgs a, uint32_t* __restrict__ order) {
-    __shared__ uint16_t s_t[kWarpsPerBlock][kMaxSeq], s_c[kWarpsPerBlock][kMaxSeq];
-    __shared__ TargetCache s_tc[kWarpsPerBlock];
-    __shared__ uint32_t s_pass[kWarpsPerBlock][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    TargetCache& tc = s_tc[w];
-    if (lane == 0) { tc.probe_id = kNoTarget; tc.flow_id = kNoTarget; }
-    __syncwarp();
+__global__ void __launch_bounds__(256) k_small(Src src, const unsigned long long* n_pairs_ptr, uint64_t n_cap,
+                                               ExhArgs a, uint32_t* __restrict__ order) {
+    __shared__ uint16_t s_ins[Src::kMaxT + Src::kMaxC][256];
+    __shared__ uint16_t s_dep[NUM_OPS][16];
+    for (int i = threadIdx.x; i < NUM_OPS * NUM_LOCS; i += blockDim.x) s_dep[i / NUM_LOCS][i % NUM_LOCS] = c_dep[i / NUM_LOCS][i % NUM_LOCS];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
     const uint64_t n = min((uint64_t)*n_pairs_ptr, n_cap);
-    const unsigned long long tbatch = a.ticket_batch ? a.ticket_batch : kTicketBatch;
-    unsigned long long next = 0, lim = 0, ahead = 0, probe_rej = 0;
-    int npass = 0;   // passed pairs staged in s_pass[w] (uniform)
-    auto flush = [&]() {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&a.cnt->probe_pass, (unsigned long long)npass);
-        base = __shfl_sync(kFull, base, 0);
-        if (lane < npass && base + lane < n_cap) order[base + lane] = s_pass[w][lane];
-        __syncwarp();
-        npass = 0;
-    };
-    if (lane == 0) ahead = atomicAdd(&a.cnt->probe_ticket, tbatch);
+    // Lanes per pair (log2): a warp while that fills the chip, then fewer.
+    int g = 5;
+    for (uint64_t warps = (uint64_t)gridDim.x * kWarpsPerBlock; g > kSmallLanesLog2 && n > warps; g--) warps <<= 1;
+    const uint32_t sub = (uint32_t)lane & ((1u << g) - 1u), lead = (uint32_t)lane - sub;
+    const uint32_t group = (g == 5 ? kFull : (1u << (1 << g)) - 1u) << lead;
+    const unsigned long long batch = 32u >> g;
+    // the pair's sequences: one column of the staging array for its lanes
+    uint16_t *st = &s_ins[0][(threadIdx.x & ~31u) + lead], *sc = st + Src::kMaxT * 256;
+    unsigned long long nstates = 0, next = 0;
+    if (lane == 0) next = atomicAdd(&a.cnt->small_ticket, batch);
     for (;;) {
-        if (next >= lim) {
-            next = __shfl_sync(kFull, ahead, 0);
-            lim = next + tbatch;
-            if (lane == 0 && next < n) ahead = atomicAdd(&a.cnt->probe_ticket, tbatch);
+        const uint64_t first = __shfl_sync(kFull, next, 0), p = first + (uint32_t)(lane >> g);
+        if (first >= n) break;
+        if (lane == 0) next = atomicAdd(&a.cnt->small_ticket, batch);
+        int tn = 0, cn = 0;
+        uint32_t dead = 0, swx = 0, written = 0;
+        if (p < n && sub == 0) src.load_lane(p, st, sc, 256, tn, cn, dead);
+        const uint32_t head = __shfl_sync(kFull, (uint32_t)tn | (uint32_t)cn << 8 | dead << 16, (int)lead);
+        tn = (int)(head & 0xFFu);
+        cn = (int)((head >> 8) & 0xFFu);
+        dead = head >> 16;
+        __syncwarp();
+        for (int i = 0; i < tn; i++) { const uint32_t op = st[i * 256] & 0xFFu; swx |= c_sweep[op]; written |= c_wr[op]; }
+        for (int i = 0; i < cn; i++) { const uint32_t op = sc[i * 256] & 0xFFu; swx |= c_sweep[op]; written |= c_wr[op]; }
+        const uint32_t live = written & ~(((dead & 0x0Fu) << L_C) | ((dead >> 6) << L_V));
+        uint32_t ut = live, uc = live;
+        for (int i = tn - 1; i >= 0; i--) ut = backward(ut, st[i * 256] & 0xFFu, s_dep);
+        for (int i = cn - 1; i >= 0; i--) uc = backward(uc, sc[i * 256] & 0xFFu, s_dep);
+        const uint32_t u = (ut | uc) & (swx | LB(L_A) | LB(L_C)), reg = u & ~LB(L_C);
+        const bool rep = a.sweep == M6502_SWEEP_REFERENCE && __popc(swx) >= 3;
+        const bool small = p < n && cone_bits(u, rep) <= 9;
+        const unsigned left = __ballot_sync(kFull, p < n && !small && sub == 0);
+        if (left) {
+            unsigned long long b = 0;
+            if (lane == 0) b = atomicAdd(&a.cnt->small_left, (unsigned long long)__popc(left));
+            b = __shfl_sync(kFull, b, 0) + __popc(left & ((1u << lane) - 1u));
+            if (((left >> lane) & 1u) && b < n_cap) order[b] = (uint32_t)p;
         }
-        const unsigned long long p = next++;
-        if (p >= n) break;
-        bool pass;
-        {
-            PairView pv;
-            pv.t = s_t[w]; pv.c = s_c[w];
-            src.load(p, s_t[w], s_c[w], pv.tn, pv.cn, pv.dead, lane);
-            const uint64_t tid = src.target_id(p);
-            __syncwarp();
-            uint32_t sw_t = 0, sw_c = 0;
-            for (int i = 0; i < pv.tn; i++) sw_t |= c_sweep[pv.t[i] & 0xFFu];
-            for (int i = 0; i < pv.cn; i++) sw_c |= c_sweep[pv.c[i] & 0xFFu];
-            const bool prep = a.sweep == M6502_SWEEP_REFERENCE && __popc(sw_t | sw_c) >= 3;
-            pass = probe_pair(pv, sw_t, sw_c, prep, tid, p, tc, lane);
-            __syncwarp();
+        auto mask = [&](uint32_t l) { return (reg & LB(l)) ? 0xFFFFFFFFu : 0u; };
+        const uint32_t ma = mask(L_A), mx = mask(L_X), my = mask(L_Y), ms = mask(L_S), mm = mask(L_M), m0 = mask(L_S0),
+                       m1 = mask(L_S1);
+        const uint32_t bs = (swx & LB(L_S)) ? 0u : 0xFDu * kB1;   // S at its first value
+        const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;
+        const bool rreg = rep && !(reg & LB(L_A));
+        const uint32_t words = reg == 0 ? 1u : rreg ? 8u : 64u;   // packed words of the register's values
+        const uint32_t total = words << ((u & LB(L_C)) ? 1 : 0);
+        bool open = small, differ = false;
+        for (uint32_t q = 2 * sub; __any_sync(kFull, open); q += 2u << g) {
+            uint32_t d = 0;
+            if (open && q < total) {
+                St t[2], c[2];
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const uint32_t j = min(q + k, total - 1), i0 = (j & (words - 1)) * 4;
+                    uint32_t v = i0 * kB1 + 0x03020100u;
+                    if (rreg) v = c_rep[i0] | (c_rep[i0 + 1] << 8) | (c_rep[i0 + 2] << 16) | (c_rep[i0 + 3] << 24);
+                    t[k] = c[k] = St{v & ma, v & mx, v & my, j >= words ? kB1 : 0u, (v & ms) | bs, v & mm, v & m0, v & m1};
+                }
+                for (int i = 0; i < tn; i++) exec_x4n(t, st[i * 256]);
+                for (int i = 0; i < cn; i++) exec_x4n(c, sc[i * 256]);
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    d |= (t[k].a ^ c[k].a) | (t[k].x ^ c[k].x) | (t[k].y ^ c[k].y) | ((t[k].p ^ c[k].p) & pm) |
+                         (t[k].s ^ c[k].s) | (t[k].m ^ c[k].m) | (t[k].s0 ^ c[k].s0) | (t[k].s1 ^ c[k].s1);
+                nstates += 4 * min(2u, total - q);
+            }
+            const unsigned bad = __ballot_sync(kFull, d != 0) & group;
+            differ = differ || bad;
+            open = open && !differ && q - 2 * sub + (2u << g) < total;   // the same for all lanes of the pair
         }
-        if (!pass) {
-            if (lane == 0) { a.fail[p] = 1u; probe_rej += src.weight(p); }
-        } else {
-            if (lane == 0) s_pass[w][npass] = (uint32_t)p;
-            __syncwarp();
-            if (++npass == 32) flush();
-        }
+        if (small && sub == 0) a.fail[p] = differ ? 1u : 0u;
+        __syncwarp();
     }
-    if (npass) flush();
-    if (lane == 0 && probe_rej) atomicAdd(&a.cnt->probe_rejects, probe_rej);
+    for (int o = 16; o; o >>= 1) nstates += __shfl_down_sync(kFull, nstates, o);
+    if (lane == 0 && nstates) atomicAdd(&a.cnt->states, nstates);
 }
 
 template <class Src>
 __global__ void __launch_bounds__(256) k_exh_items(Src src, ExhArgs a) {
     __shared__ uint16_t s_t[kWarpsPerBlock][kMaxSeq], s_c[kWarpsPerBlock][kMaxSeq];
-    __shared__ uint16_t s_dep[NUM_OPS][NUM_LOCS];
-    for (int i = threadIdx.x; i < NUM_OPS * NUM_LOCS; i += blockDim.x) (&s_dep[0][0])[i] = (&c_dep[0][0])[i];
-    __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t n = min((uint64_t)a.cnt->items, a.item_cap);
     unsigned long long nstates = 0;
@@ -1652,9 +1879,11 @@ __global__ void __launch_bounds__(256) k_exh_items(Src src, ExhArgs a) {
         pv.t = s_t[w]; pv.c = s_c[w];
         src.load(it.pair, s_t[w], s_c[w], pv.tn, pv.cn, pv.dead, lane);
         __syncwarp();
-        Flow fl = dataflow_s(pv, lane, s_dep);
-        Fields f = make_fields(it.cone, fl.swept, it.rep != 0);
-        bool ok = sweep_states<4>(pv, f, it.outmask, it.start, it.start + it.count, flag, &nstates, lane);
+        uint32_t swept = LB(L_A) | LB(L_C);
+        for (int i = 0; i < pv.tn; i++) swept |= c_sweep[pv.t[i] & 0xFFu];
+        for (int i = 0; i < pv.cn; i++) swept |= c_sweep[pv.c[i] & 0xFFu];
+        const bool ok = sweep_cone(pv, it.cone, swept, it.rep != 0, it.outmask, it.start, it.start + it.count, flag,
+                                   &nstates, lane);
         if (!ok && lane == 0) *flag = 1u;
         __syncwarp();
     }
@@ -2101,7 +2330,7 @@ struct m6502_ctx {
     std::string err;
     std::mutex mu;
     int sms = 148;
-    int exh_blocks = 0, exh_item_blocks = 0, qc_blocks = 0, fp_blocks = 0, probe_blocks = 0;
+    int exh_blocks = 0, exh_item_blocks = 0, qc_blocks = 0, fp_blocks = 0, small_blocks = 0;
     int exh_occ[5] = {};       // resident blocks per SM of k_exhaustive<SurvSource, MINB>, by MINB
     m6502_tune tune{4, 4, 11, 1, {0, 0, 0, 0}};   // scheduling knobs (m6502_tune_set / m6502_autotune)
     uint64_t pass_targets = 1ull << 21;
@@ -2115,9 +2344,11 @@ struct m6502_ctx {
     std::vector<uint16_t> h_tab;      // instructions, CUDA order (host copy)
     DevBuf go_keys, go_keys2, go_ord, go_round, go_sort_tmp;   // Go-order verification rounds
     DevBuf jitems;                                             // chunks of long length-2 equal ranges
-    DevBuf order;                                              // k_probe_pairs: the pairs it passed on
+    DevBuf order;                                              // k_small: the pairs it left
+    DevBuf match;                                              // k_qc_join: the targets that match
     DevBuf join_tab[2][256];                      // JoinTable by semantics and dead-flags mask
     DevBuf join_groups[256];                      // CandGroups of the CUDA-semantics tables
+    DevBuf join_lines[256];                       // line hashes of the candidates, [64 register sets][2863]
     struct Cand2Table {            // sorted (key, index) of all length-2 sequences for one mask
         uint32_t dead = 0xFFFFFFFFu;
         DevBuf keys, idx;
@@ -2169,19 +2400,18 @@ int ensure(m6502_ctx* ctx, DevBuf& b, size_t bytes) {
         if (rc_ != M6502_OK) return rc_; \
     } while (0)
 
-// The exhaustive kernel over survivors with the context's knobs: ticket
-// batch and work-item size in the arguments, the register-cap variant and
-// its persistent grid (SMs x resident blocks).
-int launch_exh(m6502_ctx* ctx, const SurvSource& src, const unsigned long long* n_ptr, uint64_t cap, ExhArgs ea,
-               bool split = false) {
+// ExhaustiveCheck over survivors, up to the work items, with the context's
+// knobs: ticket batch and work-item size in the arguments, the register-cap
+// variant and its persistent grid (SMs x resident blocks).  Brute force
+// sweeps every pair's whole product in k_exhaustive.
+int launch_exh(m6502_ctx* ctx, const SurvSource& src, const unsigned long long* n_ptr, uint64_t cap, ExhArgs ea) {
     ea.ticket_batch = ctx->tune.ticket_batch;
     ea.chunk_log2 = ctx->tune.chunk_log2;
-    if (split) {   // the probe first, in its own kernel; k_exhaustive then sweeps the pairs it passed on
-        k_probe_pairs<SurvSource><<<ctx->probe_blocks, 256, 0, ctx->stream>>>(src, n_ptr, cap, ea,
-                                                                               (uint32_t*)ctx->order.p);
-        CKL("k_probe_pairs");
+    if (!ea.brute) {
+        k_small<SurvSource><<<ctx->small_blocks, 256, 0, ctx->stream>>>(src, n_ptr, cap, ea, (uint32_t*)ctx->order.p);
+        CKL("k_small");
         ea.order = (const uint32_t*)ctx->order.p;
-        n_ptr = &ea.cnt->probe_pass;
+        n_ptr = &ea.cnt->small_left;
     }
     const int minb = (int)ctx->tune.exh_minb;
     const unsigned grid = (unsigned)(ctx->sms * ctx->exh_occ[minb >= 2 && minb <= 4 ? minb : 4]);
@@ -2195,6 +2425,25 @@ int launch_exh(m6502_ctx* ctx, const SurvSource& src, const unsigned long long* 
     return M6502_OK;
 }
 
+// ExhaustiveCheck of n pairs from another source, work items included; n is
+// the value at n_ptr, at most cap.
+template <class Src>
+int launch_verify(m6502_ctx* ctx, const Src& src, const unsigned long long* n_ptr, uint64_t cap, ExhArgs ea) {
+    if (!ea.brute) {
+        const uint64_t need = (cap + 255) / 256;
+        k_small<Src><<<(unsigned)std::min<uint64_t>(ctx->sms * 4, std::max<uint64_t>(need, 1)), 256, 0, ctx->stream>>>(
+            src, n_ptr, cap, ea, (uint32_t*)ctx->order.p);
+        CKL("k_small");
+        ea.order = (const uint32_t*)ctx->order.p;
+        n_ptr = &ea.cnt->small_left;
+    }
+    k_exhaustive<Src><<<ctx->exh_blocks, 256, 0, ctx->stream>>>(src, n_ptr, cap, ea);
+    CKL("k_exhaustive");
+    k_exh_items<Src><<<ctx->exh_item_blocks, 256, 0, ctx->stream>>>(src, ea);
+    CKL("k_exh_items");
+    return M6502_OK;
+}
+
 const uint16_t* join_mult(const m6502_ctx* ctx, uint32_t dead) {
     const CandGroups* g = (const CandGroups*)ctx->join_groups[dead].p;
     return g ? g->mult : nullptr;
@@ -2202,21 +2451,35 @@ const uint16_t* join_mult(const m6502_ctx* ctx, uint32_t dead) {
 
 // The length-1 QuickCheck join.  A warp takes as many targets as fill the
 // resident warps, up to a lane each: small searches spread over all SMs.
-int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt, uint32_t dead, uint32_t stages,
-                 uint64_t scap, Counters* cnt, bool go) {
+int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt, const m6502_search_cfg& cfg,
+                 uint64_t scap, Counters* cnt) {
+    const bool go = cfg.semantics == M6502_SEM_GO;
+    const uint32_t stages = cfg.stages ? cfg.stages : M6502_CHECK_ALL, dead = cfg.dead_flags;
+    // the line filter is part of ExhaustiveCheck; brute force does without
+    const bool filter = !go && (stages & M6502_CHECK_EXH) && cfg.exh_mode != M6502_EXH_BRUTE;
     const uint64_t warps = (uint64_t)ctx->sms * 4 * kWarpsPerBlock;   // 4 resident blocks per SM
     const uint32_t chunk = (uint32_t)std::min<uint64_t>(32, (nt + warps - 1) / warps);
     const uint64_t blocks = (nt + (uint64_t)chunk * kWarpsPerBlock - 1) / ((uint64_t)chunk * kWarpsPerBlock);
     const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->sms * 4, blocks));
     const JoinTable* tab = (const JoinTable*)ctx->join_tab[go][dead].p;
     const uint4* cfp4 = (const uint4*)ctx->cfp4.p;
+    Surv* match = (Surv*)ctx->match.p;
     if (go)
-        k_qc_join<true><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages,
-                                                       (Surv*)ctx->surv.p, scap, cnt, nullptr);
+        k_qc_join<true><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages, match, cnt);
     else
-        k_qc_join<false><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages,
-                                                        (Surv*)ctx->surv.p, scap, cnt, join_mult(ctx, dead));
+        k_qc_join<false><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages, match, cnt);
     CKL("k_qc_join");
+    const uint16_t* mult = go ? nullptr : join_mult(ctx, dead);
+    const uint32_t* lines = (const uint32_t*)ctx->join_lines[dead].p;
+    const uint32_t egrid = (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 4, (nt + 255) / 256);
+    auto expand = [&](auto kernel) {
+        kernel<<<egrid, 256, 0, ctx->stream>>>(match, d_t, tlen, cfp4, tab, dead, cfg.sweep, mult, lines, (Surv*)ctx->surv.p,
+                                               scap, cnt);
+    };
+    if (go) expand(k_expand<true, false>);
+    else if (filter) expand(k_expand<false, true>);
+    else expand(k_expand<false, false>);
+    CKL("k_expand");
     return M6502_OK;
 }
 
@@ -2261,6 +2524,21 @@ int init_ctx(m6502_ctx* ctx) {
         for (int f = 0; f < 8; f++) vec4[g][f] = pack4(vec + 4 * g, f);
     CK(cudaMemcpyToSymbol(c_vec, vec, sizeof vec));
     CK(cudaMemcpyToSymbol(c_vec4, vec4, sizeof vec4));
+    // Line states: A = i, the other registers a permutation of it each, the
+    // carry the parity of i.
+    uint32_t line[64][8];
+    for (int j = 0; j < 64; j++) {
+        uint64_t st[4];
+        for (int k = 0; k < 4; k++) {
+            const uint32_t i = (uint32_t)(4 * j + k);
+            const uint32_t f[8] = {i, 5 * i + 59, 13 * i + 113, (uint32_t)__builtin_parity(i),
+                                   29 * i + 7, 77 * i + 196, 141 * i + 45, 203 * i + 150};
+            st[k] = 0;
+            for (int b = 0; b < 8; b++) st[k] |= (uint64_t)(f[b] & 0xFFu) << (8 * b);
+        }
+        for (int f = 0; f < 8; f++) line[j][f] = pack4(st, f);
+    }
+    CK(cudaMemcpyToSymbol(c_line, line, sizeof line));
     CK(cudaMemcpyToSymbol(c_dep, dep, sizeof dep));
     CK(cudaMemcpyToSymbol(c_wr, wr, sizeof wr));
     CK(cudaMemcpyToSymbol(c_sweep, sw, sizeof sw));
@@ -2283,8 +2561,8 @@ int init_ctx(m6502_ctx* ctx) {
     ctx->exh_occ[3] = std::max(occ, 1);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_exhaustive<SurvSource, 2>, 256, 0));
     ctx->exh_occ[2] = std::max(occ, 1);
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_probe_pairs<SurvSource>, 256, 0));
-    ctx->probe_blocks = ctx->sms * std::max(occ, 1);
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_small<SurvSource>, 256, 0));
+    ctx->small_blocks = ctx->sms * std::max(occ, 1);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_exh_items<SurvSource>, 256, 0));
     ctx->exh_item_blocks = ctx->sms * std::max(occ, 1);
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_qc1<false>, 256, 0));
@@ -2409,6 +2687,9 @@ int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
                 for (uint32_t b = t.cand[i] >> 12; b <= 2; b++) t.weight[u][b - 1] += gr.mult[t.cand[i] & 0xFFFu];
         TRY(ensure(ctx, ctx->join_groups[dead], sizeof gr));
         CK(cudaMemcpy(ctx->join_groups[dead].p, &gr, sizeof gr, cudaMemcpyHostToDevice));
+        TRY(ensure(ctx, ctx->join_lines[dead], 64 * kNumInsns * sizeof(uint32_t)));
+        k_line_hash<<<(64 * kNumInsns + 255) / 256, 256, 0, ctx->stream>>>(dead, (uint32_t*)ctx->join_lines[dead].p);
+        CKL("k_line_hash");
     }
     TRY(ensure(ctx, ctx->join_tab[go][dead], sizeof t));
     CK(cudaMemcpy(ctx->join_tab[go][dead].p, &t, sizeof t, cudaMemcpyHostToDevice));
@@ -2488,6 +2769,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         TRY(ensure(ctx, ctx->surv, scap * sizeof(Surv)));
         TRY(ensure(ctx, ctx->fail, scap * sizeof(uint32_t)));
         TRY(ensure(ctx, ctx->order, scap * sizeof(uint32_t)));
+        if (!scan) TRY(ensure(ctx, ctx->match, nt * sizeof(Surv)));
         TRY(ensure(ctx, ctx->items, icap * sizeof(Item)));
         TRY(ensure(ctx, ctx->rules, rcap * sizeof(m6502_rule)));
         if (go) TRY(ensure(ctx, ctx->best, 2 * nt * sizeof(uint32_t)));
@@ -2524,7 +2806,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         CK(rec(ctx->sev[1]));
         uint32_t qgrid = (uint32_t)std::min<uint64_t>(ctx->qc_blocks, (nt + kQcTile - 1) / kQcTile);
         if (!scan) {
-            TRY(launch_join1(ctx, d_targets, tlen, nt, dead, stages, scap, cnt, go));
+            TRY(launch_join1(ctx, d_targets, tlen, nt, cfg, scap, cnt));
         } else if (go)
             k_qc1<true><<<qgrid, 256, 0, ctx->stream>>>((uint64_t*)ctx->tfp.p, (uint8_t*)ctx->tmeta.p,
                                                         (uint32_t)nt, (uint64_t*)ctx->cfp1.p,
@@ -2561,7 +2843,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
                                                             (uint32_t*)ctx->go_ord.p, cnt);
             CKL("k_go_ord");
             SurvSource rs{(const Surv*)ctx->go_round.p, d_targets, tlen, dead, 1, nullptr};
-            for (uint64_t lo = 0, blk = 64; lo < bound; lo += blk, blk = std::min<uint64_t>(blk * 2, 1ull << 22)) {
+            for (uint64_t lo = 0, blk = 64; lo < bound; lo += blk, blk = std::min<uint64_t>(blk * 4, 1ull << 22)) {
                 const uint64_t hi = std::min<uint64_t>(lo + blk, 0xFFFFFFFFull);
                 CK(cudaMemsetAsync(&cnt->round_n, 0, sizeof(unsigned long long), ctx->stream));
                 k_go_round<<<ctx->sms * 8, 256, 0, ctx->stream>>>(
@@ -2569,7 +2851,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
                     (uint32_t)hi, (const uint32_t*)ctx->best.p, (uint32_t)nt, (Surv*)ctx->go_round.p, cnt);
                 CKL("k_go_round");
                 // exhaustive tickets, work items and item tickets restart each round
-                CK(cudaMemsetAsync(&cnt->exh_ticket, 0, 3 * sizeof(unsigned long long), ctx->stream));
+                CK(cudaMemsetAsync(&cnt->exh_ticket, 0, kVerifyCounters * sizeof(unsigned long long), ctx->stream));
                 ExhArgs ra{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, cfg.sweep,
                            cfg.exh_mode == M6502_EXH_BRUTE};
                 TRY(launch_exh(ctx, rs, &cnt->round_n, scap, ra));
@@ -2585,7 +2867,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
             return M6502_OK;
         };
         if (go) CK(cudaMemsetAsync(ctx->best.p, 0xFF, 2 * nt * sizeof(uint32_t), ctx->stream));
-        if (exh && !rounds) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea, true));
+        if (exh && !rounds) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea));
         if (rounds) TRY(go_rounds(kNumInsns));   // a target has at most 2,863 length-1 candidates
         CK(rec(ctx->sev[3]));
         if (exh && !rounds) TRY(launch_items(ctx, src, ea));
@@ -2617,9 +2899,8 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
             // phase are checked once, after the pass.
             k_mark_phase<<<1, 1, 0, ctx->stream>>>(cnt);
             CKL("k_mark_phase");
-            // survivor, exhaustive-ticket, work-item and probe counters restart for this phase
-            CK(cudaMemsetAsync(&cnt->surv, 0, 4 * sizeof(unsigned long long), ctx->stream));
-            CK(cudaMemsetAsync(&cnt->probe_ticket, 0, 2 * sizeof(unsigned long long), ctx->stream));
+            // survivor and verification counters restart for this phase
+            CK(cudaMemsetAsync(&cnt->surv, 0, (1 + kVerifyCounters) * sizeof(unsigned long long), ctx->stream));
             CK(rec(ctx->sev2[0]));
             const uint32_t jgrid2 =
                 (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 8, (nt + kWarpsPerBlock - 1) / kWarpsPerBlock);
@@ -2638,7 +2919,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
             }
             CKL("k_qc_join2");
             CK(rec(ctx->sev2[1]));
-            if (exh && !rounds) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea, true));
+            if (exh && !rounds) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea));
             if (rounds) TRY(go_rounds((uint64_t)kNumInsns * kNumInsns));
             CK(rec(ctx->sev2[2]));
             if (exh && !rounds) TRY(launch_items(ctx, src, ea));
@@ -2664,7 +2945,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
                 (uint64_t)(uintptr_t)d_targets, nt, tlen, (uint64_t)(uintptr_t)d_ids, cfg.semantics, cfg.sweep,
                 cfg.exh_mode, stages, cfg.flags, dead, cfg.max_cand_len, scap, icap, rcap, jcap,
                 (uint64_t)(uintptr_t)ctx->surv.p, (uint64_t)(uintptr_t)ctx->fail.p, (uint64_t)(uintptr_t)ctx->items.p,
-                (uint64_t)(uintptr_t)ctx->order.p,
+                (uint64_t)(uintptr_t)ctx->order.p, (uint64_t)(uintptr_t)ctx->match.p,
                 (uint64_t)(uintptr_t)ctx->rules.p, (uint64_t)(uintptr_t)ctx->cnt.p, (uint64_t)(uintptr_t)ctx->best.p,
                 (uint64_t)(uintptr_t)ctx->tfp.p, (uint64_t)(uintptr_t)ctx->tmeta.p,
                 (uint64_t)(uintptr_t)ctx->go_keys.p, (uint64_t)(uintptr_t)ctx->go_keys2.p,
@@ -2714,12 +2995,15 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         bool redo = false;
         CK(cudaMemcpyAsync(&hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        const uint64_t surv_need = std::max<uint64_t>(hc.surv, hc.surv_need);
-        const uint64_t items_need = std::max<uint64_t>(hc.items, hc.items_need);
+        // A first phase that overflowed leaves targets open that it would have
+        // settled: what the second phase then asked for says nothing.
+        const bool first_over = phase2 && hc.surv1 > scap;
+        const uint64_t surv_need = first_over ? hc.surv1 : std::max<uint64_t>(hc.surv, hc.surv_need);
+        const uint64_t items_need = first_over ? hc.items1 : std::max<uint64_t>(hc.items, hc.items_need);
         if (surv_need > scap) { scap = surv_need + surv_need / 4 + 1024; redo = true; }
         if (items_need > icap) { icap = items_need + items_need / 4 + 1024; redo = true; }
         if (hc.rules > rlim && !count_only) { rcap = hc.rules + hc.rules / 4 + 1024; redo = true; }
-        if (hc.join_items > jcap) { jcap = hc.join_items + hc.join_items / 4 + 1024; redo = true; }
+        if (!first_over && hc.join_items > jcap) { jcap = hc.join_items + hc.join_items / 4 + 1024; redo = true; }
         if (redo) continue;
         size_t old = ctx->staging.size();
         if (!count_only) ctx->staging.resize(old + hc.rules);
@@ -2800,6 +3084,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
         TRY(ensure(ctx, ctx->surv, scap * sizeof(Surv)));
         TRY(ensure(ctx, ctx->fail, scap * sizeof(uint32_t)));
         TRY(ensure(ctx, ctx->order, scap * sizeof(uint32_t)));
+        if (!scan) TRY(ensure(ctx, ctx->match, pmax * sizeof(Surv)));
         TRY(ensure(ctx, ctx->items, icap * sizeof(Item)));
         TRY(ensure(ctx, ctx->rules, rcap * sizeof(m6502_rule)));
         // All passes, queued with no host round trip, recorded once as a CUDA
@@ -2833,13 +3118,13 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                                                                  (Surv*)ctx->surv.p, scap, cnt);
                     CKL("k_qc1");
                 } else {
-                    TRY(launch_join1(ctx, d_t, tlen, nt, dead, stages, scap, cnt, false));
+                    TRY(launch_join1(ctx, d_t, tlen, nt, cfg, scap, cnt));
                 }
                 CK(rec(ev[2]));
                 SurvSource src{(const Surv*)ctx->surv.p, d_t, tlen, dead, 0, groups ? groups->mult : nullptr};
                 ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, cfg.sweep,
                            cfg.exh_mode == M6502_EXH_BRUTE};
-                if (exh) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea, true));
+                if (exh) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea));
                 CK(rec(ev[3]));
                 if (exh) TRY(launch_items(ctx, src, ea));
                 CK(rec(ev[4]));
@@ -2859,7 +3144,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
             const std::vector<uint64_t> key = {
                 (uint64_t)(uintptr_t)targets, n, tlen, cfg.semantics, cfg.sweep, cfg.exh_mode, stages,
                 cfg.flags, dead, scap, icap, rcap, P, (uint64_t)(uintptr_t)ctx->surv.p,
-                (uint64_t)(uintptr_t)ctx->fail.p, (uint64_t)(uintptr_t)ctx->items.p, (uint64_t)(uintptr_t)ctx->order.p,
+                (uint64_t)(uintptr_t)ctx->fail.p, (uint64_t)(uintptr_t)ctx->items.p, (uint64_t)(uintptr_t)ctx->order.p, (uint64_t)(uintptr_t)ctx->match.p,
                 (uint64_t)(uintptr_t)ctx->rules.p, (uint64_t)(uintptr_t)ctx->cnt_slots.p,
                 (uint64_t)(uintptr_t)ctx->tfp.p, (uint64_t)(uintptr_t)ctx->tmeta.p,
                 (uint64_t)(uintptr_t)ctx->join_tab[0][dead].p, ctx->tune.exh_minb, ctx->tune.ticket_batch,
@@ -3140,6 +3425,7 @@ void m6502_destroy(m6502_ctx* ctx) {
         for (int g = 0; g < 2; g++)
             if (ctx->join_tab[g][i].p) cudaFree(ctx->join_tab[g][i].p);
         if (ctx->join_groups[i].p) cudaFree(ctx->join_groups[i].p);
+        if (ctx->join_lines[i].p) cudaFree(ctx->join_lines[i].p);
     }
     DevBuf* bufs[] = {&ctx->cfp4, &ctx->cfp1, &ctx->cmeta1, &ctx->targets, &ctx->ids, &ctx->tfp, &ctx->tmeta,
                       &ctx->surv, &ctx->fail, &ctx->items, &ctx->rules, &ctx->cnt, &ctx->best,
@@ -3151,7 +3437,7 @@ void m6502_destroy(m6502_ctx* ctx) {
                       &ctx->st_vlist, &ctx->st_vpos, &ctx->st_sort_tmp, &ctx->c2_keys_in, &ctx->c2_idx_in,
                       &ctx->c2_sort_tmp, &ctx->go_keys, &ctx->go_keys2, &ctx->go_ord, &ctx->go_round,
                       &ctx->go_sort_tmp, &ctx->jitems, &ctx->cnt_slots, &ctx->st_vphase, &ctx->st_pphase,
-                      &ctx->tall, &ctx->opflag, &ctx->order};
+                      &ctx->tall, &ctx->opflag, &ctx->order, &ctx->match};
     for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
     for (cudaEvent_t e : ctx->sev) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->sev2) if (e) cudaEventDestroy(e);
@@ -3198,6 +3484,7 @@ int m6502_check_pairs(m6502_ctx* ctx, uint64_t n, const uint16_t* t_insns, const
     TRY(ensure(ctx, ctx->pout, n));
     TRY(ensure(ctx, ctx->pfd, n));
     TRY(ensure(ctx, ctx->fail, n * 4));
+    TRY(ensure(ctx, ctx->order, n * 4));
     CK(cudaMemcpyAsync(ctx->pins.p, t_insns, tin * 2, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->cins.p, c_insns, cin * 2, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->poffs.p, t_offs, (n + 1) * 4, cudaMemcpyHostToDevice, ctx->stream));
@@ -3217,10 +3504,7 @@ int m6502_check_pairs(m6502_ctx* ctx, uint64_t n, const uint16_t* t_insns, const
             unsigned long long hn = n;
             CK(cudaMemcpyAsync(&cnt->surv, &hn, sizeof hn, cudaMemcpyHostToDevice, ctx->stream));
             ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, sweep, exh_mode == M6502_EXH_BRUTE};
-            k_exhaustive<CsrSource><<<ctx->exh_blocks, 256, 0, ctx->stream>>>(src, &cnt->surv, n, ea);
-            CKL("k_exhaustive");
-            k_exh_items<CsrSource><<<ctx->exh_item_blocks, 256, 0, ctx->stream>>>(src, ea);
-            CKL("k_exh_items");
+            TRY(launch_verify(ctx, src, &cnt->surv, n, ea));
             Counters hc;
             CK(cudaMemcpyAsync(&hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));

@@ -168,19 +168,6 @@ M6502_HD void exec(St& s, uint32_t insn) {
     }
 }
 
-// The same instruction on two states with one dispatch (the sweeps run two
-// states per lane so the opcode switch is paid once per pair of states).
-M6502_HD void exec2(St& s0, St& s1, uint32_t insn) {
-    const uint32_t imm = insn >> 8;
-    (void)imm;
-    switch (insn & 0xFFu) {
-#define M6502_CASE2(op, ...) case op: { { St& s = s0; __VA_ARGS__; } { St& s = s1; __VA_ARGS__; } } break;
-        M6502_OPCODES(M6502_CASE2)
-#undef M6502_CASE2
-    default: break;
-    }
-}
-
 // ---- Four states per register (SWAR) ----
 //
 // The same St holds four machine states: byte k of every field is state k.

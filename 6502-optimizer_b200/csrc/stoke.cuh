@@ -400,6 +400,7 @@ __global__ void k_stoke_vectors(StokeEntry* __restrict__ entries, uint64_t ecap,
 
 // Pairs (target, entry) of the entries that passed all vectors.
 struct StokeSource {
+    static constexpr int kMaxT = kMaxSeq, kMaxC = kMaxSeq;
     const StokeEntry* entries;
     const uint32_t* vidx;
     StokeTargets tg;
@@ -412,6 +413,15 @@ struct StokeSource {
         cn = e.len;
         if (lane < tn) st[lane] = tg.ins[t0 + lane];
         if (lane < cn) sc[lane] = e.ins[lane];
+        dead = dead_;
+    }
+    __device__ void load_lane(uint64_t p, uint16_t* st, uint16_t* sc, int ld, int& tn, int& cn, uint32_t& dead) const {
+        const StokeEntry& e = entries[vidx[p]];
+        const uint32_t t0 = tg.off[e.target];
+        tn = (int)(tg.off[e.target + 1] - t0);
+        cn = e.len;
+        for (int i = 0; i < tn; i++) st[i * ld] = tg.ins[t0 + i];
+        for (int i = 0; i < cn; i++) sc[i * ld] = e.ins[i];
         dead = dead_;
     }
     __device__ uint64_t target_id(uint64_t) const { return kNoTarget; }   // candidates may be empty
@@ -580,6 +590,7 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
     TRY(ensure(ctx, ctx->st_entries, ecap * sizeof(StokeEntry)));
     TRY(ensure(ctx, ctx->st_vidx, ecap * 4));
     TRY(ensure(ctx, ctx->fail, ecap * 4));
+    TRY(ensure(ctx, ctx->order, ecap * 4));
     TRY(ensure(ctx, ctx->st_proven, (size_t)n_targets * 4));
     TRY(ensure(ctx, ctx->st_cnt, sizeof(StokeCounters)));
     TRY(ensure(ctx, ctx->st_pidx, ecap * 4));
@@ -730,10 +741,7 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
                 CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), ctx->stream));
                 ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, cfg->sweep, 0,
                            phase == 0 ? kStokeDeferBits : 0u};
-                k_exhaustive<StokeSource><<<ctx->exh_blocks, 256, 0, ctx->stream>>>(src, &sc->round_n, ecap, ea);
-                CKL("k_exhaustive(stoke)");
-                k_exh_items<StokeSource><<<ctx->exh_item_blocks, 256, 0, ctx->stream>>>(src, ea);
-                CKL("k_exh_items(stoke)");
+                TRY(launch_verify(ctx, src, &sc->round_n, ecap, ea));
                 unsigned long long items = 0;
                 CK(cudaMemcpyAsync(&items, &cnt->items, sizeof items, cudaMemcpyDeviceToHost, ctx->stream));
                 CK(cudaStreamSynchronize(ctx->stream));
