@@ -392,6 +392,7 @@ tcg::Epilogue epi_of(int mode, float* of, __nv_bfloat16* ob, const float* bias, 
     tcg::Epilogue e;
     e.mode = mode; e.out_f32 = of; e.out_bf16 = ob; e.bias = bias; e.act = act; e.ldc = ldc;
     e.split_stride = 0;
+    e.wide = false;   // launch_gemm sets it
     return e;
 }
 
@@ -714,6 +715,7 @@ int m6502_gemm_bf16_timed(m6502_ctx* ctx, int M, int N, int K, const void* A, co
     tcg::Epilogue e;
     e.mode = tcg::EPI_F32; e.out_f32 = C; e.out_bf16 = nullptr; e.bias = nullptr; e.act = nullptr; e.ldc = N;
     e.split_stride = 0;
+    e.wide = false;   // launch_gemm sets it
     if (ms_per_launch && cudaEventRecord(ev[dev][0], st) != cudaSuccess) return M6502_E_CUDA;
     for (int r = 0; r < reps; r++)
         if (!tcg::launch_gemm((const __nv_bfloat16*)A, K, (const __nv_bfloat16*)B, K, M, N, K, e, d_err[dev], st,
