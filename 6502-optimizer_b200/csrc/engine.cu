@@ -218,8 +218,8 @@ constexpr size_t kJoinShared = offsetof(JoinTable, sub);
 static_assert(kJoinShared % 16 == 0 && kNumInsns < (1 << 12), "copied in 16-byte words; 12-bit indices");
 
 // Warp-collective key of the outputs held by lanes 0..7 (lane v: vector v).
-__device__ __forceinline__ uint64_t warp_key(uint64_t tv, uint64_t mask, int lane) {
-    uint64_t h = lane < 8 ? key_term(tv & mask, lane) : 0ull;
+__device__ __forceinline__ uint64_t warp_key(uint64_t tv, uint64_t mask, uint64_t salt, int lane) {
+    uint64_t h = lane < 8 ? key_term((tv & mask) + salt, lane) : 0ull;
     h ^= __shfl_xor_sync(kFull, h, 1);
     h ^= __shfl_xor_sync(kFull, h, 2);
     h ^= __shfl_xor_sync(kFull, h, 4);
@@ -245,8 +245,6 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const uint64_t* __restrict_
     return lo + (uint32_t)__popc(__ballot_sync(kFull, i < hi && keys[i] < key));
 }
 
-constexpr int kVerifyCounters = 5;   // exh_ticket .. small_left of Counters
-
 // Survivor record: target (index within the pass) and candidate code:
 // bits 0..22 candidate index, bit 23 length-2 candidate, bit 24 Go masked
 // pass, bits 25..30 FlagDiff (P bits 0-3, 6-7 compressed to 6 bits).
@@ -259,20 +257,28 @@ constexpr uint32_t kSurvLen2 = 1u << 23, kSurvMasked = 1u << 24;
 constexpr uint64_t kNoTarget = ~0ull;
 __host__ __device__ __forceinline__ uint32_t fd_pack(uint32_t fd) { return (fd & 0x0Fu) | ((fd >> 2) & 0x30u); }
 
+// Counters of one verification (k_small, k_exhaustive, k_exh_items over one
+// list of pairs); zero at its start.
+constexpr uint32_t kGoBlock = 64;    // survivors of a (target, pass) in the first Go-order round
+struct VerifyCounters {
+    unsigned long long n;            // pairs listed (Go-order rounds)
+    unsigned long long exh_ticket, items, item_ticket, small_ticket, small_left;
+};
+constexpr int kMaxRounds = 8;        // Go-order rounds per phase: 64 x 8^r ordinals each, 19 M before the last
+
 struct Counters {
     unsigned long long qc, mid;
-    // reset together for every verification (surv: for every phase)
-    unsigned long long surv, exh_ticket, items, item_ticket, small_ticket, small_left;
-    unsigned long long rules, exh_pass, states, algo, probe_rejects;
-    unsigned long long round_n, max_ord;   // Go-order verification rounds
+    // restart with the length-2 phase
+    unsigned long long surv, max_ord;      // max_ord: largest ordinal among the survivors (Go semantics)
     unsigned long long join_items;         // chunks of long length-2 equal ranges
+    unsigned long long rules, exh_pass, states, algo, probe_rejects;
     unsigned long long undecided;          // pairs left undecided (a cone beyond the sweep cap)
-    unsigned long long round_checked, round_items;   // Go-order rounds: pairs and work items, summed
-    unsigned long long surv1, items1;      // phase-1 survivors and work items (length-2 phase runs after)
-    unsigned long long surv_need, items_need;   // largest survivor / work-item counts seen, for the
-                                                // overflow check after the pass
+    unsigned long long round_rejects;      // pairs of a first round that the line filter settled
+    unsigned long long surv1;              // survivors of the length-1 phase
     unsigned long long join_ticket, matches;   // k_qc_join: claimed chunks of targets, matching targets
+    VerifyCounters v[2][kMaxRounds];       // by phase and round (CUDA semantics: round 0)
 };
+constexpr int kPhaseCounters = 3;   // surv, max_ord, join_items
 
 struct Item {   // one chunk of a large cone sweep
     uint32_t pair;
@@ -933,6 +939,7 @@ struct ExhArgs {
     Item* items;
     uint64_t item_cap;
     Counters* cnt;
+    VerifyCounters* v;           // this verification's counters
     uint32_t sweep;              // M6502_SWEEP_*
     uint32_t brute;
     uint32_t defer_bits;         // > 0: pairs with a cone above 2^defer_bits states get fail = 4 (deferred)
@@ -1315,6 +1322,38 @@ __global__ void __launch_bounds__(256) k_line_hash(uint32_t dead, uint32_t* __re
     }
 }
 
+// Go semantics: ordinals of survivors met in Go order, 32 at a time.
+struct GoCount {
+    uint32_t run0 = 0, run1 = 0;   // unmasked and masked survivors so far of the target that lane 31 was at
+    // This lane's ordinal within its target and pass.  `seg`: the first lane of
+    // its target in this step; `cont`: the target began in an earlier step.
+    __device__ __forceinline__ uint32_t step(bool take, bool masked, uint32_t seg, bool cont, int lane) {
+        const unsigned b0 = __ballot_sync(kFull, take && !masked), b1 = __ballot_sync(kFull, take && masked);
+        const unsigned span = (kFull << seg) & ((1u << lane) - 1u);
+        const uint32_t k0 = (cont ? run0 : 0u) + __popc(b0 & span), k1 = (cont ? run1 : 0u) + __popc(b1 & span);
+        run0 = __shfl_sync(kFull, k0, 31) + (b0 >> 31);
+        run1 = __shfl_sync(kFull, k1, 31) + (b1 >> 31);
+        return masked ? k1 : k0;
+    }
+};
+// Survivors past the first round: kept with their ordinals.
+__device__ __forceinline__ void go_late(bool late, Surv rec, uint32_t at, Surv* __restrict__ surv,
+                                        uint32_t* __restrict__ ord, uint64_t cap, Counters* __restrict__ cnt, int lane) {
+    const unsigned vote = __ballot_sync(kFull, late);
+    if (!vote) return;
+    const uint32_t top = __reduce_max_sync(kFull, late ? at : 0u);
+    unsigned long long b = 0;
+    if (lane == 0) {
+        b = atomicAdd(&cnt->surv, (unsigned long long)__popc(vote));
+        atomicMax(&cnt->max_ord, (unsigned long long)top);
+    }
+    b = __shfl_sync(kFull, b, 0) + __popc(vote & ((1u << lane) - 1u));
+    if (late && b < cap) {
+        surv[b] = rec;
+        ord[b] = at;
+    }
+}
+
 // A lane per match, or 2^g lanes while the matches alone do not fill the
 // chip; a static stride, since each costs about the same.  FILTER computes
 // the target's line hash; then the candidates of the warp's matches, numbered
@@ -1324,12 +1363,18 @@ __global__ void __launch_bounds__(256) k_line_hash(uint32_t dead, uint32_t* __re
 // enumeration (mask 0x00); the random probe it replaces (128 states, a warp
 // per pair) left 1.36 M in 2.42 ms.  Here, candidates and survivors included:
 // 0.48 ms.
+// Go semantics: the candidates of a match come in Go order, so a survivor's
+// ordinal within its (target, pass) is a running count.  The first `block` of
+// each go straight to the first round's list (there the line filter applies,
+// on the run's mask in both passes: what differs under the mask differs
+// without it), the others to `surv` with their ordinals.
 template <bool GO, bool FILTER>
 __global__ void __launch_bounds__(256, 4) k_expand(const Surv* __restrict__ match, const uint16_t* __restrict__ targets,
                                                  uint32_t tlen, const uint4* __restrict__ cfp4,
                                                  const JoinTable* __restrict__ table, uint32_t dead, uint32_t sweep,
                                                  const uint16_t* __restrict__ mult, const uint32_t* __restrict__ lines,
-                                                 Surv* __restrict__ surv, uint64_t cap, Counters* __restrict__ cnt) {
+                                                 Surv* __restrict__ surv, uint64_t cap, Counters* __restrict__ cnt,
+                                                 Surv* __restrict__ first, uint32_t* __restrict__ ord, uint32_t block) {
     __shared__ Surv s_stage[kWarpsPerBlock][kStage];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     Surv* stage = s_stage[w];
@@ -1364,7 +1409,8 @@ __global__ void __launch_bounds__(256, 4) k_expand(const Surv* __restrict__ matc
         if (FILTER) {
             hash = line_hash(regs, pm, run, sub, g);
             for (int o = 0; o < g; o++) hash += __shfl_xor_sync(kFull, hash, 1 << o);
-        } else if (GO) {
+        }
+        if (GO) {
             St v[2];
 #pragma unroll
             for (int g = 0; g < 2; g++)
@@ -1380,6 +1426,7 @@ __global__ void __launch_bounds__(256, 4) k_expand(const Surv* __restrict__ matc
             upto += lane >= o ? x : 0u;
         }
         const uint32_t total = __shfl_sync(kFull, upto, 31);
+        GoCount count;
         for (uint32_t h0 = 0; h0 < total; h0 += 32) {
             const uint32_t h = h0 + (uint32_t)lane;
             uint32_t own = 0;   // lanes whose candidates end at or before h
@@ -1415,6 +1462,22 @@ __global__ void __launch_bounds__(256, 4) k_expand(const Surv* __restrict__ matc
                 }
                 nqc += pass;
                 nmid += pass;
+                const bool masked = (code & kSurvMasked) != 0;
+                const uint32_t start = end - cnt_o;   // the match's first candidate
+                const uint32_t at = count.step(pass, masked, start <= h0 ? 0u : start - h0, start < h0, lane);
+                bool early = pass && at < block;
+                go_late(pass && !early, Surv{t, code}, at, surv, ord, cap, cnt, lane);
+                if (FILTER) {
+                    const uint32_t hash_o = __shfl_sync(kFull, hash, (int)own), regs_o = __shfl_sync(kFull, regs, (int)own);
+                    const bool filter_o = __shfl_sync(kFull, (int)filter, (int)own) != 0;
+                    if (early && filter_o && !(c_sweep[c_tab[c] & 0xFFu] & ~regs_o) &&
+                        lines[extra_bits(regs_o) * kNumInsns + c] != hash_o) {
+                        early = false;
+                        nrej++;
+                    }
+                }
+                stage_push(early, Surv{t, code}, stage, nstage, first, cap, &cnt->v[0][0].n, lane);
+                continue;
             } else {
                 const uint32_t weight = pass ? mult[c] : 0u;   // pairs this record stands for
                 nmid += weight;
@@ -1431,7 +1494,8 @@ __global__ void __launch_bounds__(256, 4) k_expand(const Surv* __restrict__ matc
             stage_push(pass, Surv{t, code}, stage, nstage, surv, cap, &cnt->surv, lane);
         }
     }
-    stage_flush(stage, nstage, surv, cap, &cnt->surv, lane);
+    if (GO) stage_flush(stage, nstage, first, cap, &cnt->v[0][0].n, lane);
+    else stage_flush(stage, nstage, surv, cap, &cnt->surv, lane);
     for (int o = 16; o; o >>= 1) {
         nqc += __shfl_down_sync(kFull, nqc, o);
         nmid += __shfl_down_sync(kFull, nmid, o);
@@ -1441,46 +1505,90 @@ __global__ void __launch_bounds__(256, 4) k_expand(const Surv* __restrict__ matc
         if (nqc) atomicAdd(&cnt->qc, nqc);
         if (nmid) atomicAdd(&cnt->mid, nmid);
         if (nrej) atomicAdd(&cnt->probe_rejects, nrej);
+        if (GO && nrej) atomicAdd(&cnt->round_rejects, nrej);
     }
 }
 
 // ---- Length-2 candidates: an exact join over all 2,863^2 sequences ----
 //
 // Per dead-flags mask, every length-2 sequence (CUDA index c0 * 2863 + c1)
-// gets the key of its 8 masked QuickCheck outputs; the (key, index) table is
+// gets the key of its 8 masked QuickCheck outputs; the (key, entry) table is
 // radix-sorted on the device once and cached.  A target's QuickCheck hits
 // among the 8.2 M candidates are then exactly the candidates with its key
 // that re-pass the 8 vectors -- found by one warp-wide search per target.
+// The sequences enter the (stable) sort in Go order, so those of one key stay
+// in Go order.  An entry holds the index, the pruner's answer and the sizes.
+constexpr uint32_t kEntryIndex = 0x7FFFFFu, kEntryPruned = 1u << 23;
+__device__ __forceinline__ uint32_t entry_bytes_cuda(uint32_t e) { return 2u + ((e >> 24) & 3u); }
+__device__ __forceinline__ uint32_t entry_bytes_go(uint32_t e) { return 2u + ((e >> 26) & 3u); }
 
-// Keys of all length-2 sequences, thread per sequence.  Consecutive threads
-// share the first instruction and mostly the second's opcode, so the
-// dispatch stays warp-uniform.
-__global__ void k_cand2_keys(uint32_t dead, uint64_t* __restrict__ keys, uint32_t* __restrict__ idx) {
+// Keys of all length-2 sequences in Go order, thread per sequence.
+__global__ void k_cand2_keys(uint32_t dead, uint64_t salt, uint64_t* __restrict__ keys, uint32_t* __restrict__ idx) {
     const uint64_t loose = cmp_mask(dead);
     const uint32_t n = (uint32_t)kNumInsns * (uint32_t)kNumInsns;
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        const uint16_t i0 = c_tab[c / kNumInsns], i1 = c_tab[c % kNumInsns];
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+        const uint32_t c0 = c_goidx[r / kNumInsns], c1 = c_goidx[r % kNumInsns];
+        const uint16_t seq[2] = {c_tab[c0], c_tab[c1]};
         uint64_t x = 0;
         for (int v = 0; v < 8; v++) {
             St s = unpack(c_vec[v]);
-            exec(s, i0);
-            exec(s, i1);
-            x ^= key_term(fp_of(s) & loose, v);
+            exec(s, seq[0]);
+            exec(s, seq[1]);
+            x ^= key_term((fp_of(s) & loose) + salt, v);
         }
-        const uint64_t key = key_final(x);
-        keys[c] = key;
-        idx[c] = c;
+        keys[r] = key_final(x);
+        const uint32_t bc = bytes_cuda(seq[0] & 0xFFu) + bytes_cuda(seq[1] & 0xFFu),
+                       bg = bytes_go(seq[0] & 0xFFu) + bytes_go(seq[1] & 0xFFu);
+        idx[r] = (c0 * kNumInsns + c1) | (should_prune(seq, 2) ? kEntryPruned : 0u) | (bc - 2) << 24 | (bg - 2) << 26;
     }
 }
 
+// The two packed words of QuickCheck outputs of a length-2 sequence.
+__device__ __forceinline__ void cand2_outputs(uint32_t c, St (&v)[2]) {
+#pragma unroll
+    for (int g = 0; g < 2; g++)
+        v[g] = St{c_vec4[g][0], c_vec4[g][1], c_vec4[g][2], c_vec4[g][3],
+                  c_vec4[g][4], c_vec4[g][5], c_vec4[g][6], c_vec4[g][7]};
+    exec_x4n(v, c_tab[c / kNumInsns]);
+    exec_x4n(v, c_tab[c % kNumInsns]);
+}
 
-// QC (+ MidCheck) of targets x all length-2 candidates through the sorted
-// table.  Lane v executes the candidate on vector v.  The byte filter and
-// the pruner are applied per candidate in the equal range.  Go semantics:
-// `best` ([2][nt], the length-1 winners) skips the passes a target has
-// already settled (the worker stops at the first candidate length that
-// finds one, worker.go:122-176).
-//
+// After the sort: P after the QuickCheck vectors of every entry (pw, for
+// FlagDiff); whether two different sets of outputs share a key (info[0]: the
+// table is then built again with another salt, so that one candidate of a
+// range decides QuickCheck for all); the longest range of one key (info[1]).
+__global__ void k_cand2_info(uint32_t dead, const uint64_t* __restrict__ keys, const uint32_t* __restrict__ idx,
+                             uint2* __restrict__ pw, uint32_t* __restrict__ info) {
+    const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;
+    const uint32_t n = (uint32_t)kNumInsns * (uint32_t)kNumInsns;
+    uint32_t longest = 0, clash = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        St v[2];
+        cand2_outputs(idx[i] & kEntryIndex, v);
+        pw[i] = make_uint2(v[0].p & (kPMask * kB1), v[1].p & (kPMask * kB1));
+        const uint64_t key = keys[i];
+        if (i > 0 && keys[i - 1] == key) {
+            St u[2];
+            cand2_outputs(idx[i - 1] & kEntryIndex, u);
+#pragma unroll
+            for (int g = 0; g < 2; g++)
+                clash |= (v[g].a ^ u[g].a) | (v[g].x ^ u[g].x) | (v[g].y ^ u[g].y) | ((v[g].p ^ u[g].p) & pm) |
+                         (v[g].s ^ u[g].s) | (v[g].m ^ u[g].m) | (v[g].s0 ^ u[g].s0) | (v[g].s1 ^ u[g].s1);
+        } else {   // first of its range: the range's end by doubling and halving
+            uint32_t step = 1;
+            while (i + step < n && keys[i + step] == key) step <<= 1;
+            uint32_t lo = i + (step >> 1), hi = min(i + step, n);   // keys[lo] == key; keys[hi] is another or past the end
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (keys[mid] == key) lo = mid; else hi = mid;
+            }
+            longest = max(longest, hi - i);
+        }
+    }
+    if (clash) info[0] = 1u;
+    atomicMax(info + 1, longest);
+}
+
 // Equal ranges are very uneven (a flags-only target under mask 0xFF matches
 // hundreds of thousands of flags-only candidates), so a range longer than
 // kJoinChunk is cut into work items that every warp drains.
@@ -1488,16 +1596,24 @@ constexpr uint32_t kJoinChunk = 1024;
 
 struct JoinItem {   // candidates [lo, hi) of one target's equal range
     uint32_t t, lo, hi, exact;
+    uint32_t seq;      // items of the same range before it (they lie next to each other)
+    uint32_t n0, n1;   // Go semantics: its survivors of each pass
+    uint32_t pad;
+};
+
+struct Cand2View {     // the sorted table of one mask
+    const uint64_t* keys;
+    const uint32_t* idx;
+    const uint2* pw;
+    uint64_t salt;
 };
 
 struct Join2Args {
     const uint64_t* tfp;
     const uint8_t* tmeta;
     uint32_t nt;
-    const uint64_t* lkeys;   // the run mask's table
-    const uint32_t* lidx;
-    const uint64_t* ekeys;   // the unmasked table (Go semantics, unmasked pass only)
-    const uint32_t* eidx;
+    Cand2View loose;         // the run mask's table
+    Cand2View exact;         // the unmasked table (Go semantics, unmasked pass only)
     uint32_t nsorted;
     uint32_t dead;
     uint32_t stages;
@@ -1507,60 +1623,35 @@ struct Join2Args {
     JoinItem* items;
     uint64_t item_cap;
     Counters* cnt;
+    Surv* first;             // Go semantics: the first round's list (see k_expand)
+    uint32_t* ord;
+    uint32_t block;
 };
 
-// Which passes a target still needs (Go semantics; both for CUDA).
-template <bool GO>
-__device__ __forceinline__ void open_passes(const Join2Args& a, uint32_t t, bool& need_u, bool& need_m) {
-    need_u = true;
-    need_m = a.dead != 0;
-    if (GO) {
-        need_u = a.best[t] == 0xFFFFFFFFu;
-        need_m = need_m && a.best[(uint64_t)a.nt + t] == 0xFFFFFFFFu;
-    }
-}
-
-template <bool GO>
-__device__ __forceinline__ void join2_range(const Join2Args& a, uint32_t t, uint32_t lo, uint32_t hi, bool use_exact,
-                                            uint64_t tv, bool need_u, bool need_m, Surv* stage, int& nstage,
-                                            unsigned long long& nqc, unsigned long long& nmid, int lane) {
-    const uint64_t loose = cmp_mask(a.dead), exact = cmp_mask(0);
-    const uint32_t* sidx = use_exact ? a.eidx : a.lidx;
-    const uint32_t tb = GO ? (a.tmeta[t] >> 4) : (a.tmeta[t] & 15u);
+// CUDA semantics: QC + MidCheck of targets x all length-2 candidates through
+// the sorted table.  Lane v executes the candidate on vector v.  The byte
+// filter and the pruner are applied per candidate in the equal range.
+__device__ __forceinline__ void join2_range(const Join2Args& a, uint32_t t, uint32_t lo, uint32_t hi, uint64_t tv,
+                                            Surv* stage, int& nstage, unsigned long long& nqc,
+                                            unsigned long long& nmid, int lane) {
+    const uint64_t loose = cmp_mask(a.dead);
+    const uint32_t tb = a.tmeta[t] & 15u;
     for (uint32_t base = lo; base < hi; base += 32) {
         const uint32_t i = base + (uint32_t)lane;
-        const unsigned run = __ballot_sync(kFull, i < hi);
-        const uint32_t mine = i < hi ? sidx[i] : 0u;
-        for (unsigned r = run; r; r &= r - 1) {
-            const uint32_t c = __shfl_sync(kFull, mine, __ffs(r) - 1);
-            uint16_t seq[2] = {c_tab[c / kNumInsns], c_tab[c % kNumInsns]};
-            const uint32_t cb = GO ? bytes_go(seq[0] & 0xFFu) + bytes_go(seq[1] & 0xFFu)
-                                   : bytes_cuda(seq[0] & 0xFFu) + bytes_cuda(seq[1] & 0xFFu);
-            if (cb >= tb || should_prune(seq, 2)) continue;   // not shorter, or pruned (uniform)
+        const uint32_t mine = i < hi ? a.loose.idx[i] : kEntryPruned;
+        // shorter, and not pruned
+        unsigned run = __ballot_sync(kFull, !(mine & kEntryPruned) && entry_bytes_cuda(mine) < tb);
+        for (; run; run &= run - 1) {
+            const uint32_t c = __shfl_sync(kFull, mine, __ffs(run) - 1) & kEntryIndex;
             St s = unpack(c_vec[lane]);
-            exec(s, seq[0]);
-            exec(s, seq[1]);
-            const uint64_t x = tv ^ fp_of(s);
-            const unsigned lo_eq = __ballot_sync(kFull, (x & loose) == 0);
-            const unsigned ex_eq = __ballot_sync(kFull, (x & exact) == 0);
-            if ((lo_eq & 0xFFu) != 0xFFu) continue;          // hash collision: QuickCheck fails
-            bool pass = false;
-            uint32_t code = c | kSurvLen2;
-            if (!GO) {
-                nqc += lane == 0;
-                const bool mid = !(a.stages & M6502_CHECK_MID) || lo_eq == kFull;
-                if (mid) { nmid += lane == 0; pass = true; }
-            } else if ((ex_eq & 0xFFu) == 0xFFu) {           // processTask: unmasked QC passes
-                if (need_u) { nqc += lane == 0; nmid += lane == 0; pass = true; }
-            } else if (need_m) {                             // processTaskMasked, FlagDiff != 0
-                uint32_t fd = lane < 8 ? ((uint32_t)(x >> 24) & kPMask) : 0u;
-                fd = __reduce_or_sync(kFull, fd);
-                if (fd) {
-                    nqc += lane == 0; nmid += lane == 0; pass = true;
-                    code |= kSurvMasked | (fd_pack(fd) << 25);
-                }
-            }
-            stage_push(pass && lane == 0, Surv{t, code}, stage, nstage, a.surv, a.cap, &a.cnt->surv, lane);
+            exec(s, c_tab[c / kNumInsns]);
+            exec(s, c_tab[c % kNumInsns]);
+            const unsigned eq = __ballot_sync(kFull, ((tv ^ fp_of(s)) & loose) == 0);
+            if ((eq & 0xFFu) != 0xFFu) continue;          // hash collision: QuickCheck fails
+            nqc += lane == 0;
+            const bool mid = !(a.stages & M6502_CHECK_MID) || eq == kFull;
+            nmid += mid && lane == 0;
+            stage_push(mid && lane == 0, Surv{t, c | kSurvLen2}, stage, nstage, a.surv, a.cap, &a.cnt->surv, lane);
         }
     }
 }
@@ -1576,46 +1667,41 @@ __device__ __forceinline__ void join_counts(Counters* cnt, unsigned long long nq
     }
 }
 
-template <bool GO>
+// The range [lo, hi) of a target's key in a table.
+__device__ __forceinline__ void key_range(const Cand2View& tab, uint32_t n, uint64_t key, uint32_t& lo, uint32_t& hi, int lane) {
+    lo = warp_lower_bound(tab.keys, n, key, lane);
+    hi = key == ~0ull ? n : warp_lower_bound(tab.keys, n, key + 1, lane);
+}
+
+// Cuts a long range into items.
+__device__ __forceinline__ void push_items(const Join2Args& a, uint32_t t, uint32_t lo, uint32_t hi, bool exact, int lane) {
+    const uint32_t nitems = (hi - lo + kJoinChunk - 1) / kJoinChunk;
+    unsigned long long b = 0;
+    if (lane == 0) b = atomicAdd(&a.cnt->join_items, (unsigned long long)nitems);
+    b = __shfl_sync(kFull, b, 0);
+    for (uint32_t j = lane; j < nitems; j += 32)
+        if (b + j < a.item_cap)
+            a.items[b + j] = JoinItem{t, lo + j * kJoinChunk, min(hi, lo + (j + 1) * kJoinChunk), exact ? 1u : 0u, j, 0, 0, 0};
+}
+
 __global__ void __launch_bounds__(256) k_qc_join2(Join2Args a) {
     __shared__ Surv s_stage[kWarpsPerBlock][kStage];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     Surv* stage = s_stage[w];
     int nstage = 0;
-    const uint64_t loose = cmp_mask(a.dead), exact = cmp_mask(0);
     unsigned long long nqc = 0, nmid = 0;
     for (uint32_t t = blockIdx.x * kWarpsPerBlock + w; t < a.nt; t += gridDim.x * kWarpsPerBlock) {
-        bool need_u, need_m;
-        open_passes<GO>(a, t, need_u, need_m);
-        if (!need_u && !need_m) continue;
         const uint64_t tv = a.tfp[(uint64_t)t * 32 + lane];
-        // Only the unmasked pass open: its candidates are the exact-key range
-        // of the unmasked table, a subset of the masked key's range.
-        const bool use_exact = GO && !need_m;
-        const uint64_t* skeys = use_exact ? a.ekeys : a.lkeys;
-        const uint64_t km = use_exact ? exact : loose;
-        const uint64_t key = warp_key(tv, km, lane);
-        const uint32_t lo = warp_lower_bound(skeys, a.nsorted, key, lane);
-        const uint32_t hi = key == ~0ull ? a.nsorted : warp_lower_bound(skeys, a.nsorted, key + 1, lane);
-        if (hi - lo <= kJoinChunk) {
-            join2_range<GO>(a, t, lo, hi, use_exact, tv, need_u, need_m, stage, nstage, nqc, nmid, lane);
-            continue;
-        }
-        const uint32_t nitems = (hi - lo + kJoinChunk - 1) / kJoinChunk;
-        unsigned long long b = 0;
-        if (lane == 0) b = atomicAdd(&a.cnt->join_items, (unsigned long long)nitems);
-        b = __shfl_sync(kFull, b, 0);
-        for (uint32_t j = lane; j < nitems; j += 32)
-            if (b + j < a.item_cap)
-                a.items[b + j] = JoinItem{t, lo + j * kJoinChunk, min(hi, lo + (j + 1) * kJoinChunk),
-                                          use_exact ? 1u : 0u};
+        uint32_t lo, hi;
+        key_range(a.loose, a.nsorted, warp_key(tv, cmp_mask(a.dead), a.loose.salt, lane), lo, hi, lane);
+        if (hi - lo <= kJoinChunk) join2_range(a, t, lo, hi, tv, stage, nstage, nqc, nmid, lane);
+        else push_items(a, t, lo, hi, false, lane);
     }
     stage_flush(stage, nstage, a.surv, a.cap, &a.cnt->surv, lane);
     join_counts(a.cnt, nqc, nmid);
 }
 
 // The chunks of the long equal ranges, a warp per chunk.
-template <bool GO>
 __global__ void __launch_bounds__(256) k_qc_join2_items(Join2Args a) {
     __shared__ Surv s_stage[kWarpsPerBlock][kStage];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1625,13 +1711,135 @@ __global__ void __launch_bounds__(256) k_qc_join2_items(Join2Args a) {
     const uint64_t n = min((uint64_t)a.cnt->join_items, a.item_cap);
     for (uint64_t q = (uint64_t)blockIdx.x * kWarpsPerBlock + w; q < n; q += (uint64_t)gridDim.x * kWarpsPerBlock) {
         const JoinItem it = a.items[q];
-        bool need_u, need_m;
-        open_passes<GO>(a, it.t, need_u, need_m);
-        const uint64_t tv = a.tfp[(uint64_t)it.t * 32 + lane];
-        join2_range<GO>(a, it.t, it.lo, it.hi, it.exact != 0, tv, need_u, need_m, stage, nstage, nqc, nmid, lane);
+        join2_range(a, it.t, it.lo, it.hi, a.tfp[(uint64_t)it.t * 32 + lane], stage, nstage, nqc, nmid, lane);
     }
     stage_flush(stage, nstage, a.surv, a.cap, &a.cnt->surv, lane);
     join_counts(a.cnt, nqc, nmid);
+}
+
+// Go semantics: QuickCheck of targets x all length-2 candidates.  No
+// MidCheck, and the candidates of a range have one set of masked outputs (the
+// table is built so), so one of them decides for all; what is left per
+// candidate is its entry (pruned, size) and its FlagDiff from the tabulated P
+// words: a lane each, where a warp per candidate ran it on the vectors before
+// (4,096 length-3 targets, mask 0xC3: 2.36 ms, now 0.14).
+// `best` ([2][nt], the length-1 winners) skips the passes a target has already
+// settled (the worker stops at the first candidate length that finds one,
+// worker.go:122-176).  Candidates come in Go order; a long range's items are
+// counted first (k_go_join2_count), so that each knows the ordinals before it.
+struct GoRange {
+    bool need_u, need_m, use_exact;
+    uint32_t tb, p0, p1;   // Go byte size; P after the QuickCheck vectors
+};
+
+__device__ __forceinline__ GoRange go_range(const Join2Args& a, uint32_t t, uint64_t tv, int lane) {
+    GoRange r;
+    r.need_u = a.best[t] == 0xFFFFFFFFu;
+    r.need_m = a.dead != 0 && a.best[(uint64_t)a.nt + t] == 0xFFFFFFFFu;
+    // Only the unmasked pass open: its candidates are the exact-key range of
+    // the unmasked table, a subset of the masked key's range.
+    r.use_exact = !r.need_m;
+    r.tb = a.tmeta[t] >> 4;
+    const uint32_t p = (uint32_t)(tv >> 24) & 0xFFu;
+    r.p0 = __reduce_or_sync(kFull, lane < 4 ? p << (8 * lane) : 0u);
+    r.p1 = __reduce_or_sync(kFull, lane >= 4 && lane < 8 ? p << (8 * (lane - 4)) : 0u);
+    return r;
+}
+
+// One step of 32 candidates from `base`: whether this lane's is a survivor
+// of an open pass, which, and its index.
+__device__ __forceinline__ bool go_candidate(const Join2Args& a, const GoRange& r, uint32_t i, uint32_t hi, bool& masked,
+                                             uint32_t& c) {
+    masked = false;
+    if (i >= hi) return false;
+    const uint32_t e = r.use_exact ? a.exact.idx[i] : a.loose.idx[i];
+    c = e & kEntryIndex;
+    if ((e & kEntryPruned) || entry_bytes_go(e) >= r.tb) return false;
+    if (!r.use_exact) {
+        const uint2 p = a.loose.pw[i];
+        masked = (((p.x ^ r.p0) | (p.y ^ r.p1)) & (kPMask * kB1)) != 0;   // FlagDiff != 0: processTaskMasked
+    }
+    return masked ? r.need_m : r.need_u;
+}
+
+__device__ __forceinline__ void go_scan(const Join2Args& a, const GoRange& r, uint32_t t, uint32_t lo, uint32_t hi,
+                                        uint32_t n0, uint32_t n1, Surv* stage, int& nstage, unsigned long long& nqc, int lane) {
+    GoCount count{n0, n1};
+    for (uint32_t base = lo; base < hi; base += 32) {
+        bool masked;
+        uint32_t c = 0;
+        const bool take = go_candidate(a, r, base + lane, hi, masked, c);
+        nqc += take;
+        const uint32_t at = count.step(take, masked, 0, true, lane);
+        const Surv rec{t, c | kSurvLen2 | (masked ? kSurvMasked : 0u)};
+        go_late(take && at >= a.block, rec, at, a.surv, a.ord, a.cap, a.cnt, lane);
+        stage_push(take && at < a.block, rec, stage, nstage, a.first, a.cap, &a.cnt->v[1][0].n, lane);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_go_join2(Join2Args a) {
+    __shared__ Surv s_stage[kWarpsPerBlock][kStage];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    Surv* stage = s_stage[w];
+    int nstage = 0;
+    unsigned long long nqc = 0;
+    for (uint32_t t = blockIdx.x * kWarpsPerBlock + w; t < a.nt; t += gridDim.x * kWarpsPerBlock) {
+        const uint64_t tv = a.tfp[(uint64_t)t * 32 + lane];
+        const GoRange r = go_range(a, t, tv, lane);
+        if (!r.need_u && !r.need_m) continue;
+        const Cand2View& tab = r.use_exact ? a.exact : a.loose;
+        const uint64_t km = r.use_exact ? cmp_mask(0) : cmp_mask(a.dead);
+        uint32_t lo, hi;
+        key_range(tab, a.nsorted, warp_key(tv, km, tab.salt, lane), lo, hi, lane);
+        if (lo == hi) continue;
+        const uint32_t c = tab.idx[lo] & kEntryIndex;   // the range's QuickCheck
+        St s = unpack(c_vec[lane]);
+        exec(s, c_tab[c / kNumInsns]);
+        exec(s, c_tab[c % kNumInsns]);
+        if ((__ballot_sync(kFull, ((tv ^ fp_of(s)) & km) == 0) & 0xFFu) != 0xFFu) continue;
+        if (hi - lo <= kJoinChunk) go_scan(a, r, t, lo, hi, 0, 0, stage, nstage, nqc, lane);
+        else push_items(a, t, lo, hi, r.use_exact, lane);
+    }
+    stage_flush(stage, nstage, a.first, a.cap, &a.cnt->v[1][0].n, lane);
+    join_counts(a.cnt, nqc, nqc);
+}
+
+__global__ void __launch_bounds__(256) k_go_join2_count(Join2Args a) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t n = min((uint64_t)a.cnt->join_items, a.item_cap);
+    for (uint64_t q = (uint64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); q < n; q += (uint64_t)gridDim.x * kWarpsPerBlock) {
+        const JoinItem it = a.items[q];
+        const GoRange r = go_range(a, it.t, a.tfp[(uint64_t)it.t * 32 + lane], lane);
+        uint32_t n0 = 0, n1 = 0;
+        for (uint32_t base = it.lo; base < it.hi; base += 32) {
+            bool masked;
+            uint32_t c;
+            const bool take = go_candidate(a, r, base + lane, it.hi, masked, c);
+            n0 += __popc(__ballot_sync(kFull, take && !masked));
+            n1 += __popc(__ballot_sync(kFull, take && masked));
+        }
+        if (lane == 0) { a.items[q].n0 = n0; a.items[q].n1 = n1; }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_go_join2_items(Join2Args a) {
+    __shared__ Surv s_stage[kWarpsPerBlock][kStage];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    Surv* stage = s_stage[w];
+    int nstage = 0;
+    unsigned long long nqc = 0;
+    const uint64_t n = min((uint64_t)a.cnt->join_items, a.item_cap);
+    for (uint64_t q = (uint64_t)blockIdx.x * kWarpsPerBlock + w; q < n; q += (uint64_t)gridDim.x * kWarpsPerBlock) {
+        const JoinItem it = a.items[q];
+        const GoRange r = go_range(a, it.t, a.tfp[(uint64_t)it.t * 32 + lane], lane);
+        uint32_t n0 = 0, n1 = 0;   // survivors of the items before it
+        for (uint32_t j = lane; j < it.seq; j += 32) { n0 += a.items[q - 1 - j].n0; n1 += a.items[q - 1 - j].n1; }
+        n0 = __reduce_add_sync(kFull, n0);
+        n1 = __reduce_add_sync(kFull, n1);
+        go_scan(a, r, it.t, it.lo, it.hi, n0, n1, stage, nstage, nqc, lane);
+    }
+    stage_flush(stage, nstage, a.first, a.cap, &a.cnt->v[1][0].n, lane);
+    join_counts(a.cnt, nqc, nqc);
 }
 
 // Exhaustive check, one pair per warp (persistent, device ticket).
@@ -1657,12 +1865,12 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
     // Lane 0 claims the following batch while the warp works on the current
     // one, so the atomic's latency is hidden behind a batch of pairs.
     unsigned long long ahead = 0;
-    if (lane == 0) ahead = atomicAdd(&a.cnt->exh_ticket, tbatch);
+    if (lane == 0) ahead = atomicAdd(&a.v->exh_ticket, tbatch);
     for (;;) {
         if (next >= lim) {
             next = __shfl_sync(kFull, ahead, 0);
             lim = next + tbatch;
-            if (lane == 0 && next < n) ahead = atomicAdd(&a.cnt->exh_ticket, tbatch);
+            if (lane == 0 && next < n) ahead = atomicAdd(&a.v->exh_ticket, tbatch);
         }
         const unsigned long long q = next++;
         if (q >= n) break;
@@ -1728,7 +1936,7 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
                 const uint64_t chunk = max(chunk_min, (total + kMaxItemsPerCone - 1) / kMaxItemsPerCone);
                 const uint64_t nitems = (total - kProbe + chunk - 1) / chunk;
                 unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(&a.cnt->items, (unsigned long long)nitems);
+                if (lane == 0) base = atomicAdd(&a.v->items, (unsigned long long)nitems);
                 base = __shfl_sync(kFull, base, 0);
                 for (uint64_t j = lane; j < nitems; j += 32) {
                     if (base + j >= a.item_cap) break;
@@ -1792,11 +2000,11 @@ __global__ void __launch_bounds__(256) k_small(Src src, const unsigned long long
     // the pair's sequences: one column of the staging array for its lanes
     uint16_t *st = &s_ins[0][(threadIdx.x & ~31u) + lead], *sc = st + Src::kMaxT * 256;
     unsigned long long nstates = 0, next = 0;
-    if (lane == 0) next = atomicAdd(&a.cnt->small_ticket, batch);
+    if (lane == 0) next = atomicAdd(&a.v->small_ticket, batch);
     for (;;) {
         const uint64_t first = __shfl_sync(kFull, next, 0), p = first + (uint32_t)(lane >> g);
         if (first >= n) break;
-        if (lane == 0) next = atomicAdd(&a.cnt->small_ticket, batch);
+        if (lane == 0) next = atomicAdd(&a.v->small_ticket, batch);
         int tn = 0, cn = 0;
         uint32_t dead = 0, swx = 0, written = 0;
         if (p < n && sub == 0) src.load_lane(p, st, sc, 256, tn, cn, dead);
@@ -1817,7 +2025,7 @@ __global__ void __launch_bounds__(256) k_small(Src src, const unsigned long long
         const unsigned left = __ballot_sync(kFull, p < n && !small && sub == 0);
         if (left) {
             unsigned long long b = 0;
-            if (lane == 0) b = atomicAdd(&a.cnt->small_left, (unsigned long long)__popc(left));
+            if (lane == 0) b = atomicAdd(&a.v->small_left, (unsigned long long)__popc(left));
             b = __shfl_sync(kFull, b, 0) + __popc(left & ((1u << lane) - 1u));
             if (((left >> lane) & 1u) && b < n_cap) order[b] = (uint32_t)p;
         }
@@ -1864,11 +2072,11 @@ template <class Src>
 __global__ void __launch_bounds__(256) k_exh_items(Src src, ExhArgs a) {
     __shared__ uint16_t s_t[kWarpsPerBlock][kMaxSeq], s_c[kWarpsPerBlock][kMaxSeq];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint64_t n = min((uint64_t)a.cnt->items, a.item_cap);
+    const uint64_t n = min((uint64_t)a.v->items, a.item_cap);
     unsigned long long nstates = 0;
     for (;;) {
         unsigned long long q = 0;
-        if (lane == 0) q = atomicAdd(&a.cnt->item_ticket, 1ull);
+        if (lane == 0) q = atomicAdd(&a.v->item_ticket, 1ull);
         q = __shfl_sync(kFull, q, 0);
         if (q >= n) break;
         const Item it = a.items[q];
@@ -2042,14 +2250,14 @@ __global__ void k_go_emit(const uint32_t* __restrict__ best, uint32_t nt, const 
 // ---- Go semantics: verification in Go order, in rounds ----
 //
 // The Go worker stops at the first candidate (in Go order) that passes
-// ExhaustiveCheck (worker.go:125-173).  The survivors of a pass are sorted by
-// (target, pass kind, Go rank); round r verifies, for every (target, kind)
-// not yet settled, the next block of its survivors (block sizes 64, 128,
-// 256, ...), and the smallest passing rank of a block settles it.  Only the
-// blocks up to the first pass are swept -- the work the Go worker does.
+// ExhaustiveCheck (worker.go:125-173).  Every survivor has an ordinal within
+// its (target, pass) in Go order; round r verifies, for every (target, pass)
+// not yet settled, the next block of its survivors (block sizes 64, 512,
+// 4096, ...), and the smallest passing rank of a block settles it.  Only the
+// blocks up to the first pass are swept.  The joins meet the candidates in Go
+// order and number them as they go (GoCount); the scan's survivors are sorted.
 
-// Sort key of a survivor: target << 30 | masked pass << 29 | go_rank_of.
-
+// Sort key of a scanned survivor: target << 30 | masked pass << 29 | go_rank_of.
 // Entries from the survivor count up to the capacity get `pad`, which sorts
 // after every real key.
 __global__ void k_go_keys(const Surv* __restrict__ surv, const unsigned long long* n_ptr, uint64_t cap, uint64_t pad,
@@ -2062,67 +2270,46 @@ __global__ void k_go_keys(const Surv* __restrict__ surv, const unsigned long lon
     }
 }
 
-// Ordinal of each sorted survivor within its (target, kind) group.
+// The sorted survivors, rebuilt from their keys, with their ordinals.
 __global__ void k_go_ord(const uint64_t* __restrict__ keys, const unsigned long long* n_ptr, uint64_t cap,
-                         uint32_t* __restrict__ ord, Counters* __restrict__ cnt) {
+                         Surv* __restrict__ surv, uint32_t* __restrict__ ord, Counters* __restrict__ cnt) {
     const uint64_t n = min((uint64_t)*n_ptr, cap);
     unsigned long long mx = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t g = keys[i] >> 29;
+        const uint64_t k = keys[i], g = k >> 29;
         uint64_t lo = 0, hi = i;   // first index of the group
         while (lo < hi) {
             const uint64_t mid = (lo + hi) >> 1;
             if ((keys[mid] >> 29) < g) lo = mid + 1; else hi = mid;
         }
-        ord[i] = (uint32_t)min((unsigned long long)(i - lo), 0xFFFFFFFFull);
+        surv[i] = Surv{(uint32_t)(k >> 30), c_goidx[(uint32_t)k & 0x1FFFFFFFu] | ((g & 1u) ? kSurvMasked : 0u)};
+        ord[i] = (uint32_t)(i - lo);
         mx = max(mx, (unsigned long long)(i - lo));
     }
     for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_down_sync(kFull, mx, o));
     if ((threadIdx.x & 31) == 0 && mx) atomicMax(&cnt->max_ord, mx);
 }
 
-// The survivors of one round, rebuilt as Surv records from their keys.
-// A round whose first ordinal lies past the largest one finds nothing.
-__global__ void k_go_round(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ ord,
+// The survivors of one round: ordinals [lo, hi) of what is still open.  A
+// round whose first ordinal lies past the largest one finds nothing.
+__global__ void k_go_round(const Surv* __restrict__ surv, const uint32_t* __restrict__ ord,
                            const unsigned long long* n_ptr, uint64_t cap, uint32_t lo, uint32_t hi,
                            const uint32_t* __restrict__ best, uint32_t nt, Surv* __restrict__ out,
-                           Counters* __restrict__ cnt) {
+                           const Counters* __restrict__ cnt, VerifyCounters* __restrict__ v) {
     if ((unsigned long long)lo > cnt->max_ord) return;
     const uint64_t n = min((uint64_t)*n_ptr, cap);
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t o = ord[i];
         if (o < lo || o >= hi) continue;
-        const uint64_t k = keys[i];
-        const uint32_t t = (uint32_t)(k >> 30), kind = (uint32_t)(k >> 29) & 1u, rank = (uint32_t)k & 0x1FFFFFFFu;
-        if (best[(uint64_t)kind * nt + t] != 0xFFFFFFFFu) continue;   // settled by an earlier round
-        uint32_t code;
-        if (rank >> 28) {
-            const uint32_t r = rank & 0x0FFFFFFFu;
-            code = kSurvLen2 | ((uint32_t)c_goidx[r / kNumInsns] * kNumInsns + c_goidx[r % kNumInsns]);
-        } else {
-            code = c_goidx[rank];
-        }
-        if (kind) code |= kSurvMasked;
-        out[atomicAdd(&cnt->round_n, 1ull)] = Surv{t, code};
+        const Surv s = surv[i];
+        const uint32_t kind = (s.c & kSurvMasked) ? 1u : 0u;
+        if (best[(uint64_t)kind * nt + s.t] != 0xFFFFFFFFu) continue;   // settled by an earlier round
+        out[atomicAdd(&v->n, 1ull)] = s;
     }
 }
 
-// After a round: its pairs and work items join the totals; the largest
-// item count is kept for the overflow check after the pass.
-__global__ void k_go_tally(Counters* cnt) {
-    cnt->round_checked += cnt->round_n;
-    cnt->round_items += cnt->items;
-    cnt->items_need = max(cnt->items_need, cnt->items);
-}
-
-// Before the length-2 phase resets the survivor and item counters: the
-// first phase's counts are kept.
-__global__ void k_mark_phase(Counters* cnt) {
-    cnt->surv1 = cnt->surv;
-    cnt->items1 = cnt->items;
-    cnt->surv_need = max(cnt->surv_need, cnt->surv);
-    cnt->items_need = max(cnt->items_need, cnt->items);
-}
+// Before the length-2 phase resets the survivor counter.
+__global__ void k_mark_phase(Counters* cnt) { cnt->surv1 = cnt->surv; }
 
 // Pairwise QC / MidCheck / FlagDiff: warp per pair, lane = vector.
 __global__ void __launch_bounds__(256) k_pair_vectors(CsrSource src, uint64_t n, uint8_t* __restrict__ out,
@@ -2255,7 +2442,7 @@ __global__ void __launch_bounds__(256) k_exhaustive_static(StaticCsrSource src, 
     unsigned long long nstates = 0;
     for (;;) {
         unsigned long long p = 0;
-        if (lane == 0) p = atomicAdd(&scr->cnt.exh_ticket, 1ull);
+        if (lane == 0) p = atomicAdd(&scr->cnt.v[0][0].exh_ticket, 1ull);
         p = __shfl_sync(kFull, p, 0);
         if (p >= n) break;
         PairView pv;
@@ -2342,6 +2529,8 @@ struct m6502_ctx {
     std::vector<uint32_t> h_cfp4;     // host copy
     std::vector<uint8_t> h_cmeta;
     std::vector<uint16_t> h_tab;      // instructions, CUDA order (host copy)
+    std::vector<uint32_t> h_gorank;   // Go-order rank of each
+    uint32_t join_longest[256] = {};  // most candidates of one entry of the Go-semantics table
     DevBuf go_keys, go_keys2, go_ord, go_round, go_sort_tmp;   // Go-order verification rounds
     DevBuf jitems;                                             // chunks of long length-2 equal ranges
     DevBuf order;                                              // k_small: the pairs it left
@@ -2349,9 +2538,11 @@ struct m6502_ctx {
     DevBuf join_tab[2][256];                      // JoinTable by semantics and dead-flags mask
     DevBuf join_groups[256];                      // CandGroups of the CUDA-semantics tables
     DevBuf join_lines[256];                       // line hashes of the candidates, [64 register sets][2863]
-    struct Cand2Table {            // sorted (key, index) of all length-2 sequences for one mask
+    struct Cand2Table {            // sorted (key, entry) of all length-2 sequences for one mask
         uint32_t dead = 0xFFFFFFFFu;
-        DevBuf keys, idx;
+        uint32_t longest = 0;      // longest range of one key
+        uint64_t salt = 0;
+        DevBuf keys, idx, pw;
         uint64_t stamp = 0;
     } cand2[4];                    // least recently used mask is rebuilt
     uint64_t cand2_clock = 0;
@@ -2411,7 +2602,7 @@ int launch_exh(m6502_ctx* ctx, const SurvSource& src, const unsigned long long* 
         k_small<SurvSource><<<ctx->small_blocks, 256, 0, ctx->stream>>>(src, n_ptr, cap, ea, (uint32_t*)ctx->order.p);
         CKL("k_small");
         ea.order = (const uint32_t*)ctx->order.p;
-        n_ptr = &ea.cnt->small_left;
+        n_ptr = &ea.v->small_left;
     }
     const int minb = (int)ctx->tune.exh_minb;
     const unsigned grid = (unsigned)(ctx->sms * ctx->exh_occ[minb >= 2 && minb <= 4 ? minb : 4]);
@@ -2435,7 +2626,7 @@ int launch_verify(m6502_ctx* ctx, const Src& src, const unsigned long long* n_pt
             src, n_ptr, cap, ea, (uint32_t*)ctx->order.p);
         CKL("k_small");
         ea.order = (const uint32_t*)ctx->order.p;
-        n_ptr = &ea.cnt->small_left;
+        n_ptr = &ea.v->small_left;
     }
     k_exhaustive<Src><<<ctx->exh_blocks, 256, 0, ctx->stream>>>(src, n_ptr, cap, ea);
     CKL("k_exhaustive");
@@ -2456,7 +2647,7 @@ int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt
     const bool go = cfg.semantics == M6502_SEM_GO;
     const uint32_t stages = cfg.stages ? cfg.stages : M6502_CHECK_ALL, dead = cfg.dead_flags;
     // the line filter is part of ExhaustiveCheck; brute force does without
-    const bool filter = !go && (stages & M6502_CHECK_EXH) && cfg.exh_mode != M6502_EXH_BRUTE;
+    const bool exh = (stages & M6502_CHECK_EXH) != 0, filter = exh && cfg.exh_mode != M6502_EXH_BRUTE;
     const uint64_t warps = (uint64_t)ctx->sms * 4 * kWarpsPerBlock;   // 4 resident blocks per SM
     const uint32_t chunk = (uint32_t)std::min<uint64_t>(32, (nt + warps - 1) / warps);
     const uint64_t blocks = (nt + (uint64_t)chunk * kWarpsPerBlock - 1) / ((uint64_t)chunk * kWarpsPerBlock);
@@ -2474,9 +2665,11 @@ int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt
     const uint32_t egrid = (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 4, (nt + 255) / 256);
     auto expand = [&](auto kernel) {
         kernel<<<egrid, 256, 0, ctx->stream>>>(match, d_t, tlen, cfp4, tab, dead, cfg.sweep, mult, lines, (Surv*)ctx->surv.p,
-                                               scap, cnt);
+                                               scap, cnt, (Surv*)ctx->go_round.p, (uint32_t*)ctx->go_ord.p,
+                                               exh ? kGoBlock : 0u);
     };
-    if (go) expand(k_expand<true, false>);
+    if (go && filter) expand(k_expand<true, true>);
+    else if (go) expand(k_expand<true, false>);
     else if (filter) expand(k_expand<false, true>);
     else expand(k_expand<false, false>);
     CKL("k_expand");
@@ -2598,6 +2791,7 @@ int init_ctx(m6502_ctx* ctx) {
                        ctx->stream));
     ctx->h_cmeta = meta;
     ctx->h_tab.assign(tab, tab + kNumInsns);
+    ctx->h_gorank.assign(gorank, gorank + kNumInsns);
     CK(cudaMemcpyAsync(ctx->cfp1.p, tr.data(), tr.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->cmeta1.p, meta.data(), meta.size(), cudaMemcpyHostToDevice, ctx->stream));
     TRY(ensure(ctx, ctx->cnt, sizeof(Counters)));
@@ -2629,7 +2823,8 @@ int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
     const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;
     struct Entry {
         uint64_t key;
-        std::vector<uint32_t> words;
+        std::vector<uint32_t> words;   // Go semantics has no MidCheck: QuickCheck's 16 only
+        uint32_t rank;                 // order among equals: CUDA or Go enumeration
         uint16_t cand;
     };
     std::vector<Entry> v;
@@ -2649,10 +2844,11 @@ int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
         for (int g = 0; g < 8; g++) words[8 * g + 3] &= pm;
         uint32_t qc[16];
         std::copy(words.begin(), words.begin() + 16, qc);
-        v.push_back({join_key(qc), std::move(words), (uint16_t)c});
+        if (go) words.resize(16);
+        v.push_back({join_key(qc), std::move(words), go ? ctx->h_gorank[c] : (uint32_t)c, (uint16_t)c});
     }
     std::sort(v.begin(), v.end(), [](const Entry& a, const Entry& b) {
-        return std::tie(a.key, a.words, a.cand) < std::tie(b.key, b.words, b.cand);
+        return std::tie(a.key, a.words, a.rank) < std::tie(b.key, b.words, b.rank);
     });
     std::vector<JoinTable> tab(1);
     JoinTable& t = tab[0];
@@ -2675,6 +2871,13 @@ int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
     t.sub[nu] = (uint16_t)nj;
     t.start[nj] = (uint16_t)v.size();
     for (; bucket <= (1u << kDirBits); bucket++) t.dir[bucket] = (uint16_t)nu;
+    for (uint32_t u = 0; go && u < nu; u++)
+        ctx->join_longest[dead] = std::max<uint32_t>(ctx->join_longest[dead], t.start[t.sub[u + 1]] - t.start[t.sub[u]]);
+    if (!ctx->join_lines[dead].p) {
+        TRY(ensure(ctx, ctx->join_lines[dead], 64 * kNumInsns * sizeof(uint32_t)));
+        k_line_hash<<<(64 * kNumInsns + 255) / 256, 256, 0, ctx->stream>>>(dead, (uint32_t*)ctx->join_lines[dead].p);
+        CKL("k_line_hash");
+    }
     if (!go) {
         uint16_t at = 0;
         for (const auto& e : groups) {
@@ -2687,9 +2890,6 @@ int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
                 for (uint32_t b = t.cand[i] >> 12; b <= 2; b++) t.weight[u][b - 1] += gr.mult[t.cand[i] & 0xFFFu];
         TRY(ensure(ctx, ctx->join_groups[dead], sizeof gr));
         CK(cudaMemcpy(ctx->join_groups[dead].p, &gr, sizeof gr, cudaMemcpyHostToDevice));
-        TRY(ensure(ctx, ctx->join_lines[dead], 64 * kNumInsns * sizeof(uint32_t)));
-        k_line_hash<<<(64 * kNumInsns + 255) / 256, 256, 0, ctx->stream>>>(dead, (uint32_t*)ctx->join_lines[dead].p);
-        CKL("k_line_hash");
     }
     TRY(ensure(ctx, ctx->join_tab[go][dead], sizeof t));
     CK(cudaMemcpy(ctx->join_tab[go][dead].p, &t, sizeof t, cudaMemcpyHostToDevice));
@@ -2715,13 +2915,28 @@ int cand2_table(m6502_ctx* ctx, uint32_t dead, m6502_ctx::Cand2Table** out) {
         CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, (const uint64_t*)nullptr, (uint64_t*)nullptr,
                                            (const uint32_t*)nullptr, (uint32_t*)nullptr, (int)n, 0, 64, ctx->stream));
         TRY(ensure(ctx, ctx->c2_sort_tmp, tb));
-        k_cand2_keys<<<ctx->sms * 8, 256, 0, ctx->stream>>>(dead, (uint64_t*)ctx->c2_keys_in.p,
-                                                            (uint32_t*)ctx->c2_idx_in.p);
-        CKL("k_cand2_keys");
-        tb = ctx->c2_sort_tmp.bytes;
-        CK(cub::DeviceRadixSort::SortPairs(ctx->c2_sort_tmp.p, tb, (const uint64_t*)ctx->c2_keys_in.p,
-                                           (uint64_t*)slot->keys.p, (const uint32_t*)ctx->c2_idx_in.p,
-                                           (uint32_t*)slot->idx.p, (int)n, 0, 64, ctx->stream));
+        TRY(ensure(ctx, slot->pw, (size_t)n * sizeof(uint2)));
+        TRY(ensure(ctx, ctx->opflag, 2 * sizeof(uint32_t)));
+        uint32_t info[2] = {1, 0};
+        for (int attempt = 0; info[0]; attempt++) {   // two sets of outputs with one 64-bit key: another salt
+            if (attempt == 8) return set_err(ctx, M6502_E_CUDA, "no salt separates the length-2 candidates");
+            slot->salt = 0x9E3779B97F4A7C15ull * (uint64_t)attempt;
+            k_cand2_keys<<<ctx->sms * 8, 256, 0, ctx->stream>>>(dead, slot->salt, (uint64_t*)ctx->c2_keys_in.p,
+                                                                (uint32_t*)ctx->c2_idx_in.p);
+            CKL("k_cand2_keys");
+            tb = ctx->c2_sort_tmp.bytes;
+            CK(cub::DeviceRadixSort::SortPairs(ctx->c2_sort_tmp.p, tb, (const uint64_t*)ctx->c2_keys_in.p,
+                                               (uint64_t*)slot->keys.p, (const uint32_t*)ctx->c2_idx_in.p,
+                                               (uint32_t*)slot->idx.p, (int)n, 0, 64, ctx->stream));
+            CK(cudaMemsetAsync(ctx->opflag.p, 0, 2 * sizeof(uint32_t), ctx->stream));
+            k_cand2_info<<<ctx->sms * 8, 256, 0, ctx->stream>>>(dead, (const uint64_t*)slot->keys.p,
+                                                                (const uint32_t*)slot->idx.p, (uint2*)slot->pw.p,
+                                                                (uint32_t*)ctx->opflag.p);
+            CKL("k_cand2_info");
+            CK(cudaMemcpyAsync(info, ctx->opflag.p, sizeof info, cudaMemcpyDeviceToHost, ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
+        }
+        slot->longest = info[1];
         slot->dead = dead;
     }
     slot->stamp = ++ctx->cand2_clock;
@@ -2772,14 +2987,16 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         if (!scan) TRY(ensure(ctx, ctx->match, nt * sizeof(Surv)));
         TRY(ensure(ctx, ctx->items, icap * sizeof(Item)));
         TRY(ensure(ctx, ctx->rules, rcap * sizeof(m6502_rule)));
-        if (go) TRY(ensure(ctx, ctx->best, 2 * nt * sizeof(uint32_t)));
-        int end_bit = 30;   // Go-order sort keys: target << 30 | pass << 29 | rank
-        while (end_bit < 63 && (nt >> (end_bit - 30)) != 0) end_bit++;
-        if (rounds) {
-            TRY(ensure(ctx, ctx->go_keys, scap * 8));
-            TRY(ensure(ctx, ctx->go_keys2, scap * 8));
+        if (go) {
+            TRY(ensure(ctx, ctx->best, 2 * nt * sizeof(uint32_t)));
             TRY(ensure(ctx, ctx->go_ord, scap * 4));
             TRY(ensure(ctx, ctx->go_round, scap * sizeof(Surv)));
+        }
+        int end_bit = 30;   // Go-order sort keys: target << 30 | pass << 29 | rank
+        while (end_bit < 63 && (nt >> (end_bit - 30)) != 0) end_bit++;
+        if (rounds && scan) {
+            TRY(ensure(ctx, ctx->go_keys, scap * 8));
+            TRY(ensure(ctx, ctx->go_keys2, scap * 8));
             size_t tb = 0;
             CK(cub::DeviceRadixSort::SortKeys(nullptr, tb, (const uint64_t*)nullptr, (uint64_t*)nullptr, (int)scap, 0,
                                               end_bit, ctx->stream));
@@ -2820,55 +3037,54 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         CKL("k_qc1");
         CK(rec(ctx->sev[2]));
         SurvSource src{(const Surv*)ctx->surv.p, d_targets, tlen, dead, go ? 1 : 0, mult};
-        ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, cfg.sweep, cfg.exh_mode == M6502_EXH_BRUTE};
-        // Go-order verification rounds over the survivors in ctx->surv; on
-        // return `best` holds the first passing candidate per target and pass.
-        // Go-order verification rounds over the survivors in ctx->surv, queued
-        // with no read-back: the survivors are sorted over the buffer's whole
-        // capacity (entries past the device's count get a key that sorts last),
-        // and every round a group of `bound` candidates could need is launched;
-        // a round past the largest ordinal finds nothing to do.  On return
-        // `best` holds the first passing candidate per target and pass; the
-        // rounds' pair and item counts are summed on the device.
-        auto go_rounds = [&](uint64_t bound) -> int {
-            const uint64_t pad = (1ull << end_bit) - 1;   // above every real key (target < nt)
-            k_go_keys<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const Surv*)ctx->surv.p, &cnt->surv, scap, pad,
-                                                             (uint64_t*)ctx->go_keys.p);
-            CKL("k_go_keys");
-            size_t tb = ctx->go_sort_tmp.bytes;
-            CK(cub::DeviceRadixSort::SortKeys(ctx->go_sort_tmp.p, tb, (const uint64_t*)ctx->go_keys.p,
-                                              (uint64_t*)ctx->go_keys2.p, (int)scap, 0, end_bit, ctx->stream));
-            CK(cudaMemsetAsync(&cnt->max_ord, 0, sizeof(unsigned long long), ctx->stream));
-            k_go_ord<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const uint64_t*)ctx->go_keys2.p, &cnt->surv, scap,
-                                                            (uint32_t*)ctx->go_ord.p, cnt);
-            CKL("k_go_ord");
+        ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, &cnt->v[0][0], cfg.sweep,
+                   cfg.exh_mode == M6502_EXH_BRUTE};
+        // Go-order verification rounds of a phase, queued with no read-back: the
+        // first round's list is in ctx->go_round and the later survivors in
+        // ctx->surv with their ordinals (after a scan: all of them in ctx->surv,
+        // to be sorted, over the buffer's whole capacity; entries past the
+        // device's count get a key that sorts last).  Every round that a range of
+        // `bound` candidates could need is launched.  On return `best` holds the
+        // first passing candidate per target and pass.
+        auto go_rounds = [&](int phase, uint64_t bound) -> int {
+            const bool sorted = scan && phase == 0;
+            if (sorted) {
+                const uint64_t pad = (1ull << end_bit) - 1;   // above every real key (target < nt)
+                k_go_keys<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const Surv*)ctx->surv.p, &cnt->surv, scap, pad,
+                                                                 (uint64_t*)ctx->go_keys.p);
+                CKL("k_go_keys");
+                size_t tb = ctx->go_sort_tmp.bytes;
+                CK(cub::DeviceRadixSort::SortKeys(ctx->go_sort_tmp.p, tb, (const uint64_t*)ctx->go_keys.p,
+                                                  (uint64_t*)ctx->go_keys2.p, (int)scap, 0, end_bit, ctx->stream));
+                k_go_ord<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const uint64_t*)ctx->go_keys2.p, &cnt->surv, scap,
+                                                                (Surv*)ctx->surv.p, (uint32_t*)ctx->go_ord.p, cnt);
+                CKL("k_go_ord");
+            }
             SurvSource rs{(const Surv*)ctx->go_round.p, d_targets, tlen, dead, 1, nullptr};
-            for (uint64_t lo = 0, blk = 64; lo < bound; lo += blk, blk = std::min<uint64_t>(blk * 4, 1ull << 22)) {
-                const uint64_t hi = std::min<uint64_t>(lo + blk, 0xFFFFFFFFull);
-                CK(cudaMemsetAsync(&cnt->round_n, 0, sizeof(unsigned long long), ctx->stream));
-                k_go_round<<<ctx->sms * 8, 256, 0, ctx->stream>>>(
-                    (const uint64_t*)ctx->go_keys2.p, (const uint32_t*)ctx->go_ord.p, &cnt->surv, scap, (uint32_t)lo,
-                    (uint32_t)hi, (const uint32_t*)ctx->best.p, (uint32_t)nt, (Surv*)ctx->go_round.p, cnt);
-                CKL("k_go_round");
-                // exhaustive tickets, work items and item tickets restart each round
-                CK(cudaMemsetAsync(&cnt->exh_ticket, 0, kVerifyCounters * sizeof(unsigned long long), ctx->stream));
-                ExhArgs ra{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, cfg.sweep,
+            int r = 0;
+            for (uint64_t lo = 0, blk = kGoBlock; lo < bound; lo += blk, blk *= 8, r++) {
+                VerifyCounters* v = &cnt->v[phase][r];
+                if (r > 0 || sorted) {
+                    k_go_round<<<ctx->sms * 8, 256, 0, ctx->stream>>>(
+                        (const Surv*)ctx->surv.p, (const uint32_t*)ctx->go_ord.p, &cnt->surv, scap, (uint32_t)lo,
+                        (uint32_t)(lo + blk), (const uint32_t*)ctx->best.p, (uint32_t)nt, (Surv*)ctx->go_round.p, cnt, v);
+                    CKL("k_go_round");
+                }
+                ExhArgs ra{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, v, cfg.sweep,
                            cfg.exh_mode == M6502_EXH_BRUTE};
-                TRY(launch_exh(ctx, rs, &cnt->round_n, scap, ra));
+                TRY(launch_exh(ctx, rs, &v->n, scap, ra));
                 TRY(launch_items(ctx, rs, ra));
-                k_go_select<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const Surv*)ctx->go_round.p, &cnt->round_n, scap,
+                k_go_select<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const Surv*)ctx->go_round.p, &v->n, scap,
                                                                    (const uint32_t*)ctx->fail.p, (uint32_t)nt,
                                                                    (uint32_t*)ctx->best.p, cnt, d_targets, tlen,
                                                                    cfg.sweep);
                 CKL("k_go_select");
-                k_go_tally<<<1, 1, 0, ctx->stream>>>(cnt);
-                CKL("k_go_tally");
             }
             return M6502_OK;
         };
         if (go) CK(cudaMemsetAsync(ctx->best.p, 0xFF, 2 * nt * sizeof(uint32_t), ctx->stream));
         if (exh && !rounds) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea));
-        if (rounds) TRY(go_rounds(kNumInsns));   // a target has at most 2,863 length-1 candidates
+        if (rounds) TRY(go_rounds(0, scan ? (uint64_t)kNumInsns : ctx->join_longest[dead]));
         CK(rec(ctx->sev[3]));
         if (exh && !rounds) TRY(launch_items(ctx, src, ea));
         CK(rec(ctx->sev[4]));
@@ -2899,30 +3115,34 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
             // phase are checked once, after the pass.
             k_mark_phase<<<1, 1, 0, ctx->stream>>>(cnt);
             CKL("k_mark_phase");
-            // survivor and verification counters restart for this phase
-            CK(cudaMemsetAsync(&cnt->surv, 0, (1 + kVerifyCounters) * sizeof(unsigned long long), ctx->stream));
+            CK(cudaMemsetAsync(&cnt->surv, 0, kPhaseCounters * sizeof(unsigned long long), ctx->stream));
             CK(rec(ctx->sev2[0]));
             const uint32_t jgrid2 =
                 (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 8, (nt + kWarpsPerBlock - 1) / kWarpsPerBlock);
             const uint32_t n2 = (uint32_t)kNumInsns * (uint32_t)kNumInsns;
-            CK(cudaMemsetAsync(&cnt->join_items, 0, sizeof(unsigned long long), ctx->stream));
-            Join2Args ja{(const uint64_t*)ctx->tfp.p, (const uint8_t*)ctx->tmeta.p, (uint32_t)nt,
-                         (const uint64_t*)c2->keys.p, (const uint32_t*)c2->idx.p, (const uint64_t*)c2e->keys.p,
-                         (const uint32_t*)c2e->idx.p, n2, dead, stages, go ? (const uint32_t*)ctx->best.p : nullptr,
-                         (Surv*)ctx->surv.p, scap, (JoinItem*)ctx->jitems.p, jcap, cnt};
+            auto view = [](const m6502_ctx::Cand2Table* t) {
+                return Cand2View{(const uint64_t*)t->keys.p, (const uint32_t*)t->idx.p, (const uint2*)t->pw.p, t->salt};
+            };
+            Join2Args ja{(const uint64_t*)ctx->tfp.p, (const uint8_t*)ctx->tmeta.p, (uint32_t)nt, view(c2), view(c2e), n2,
+                         dead, stages, go ? (const uint32_t*)ctx->best.p : nullptr, (Surv*)ctx->surv.p, scap,
+                         (JoinItem*)ctx->jitems.p, jcap, cnt, (Surv*)ctx->go_round.p, (uint32_t*)ctx->go_ord.p,
+                         rounds ? kGoBlock : 0u};
             if (go) {
-                k_qc_join2<true><<<jgrid2, 256, 0, ctx->stream>>>(ja);
-                k_qc_join2_items<true><<<ctx->sms * 8, 256, 0, ctx->stream>>>(ja);
+                k_go_join2<<<jgrid2, 256, 0, ctx->stream>>>(ja);
+                k_go_join2_count<<<ctx->sms * 8, 256, 0, ctx->stream>>>(ja);
+                k_go_join2_items<<<ctx->sms * 8, 256, 0, ctx->stream>>>(ja);
             } else {
-                k_qc_join2<false><<<jgrid2, 256, 0, ctx->stream>>>(ja);
-                k_qc_join2_items<false><<<ctx->sms * 8, 256, 0, ctx->stream>>>(ja);
+                k_qc_join2<<<jgrid2, 256, 0, ctx->stream>>>(ja);
+                k_qc_join2_items<<<ctx->sms * 8, 256, 0, ctx->stream>>>(ja);
             }
             CKL("k_qc_join2");
             CK(rec(ctx->sev2[1]));
-            if (exh && !rounds) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea));
-            if (rounds) TRY(go_rounds((uint64_t)kNumInsns * kNumInsns));
+            ExhArgs ea2 = ea;
+            ea2.v = &cnt->v[1][0];
+            if (exh && !rounds) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea2));
+            if (rounds) TRY(go_rounds(1, std::max(c2->longest, c2e->longest)));
             CK(rec(ctx->sev2[2]));
-            if (exh && !rounds) TRY(launch_items(ctx, src, ea));
+            if (exh && !rounds) TRY(launch_items(ctx, src, ea2));
             CK(rec(ctx->sev2[3]));
             TRY(select_or_emit());
             CK(rec(ctx->sev2[4]));
@@ -2995,11 +3215,23 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         bool redo = false;
         CK(cudaMemcpyAsync(&hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        // A first phase that overflowed leaves targets open that it would have
-        // settled: what the second phase then asked for says nothing.
-        const bool first_over = phase2 && hc.surv1 > scap;
-        const uint64_t surv_need = first_over ? hc.surv1 : std::max<uint64_t>(hc.surv, hc.surv_need);
-        const uint64_t items_need = first_over ? hc.items1 : std::max<uint64_t>(hc.items, hc.items_need);
+        uint64_t surv_need = std::max<uint64_t>(hc.surv1, phase2 ? 0 : hc.surv), items_need = 0, listed = 0, items = 0;
+        bool first_over = false;
+        for (int ph = 0; ph < 2; ph++) {
+            if (ph == 1) {
+                // A first phase that overflowed leaves targets open that it would
+                // have settled: what the second phase then asked for says nothing.
+                first_over = surv_need > scap;
+                if (first_over) break;
+                if (phase2) surv_need = std::max<uint64_t>(surv_need, hc.surv);
+            }
+            for (const VerifyCounters& v : hc.v[ph]) {
+                surv_need = std::max<uint64_t>(surv_need, v.n);
+                items_need = std::max<uint64_t>(items_need, v.items);
+                listed += v.n;
+                items += v.items;
+            }
+        }
         if (surv_need > scap) { scap = surv_need + surv_need / 4 + 1024; redo = true; }
         if (items_need > icap) { icap = items_need + items_need / 4 + 1024; redo = true; }
         if (hc.rules > rlim && !count_only) { rcap = hc.rules + hc.rules / 4 + 1024; redo = true; }
@@ -3018,11 +3250,11 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
             st->pairs += nt * ((uint64_t)kNumInsns + (phase2 ? (uint64_t)kNumInsns * kNumInsns : 0u));
             st->qc_hits += hc.qc;
             st->mid_hits += hc.mid;
-            st->exh_checked += !exh ? 0 : rounds ? hc.round_checked : hc.mid;
+            st->exh_checked += !exh ? 0 : rounds ? listed + hc.round_rejects : hc.mid;
             st->exh_passed += hc.exh_pass;
             st->rules += hc.rules;
             st->exh_states += hc.states;
-            st->exh_items += rounds ? hc.round_items : hc.items + hc.items1;
+            st->exh_items += items;
             st->exh_algo_ops += hc.algo;
             st->exh_probe_rejects += hc.probe_rejects;
             st->exh_undecided += hc.undecided;
@@ -3122,7 +3354,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 }
                 CK(rec(ev[2]));
                 SurvSource src{(const Surv*)ctx->surv.p, d_t, tlen, dead, 0, groups ? groups->mult : nullptr};
-                ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, cfg.sweep,
+                ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, &cnt->v[0][0], cfg.sweep,
                            cfg.exh_mode == M6502_EXH_BRUTE};
                 if (exh) TRY(launch_exh(ctx, src, &cnt->surv, scap, ea));
                 CK(rec(ev[3]));
@@ -3187,7 +3419,8 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
         bool redo = false;
         for (const Counters& c : hc) {
             if (c.surv > scap) { scap = std::max<uint64_t>(scap, c.surv + c.surv / 4 + 1024); redo = true; }
-            if (c.items > icap) { icap = std::max<uint64_t>(icap, c.items + c.items / 4 + 1024); redo = true; }
+            const uint64_t items = c.v[0][0].items;
+            if (items > icap) { icap = std::max<uint64_t>(icap, items + items / 4 + 1024); redo = true; }
         }
         const uint64_t nrules = hc[0].rules;
         if (nrules > rcap && !count_only) { rcap = nrules + nrules / 4 + 1024; redo = true; }
@@ -3218,7 +3451,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 st->exh_checked += exh ? c.mid : 0;   // every MidCheck survivor, the join's probe included
                 st->exh_passed += c.exh_pass;
                 st->exh_states += c.states;
-                st->exh_items += c.items;
+                st->exh_items += c.v[0][0].items;
                 st->exh_algo_ops += c.algo;
                 st->exh_probe_rejects += c.probe_rejects;
                 st->exh_undecided += c.undecided;
@@ -3448,6 +3681,7 @@ void m6502_destroy(m6502_ctx* ctx) {
     for (auto& t : ctx->cand2) {
         if (t.keys.p) cudaFree(t.keys.p);
         if (t.idx.p) cudaFree(t.idx.p);
+        if (t.pw.p) cudaFree(t.pw.p);
     }
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
@@ -3503,14 +3737,16 @@ int m6502_check_pairs(m6502_ctx* ctx, uint64_t n, const uint16_t* t_insns, const
             CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), ctx->stream));
             unsigned long long hn = n;
             CK(cudaMemcpyAsync(&cnt->surv, &hn, sizeof hn, cudaMemcpyHostToDevice, ctx->stream));
-            ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, sweep, exh_mode == M6502_EXH_BRUTE};
+            ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, &cnt->v[0][0], sweep,
+                       exh_mode == M6502_EXH_BRUTE};
             TRY(launch_verify(ctx, src, &cnt->surv, n, ea));
             Counters hc;
             CK(cudaMemcpyAsync(&hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
-            if (hc.items <= icap) break;
+            const uint64_t items = hc.v[0][0].items;
+            if (items <= icap) break;
             if (attempt >= 4) return set_err(ctx, M6502_E_NOMEM, "work-item queue kept overflowing");
-            icap = hc.items + hc.items / 4 + 1024;
+            icap = items + items / 4 + 1024;
         }
         fl.resize(n * 4);
         CK(cudaMemcpyAsync(fl.data(), ctx->fail.p, n * 4, cudaMemcpyDeviceToHost, ctx->stream));

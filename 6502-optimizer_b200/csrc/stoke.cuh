@@ -739,11 +739,11 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
             for (int attempt = 0;; attempt++) {
                 TRY(ensure(ctx, ctx->items, icap * sizeof(Item)));
                 CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), ctx->stream));
-                ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, cfg->sweep, 0,
+                ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, &cnt->v[0][0], cfg->sweep, 0,
                            phase == 0 ? kStokeDeferBits : 0u};
                 TRY(launch_verify(ctx, src, &sc->round_n, ecap, ea));
                 unsigned long long items = 0;
-                CK(cudaMemcpyAsync(&items, &cnt->items, sizeof items, cudaMemcpyDeviceToHost, ctx->stream));
+                CK(cudaMemcpyAsync(&items, &cnt->v[0][0].items, sizeof items, cudaMemcpyDeviceToHost, ctx->stream));
                 CK(cudaStreamSynchronize(ctx->stream));
                 if (items <= icap) break;
                 if (attempt >= 4) return set_err(ctx, M6502_E_NOMEM, "work-item queue kept overflowing");
