@@ -109,6 +109,7 @@ __constant__ uint16_t c_gotab[kNumInsns];     // instructions, Go order
 __constant__ uint32_t c_gorank[kNumInsns];    // Go-order rank of CUDA index i
 __constant__ uint16_t c_goidx[kNumInsns];     // CUDA index of Go rank r
 __constant__ uint32_t c_rep[32];
+__device__ uint4 g_x4row[NUM_OPS * 3];        // X4Row by opcode (the STOKE chains' executor)
 
 // Packed-executor descriptor of an instruction (an opcode outside the table
 // runs as NOP, as exec leaves the state unchanged for it).
@@ -2550,7 +2551,7 @@ struct m6502_ctx {
     DevBuf st_tins, st_toffs, st_tout, st_tbytes, st_chains, st_entries, st_vidx, st_proven, st_cnt, st_pidx,
         st_mex, st_probs, st_traj, st_row;
     DevBuf st_keys, st_keys2, st_vals2, st_rep, st_ord, st_verdict, st_vlist, st_vpos, st_sort_tmp, st_vphase,
-        st_pphase;
+        st_pphase, st_live, st_rounds, st_proven_was;
 };
 
 namespace {
@@ -2738,6 +2739,10 @@ int init_ctx(m6502_ctx* ctx) {
     uint32_t x4[NUM_OPS];
     for (uint32_t op = 0; op < NUM_OPS; op++) x4[op] = x4_desc(op);
     CK(cudaMemcpyToSymbol(c_x4d, x4, sizeof x4));
+    X4Row rows[NUM_OPS];
+    static_assert(sizeof(X4Row) == 3 * sizeof(uint4), "three words of 16 bytes");
+    for (uint32_t op = 0; op < NUM_OPS; op++) rows[op] = x4_row(op);
+    CK(cudaMemcpyToSymbol(g_x4row, rows, sizeof rows));
     CK(cudaMemcpyToSymbol(c_tab, tab, sizeof tab));
     CK(cudaMemcpyToSymbol(c_gotab, gotab, sizeof gotab));
     CK(cudaMemcpyToSymbol(c_gorank, gorank, sizeof gorank));
@@ -3670,6 +3675,7 @@ void m6502_destroy(m6502_ctx* ctx) {
                       &ctx->st_vlist, &ctx->st_vpos, &ctx->st_sort_tmp, &ctx->c2_keys_in, &ctx->c2_idx_in,
                       &ctx->c2_sort_tmp, &ctx->go_keys, &ctx->go_keys2, &ctx->go_ord, &ctx->go_round,
                       &ctx->go_sort_tmp, &ctx->jitems, &ctx->cnt_slots, &ctx->st_vphase, &ctx->st_pphase,
+                      &ctx->st_live, &ctx->st_rounds, &ctx->st_proven_was,
                       &ctx->tall, &ctx->opflag, &ctx->order, &ctx->match};
     for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
     for (cudaEvent_t e : ctx->sev) if (e) cudaEventDestroy(e);

@@ -476,6 +476,98 @@ M6502_HD void exec_x4d(St& s, uint32_t insn, uint32_t d) {
     }
 }
 
+// ---- Four states per register by table, without branches ----
+//
+// exec_x4r runs an instruction from a row of masks (x4_row): its operands are
+// read from and its result written to an array of registers (slot i at
+// st[i * stride]), and one adder, one logic unit and one right shift are
+// computed for every instruction, of which the row keeps one.  Only the stack
+// instructions and BIT branch.  For lanes that run different instructions.
+// Results equal exec_x4's (tests/x4r_check.cpp checks every instruction).
+enum : uint32_t { X4S_A, X4S_X, X4S_Y, X4S_S, X4S_M, X4S_S0, X4S_S1, X4S_NONE, X4S_COUNT };
+enum : uint32_t { X4C_IMM = 1u << 9, X4C_DUP = 1u << 10, X4C_ADD = 1u << 11, X4C_RIGHT = 1u << 12, X4C_KIND = 13 };
+struct X4Row {
+    uint32_t ctl;       // slots of a (bits 0-2), m (3-5) and the result (6-8), X4C_*, kind of the branching ones (13-15)
+    uint32_t konst;     // added to the operand word (INC, DEC)
+    uint32_t pad[2];
+    uint32_t keep, upd, set;   // P: bits kept, taken from the new flags, set
+    uint32_t inv;       // operand inverted
+    uint32_t ka, k1, k2;       // logic unit: ((a & ka) & m & k1) | (((a & ka) ^ m) & k2)
+    uint32_t carry;     // per byte: bit 0 carry in from C, bit 1 carry in 1, bit 7 right shift takes C
+};
+
+M6502_HD X4Row x4_row(uint32_t op) {
+    const uint32_t d = x4_desc(op), src = (d >> 4) & 7u, dst = (d >> 7) & 7u, sub = (d >> 10) & 3u;
+    const uint32_t all = 0xFFFFFFFFu, nz = (kFlagN | kFlagZ) * kB1, nzc = nz | kFlagC * kB1;
+    X4Row r{X4S_NONE << 6, 0, {0, 0}, all, 0, 0, 0, 0, 0, 0, 0};
+    // The register numbers of x4_desc (A X Y S M, 7 = immediate) are the slots'.
+    auto ctl = [&](uint32_t a, uint32_t m, uint32_t out) {
+        r.ctl = a | (m == X4R_IMM ? X4C_IMM : m << 3) | out << 6;
+    };
+    auto flags = [&](uint32_t u) { r.upd = u; r.keep = ~u; };
+    switch (d & 15u) {
+    case X4_MOVE_NZ: ctl(0, src, dst); r.k2 = all; flags(nz); break;
+    case X4_MOVE: ctl(0, src, dst); r.k2 = all; break;
+    case X4_INCDEC: ctl(dst, X4R_IMM, dst); r.ctl |= X4C_ADD; r.konst = sub ? all : kB1; flags(nz); break;
+    case X4_SHIFT:
+        ctl(dst, 0, dst);
+        r.ctl |= (sub & 1u) ? X4C_RIGHT : X4C_ADD | X4C_DUP;   // left: a + a
+        if (sub == 2) r.carry = kB1;
+        if (sub == 3) r.carry = kH;
+        flags(nzc);
+        break;
+    case X4_FLAG: r.keep = ~(((d >> 16) & 0xFFu) * kB1); r.set = (d >> 24) * kB1; break;
+    case X4_ADDSUB: ctl(X4S_A, src, X4S_A); r.ctl |= X4C_ADD; r.inv = sub ? all : 0; r.carry = kB1; flags(nzc | kFlagV * kB1); break;
+    case X4_LOGIC: ctl(X4S_A, src, X4S_A); r.ka = all; r.k1 = sub < 2 ? all : 0; r.k2 = sub ? all : 0; flags(nz); break;
+    case X4_CMP: ctl(dst, src, X4S_NONE); r.ctl |= X4C_ADD; r.inv = all; r.carry = 2 * kB1; flags(nzc); break;
+    case X4_PUSH: r.ctl |= (sub ? 2u : 1u) << X4C_KIND; break;
+    case X4_PLA: r.ctl |= 3u << X4C_KIND; break;
+    case X4_PLP: r.ctl |= 4u << X4C_KIND; break;
+    case X4_BIT: r.ctl |= 5u << X4C_KIND; break;
+    default: break;
+    }
+    return r;
+}
+
+// One instruction (insn = op | imm << 8, q = x4_row(op)) on the four states
+// in st and p.
+M6502_HD void exec_x4r(uint32_t* st, int stride, uint32_t& p, const X4Row& q, uint32_t insn) {
+    const uint32_t a = st[(q.ctl & 7u) * stride], mr = st[((q.ctl >> 3) & 7u) * stride];
+    const uint32_t m = (q.ctl & X4C_IMM) ? (insn >> 8) * kB1 + q.konst : mr;
+    const uint32_t b = (q.ctl & X4C_DUP) ? a : m ^ q.inv;
+    uint32_t co;
+    const uint32_t sum = x4_add(a, b, (p & q.carry & kB1) | ((q.carry >> 1) & kB1), co);
+    const uint32_t al = a & q.ka;
+    const uint32_t logic = (al & m & q.k1) | ((al ^ m) & q.k2);
+    const uint32_t right = ((a >> 1) & kL7) | ((p << 7) & q.carry & kH);
+    const bool add = (q.ctl & X4C_ADD) != 0, rs = (q.ctl & X4C_RIGHT) != 0;
+    const uint32_t r = add ? sum : rs ? right : logic;
+    const uint32_t c = rs ? a & kB1 : co;
+    const uint32_t v = ((a ^ r) & (b ^ r) & kH) >> 1;
+    const uint32_t was = p;
+    p = (p & q.keep) | ((x4_nzf(r) | c | v) & q.upd) | q.set;
+    st[((q.ctl >> 6) & 7u) * stride] = r;
+    const uint32_t kind = q.ctl >> X4C_KIND;
+    if (kind) {
+        uint32_t &ra = st[X4S_A * stride], &rsp = st[X4S_S * stride], &s0 = st[X4S_S0 * stride], &s1 = st[X4S_S1 * stride];
+        if (kind <= 2) {   // PHA, PHP
+            s1 = s0;
+            s0 = kind == 1 ? ra : was | (kFlagB | kFlagU) * kB1;
+            rsp = x4_dec(rsp);
+        } else if (kind <= 4) {   // PLA, PLP
+            const uint32_t t = s0;
+            s0 = s1;
+            s1 = 0;
+            rsp = x4_inc(rsp);
+            if (kind == 3) { ra = t; p = (was & (0x7Du * kB1)) | x4_nzf(t); }
+            else p = t;
+        } else {           // BIT
+            const uint32_t w = st[X4S_M * stride];
+            p = (was & (0x3Du * kB1)) | (w & (0xC0u * kB1)) | (x4_zero(ra & w) >> 6);
+        }
+    }
+}
+
 M6502_HD uint64_t pack(const St& s) {
     return (uint64_t)(s.a | (s.x << 8) | (s.y << 16) | (s.p << 24)) |
            ((uint64_t)(s.s | (s.m << 8) | (s.s0 << 16) | (s.s1 << 24)) << 32);

@@ -5,10 +5,10 @@
 // The reference runs one goroutine per MCMC chain (pkg/stoke/search.go:88-163):
 // mutate (mutator.go:30-115), cost on the test vectors (cost.go:32-81),
 // Metropolis accept with T *= decay (mcmc.go:51-81), and ExhaustiveCheck of
-// every shorter zero-mismatch best (search.go:102-155).  Here one warp runs
-// one chain: all 32 lanes draw the same random numbers (one splitmix64 state
-// per chain, so the control flow is warp-uniform), lane v evaluates the
-// candidate on test vector v, and the cost is a warp reduction.  Chains run in
+// every shorter zero-mismatch best (search.go:102-155).  Here eight lanes run
+// one chain: they draw the same random numbers (one splitmix64 state per
+// chain), each evaluates the candidate on four of the test vectors, and the
+// cost is a reduction over them.  Chains run in
 // epochs of S steps; after each epoch the shorter zero-cost bests found during
 // it are checked on all 32 vectors and proved by the exhaustive kernels, and
 // the chains of proven targets restart (the reference's NewChain) or stop.
@@ -43,6 +43,7 @@ struct StokeCounters {
     unsigned long long round_n;   // pairs verified in the current round
     unsigned long long verified;  // pairs verified this epoch (all rounds)
     unsigned long long ex_rows;   // chains given a row of the learned proposal this epoch
+    unsigned long long live;      // chains still searching this epoch
 };
 
 constexpr uint32_t kVerifyBatch = 8;   // distinct candidates per target per round under stop_on_proof
@@ -89,68 +90,33 @@ struct StokeParams {
     uint64_t traj_cap;
 };
 
-__device__ __forceinline__ uint64_t sm_next(uint64_t& x) {
-    uint64_t z = (x += 0x9E3779B97F4A7C15ull);
+constexpr uint64_t kSmStep = 0x9E3779B97F4A7C15ull;
+__device__ __forceinline__ uint64_t sm_mix(uint64_t z) {
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
     return z ^ (z >> 31);
 }
-// Uniform integer in [0, n): high half of a 32x32 product (bias < n / 2^32).
-__device__ __forceinline__ uint32_t sm_below(uint64_t& x, uint32_t n) {
-    return (uint32_t)(((sm_next(x) >> 32) * (uint64_t)n) >> 32);
-}
-__device__ __forceinline__ float sm_unit(uint64_t& x) { return (float)(sm_next(x) >> 40) * (1.0f / 16777216.0f); }
-
-// randomInstruction (mutator.go:108-115): opcode uniform over the 58 opcodes,
-// immediate uniform over 0..255 when the opcode takes one.
-__device__ __forceinline__ uint16_t random_insn(uint64_t& rng) {
-    uint32_t op = sm_below(rng, NUM_OPS);
-    uint32_t imm = has_imm(op) ? sm_below(rng, 256) : 0u;
-    return (uint16_t)(op | (imm << 8));
-}
-
-// Cost of the sequence in seq[0..len) against the target outputs `tv` (this
-// lane's vector).  COST_REF: 1000 x mismatching QC vectors + bytes +
-// cycles / 100 (cost.go:32-81); COST_HAMMING: differing output bits over the
-// 32 vectors + bytes + cycles / 100.  `zero` is true when no vector differs.
-__device__ __forceinline__ int32_t stoke_cost(const uint16_t* seq, int len, uint64_t tv, uint64_t mask,
-                                              uint32_t mode, int lane, bool& zero, uint32_t& vmask) {
-    St s = unpack(c_vec[lane]);
-    for (int i = 0; i < len; i++) exec(s, seq[i]);
-    const uint64_t x = (fp_of(s) ^ tv) & mask;
-    uint32_t b = 0, c = 0;
-    if (lane < len) { b = bytes_go(seq[lane] & 0xFFu); c = cycles(seq[lane] & 0xFFu); }
-    b = __reduce_add_sync(kFull, b);
-    c = __reduce_add_sync(kFull, c);
-    int32_t base = (int32_t)(b + c / 100u);
-    vmask = __ballot_sync(kFull, x != 0);
-    if (mode == M6502_COST_REF) {
-        unsigned mism = __ballot_sync(kFull, x != 0) & 0xFFu;
-        zero = mism == 0;
-        return 1000 * __popc(mism) + base;
-    }
-    uint32_t h = __reduce_add_sync(kFull, (uint32_t)__popcll(x));
-    zero = h == 0;
-    return (int32_t)h + base;
-}
+__device__ __forceinline__ uint64_t sm_next(uint64_t& x) { return sm_mix(x += kSmStep); }
+// Uniform integer in [0, n) from the top half of a draw: high half of a
+// 32x32 product (bias < n / 2^32).
+__device__ __forceinline__ uint32_t below(uint32_t top, uint32_t n) { return __umulhi(top, n); }
+__device__ __forceinline__ float unit(uint32_t top) { return (float)(top >> 8) * (1.0f / 16777216.0f); }
+__device__ __forceinline__ uint32_t sm_below(uint64_t& x, uint32_t n) { return below((uint32_t)(sm_next(x) >> 32), n); }
+__device__ __forceinline__ float sm_unit(uint64_t& x) { return unit((uint32_t)(sm_next(x) >> 32)); }
 
 // Index drawn from one head of a chain's cumulative distribution (entries
 // [a, b) of the chain's row in shared memory hold running sums): the first
 // entry above a uniform point of the head's range (the last one if rounding
-// leaves none).  Warp-collective, two ballots: lane i tests the last entry
-// of block i (blocks of ceil((b - a) / 32) entries), then the lanes of the
-// first block above the point test its entries.
-__device__ __forceinline__ int cdf_sample(const float* cdf, int a, int b, uint64_t& rng, int lane) {
+// leaves none).
+__device__ __forceinline__ int cdf_sample(const float* cdf, int a, int b, uint64_t& rng) {
     const float base = a > 0 ? cdf[a - 1] : 0.0f;
     const float r = base + sm_unit(rng) * (cdf[b - 1] - base);
-    const int n = b - a, bs = (n + 31) >> 5;
-    const int last = min((lane + 1) * bs, n) - 1;
-    const unsigned above = __ballot_sync(kFull, lane * bs < n && cdf[a + last] > r);
-    if (!above) return n - 1;
-    const int blk = __ffs(above) - 1;
-    const int j = blk * bs + lane;
-    const unsigned in = __ballot_sync(kFull, lane < bs && j < n && cdf[a + j] > r);
-    return in ? blk * bs + __ffs(in) - 1 : min((blk + 1) * bs, n) - 1;
+    int lo = a, hi = b - 1;   // the answer lies in [lo, hi]
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cdf[mid] > r) hi = mid; else lo = mid + 1;
+    }
+    return lo - a;
 }
 
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;
@@ -205,121 +171,256 @@ __global__ void k_cdf(float* __restrict__ p, uint32_t n) {
     }
 }
 
-// One epoch of every chain: warp per chain.
-__global__ void __launch_bounds__(256) k_stoke_epoch(StokeChain* __restrict__ chains, uint32_t n_chains,
+// The chains still searching, listed (their order does not matter: a chain's
+// course depends on its own state alone); chains of proved targets stop.
+__global__ void k_stoke_live(StokeChain* __restrict__ chains, uint32_t n_chains, uint32_t cpt,
+                             const uint32_t* __restrict__ proven, uint32_t stop_on_proof, uint32_t* __restrict__ list,
+                             StokeCounters* __restrict__ sc) {
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n_chains; base += gridDim.x * blockDim.x) {
+        const uint32_t ci = base + threadIdx.x;
+        bool live = ci < n_chains && chains[ci].status != 2;
+        if (live && stop_on_proof && proven[ci / cpt]) {
+            chains[ci].status = 2;
+            live = false;
+        }
+        const unsigned vote = __ballot_sync(kFull, live);
+        const int lane = threadIdx.x & 31;
+        unsigned long long b = 0;
+        if (lane == 0 && vote) b = atomicAdd(&sc->live, (unsigned long long)__popc(vote));
+        b = __shfl_sync(kFull, b, 0) + __popc(vote & ((1u << lane) - 1u));
+        if (live) list[b] = ci;
+    }
+}
+
+__device__ __forceinline__ X4Row load_row(const uint4 (&q)[3]) {
+    const uint4 a = q[0], b = q[1], c = q[2];
+    return X4Row{a.x, a.y, {0, 0}, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+}
+// One epoch of the listed chains: eight lanes per chain, up to four chains per
+// warp.  Lane `sub` of a chain runs the candidate on vectors 4 sub .. 4 sub +
+// 3, packed in one word per register; the chain's random numbers are drawn by
+// all its lanes alike.  Cost of a candidate: COST_REF: 1000 x mismatching QC
+// vectors + bytes + cycles / 100 (cost.go:32-81); COST_HAMMING: differing
+// output bits over the 32 vectors + bytes + cycles / 100.
+// Bound by issue and by each chain's serial steps.  A warp per chain paid the
+// random numbers, the mutation and the acceptance (two thirds of its
+// instructions) for one chain; here up to four chains pay them together,
+// written without branches on the kind of move and with the table-driven
+// executor (four opcodes in a warp: one course instead of four arms of the
+// switch; 21.3 -> 20.1 ms for the whole run).  A warp's steps are a serial
+// chain at seven cycles per instruction, so few chains spread over more warps
+// first (kEpochWarps: three per scheduler; 20.1 ms, with four 20.7, six 23.4),
+// and only listed chains get a warp: the ones of a proved target lie together
+// and left some SMs idle, others twice as busy.
+// 256 targets x 128 chains x 4,000 steps: all epochs 20.3 -> 11.4 ms.
+constexpr int kEpochChains = 8;               // chains per block of 64 threads, at most
+constexpr uint32_t kEpochWarps = 148 * 4 * 3;
+__global__ void __launch_bounds__(64) k_stoke_epoch(StokeChain* __restrict__ chains, const uint32_t* __restrict__ list,
                                                       StokeTargets tg, StokeParams prm,
                                                       StokeEntry* __restrict__ entries, uint64_t ecap,
                                                       StokeCounters* __restrict__ sc) {
-    __shared__ uint16_t s_buf[kWarpsPerBlock][2][kMaxSeq];
-    __shared__ uint16_t s_best[kWarpsPerBlock][kMaxSeq];
-    __shared__ float s_cdf[kWarpsPerBlock][330];   // the chain's learned distributions, staged once
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t ci = blockIdx.x * kWarpsPerBlock + (uint32_t)w;
-    if (ci >= n_chains) return;
+    __shared__ uint16_t s_seq[kEpochChains][3][kMaxSeq];   // two candidates in turn, the best
+    __shared__ float s_cdf[kEpochChains][330];             // the chain's learned distributions, staged once
+    __shared__ uint8_t s_size[64];                         // bytes | cycles << 4 by opcode
+    __shared__ uint4 s_row[NUM_OPS][3];                    // X4Row by opcode
+    __shared__ uint32_t s_st[X4S_COUNT][64];               // each lane's registers
+    for (int i = threadIdx.x; i < (int)NUM_OPS * 3; i += 64) (&s_row[0][0])[i] = g_x4row[i];
+    if (threadIdx.x < 64)
+        s_size[threadIdx.x] = (uint8_t)(bytes_go(threadIdx.x) | cycles(threadIdx.x) << 4);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, sub = lane & 7, g = threadIdx.x >> 3, shift = lane & 24;
+    const unsigned gmask = 0xFFu << shift;   // the chain's lanes
+    const uint32_t live = (uint32_t)sc->live;
+    const uint32_t per = min(4u, (live + kEpochWarps - 1) / kEpochWarps);   // chains per warp
+    const uint32_t li = (blockIdx.x * 2u + (threadIdx.x >> 5)) * per + (uint32_t)(lane >> 3);
+    const bool on = (uint32_t)(lane >> 3) < per && li < live;
+    if (!__any_sync(kFull, on)) return;
+    const uint32_t ci = list[on ? li : 0];
     StokeChain& ch = chains[ci];
-    const uint32_t t = ci / prm.chains_per_target;
-    uint32_t status = ch.status;
-    if (prm.stop_on_proof && prm.proven[t]) status = 2;
-    if (status == 2) {
-        if (lane == 0) ch.status = 2;
-        return;
-    }
+    const uint32_t t = ci / prm.chains_per_target, status = ch.status;
     const uint32_t t0 = tg.off[t], tlen = tg.off[t + 1] - t0;
-    const uint64_t tv = tg.out[(uint64_t)t * 32 + lane];
     const uint32_t tbytes = tg.bytes[t];
-    const uint64_t mask = cmp_mask(prm.dead);
+    const uint32_t pm = (kPMask & ~prm.dead & 0xFFu) * kB1;
     const int max_len = (int)(prm.max_len ? prm.max_len : max(tlen + 2u, 10u));
-    uint16_t* cur = s_buf[w][0];
-    uint16_t* cand = s_buf[w][1];
-    uint16_t* best = s_best[w];
-    int len, best_len;
-    int32_t cost, best_cost;
-    float temp;
-    uint64_t rng, step = ch.step, since = ch.since;
-    uint32_t accepted = 0, diff = 0;
-    bool zero;
-    const uint32_t crow = prm.cdf ? prm.row[ci] : kNoRow;
-    const float* cdf = nullptr;
-    if (crow != kNoRow) {   // uniform
-        const float* g = prm.cdf + (size_t)crow * 330;
-        for (int i = lane; i < 330; i += 32) s_cdf[w][i] = g[i];
-        __syncwarp();
-        cdf = s_cdf[w];
+    uint16_t *cur = s_seq[g][0], *cand = s_seq[g][1], *best = s_seq[g][2];
+    const int p0 = sub, p1 = sub + 8;   // the two positions this lane moves
+    // this lane's four vectors and the target's outputs on them
+    const uint32_t* vw = c_vec4[sub];
+    const St vin{vw[0], vw[1], vw[2], vw[3], vw[4], vw[5], vw[6], vw[7]};
+    St want{0, 0, 0, 0, 0, 0, 0, 0};
+    for (int k = 0; k < 4; k++) {
+        const St o = unpack(tg.out[(uint64_t)t * 32 + 4 * sub + k]);
+        want.a |= o.a << (8 * k); want.x |= o.x << (8 * k); want.y |= o.y << (8 * k); want.p |= o.p << (8 * k);
+        want.s |= o.s << (8 * k); want.m |= o.m << (8 * k); want.s0 |= o.s0 << (8 * k); want.s1 |= o.s1 << (8 * k);
     }
-    if (status == 0) {   // NewChain (mcmc.go:28-49): start from the target
-        if (lane < (int)tlen) { cur[lane] = tg.ins[t0 + lane]; best[lane] = cur[lane]; }
-        __syncwarp();
-        len = best_len = (int)tlen;
-        rng = prm.seed + (uint64_t)ci * 0x9E3779B97F4A7C15ull + step;
-        temp = prm.t_start;
-        since = 0;
-        cost = best_cost = stoke_cost(cur, len, tv, mask, prm.cost_mode, lane, zero, diff);
-
-    } else {
-        if (lane < kMaxSeq) { cur[lane] = ch.cur[lane]; best[lane] = ch.best[lane]; }
-        __syncwarp();
-        len = ch.len; best_len = ch.best_len;
-        cost = ch.cost; best_cost = ch.best_cost;
-        temp = ch.temp; rng = ch.rng;
-        diff = ch.diff;
+    // Cost of seq[0..n): every lane of the chain gets it; `zero`: no vector
+    // differs; `vm`: the vectors that do.  All chains of the warp call it together.
+    auto cost_of = [&](const uint16_t* seq, int n, bool& zero, uint32_t& vm, uint32_t& size) -> int32_t {
+        uint32_t* st = &s_st[0][threadIdx.x];
+        st[X4S_A * 64] = vin.a; st[X4S_X * 64] = vin.x; st[X4S_Y * 64] = vin.y; st[X4S_S * 64] = vin.s;
+        st[X4S_M * 64] = vin.m; st[X4S_S0 * 64] = vin.s0; st[X4S_S1 * 64] = vin.s1;
+        uint32_t p = vin.p, insn = seq[0];
+        X4Row row = load_row(s_row[min(insn & 0xFFu, NUM_OPS - 1u)]);
+        for (int i = 0; i < n; i++) {
+            const uint32_t next = seq[min(i + 1, kMaxSeq - 1)];   // it and its row in flight while this one runs
+            const X4Row next_row = load_row(s_row[min(next & 0xFFu, NUM_OPS - 1u)]);
+            exec_x4r(st, 64, p, row, insn);
+            insn = next;
+            row = next_row;
+        }
+        const St s{st[X4S_A * 64], st[X4S_X * 64], st[X4S_Y * 64], p, st[X4S_S * 64], st[X4S_M * 64], st[X4S_S0 * 64],
+                   st[X4S_S1 * 64]};
+        const uint32_t da = s.a ^ want.a, dx = s.x ^ want.x, dy = s.y ^ want.y, dp = (s.p ^ want.p) & pm, ds = s.s ^ want.s,
+                       dm = s.m ^ want.m, d0 = s.s0 ^ want.s0, d1 = s.s1 ^ want.s1;
+        const uint32_t differ = ~x4_zero(da | dx | dy | dp | ds | dm | d0 | d1) & kH;   // 0x80 in the bytes that do
+        uint32_t v = ((differ >> 7) * 0x10204080u) >> 28;                               // their four bits, gathered
+        v <<= 4 * sub;
+        const uint32_t h = (uint32_t)(__popc(da) + __popc(dx) + __popc(dy) + __popc(dp) + __popc(ds) + __popc(dm) +
+                                      __popc(d0) + __popc(d1));
+        const uint32_t z0 = p0 < n ? s_size[seq[p0] & 63u] : 0u, z1 = p1 < n ? s_size[seq[p1] & 63u] : 0u;
+        uint32_t sum = h | ((z0 & 15u) + (z1 & 15u)) << 12 | ((z0 >> 4) + (z1 >> 4)) << 20;   // no field overflows in 8 lanes
+        for (int o = 1; o < 8; o <<= 1) {
+            sum += __shfl_xor_sync(kFull, sum, o);
+            v |= __shfl_xor_sync(kFull, v, o);
+        }
+        vm = v;
+        size = (sum >> 12) & 0xFFu;
+        const int32_t base = (int32_t)(size + (sum >> 20) / 100u);
+        if (prm.cost_mode == M6502_COST_REF) {
+            zero = (v & 0xFFu) == 0;
+            return 1000 * __popc(v & 0xFFu) + base;
+        }
+        zero = (sum & 0xFFFu) == 0;
+        return (int32_t)(sum & 0xFFFu) + base;
+    };
+    int len = 0, best_len = 0;
+    int32_t cost = 0, best_cost = 0;
+    float temp = 0.0f;
+    uint64_t rng = 0, step = ch.step, since = ch.since;
+    uint32_t accepted = 0, diff = 0, size = 0;
+    bool zero = false;
+    const uint32_t crow = on && prm.cdf ? prm.row[ci] : kNoRow;
+    const float* cdf = nullptr;
+    if (crow != kNoRow) {
+        const float* r = prm.cdf + (size_t)crow * 330;
+        for (int i = sub; i < 330; i += 8) s_cdf[g][i] = r[i];
+        cdf = s_cdf[g];
+    }
+    const bool fresh = on && status == 0;   // NewChain (mcmc.go:28-49): start from the target
+    for (int p = p0; p < kMaxSeq; p += 8) {
+        const uint16_t c = fresh ? (p < (int)tlen ? tg.ins[t0 + p] : (uint16_t)0) : ch.cur[p];
+        cur[p] = c;
+        cand[p] = 0;
+        best[p] = fresh ? c : ch.best[p];
+    }
+    __syncwarp();
+    {
+        const int32_t c0 = cost_of(cur, fresh ? (int)tlen : 0, zero, diff, size);
+        if (fresh) {
+            len = best_len = (int)tlen;
+            rng = prm.seed + (uint64_t)ci * 0x9E3779B97F4A7C15ull + step;
+            temp = prm.t_start;
+            since = 0;
+            cost = best_cost = c0;
+        } else if (on) {
+            len = ch.len; best_len = ch.best_len;
+            cost = ch.cost; best_cost = ch.best_cost;
+            temp = ch.temp; rng = ch.rng;
+            diff = ch.diff;
+        }
     }
     for (uint32_t it = 0; it < prm.steps; it++, step++, since++) {
         // Mutate (mutator.go:30-44): replace 40%, swap 20%, delete 20%,
         // insert 10%, change immediate 10%.
-        const uint32_t r = sm_below(rng, 100);
+        // The generator's next values do not depend on each other: the five
+        // that a step can use are computed side by side.
+        uint32_t z[5];
+#pragma unroll
+        for (int k = 0; k < 5; k++) z[k] = (uint32_t)(sm_mix(rng + (uint64_t)(k + 1) * kSmStep) >> 32);
+        const uint32_t r = below(z[0], 100);
+        uint32_t unit_z;   // the value the acceptance draws if it needs one
         int kind = r < 40 ? 0 : r < 60 ? 1 : r < 80 ? 2 : r < 90 ? 3 : 4;
-        int nlen = len, pos = 0;
-        uint16_t ins = 0;
         if (kind == 3 && len >= max_len) kind = 0;              // InsertInstruction falls back
-        if (kind == 4) {
-            const unsigned immpos = __ballot_sync(kFull, lane < len && has_imm(cur[lane] & 0xFFu));
-            if (!immpos) kind = 0;                                // ChangeImmediate falls back
-            else {
-                uint32_t j = sm_below(rng, (uint32_t)__popc(immpos));
-                unsigned m = immpos;
-                for (uint32_t q = 0; q < j; q++) m &= m - 1;
-                pos = __ffs(m) - 1;
-                ins = (uint16_t)((cur[pos] & 0xFFu) | (sm_below(rng, 256) << 8));
-            }
+        uint32_t immpos = 0;                                    // positions with an operand
+        if (__any_sync(kFull, kind == 4)) {
+            const unsigned b0 = __ballot_sync(kFull, p0 < len && has_imm(cur[p0] & 0xFFu));
+            const unsigned b1 = __ballot_sync(kFull, p1 < len && has_imm(cur[p1] & 0xFFu));
+            immpos = ((b0 >> shift) & 0xFFu) | ((b1 >> shift) & 0xFFu) << 8;
+            if (kind == 4 && !immpos) kind = 0;                 // ChangeImmediate falls back
         }
-        const bool learned = cdf && (kind == 0 || kind == 3) && sm_unit(rng) < prm.learned_frac;
+        int pos = 0;
+        uint32_t op = 0, imm = 0;
+        const bool fresh_insn = kind == 0 || kind == 3;
+        bool learned = false;
+        if (cdf && fresh_insn) learned = unit(z[1]) < prm.learned_frac;
         if (learned) {   // position, opcode, operand from the model's distributions
+            rng += 2 * kSmStep;
             const int lim = kind == 0 ? len : len + 1;
-            pos = cdf_sample(cdf, 0, 16, rng, lane);
+            pos = cdf_sample(cdf, 0, 16, rng);
             if (pos >= lim) pos = (int)sm_below(rng, (uint32_t)lim);
-            const uint32_t op = (uint32_t)cdf_sample(cdf, 16, 74, rng, lane);
-            const uint32_t imm = has_imm(op) ? (uint32_t)cdf_sample(cdf, 74, 330, rng, lane) : 0u;
-            ins = (uint16_t)(op | (imm << 8));
-            if (kind == 3) nlen = len + 1;
+            op = (uint32_t)cdf_sample(cdf, 16, 74, rng);
+            imm = has_imm(op) ? (uint32_t)cdf_sample(cdf, 74, 330, rng) : 0u;
+            unit_z = (uint32_t)(sm_mix(rng + kSmStep) >> 32);
+        } else {         // uniform: position, then opcode over the 58, then operand (mutator.go:108-115), as far as the move has them
+            if (cdf && fresh_insn) {   // one value went to the choice above
+                rng += kSmStep;
+                z[1] = z[2]; z[2] = z[3]; z[3] = z[4];
+                z[4] = (uint32_t)(sm_mix(rng + 5 * kSmStep) >> 32);
+            }
+            const uint32_t places = kind == 4 ? (uint32_t)__popc(immpos) : (uint32_t)(kind == 3 ? len + 1 : kind == 1 ? len - 1 : len);
+            const bool placed = kind == 1 || kind == 2 ? len > 1 : true;
+            uint32_t used = 1;
+            if (placed) { pos = (int)below(z[1], places); used = 2; }
+            if (fresh_insn) { op = below(z[2], NUM_OPS); used = 3; }
+            if (kind == 4) {
+                uint32_t m = immpos;
+                for (int q = 0; q < pos; q++) m &= m - 1;
+                pos = __ffs(m) - 1;
+                op = cur[pos] & 0xFFu;
+            }
+            unit_z = used == 1 ? z[1] : used == 2 ? z[2] : z[3];
+            if ((fresh_insn || kind == 4) && has_imm(op)) {
+                imm = below(unit_z, 256);
+                unit_z = used == 2 ? z[3] : z[4];
+                used++;
+            }
+            rng += used * kSmStep;
         }
-        else if (kind == 0) { pos = (int)sm_below(rng, (uint32_t)len); ins = random_insn(rng); }
-        else if (kind == 1) { if (len >= 2) pos = (int)sm_below(rng, (uint32_t)(len - 1)); }
-        else if (kind == 2) { if (len > 1) { pos = (int)sm_below(rng, (uint32_t)len); nlen = len - 1; } }
-        else if (kind == 3) { pos = (int)sm_below(rng, (uint32_t)(len + 1)); ins = random_insn(rng); nlen = len + 1; }
-        if (lane < kMaxSeq) {
-            uint16_t v = cur[lane];
-            if (kind == 0 || kind == 4) v = lane == pos ? ins : cur[lane];
-            else if (kind == 1 && len >= 2) v = lane == pos ? cur[pos + 1] : (lane == pos + 1 ? cur[pos] : cur[lane]);
-            else if (kind == 2 && len > 1) v = lane < pos ? cur[lane] : (lane + 1 < kMaxSeq ? cur[lane + 1] : 0);
-            else if (kind == 3) v = lane < pos ? cur[lane] : (lane == pos ? ins : cur[lane - 1]);
-            cand[lane] = v;
+        const uint16_t ins = (uint16_t)(op | imm << 8);
+        const bool moved = kind == 1 ? len >= 2 : kind == 2 ? len > 1 : true;
+        const int nlen = kind == 3 ? len + 1 : kind == 2 && moved ? len - 1 : len;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int p = k ? p1 : p0;
+            int q = p;   // the position the instruction comes from
+            if (kind == 1 && moved) q = p == pos ? p + 1 : p == pos + 1 ? p - 1 : p;
+            if (kind == 2 && moved) q = p < pos ? p : p + 1;
+            if (kind == 3) q = p <= pos ? p : p - 1;
+            uint16_t v = q < kMaxSeq ? cur[q] : (uint16_t)0;
+            if ((kind == 0 || kind >= 3) && p == pos) v = ins;
+            cand[p] = v;
         }
         __syncwarp();
         uint32_t ndiff;
-        const int32_t ncost = stoke_cost(cand, nlen, tv, mask, prm.cost_mode, lane, zero, ndiff);
+        const int32_t ncost = cost_of(cand, on ? nlen : 0, zero, ndiff, size);
         // Metropolis accept (mcmc.go:51-81)
         const int32_t delta = ncost - cost;
         bool acc = delta <= 0;
-        if (!acc && temp > 0.0f) acc = sm_unit(rng) < __expf(-(float)delta / temp);
+        if (!acc && temp > 0.0f) {
+            rng += kSmStep;
+            acc = unit(unit_z) < __expf(-(float)delta / temp);
+        }
+        acc = acc && on;
         if (acc && prm.traj && delta < 0 && (kind == 0 || kind == 3)) {   // an improving move: training example
             unsigned long long e = 0;
-            if (lane == 0) e = atomicAdd(&sc->traj, 1ull);
-            e = __shfl_sync(kFull, e, 0);
+            if (sub == 0) e = atomicAdd(&sc->traj, 1ull);
+            e = __shfl_sync(gmask, e, shift);
             if (e < prm.traj_cap) {
                 m6502_mlp_example& x = prm.traj[e];
-                if (lane < 8) x.target[lane] = lane < (int)tlen ? tg.ins[t0 + lane] : 0;
-                if (lane < 16) x.cand[lane] = lane < len ? cur[lane] : 0;
-                if (lane == 0) {
+                x.target[sub] = sub < (int)tlen ? tg.ins[t0 + sub] : 0;
+                x.cand[p0] = p0 < len ? cur[p0] : 0;
+                x.cand[p1] = p1 < len ? cur[p1] : 0;
+                if (sub == 0) {
                     x.diff = diff; x.tlen = (uint8_t)min(tlen, 8u); x.clen = (uint8_t)len;
                     x.pos = (uint8_t)pos; x.op = (uint8_t)(ins & 0xFFu); x.imm = (uint8_t)(ins >> 8);
                     x.weight = 1;
@@ -333,20 +434,19 @@ __global__ void __launch_bounds__(256) k_stoke_epoch(StokeChain* __restrict__ ch
             cost = ncost;
             accepted++;
             if (ncost < best_cost) {
-                if (lane < kMaxSeq) best[lane] = cur[lane];
-                __syncwarp();
+                best[p0] = cur[p0];
+                best[p1] = cur[p1];
                 best_len = len;
                 best_cost = ncost;
                 // verification trigger (search.go:101): zero mismatches and shorter
-                uint32_t bb = (lane < best_len) ? bytes_go(best[lane] & 0xFFu) : 0u;
-                bb = __reduce_add_sync(kFull, bb);
-                if (zero && bb < tbytes) {
+                if (zero && size < tbytes) {
                     unsigned long long e = 0;
-                    if (lane == 0) e = atomicAdd(&sc->entries, 1ull);
-                    e = __shfl_sync(kFull, e, 0);
+                    if (sub == 0) e = atomicAdd(&sc->entries, 1ull);
+                    e = __shfl_sync(gmask, e, shift);
                     if (e < ecap) {
-                        if (lane < kMaxSeq) entries[e].ins[lane] = best[lane];
-                        if (lane == 0) {
+                        entries[e].ins[p0] = cur[p0];
+                        entries[e].ins[p1] = cur[p1];
+                        if (sub == 0) {
                             entries[e].chain = ci; entries[e].target = t; entries[e].step = step;
                             entries[e].len = (uint8_t)best_len; entries[e].dead_flags = 0;
                         }
@@ -357,8 +457,10 @@ __global__ void __launch_bounds__(256) k_stoke_epoch(StokeChain* __restrict__ ch
         temp *= prm.decay;
         __syncwarp();
     }
-    if (lane < kMaxSeq) { ch.cur[lane] = cur[lane]; ch.best[lane] = best[lane]; }
-    if (lane == 0) {
+    if (!on) return;
+    ch.cur[p0] = cur[p0]; ch.cur[p1] = cur[p1];
+    ch.best[p0] = best[p0]; ch.best[p1] = best[p1];
+    if (sub == 0) {
         ch.len = (uint8_t)len; ch.best_len = (uint8_t)best_len;
         ch.cost = cost; ch.best_cost = best_cost;
         ch.temp = temp; ch.rng = rng; ch.step = step; ch.since = since;
@@ -592,6 +694,8 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
     TRY(ensure(ctx, ctx->fail, ecap * 4));
     TRY(ensure(ctx, ctx->order, ecap * 4));
     TRY(ensure(ctx, ctx->st_proven, (size_t)n_targets * 4));
+    TRY(ensure(ctx, ctx->st_live, (size_t)n_chains * 4));
+    TRY(ensure(ctx, ctx->st_proven_was, (size_t)n_targets * 4));
     TRY(ensure(ctx, ctx->st_cnt, sizeof(StokeCounters)));
     TRY(ensure(ctx, ctx->st_pidx, ecap * 4));
     TRY(ensure(ctx, ctx->st_keys, ecap * 8));
@@ -689,8 +793,13 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
                 prm.row = (const uint32_t*)ctx->st_row.p;
             }
         }
-        k_stoke_epoch<<<(n_chains + kWarpsPerBlock - 1) / kWarpsPerBlock, 256, 0, ctx->stream>>>(
-            (StokeChain*)ctx->st_chains.p, n_chains, tg, prm, (StokeEntry*)ctx->st_entries.p, ecap, sc);
+        k_stoke_live<<<std::min<uint32_t>((n_chains + 255) / 256, (uint32_t)ctx->sms * 8), 256, 0, ctx->stream>>>(
+            (StokeChain*)ctx->st_chains.p, n_chains, cpt, (const uint32_t*)ctx->st_proven.p, cfg->stop_on_proof,
+            (uint32_t*)ctx->st_live.p, sc);
+        CKL("k_stoke_live");
+        const uint32_t eblocks = std::max<uint32_t>(std::min<uint32_t>(kEpochWarps, n_chains) / 2 + 1,
+                                                    (n_chains + kEpochChains - 1) / kEpochChains);
+        k_stoke_epoch<<<eblocks, 64, 0, ctx->stream>>>((StokeChain*)ctx->st_chains.p, (const uint32_t*)ctx->st_live.p, tg, prm, (StokeEntry*)ctx->st_entries.p, ecap, sc);
         CKL("k_stoke_epoch");
         CK(cudaEventRecord(ctx->sev[1], ctx->stream));
         k_stoke_vectors<<<ctx->sms * 8, 256, 0, ctx->stream>>>((StokeEntry*)ctx->st_entries.p, ecap, tg,
@@ -715,7 +824,6 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
                                                         (const StokeEntry*)ctx->st_entries.p, (uint32_t*)ctx->st_rep.p,
                                                         (uint32_t*)ctx->st_ord.p, sc);
             CKL("k_stoke_dedupe");
-            CK(cudaMemsetAsync(ctx->st_verdict.p, 0xFF, (size_t)n_ok * 4, ctx->stream));
             CK(cudaMemcpyAsync(&hv, sc, sizeof hv, cudaMemcpyDeviceToHost, ctx->stream));
             CK(cudaStreamSynchronize(ctx->stream));
             max_ord = (uint32_t)hv.max_ord;
@@ -726,9 +834,13 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
         // pairs whose cones stay within 2^kStokeDeferBits states.  Phase 1:
         // the deferred pairs of targets still unproved.  Proofs of phase 0 are
         // timed at its end, so one expensive pair does not delay the rest.
-        const uint32_t batch = cfg->stop_on_proof ? kVerifyBatch : 0xFFFFFFFFu;
         StokeSource src{(const StokeEntry*)ctx->st_entries.p, (const uint32_t*)ctx->st_vlist.p, tg, cfg->dead_flags};
-        auto verify_round = [&](uint32_t lo, uint32_t hi, uint32_t phase) -> int {
+        // The rounds of an epoch are queued with no read-back in between, each
+        // with its own counters; the host looks at their work items once, and
+        // only if a round's did not fit is the epoch's verification run again
+        // with a larger queue, from the targets proved before it.
+        const uint32_t n_rounds = !n_ok ? 0u : cfg->stop_on_proof ? max_ord / kVerifyBatch + 1u : 1u;
+        auto verify_round = [&](uint32_t lo, uint32_t hi, uint32_t phase, VerifyCounters* v) -> int {
             CK(cudaMemsetAsync(&sc->round_n, 0, sizeof(unsigned long long), ctx->stream));
             k_stoke_select<<<ctx->sms * 4, 256, 0, ctx->stream>>>(
                 (const uint64_t*)ctx->st_keys2.p, (const uint32_t*)ctx->st_vals2.p, (const uint32_t*)ctx->st_rep.p,
@@ -736,32 +848,46 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
                 (const uint32_t*)ctx->st_verdict.p, phase, (uint32_t*)ctx->st_vlist.p, (uint32_t*)ctx->st_vpos.p,
                 sc);
             CKL("k_stoke_select");
-            for (int attempt = 0;; attempt++) {
-                TRY(ensure(ctx, ctx->items, icap * sizeof(Item)));
-                CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), ctx->stream));
-                ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, &cnt->v[0][0], cfg->sweep, 0,
-                           phase == 0 ? kStokeDeferBits : 0u};
-                TRY(launch_verify(ctx, src, &sc->round_n, ecap, ea));
-                unsigned long long items = 0;
-                CK(cudaMemcpyAsync(&items, &cnt->v[0][0].items, sizeof items, cudaMemcpyDeviceToHost, ctx->stream));
-                CK(cudaStreamSynchronize(ctx->stream));
-                if (items <= icap) break;
-                if (attempt >= 4) return set_err(ctx, M6502_E_NOMEM, "work-item queue kept overflowing");
-                icap = items + items / 4 + 1024;
-            }
+            ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, v, cfg->sweep, 0,
+                       phase == 0 ? kStokeDeferBits : 0u};
+            TRY(launch_verify(ctx, src, &sc->round_n, ecap, ea));
             k_stoke_verdicts<<<ctx->sms * 4, 256, 0, ctx->stream>>>(
                 (const uint32_t*)ctx->fail.p, (const uint32_t*)ctx->st_vpos.p, (const uint64_t*)ctx->st_keys2.p,
                 (uint32_t*)ctx->st_verdict.p, (uint8_t*)ctx->st_vphase.p, phase, (uint32_t*)ctx->st_proven.p, sc);
             CKL("k_stoke_verdicts");
             return M6502_OK;
         };
-        for (uint32_t lo = 0; n_ok && lo <= max_ord; lo = (batch > 0xFFFFFFFFu - lo) ? 0xFFFFFFFFu : lo + batch) {
-            const uint32_t hi = batch > 0xFFFFFFFFu - lo ? 0xFFFFFFFFu : lo + batch;
-            TRY(verify_round(lo, hi, 0));
-            if (hi == 0xFFFFFFFFu) break;
+        for (int attempt = 0;; attempt++) {
+            if (n_rounds) {
+                TRY(ensure(ctx, ctx->items, icap * sizeof(Item)));
+                TRY(ensure(ctx, ctx->st_rounds, ((size_t)n_rounds + 1) * sizeof(VerifyCounters)));
+                CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), ctx->stream));
+                CK(cudaMemsetAsync(ctx->st_rounds.p, 0, ((size_t)n_rounds + 1) * sizeof(VerifyCounters), ctx->stream));
+                CK(cudaMemsetAsync(ctx->st_verdict.p, 0xFF, (size_t)n_ok * 4, ctx->stream));
+                CK(cudaMemcpyAsync(ctx->st_proven_was.p, ctx->st_proven.p, (size_t)n_targets * 4, cudaMemcpyDeviceToDevice,
+                                   ctx->stream));
+            }
+            VerifyCounters* v = (VerifyCounters*)ctx->st_rounds.p;
+            for (uint32_t r = 0; r < n_rounds; r++)
+                TRY(verify_round(r * (cfg->stop_on_proof ? kVerifyBatch : 0u),
+                                 cfg->stop_on_proof ? (r + 1) * kVerifyBatch : 0xFFFFFFFFu, 0, v + r));
+            CK(cudaEventRecord(ctx->sev[3], ctx->stream));   // phase-0 proofs are complete here
+            if (!n_rounds) break;
+            TRY(verify_round(0, 0, 1, v + n_rounds));
+            std::vector<VerifyCounters> hr((size_t)n_rounds + 1);
+            CK(cudaMemcpyAsync(hr.data(), ctx->st_rounds.p, hr.size() * sizeof(VerifyCounters), cudaMemcpyDeviceToHost,
+                               ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
+            uint64_t items = 0;
+            for (const VerifyCounters& c : hr) items = std::max<uint64_t>(items, c.items);
+            if (items <= icap) break;
+            if (attempt >= 4) return set_err(ctx, M6502_E_NOMEM, "work-item queue kept overflowing");
+            icap = items + items / 4 + 1024;
+            CK(cudaMemcpyAsync(ctx->st_proven.p, ctx->st_proven_was.p, (size_t)n_targets * 4, cudaMemcpyDeviceToDevice,
+                               ctx->stream));
+            CK(cudaMemsetAsync(&sc->undecided, 0, sizeof(unsigned long long), ctx->stream));
+            CK(cudaMemsetAsync(&sc->verified, 0, sizeof(unsigned long long), ctx->stream));
         }
-        CK(cudaEventRecord(ctx->sev[3], ctx->stream));   // phase-0 proofs are complete here
-        if (n_ok) TRY(verify_round(0, 0, 1));
         if (n_ok) {
             k_stoke_collect<<<ctx->sms * 4, 256, 0, ctx->stream>>>(
                 (const uint32_t*)ctx->st_vals2.p, (const uint32_t*)ctx->st_rep.p, (const uint32_t*)ctx->st_verdict.p,
