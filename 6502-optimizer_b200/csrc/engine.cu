@@ -109,6 +109,7 @@ __constant__ uint16_t c_gotab[kNumInsns];     // instructions, Go order
 __constant__ uint32_t c_gorank[kNumInsns];    // Go-order rank of CUDA index i
 __constant__ uint16_t c_goidx[kNumInsns];     // CUDA index of Go rank r
 __constant__ uint32_t c_rep[32];
+__device__ uint4 g_dep16[NUM_OPS * 2];         // c_dep padded to 16 entries per opcode, for copies into shared memory
 __device__ uint4 g_x4row[NUM_OPS * 3];        // X4Row by opcode (the STOKE chains' executor)
 
 // Packed-executor descriptor of an instruction (an opcode outside the table
@@ -845,7 +846,7 @@ __device__ Groups make_groups(const Flow& fl, uint32_t dead, bool rep, bool brut
 // so only the locations that feed another one (`cross`, a few per
 // instruction) are fetched from their lanes.
 __device__ __forceinline__ uint32_t compose_s(uint32_t D, const uint16_t* seq, int n, int lane, uint32_t& written,
-                                              uint32_t& sweep, const uint16_t (*dep_tab)[NUM_LOCS]) {
+                                              uint32_t& sweep, const uint16_t (*dep_tab)[16]) {
     for (int i = 0; i < n; i++) {
         uint32_t op = seq[i] & 0xFFu;
         uint32_t dep = (lane < NUM_LOCS) ? dep_tab[op][lane] : 0u;
@@ -866,7 +867,7 @@ __device__ __forceinline__ uint32_t compose_s(uint32_t D, const uint16_t* seq, i
 // The same composition with the target's half kept in the warp's cache:
 // pairs of one target (consecutive survivors) compose only their candidate.
 // The two halves are independent: each starts from the identity.
-__device__ __forceinline__ Flow dataflow_cached(const PairView& pv, int lane, const uint16_t (*dep_tab)[NUM_LOCS],
+__device__ __forceinline__ Flow dataflow_cached(const PairView& pv, int lane, const uint16_t (*dep_tab)[16],
                                                 uint64_t tid, TargetCache& tc) {
     const uint32_t id = (lane < NUM_LOCS) ? (1u << lane) : 0u;
     uint32_t dt, wt, st;
@@ -1850,8 +1851,8 @@ template <class Src, int MINB = 4>
 __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigned long long* n_pairs_ptr,
                                                         uint64_t n_cap, ExhArgs a) {
     __shared__ uint16_t s_t[kWarpsPerBlock][kMaxSeq], s_c[kWarpsPerBlock][kMaxSeq];
-    __shared__ uint16_t s_dep[NUM_OPS][NUM_LOCS];
-    for (int i = threadIdx.x; i < NUM_OPS * NUM_LOCS; i += blockDim.x) (&s_dep[0][0])[i] = (&c_dep[0][0])[i];
+    __shared__ alignas(16) uint16_t s_dep[NUM_OPS][16];
+    for (int i = threadIdx.x; i < (int)NUM_OPS * 2; i += blockDim.x) reinterpret_cast<uint4*>(&s_dep[0][0])[i] = g_dep16[i];
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t n = min((uint64_t)*n_pairs_ptr, n_cap);
@@ -1861,7 +1862,11 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
     if ((threadIdx.x & 31) == 0) { tc.probe_id = kNoTarget; tc.flow_id = kNoTarget; }
     __syncwarp();
     unsigned long long next = 0, lim = 0;   // this warp's batch of tickets
-    const unsigned long long tbatch = a.ticket_batch ? a.ticket_batch : kTicketBatch;
+    // Pairs per ticket: the knob's, but no more than leaves every warp one (few
+    // large pairs in the hands of one warp: 185 us for the 1,000 that k_small
+    // leaves of a pass of 2 M length-2 targets, one at a time 43).
+    const unsigned long long share = n / ((uint64_t)gridDim.x * kWarpsPerBlock);
+    const unsigned long long tbatch = max(1ull, min(share, (unsigned long long)(a.ticket_batch ? a.ticket_batch : kTicketBatch)));
     const uint64_t chunk_min = a.chunk_log2 ? (1ull << a.chunk_log2) : kChunk;
     // Lane 0 claims the following batch while the warp works on the current
     // one, so the atomic's latency is hidden behind a batch of pairs.
@@ -1987,8 +1992,8 @@ template <class Src>
 __global__ void __launch_bounds__(256) k_small(Src src, const unsigned long long* n_pairs_ptr, uint64_t n_cap,
                                                ExhArgs a, uint32_t* __restrict__ order) {
     __shared__ uint16_t s_ins[Src::kMaxT + Src::kMaxC][256];
-    __shared__ uint16_t s_dep[NUM_OPS][16];
-    for (int i = threadIdx.x; i < NUM_OPS * NUM_LOCS; i += blockDim.x) s_dep[i / NUM_LOCS][i % NUM_LOCS] = c_dep[i / NUM_LOCS][i % NUM_LOCS];
+    __shared__ alignas(16) uint16_t s_dep[NUM_OPS][16];
+    for (int i = threadIdx.x; i < (int)NUM_OPS * 2; i += blockDim.x) reinterpret_cast<uint4*>(&s_dep[0][0])[i] = g_dep16[i];
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const uint64_t n = min((uint64_t)*n_pairs_ptr, n_cap);
@@ -1997,15 +2002,24 @@ __global__ void __launch_bounds__(256) k_small(Src src, const unsigned long long
     for (uint64_t warps = (uint64_t)gridDim.x * kWarpsPerBlock; g > kSmallLanesLog2 && n > warps; g--) warps <<= 1;
     const uint32_t sub = (uint32_t)lane & ((1u << g) - 1u), lead = (uint32_t)lane - sub;
     const uint32_t group = (g == 5 ? kFull : (1u << (1 << g)) - 1u) << lead;
-    const unsigned long long batch = 32u >> g;
+    // A ticket is up to 16 steps of the warp: with one each, a million pairs
+    // wait for 130,000 atomics on one counter.
+    const uint32_t per = 32u >> g;
+    const uint64_t steps = n / ((uint64_t)gridDim.x * kWarpsPerBlock * per * 4);
+    const uint64_t batch = (uint64_t)per * (steps < 1 ? 1 : steps > 16 ? 16 : steps);
     // the pair's sequences: one column of the staging array for its lanes
     uint16_t *st = &s_ins[0][(threadIdx.x & ~31u) + lead], *sc = st + Src::kMaxT * 256;
     unsigned long long nstates = 0, next = 0;
     if (lane == 0) next = atomicAdd(&a.v->small_ticket, batch);
-    for (;;) {
-        const uint64_t first = __shfl_sync(kFull, next, 0), p = first + (uint32_t)(lane >> g);
-        if (first >= n) break;
-        if (lane == 0) next = atomicAdd(&a.v->small_ticket, batch);
+    uint64_t first = 0, upto = 0;
+    for (;; first += per) {
+        if (first >= upto) {
+            first = __shfl_sync(kFull, next, 0);
+            if (first >= n) break;
+            upto = first + batch;
+            if (lane == 0) next = atomicAdd(&a.v->small_ticket, batch);
+        }
+        const uint64_t p = first + (uint32_t)(lane >> g);
         int tn = 0, cn = 0;
         uint32_t dead = 0, swx = 0, written = 0;
         if (p < n && sub == 0) src.load_lane(p, st, sc, 256, tn, cn, dead);
@@ -2038,7 +2052,7 @@ __global__ void __launch_bounds__(256) k_small(Src src, const unsigned long long
         const bool rreg = rep && !(reg & LB(L_A));
         const uint32_t words = reg == 0 ? 1u : rreg ? 8u : 64u;   // packed words of the register's values
         const uint32_t total = words << ((u & LB(L_C)) ? 1 : 0);
-        bool open = small, differ = false;
+        bool open = small && live, differ = false;   // no live output is written: equal
         for (uint32_t q = 2 * sub; __any_sync(kFull, open); q += 2u << g) {
             uint32_t d = 0;
             if (open && q < total) {
@@ -2211,9 +2225,16 @@ __global__ void k_go_select(const Surv* __restrict__ surv, const unsigned long l
         else cand[0] = c_tab[idx];
         algo += algo_ops(targets + (uint64_t)s.t * tlen, tlen, cand, cn, sweep_mode);
     }
-    if (npass) atomicAdd(&cnt->exh_pass, npass);
-    if (algo) atomicAdd(&cnt->algo, algo);
-    if (nund) atomicAdd(&cnt->undecided, nund);
+    for (int o = 16; o; o >>= 1) {   // one atomic per warp: one per thread took 250 us of a 2 M target pass
+        npass += __shfl_down_sync(kFull, npass, o);
+        algo += __shfl_down_sync(kFull, algo, o);
+        nund += __shfl_down_sync(kFull, nund, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (npass) atomicAdd(&cnt->exh_pass, npass);
+        if (algo) atomicAdd(&cnt->algo, algo);
+        if (nund) atomicAdd(&cnt->undecided, nund);
+    }
 }
 
 __global__ void k_go_emit(const uint32_t* __restrict__ best, uint32_t nt, const uint16_t* __restrict__ targets,
@@ -2735,6 +2756,10 @@ int init_ctx(m6502_ctx* ctx) {
     CK(cudaMemcpyToSymbol(c_line, line, sizeof line));
     CK(cudaMemcpyToSymbol(c_dep, dep, sizeof dep));
     CK(cudaMemcpyToSymbol(c_wr, wr, sizeof wr));
+    uint16_t dep16[NUM_OPS][16] = {};
+    for (uint32_t op = 0; op < NUM_OPS; op++)
+        for (uint32_t l = 0; l < NUM_LOCS; l++) dep16[op][l] = dep[op][l];
+    CK(cudaMemcpyToSymbol(g_dep16, dep16, sizeof dep16));
     CK(cudaMemcpyToSymbol(c_sweep, sw, sizeof sw));
     uint32_t x4[NUM_OPS];
     for (uint32_t op = 0; op < NUM_OPS; op++) x4[op] = x4_desc(op);
