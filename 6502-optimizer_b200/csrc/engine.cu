@@ -1977,10 +1977,12 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
 // instructions per pair (cone analysis by shuffles, ticket, staging) on 64
 // packed words of states.  The line at 9 bits: a lane takes 64 dispatches per
 // instruction for 512 states; one more register would make it 16,384.
-// Several lanes share a pair (a warp while that fills the chip, else four:
-// lanes whose candidates differ in opcode diverge).  The same enumeration:
+// Several lanes share a pair (a warp while that fills the chip, else eight:
+// lanes whose pairs differ in opcode diverge.  Four, eight, sixteen lanes:
+// the count at 0xFF 7.77, 7.19, 7.54 ms, 20,011 checked pairs 495, 460, 453 us,
+// this enumeration alike).  The same enumeration:
 // 0.56 ms for 1.1 M pairs; k_exhaustive took 2.63 ms for 1.36 M.
-constexpr int kSmallLanesLog2 = 2;   // lanes per pair once the pairs alone fill the chip: 2^2
+constexpr int kSmallLanesLog2 = 3;   // lanes per pair once the pairs alone fill the chip: 2^3
 __device__ __forceinline__ uint32_t backward(uint32_t locs, uint32_t op, const uint16_t (*dep)[16]) {
     const uint32_t wr = c_wr[op];
     uint32_t r = locs & ~wr;
