@@ -68,6 +68,7 @@ constexpr uint64_t kMaxItemsPerCone = 1ull << 16;   // larger cones get larger i
 constexpr uint32_t kMaxConeBits = 34;
 constexpr unsigned kTicketBatch = 4;           // pairs a warp takes per ticket atomic
 constexpr int kDirBits = 12;                   // key-bucket directory of the length-1 join (4,096 buckets)
+constexpr size_t kPairsStaged = 64u << 20;     // m6502_check_pairs: page-locked staging, at most
 constexpr int kMaxAsyncPasses = 64;            // passes of one search queued without a host round trip
 
 // Test vectors: TestVectors + MidCheckVectors of pkg/search/verifier.go:18-67
@@ -1087,7 +1088,8 @@ __global__ void __launch_bounds__(256) k_qc1(const uint64_t* __restrict__ tfp, c
                                               uint32_t nt, const uint64_t* __restrict__ cfp,
                                               const uint8_t* __restrict__ cmeta, uint32_t dead,
                                               uint32_t stages, Surv* __restrict__ surv, uint64_t cap,
-                                              Counters* __restrict__ cnt) {
+                                              Counters* __restrict__ cnt, const uint32_t* __restrict__ bad = nullptr) {
+    if (bad && *bad) return;
     __shared__ uint64_t s_t0[kQcTile];
     __shared__ uint8_t s_tb[kQcTile];
     __shared__ Surv s_stage[kWarpsPerBlock][kStage];
@@ -1168,7 +1170,8 @@ __global__ void __launch_bounds__(256, 4) k_qc_join(const uint16_t* __restrict__
                                                   uint32_t chunk, const uint4* __restrict__ cfp4,
                                                   const JoinTable* __restrict__ table, uint32_t dead,
                                                   uint32_t stages, Surv* __restrict__ match,
-                                                  Counters* __restrict__ cnt) {
+                                                  Counters* __restrict__ cnt, const uint32_t* __restrict__ bad) {
+    if (bad && *bad) return;   // an opcode outside the table: nothing of this search counts
     __shared__ alignas(16) uint8_t s_raw[kJoinShared];
     const JoinTable& s_tab = *reinterpret_cast<const JoinTable*>(s_raw);   // key and dir only
     __shared__ Surv s_stage[kWarpsPerBlock][kStage];
@@ -2240,15 +2243,15 @@ __global__ void k_go_select(const Surv* __restrict__ surv, const unsigned long l
 }
 
 __global__ void k_go_emit(const uint32_t* __restrict__ best, uint32_t nt, const uint16_t* __restrict__ targets,
-                          uint32_t tlen, const uint64_t* __restrict__ ids, m6502_rule* __restrict__ rules,
-                          uint64_t rcap, Counters* cnt) {
+                          uint32_t tlen, const uint64_t* __restrict__ ids, uint64_t tbase,
+                          m6502_rule* __restrict__ rules, uint64_t rcap, Counters* cnt) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
         for (int pass = 0; pass < 2; pass++) {
             uint32_t key = best[(uint64_t)pass * nt + t];
             if (key == 0xFFFFFFFFu) continue;
             m6502_rule r;
             memset(&r, 0, sizeof r);
-            r.target = ids ? ids[t] : t;
+            r.target = ids ? ids[t] : tbase + t;
             if (key >> 28) {
                 uint32_t rk = key & 0x0FFFFFFFu;
                 r.cand_len = 2; r.cand[0] = c_gotab[rk / kNumInsns]; r.cand[1] = c_gotab[rk % kNumInsns];
@@ -2363,6 +2366,16 @@ __global__ void __launch_bounds__(256) k_pair_vectors(CsrSource src, uint64_t n,
             if (fdiff) fdiff[p] = (uint8_t)(((nv & 0xFFu) == 0xFFu) ? pd : 0u);
         }
         __syncwarp();
+    }
+}
+
+// The pairs' verdict bits: the vector checks asked for (already in out, when
+// vec is not 0) and ExhaustiveCheck's verdict.
+__global__ void k_pair_verdicts(uint64_t n, uint32_t vec, const uint32_t* __restrict__ fail, uint8_t* __restrict__ out) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t r = vec ? out[i] & vec : 0u;
+        if (fail) r |= fail[i] == 0 ? 4u : fail[i] == 3 ? 8u : 0u;   // 3: undecided
+        out[i] = (uint8_t)r;
     }
 }
 
@@ -2522,8 +2535,8 @@ struct m6502_ctx {
     cudaEvent_t sev[6] = {};   // stage boundaries of one pass
     cudaEvent_t sev2[6] = {};  // stage boundaries of the length-2 candidate phase
     cudaEvent_t aev[6 * kMaxAsyncPasses] = {};   // stage boundaries of the queued passes
-    struct SearchGraph {       // the queued passes of the last device-resident search, recorded
-        cudaGraphExec_t exec = nullptr;
+    struct SearchGraph {       // the queued passes of the last search, recorded one by one
+        std::vector<cudaGraphExec_t> exec;
         std::vector<uint64_t> key;   // everything the recorded launches depend on
         bool broken = false;         // recording failed once: launch directly from then on
         std::string why;             // the error that stopped recording
@@ -2538,6 +2551,11 @@ struct m6502_ctx {
     DevBuf cnt_slots;          // Counters of the queued passes
     DevBuf tall;               // host targets of a queued search, copied to the device at once
     DevBuf opflag;             // k_check_ops result
+    cudaStream_t copy = nullptr;                  // host targets of the next pass, beside the kernels of this one
+    cudaEvent_t cev[kMaxAsyncPasses] = {};        // its copies
+    DevBuf pairs_io;                              // m6502_check_pairs: inputs, then results, in one block each way
+    void* h_io = nullptr;                         // page-locked side of it
+    size_t h_io_bytes = 0;
     std::string err;
     std::mutex mu;
     int sms = 148;
@@ -2547,7 +2565,7 @@ struct m6502_ctx {
     uint64_t pass_targets = 1ull << 21;
     bool ready = false;
     DevBuf cfp1, cmeta1, targets, ids, tfp, tmeta, surv, fail, items, rules, cnt, best, pins, poffs,
-        cins, coffs, pout, pfd, enum_count;
+        enum_count;
     std::vector<m6502_rule> staging;
     DevBuf cfp4;                      // packed outputs of the length-1 candidates: [2863][8 groups of 4 vectors][8 fields]
     std::vector<uint32_t> h_cfp4;     // host copy
@@ -2667,7 +2685,7 @@ const uint16_t* join_mult(const m6502_ctx* ctx, uint32_t dead) {
 // The length-1 QuickCheck join.  A warp takes as many targets as fill the
 // resident warps, up to a lane each: small searches spread over all SMs.
 int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt, const m6502_search_cfg& cfg,
-                 uint64_t scap, Counters* cnt) {
+                 uint64_t scap, Counters* cnt, const uint32_t* bad = nullptr) {
     const bool go = cfg.semantics == M6502_SEM_GO;
     const uint32_t stages = cfg.stages ? cfg.stages : M6502_CHECK_ALL, dead = cfg.dead_flags;
     // the line filter is part of ExhaustiveCheck; brute force does without
@@ -2680,9 +2698,9 @@ int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt
     const uint4* cfp4 = (const uint4*)ctx->cfp4.p;
     Surv* match = (Surv*)ctx->match.p;
     if (go)
-        k_qc_join<true><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages, match, cnt);
+        k_qc_join<true><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages, match, cnt, bad);
     else
-        k_qc_join<false><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages, match, cnt);
+        k_qc_join<false><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages, match, cnt, bad);
     CKL("k_qc_join");
     const uint16_t* mult = go ? nullptr : join_mult(ctx, dead);
     const uint32_t* lines = (const uint32_t*)ctx->join_lines[dead].p;
@@ -2976,14 +2994,32 @@ int cand2_table(m6502_ctx* ctx, uint32_t dead, m6502_ctx::Cand2Table** out) {
     return M6502_OK;
 }
 
-struct PassOut {
-    Counters c;
+// Where a search's rules go: the caller's buffer while they fit, then the
+// context's staging vector (m6502_fetch_rules).
+struct RuleSink {
+    m6502_rule* out;
+    uint64_t cap, n;   // room, rules written
 };
 
-// One device pass: nt targets (device pointer) of length tlen.  Appends the
-// rules to ctx->staging (target index = base + local, or ids[local]).
+// `n` device rules to the sink, on the stream (not synchronised).
+int deliver(m6502_ctx* ctx, RuleSink& sink, const m6502_rule* rules, uint64_t n) {
+    const uint64_t k = sink.out ? std::min(n, sink.cap - sink.n) : 0;
+    if (k)
+        CK(cudaMemcpyAsync(sink.out + sink.n, rules, k * sizeof(m6502_rule), cudaMemcpyDeviceToHost, ctx->stream));
+    sink.n += k;
+    if (k < n) {
+        const size_t old = ctx->staging.size();
+        ctx->staging.resize(old + (n - k));
+        CK(cudaMemcpyAsync(ctx->staging.data() + old, rules + k, (n - k) * sizeof(m6502_rule), cudaMemcpyDeviceToHost,
+                           ctx->stream));
+    }
+    return M6502_OK;
+}
+
+// One device pass: nt targets (device pointer) of length tlen.  Hands its
+// rules to the sink (target index = base + local, or ids[local]).
 int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targets, uint64_t nt,
-             uint32_t tlen, const uint64_t* d_ids, uint64_t base, m6502_stats* st) {
+             uint32_t tlen, const uint64_t* d_ids, uint64_t base, RuleSink& sink, m6502_stats* st) {
     const bool go = cfg.semantics == M6502_SEM_GO;
     const uint32_t stages = cfg.stages ? cfg.stages : M6502_CHECK_ALL;
     const uint32_t dead = cfg.dead_flags;
@@ -3060,12 +3096,12 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
             k_qc1<true><<<qgrid, 256, 0, ctx->stream>>>((uint64_t*)ctx->tfp.p, (uint8_t*)ctx->tmeta.p,
                                                         (uint32_t)nt, (uint64_t*)ctx->cfp1.p,
                                                         (uint8_t*)ctx->cmeta1.p, dead, stages,
-                                                        (Surv*)ctx->surv.p, scap, cnt);
+                                                        (Surv*)ctx->surv.p, scap, cnt, nullptr);
         else
             k_qc1<false><<<qgrid, 256, 0, ctx->stream>>>((uint64_t*)ctx->tfp.p, (uint8_t*)ctx->tmeta.p,
                                                          (uint32_t)nt, (uint64_t*)ctx->cfp1.p,
                                                          (uint8_t*)ctx->cmeta1.p, dead, stages,
-                                                         (Surv*)ctx->surv.p, scap, cnt);
+                                                         (Surv*)ctx->surv.p, scap, cnt, nullptr);
         CKL("k_qc1");
         CK(rec(ctx->sev[2]));
         SurvSource src{(const Surv*)ctx->surv.p, d_targets, tlen, dead, go ? 1 : 0, mult};
@@ -3132,7 +3168,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
                 CKL("k_go_select");
             } else {
                 k_emit_all<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const Surv*)ctx->surv.p, &cnt->surv, scap,
-                                                                  (const uint32_t*)ctx->fail.p, d_ids, 0, dead,
+                                                                  (const uint32_t*)ctx->fail.p, d_ids, base, dead,
                                                                   (m6502_rule*)ctx->rules.p, rlim, &cnt->rules, cnt,
                                                                   exh ? 1 : 0, d_targets, tlen, cfg.sweep, groups);
                 CKL("k_emit_all");
@@ -3182,7 +3218,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         if (!phase2) CK(rec(ctx->sev2[4]));
         if (go) {
             k_go_emit<<<ctx->sms * 8, 256, 0, ctx->stream>>>((const uint32_t*)ctx->best.p, (uint32_t)nt,
-                                                             d_targets, tlen, d_ids,
+                                                             d_targets, tlen, d_ids, base,
                                                              (m6502_rule*)ctx->rules.p, rlim, cnt);
             CKL("k_go_emit");
         }
@@ -3194,7 +3230,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         bool launched = false;
         if (!(cfg.flags & M6502_NO_GRAPH) && !ctx->graph.broken) {
             const std::vector<uint64_t> key = {
-                (uint64_t)(uintptr_t)d_targets, nt, tlen, (uint64_t)(uintptr_t)d_ids, cfg.semantics, cfg.sweep,
+                (uint64_t)(uintptr_t)d_targets, nt, tlen, (uint64_t)(uintptr_t)d_ids, base, cfg.semantics, cfg.sweep,
                 cfg.exh_mode, stages, cfg.flags, dead, cfg.max_cand_len, scap, icap, rcap, jcap,
                 (uint64_t)(uintptr_t)ctx->surv.p, (uint64_t)(uintptr_t)ctx->fail.p, (uint64_t)(uintptr_t)ctx->items.p,
                 (uint64_t)(uintptr_t)ctx->order.p, (uint64_t)(uintptr_t)ctx->match.p,
@@ -3269,14 +3305,8 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
         if (hc.rules > rlim && !count_only) { rcap = hc.rules + hc.rules / 4 + 1024; redo = true; }
         if (!first_over && hc.join_items > jcap) { jcap = hc.join_items + hc.join_items / 4 + 1024; redo = true; }
         if (redo) continue;
-        size_t old = ctx->staging.size();
-        if (!count_only) ctx->staging.resize(old + hc.rules);
-        if (hc.rules && !count_only)
-            CK(cudaMemcpyAsync(ctx->staging.data() + old, ctx->rules.p, hc.rules * sizeof(m6502_rule),
-                               cudaMemcpyDeviceToHost, ctx->stream));
+        if (!count_only) TRY(deliver(ctx, sink, (const m6502_rule*)ctx->rules.p, hc.rules));
         CK(cudaStreamSynchronize(ctx->stream));
-        if (!d_ids)
-            for (size_t i = old; i < ctx->staging.size(); i++) ctx->staging[i].target += base;
         if (st) {
             st->targets += nt;
             st->pairs += nt * ((uint64_t)kNumInsns + (phase2 ? (uint64_t)kNumInsns * kNumInsns : 0u));
@@ -3320,10 +3350,13 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
 // global target index.  One synchronisation at the end reads every pass's
 // counters; if any buffer overflowed, the whole search is re-run with larger
 // buffers (nothing is dropped).  Returns M6502_E_INVAL when the search does
-// not fit this path.  `targets` is in device memory.
-int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* targets, uint64_t n, uint32_t tlen,
-                 m6502_stats* st, m6502_rule* out, uint64_t out_cap, bool* delivered) {
-    *delivered = false;
+// not fit this path, or for an opcode outside the table: every pass checks its
+// targets first, and from the first bad one on the join finds nothing.
+// `targets` is in device memory; with `host` set it is filled from there pass
+// by pass on a second stream, so that the copies (pageable memory: 30 MB of
+// length-2 targets take longer than their search) run beside the kernels.
+int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* targets, const uint16_t* host, uint64_t n,
+                 uint32_t tlen, m6502_stats* st, RuleSink& sink) {
     const uint64_t P = ctx->pass_targets;
     const uint64_t npass = (n + P - 1) / P;
     if (npass == 0 || npass > (uint64_t)kMaxAsyncPasses) return set_err(ctx, M6502_E_INVAL, "too many passes");
@@ -3344,6 +3377,8 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
     const CandGroups* groups = scan ? nullptr : (const CandGroups*)ctx->join_groups[dead].p;
     TRY(ensure(ctx, ctx->cnt_slots, npass * sizeof(Counters)));
     Counters* slots = (Counters*)ctx->cnt_slots.p;
+    TRY(ensure(ctx, ctx->opflag, 2 * sizeof(uint32_t)));
+    uint32_t* bad = (uint32_t*)ctx->opflag.p;
     for (int attempt = 0; attempt < 6; attempt++) {
         TRY(ensure(ctx, ctx->surv, scap * sizeof(Surv)));
         TRY(ensure(ctx, ctx->fail, scap * sizeof(uint32_t)));
@@ -3360,13 +3395,20 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
             return capturing ? cudaEventRecordWithFlags(e, ctx->stream, cudaEventRecordExternal)
                              : cudaEventRecord(e, ctx->stream);
         };
-        auto enqueue = [&]() -> int {
-            CK(cudaMemsetAsync(slots, 0, npass * sizeof(Counters), ctx->stream));
-            for (uint64_t p = 0; p < npass; p++) {
+        // Pass p; the first also clears every pass's counters.
+        auto enqueue = [&](uint64_t p) -> int {
+            if (p == 0) {
+                CK(cudaMemsetAsync(slots, 0, npass * sizeof(Counters), ctx->stream));
+                CK(cudaMemsetAsync(bad, 0, sizeof(uint32_t), ctx->stream));
+            }
+            {
                 const uint64_t b = p * P, nt = std::min(P, n - b);
                 const uint16_t* d_t = targets + b * tlen;
                 Counters* cnt = slots + p;
                 cudaEvent_t* ev = ctx->aev + 6 * p;
+                const uint32_t cgrid = (uint32_t)std::min<uint64_t>((nt * tlen + 255) / 256, (uint64_t)ctx->sms * 16);
+                k_check_ops<<<cgrid, 256, 0, ctx->stream>>>(d_t, nt * tlen, bad);
+                CKL("k_check_ops");
                 CK(rec(ev[0]));
                 if (scan) {
                     k_fingerprint<FixedSeqs><<<ctx->fp_blocks, 256, 0, ctx->stream>>>(
@@ -3379,10 +3421,10 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                     k_qc1<false><<<qgrid, 256, 0, ctx->stream>>>((uint64_t*)ctx->tfp.p, (uint8_t*)ctx->tmeta.p,
                                                                  (uint32_t)nt, (uint64_t*)ctx->cfp1.p,
                                                                  (uint8_t*)ctx->cmeta1.p, dead, stages,
-                                                                 (Surv*)ctx->surv.p, scap, cnt);
+                                                                 (Surv*)ctx->surv.p, scap, cnt, bad);
                     CKL("k_qc1");
                 } else {
-                    TRY(launch_join1(ctx, d_t, tlen, nt, cfg, scap, cnt));
+                    TRY(launch_join1(ctx, d_t, tlen, nt, cfg, scap, cnt, bad));
                 }
                 CK(rec(ev[2]));
                 SurvSource src{(const Surv*)ctx->surv.p, d_t, tlen, dead, 0, groups ? groups->mult : nullptr};
@@ -3403,32 +3445,41 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
             return M6502_OK;
         };
         const bool use_graph = !(cfg.flags & M6502_NO_GRAPH) && !ctx->graph.broken;
-        bool replayed = false, launched = false;
+        bool replayed = false;
         if (use_graph) {
             const std::vector<uint64_t> key = {
                 (uint64_t)(uintptr_t)targets, n, tlen, cfg.semantics, cfg.sweep, cfg.exh_mode, stages,
                 cfg.flags, dead, scap, icap, rcap, P, (uint64_t)(uintptr_t)ctx->surv.p,
-                (uint64_t)(uintptr_t)ctx->fail.p, (uint64_t)(uintptr_t)ctx->items.p, (uint64_t)(uintptr_t)ctx->order.p, (uint64_t)(uintptr_t)ctx->match.p,
+                (uint64_t)(uintptr_t)ctx->fail.p, (uint64_t)(uintptr_t)ctx->items.p, (uint64_t)(uintptr_t)ctx->order.p,
+                (uint64_t)(uintptr_t)ctx->match.p,
                 (uint64_t)(uintptr_t)ctx->rules.p, (uint64_t)(uintptr_t)ctx->cnt_slots.p,
-                (uint64_t)(uintptr_t)ctx->tfp.p, (uint64_t)(uintptr_t)ctx->tmeta.p,
+                (uint64_t)(uintptr_t)ctx->tfp.p, (uint64_t)(uintptr_t)ctx->tmeta.p, (uint64_t)(uintptr_t)ctx->opflag.p,
                 (uint64_t)(uintptr_t)ctx->join_tab[0][dead].p, ctx->tune.exh_minb, ctx->tune.ticket_batch,
                 ctx->tune.chunk_log2};
-            if (!(ctx->graph.exec && ctx->graph.key == key)) {
-                if (ctx->graph.exec) { cudaGraphExecDestroy(ctx->graph.exec); ctx->graph.exec = nullptr; }
+            replayed = ctx->graph.exec.size() == npass && ctx->graph.key == key;
+            if (!replayed) {
+                for (cudaGraphExec_t e : ctx->graph.exec) cudaGraphExecDestroy(e);
+                ctx->graph.exec.clear();
                 // Record; if recording or instantiation fails, this context stops
                 // using graphs and the passes are launched directly below.
-                cudaGraph_t g = nullptr;
-                bool ok = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-                if (ok) {
-                    capturing = true;
-                    const int rc = enqueue();
-                    capturing = false;
-                    ok = cudaStreamEndCapture(ctx->stream, &g) == cudaSuccess && rc == M6502_OK && g;
-                    ok = ok && cudaGraphInstantiate(&ctx->graph.exec, g, 0) == cudaSuccess;
-                    if (g) cudaGraphDestroy(g);
+                bool ok = true;
+                for (uint64_t p = 0; p < npass && ok; p++) {
+                    cudaGraph_t g = nullptr;
+                    cudaGraphExec_t e = nullptr;
+                    ok = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+                    if (ok) {
+                        capturing = true;
+                        const int rc = enqueue(p);
+                        capturing = false;
+                        ok = cudaStreamEndCapture(ctx->stream, &g) == cudaSuccess && rc == M6502_OK && g;
+                        ok = ok && cudaGraphInstantiate(&e, g, 0) == cudaSuccess;
+                        if (g) cudaGraphDestroy(g);
+                    }
+                    if (ok) ctx->graph.exec.push_back(e);
                 }
                 if (!ok) {
-                    ctx->graph.exec = nullptr;
+                    for (cudaGraphExec_t e : ctx->graph.exec) cudaGraphExecDestroy(e);
+                    ctx->graph.exec.clear();
                     ctx->graph.broken = true;
                     ctx->graph.why = cudaGetErrorString(cudaGetLastError());   // clears the launch error
                     set_err(ctx, M6502_OK, "CUDA graph recording failed (" + ctx->graph.why +
@@ -3436,18 +3487,29 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 } else {
                     ctx->graph.key = key;
                 }
-            } else {
-                replayed = true;
-            }
-            if (ctx->graph.exec) {
-                CK(cudaGraphLaunch(ctx->graph.exec, ctx->stream));
-                launched = true;
             }
         }
-        if (!launched) TRY(enqueue());
+        for (uint64_t p = 0; p < npass; p++) {
+            if (host && attempt == 0) {
+                const uint64_t b = p * P, nt = std::min(P, n - b);
+                // a single pass has nothing to run beside: its copy goes on the same stream
+                const cudaStream_t cs = npass > 1 ? ctx->copy : ctx->stream;
+                CK(cudaMemcpyAsync((void*)(targets + b * tlen), host + b * tlen, nt * tlen * sizeof(uint16_t),
+                                   cudaMemcpyHostToDevice, cs));
+                if (npass > 1) {
+                    CK(cudaEventRecord(ctx->cev[p], ctx->copy));
+                    CK(cudaStreamWaitEvent(ctx->stream, ctx->cev[p], 0));
+                }
+            }
+            if (use_graph && !ctx->graph.broken) CK(cudaGraphLaunch(ctx->graph.exec[p], ctx->stream));
+            else TRY(enqueue(p));
+        }
         std::vector<Counters> hc(npass);
+        uint32_t any_bad = 0;
         CK(cudaMemcpyAsync(hc.data(), slots, npass * sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemcpyAsync(&any_bad, bad, sizeof any_bad, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
+        if (any_bad) return set_err(ctx, M6502_E_INVAL, "opcode out of range");
         bool redo = false;
         for (const Counters& c : hc) {
             if (c.surv > scap) { scap = std::max<uint64_t>(scap, c.surv + c.surv / 4 + 1024); redo = true; }
@@ -3457,20 +3519,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
         const uint64_t nrules = hc[0].rules;
         if (nrules > rcap && !count_only) { rcap = nrules + nrules / 4 + 1024; redo = true; }
         if (redo) continue;
-        if (count_only) {
-            *delivered = true;   // counted, nothing to hand over
-        } else if (out && nrules <= out_cap && ctx->staging.empty()) {   // straight into the caller's buffer
-            if (nrules)
-                CK(cudaMemcpyAsync(out, ctx->rules.p, nrules * sizeof(m6502_rule), cudaMemcpyDeviceToHost,
-                                   ctx->stream));
-            *delivered = true;
-        } else {
-            const size_t old = ctx->staging.size();
-            ctx->staging.resize(old + nrules);
-            if (nrules)
-                CK(cudaMemcpyAsync(ctx->staging.data() + old, ctx->rules.p, nrules * sizeof(m6502_rule),
-                                   cudaMemcpyDeviceToHost, ctx->stream));
-        }
+        if (!count_only) TRY(deliver(ctx, sink, (const m6502_rule*)ctx->rules.p, nrules));
         CK(cudaStreamSynchronize(ctx->stream));
         if (st) {
             for (uint64_t p = 0; p < npass; p++) {
@@ -3514,8 +3563,8 @@ int check_cfg(m6502_ctx* ctx, const m6502_search_cfg* cfg) {
     return M6502_OK;
 }
 
-// Hands the staged rules to the caller; what does not fit stays staged for
-// m6502_fetch_rules.
+// Hands staged rules to the caller; what does not fit stays staged for the
+// next m6502_fetch_rules.
 int finish(m6502_ctx* ctx, m6502_rule* out, uint64_t cap, uint64_t* n_out) {
     const uint64_t n = ctx->staging.size();
     if (n_out) *n_out = n;
@@ -3523,6 +3572,15 @@ int finish(m6502_ctx* ctx, m6502_rule* out, uint64_t cap, uint64_t* n_out) {
     if (k) std::memcpy(out, ctx->staging.data(), k * sizeof(m6502_rule));
     ctx->staging.erase(ctx->staging.begin(), ctx->staging.begin() + (long)k);
     if (n > k) return set_err(ctx, M6502_E_OVERFLOW, "rule buffer too small: the rest stays staged");
+    ctx->staging.shrink_to_fit();
+    return M6502_OK;
+}
+
+// The end of a search: its rules are in the caller's buffer, the rest staged.
+int finish_search(m6502_ctx* ctx, const RuleSink& sink, uint64_t* n_out) {
+    const uint64_t rest = ctx->staging.size();
+    if (n_out) *n_out = sink.n + rest;
+    if (rest) return set_err(ctx, M6502_E_OVERFLOW, "rule buffer too small: the rest stays staged");
     ctx->staging.shrink_to_fit();
     return M6502_OK;
 }
@@ -3662,6 +3720,8 @@ int m6502_create(m6502_ctx** out, const m6502_opts* opts) {
     for (cudaEvent_t& e : ctx->sev) ev_ok = ev_ok && cudaEventCreate(&e) == cudaSuccess;
     for (cudaEvent_t& e : ctx->sev2) ev_ok = ev_ok && cudaEventCreate(&e) == cudaSuccess;
     for (cudaEvent_t& e : ctx->aev) ev_ok = ev_ok && cudaEventCreate(&e) == cudaSuccess;
+    for (cudaEvent_t& e : ctx->cev) ev_ok = ev_ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    ev_ok = ev_ok && cudaStreamCreateWithFlags(&ctx->copy, cudaStreamNonBlocking) == cudaSuccess;
     if (!ev_ok) {
         delete ctx;
         return M6502_E_CUDA;
@@ -3694,7 +3754,7 @@ void m6502_destroy(m6502_ctx* ctx) {
     }
     DevBuf* bufs[] = {&ctx->cfp4, &ctx->cfp1, &ctx->cmeta1, &ctx->targets, &ctx->ids, &ctx->tfp, &ctx->tmeta,
                       &ctx->surv, &ctx->fail, &ctx->items, &ctx->rules, &ctx->cnt, &ctx->best,
-                      &ctx->pins, &ctx->poffs, &ctx->cins, &ctx->coffs, &ctx->pout, &ctx->pfd,
+                      &ctx->pins, &ctx->poffs,
                       &ctx->enum_count, &ctx->st_tins, &ctx->st_toffs, &ctx->st_tout, &ctx->st_tbytes,
                       &ctx->st_chains, &ctx->st_entries, &ctx->st_vidx, &ctx->st_proven, &ctx->st_cnt,
                       &ctx->st_pidx, &ctx->st_mex, &ctx->st_probs, &ctx->st_traj, &ctx->st_row, &ctx->st_keys,
@@ -3703,12 +3763,15 @@ void m6502_destroy(m6502_ctx* ctx) {
                       &ctx->c2_sort_tmp, &ctx->go_keys, &ctx->go_keys2, &ctx->go_ord, &ctx->go_round,
                       &ctx->go_sort_tmp, &ctx->jitems, &ctx->cnt_slots, &ctx->st_vphase, &ctx->st_pphase,
                       &ctx->st_live, &ctx->st_rounds, &ctx->st_proven_was,
-                      &ctx->tall, &ctx->opflag, &ctx->order, &ctx->match};
+                      &ctx->tall, &ctx->opflag, &ctx->order, &ctx->match, &ctx->pairs_io};
     for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
     for (cudaEvent_t e : ctx->sev) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->sev2) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->aev) if (e) cudaEventDestroy(e);
-    if (ctx->graph.exec) cudaGraphExecDestroy(ctx->graph.exec);
+    for (cudaGraphExec_t e : ctx->graph.exec) cudaGraphExecDestroy(e);
+    for (cudaEvent_t e : ctx->cev) if (e) cudaEventDestroy(e);
+    if (ctx->copy) cudaStreamDestroy(ctx->copy);
+    if (ctx->h_io) cudaFreeHost(ctx->h_io);
     for (m6502_ctx::PassGraph& g : ctx->pass_graphs)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     for (auto& t : ctx->cand2) {
@@ -3743,56 +3806,74 @@ int m6502_check_pairs(m6502_ctx* ctx, uint64_t n, const uint16_t* t_insns, const
     if (!valid_seq(t_insns + t_offs[0], t_offs[n] - t_offs[0]) || !valid_seq(c_insns + c_offs[0], c_offs[n] - c_offs[0]))
         return set_err(ctx, M6502_E_INVAL, "opcode out of range");
     CK(cudaSetDevice(ctx->device));
+    // One block on the device: verdicts, FlagDiffs and counters (copied back),
+    // counters, offsets and instructions (copied in).  Up to kPairsStaged bytes
+    // each way go through page-locked memory in one copy; more go from and to
+    // the caller's buffers.
+    const bool exh = (checks & M6502_CHECK_EXH) != 0, vectors = (checks & 3u) || flagdiff;
     const size_t tin = t_offs[n], cin = c_offs[n];
-    TRY(ensure(ctx, ctx->pins, tin * 2));
-    TRY(ensure(ctx, ctx->cins, cin * 2));
-    TRY(ensure(ctx, ctx->poffs, (n + 1) * 4));
-    TRY(ensure(ctx, ctx->coffs, (n + 1) * 4));
-    TRY(ensure(ctx, ctx->pout, n));
-    TRY(ensure(ctx, ctx->pfd, n));
+    auto up16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
+    const size_t o_fd = n, o_cnt = up16(2 * n), o_to = up16(o_cnt + sizeof(Counters)), o_co = o_to + up16((n + 1) * 4),
+                 o_ti = o_co + up16((n + 1) * 4), o_ci = o_ti + up16(tin * 2), total = o_ci + up16(cin * 2);
+    const bool staged = total <= kPairsStaged;
+    TRY(ensure(ctx, ctx->pairs_io, total));
     TRY(ensure(ctx, ctx->fail, n * 4));
     TRY(ensure(ctx, ctx->order, n * 4));
-    CK(cudaMemcpyAsync(ctx->pins.p, t_insns, tin * 2, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->cins.p, c_insns, cin * 2, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->poffs.p, t_offs, (n + 1) * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->coffs.p, c_offs, (n + 1) * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CsrSource src{(const uint16_t*)ctx->pins.p, (const uint32_t*)ctx->poffs.p, (const uint16_t*)ctx->cins.p,
-                  (const uint32_t*)ctx->coffs.p, dead_flags};
-    uint32_t grid = (uint32_t)std::min<uint64_t>((n + kWarpsPerBlock - 1) / kWarpsPerBlock, (uint64_t)ctx->sms * 16);
-    k_pair_vectors<<<grid, 256, 0, ctx->stream>>>(src, n, (uint8_t*)ctx->pout.p, (uint8_t*)ctx->pfd.p);
-    CKL("k_pair_vectors");
-    std::vector<uint8_t> fl;
-    if (checks & M6502_CHECK_EXH) {
-        Counters* cnt = (Counters*)ctx->cnt.p;
-        uint64_t icap = std::max<uint64_t>(ctx->items.bytes / sizeof(Item), 1u << 16);
-        for (int attempt = 0;; attempt++) {
+    if (staged && ctx->h_io_bytes < total) {
+        if (ctx->h_io) cudaFreeHost(ctx->h_io);
+        ctx->h_io = nullptr;
+        ctx->h_io_bytes = 0;
+        CK(cudaHostAlloc(&ctx->h_io, total, cudaHostAllocDefault));
+        ctx->h_io_bytes = total;
+    }
+    uint8_t* d = (uint8_t*)ctx->pairs_io.p;
+    uint8_t* h = (uint8_t*)ctx->h_io;
+    Counters hc;
+    std::memset(&hc, 0, sizeof hc);
+    hc.surv = n;
+    const struct { size_t at, bytes; const void* from; } parts[] = {
+        {o_cnt, sizeof hc, &hc}, {o_to, (n + 1) * 4, t_offs}, {o_co, (n + 1) * 4, c_offs}, {o_ti, tin * 2, t_insns},
+        {o_ci, cin * 2, c_insns}};
+    for (const auto& p : parts) {
+        if (staged) std::memcpy(h + p.at, p.from, p.bytes);
+        else CK(cudaMemcpyAsync(d + p.at, p.from, p.bytes, cudaMemcpyHostToDevice, ctx->stream));
+    }
+    if (staged) CK(cudaMemcpyAsync(d + o_cnt, h + o_cnt, total - o_cnt, cudaMemcpyHostToDevice, ctx->stream));
+    CsrSource src{(const uint16_t*)(d + o_ti), (const uint32_t*)(d + o_to), (const uint16_t*)(d + o_ci),
+                  (const uint32_t*)(d + o_co), dead_flags};
+    Counters* cnt = (Counters*)(d + o_cnt);
+    if (vectors) {
+        const uint32_t grid = (uint32_t)std::min<uint64_t>((n + kWarpsPerBlock - 1) / kWarpsPerBlock, (uint64_t)ctx->sms * 16);
+        k_pair_vectors<<<grid, 256, 0, ctx->stream>>>(src, n, d, d + o_fd);
+        CKL("k_pair_vectors");
+    }
+    uint64_t icap = std::max<uint64_t>(ctx->items.bytes / sizeof(Item), 1u << 16);
+    for (int attempt = 0;; attempt++) {
+        if (exh) {
             TRY(ensure(ctx, ctx->items, icap * sizeof(Item)));
-            CK(cudaMemsetAsync(cnt, 0, sizeof(Counters), ctx->stream));
-            unsigned long long hn = n;
-            CK(cudaMemcpyAsync(&cnt->surv, &hn, sizeof hn, cudaMemcpyHostToDevice, ctx->stream));
             ExhArgs ea{(uint32_t*)ctx->fail.p, (Item*)ctx->items.p, icap, cnt, &cnt->v[0][0], sweep,
                        exh_mode == M6502_EXH_BRUTE};
             TRY(launch_verify(ctx, src, &cnt->surv, n, ea));
-            Counters hc;
-            CK(cudaMemcpyAsync(&hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, ctx->stream));
-            CK(cudaStreamSynchronize(ctx->stream));
-            const uint64_t items = hc.v[0][0].items;
-            if (items <= icap) break;
-            if (attempt >= 4) return set_err(ctx, M6502_E_NOMEM, "work-item queue kept overflowing");
-            icap = items + items / 4 + 1024;
         }
-        fl.resize(n * 4);
-        CK(cudaMemcpyAsync(fl.data(), ctx->fail.p, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        k_pair_verdicts<<<(uint32_t)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx->sms * 8), 256, 0, ctx->stream>>>(
+            n, vectors ? checks & 3u : 0u, exh ? (const uint32_t*)ctx->fail.p : nullptr, d);
+        CKL("k_pair_verdicts");
+        CK(cudaMemcpyAsync(staged ? (void*)(h + o_cnt) : (void*)&hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemcpyAsync(staged ? h : out, d, n, cudaMemcpyDeviceToHost, ctx->stream));
+        if (flagdiff) CK(cudaMemcpyAsync(staged ? h + o_fd : flagdiff, d + o_fd, n, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (staged) std::memcpy(&hc, h + o_cnt, sizeof hc);
+        const uint64_t items = hc.v[0][0].items;
+        if (items <= icap) break;
+        if (attempt >= 4) return set_err(ctx, M6502_E_NOMEM, "work-item queue kept overflowing");
+        icap = items + items / 4 + 1024;
+        std::memset(&hc, 0, sizeof hc);
+        hc.surv = n;
+        CK(cudaMemcpyAsync(cnt, &hc, sizeof hc, cudaMemcpyHostToDevice, ctx->stream));
     }
-    CK(cudaMemcpyAsync(out, ctx->pout.p, n, cudaMemcpyDeviceToHost, ctx->stream));
-    if (flagdiff) CK(cudaMemcpyAsync(flagdiff, ctx->pfd.p, n, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    const uint32_t* f32 = (const uint32_t*)fl.data();
-    for (uint64_t i = 0; i < n; i++) {
-        uint8_t r = out[i] & (uint8_t)(checks & 3u);
-        if ((checks & M6502_CHECK_EXH) && f32[i] == 0) r |= 4;
-        if ((checks & M6502_CHECK_EXH) && f32[i] == 3) r |= 8;
-        out[i] = r;
+    if (staged) {
+        std::memcpy(out, h, n);
+        if (flagdiff) std::memcpy(flagdiff, h + o_fd, n);
     }
     return M6502_OK;
 }
@@ -3871,7 +3952,7 @@ int m6502_search(m6502_ctx* ctx, const m6502_search_cfg* cfg, const uint16_t* ta
     const bool async_ok = cfg->semantics == M6502_SEM_CUDA && cfg->max_cand_len <= 1 &&
                           n <= (uint64_t)kMaxAsyncPasses * ctx->pass_targets;
     // Opcodes are checked on the host only for host targets searched pass
-    // by pass; queued searches check them on the device.
+    // by pass; queued searches check them on the device, in every pass.
     if (!on_dev && !async_ok && !valid_seq(targets, n * tlen))
         return set_err(ctx, M6502_E_INVAL, "opcode out of range");
     CK(cudaSetDevice(ctx->device));
@@ -3879,15 +3960,15 @@ int m6502_search(m6502_ctx* ctx, const m6502_search_cfg* cfg, const uint16_t* ta
     std::memset(&st, 0, sizeof st);
     ctx->staging.clear();
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    // A queued search of host targets copies them all to the device first and
-    // then runs exactly as a device-resident one (CUDA graph included).
+    RuleSink sink{out, cap, 0};
+    // A queued search of host targets copies them to the device pass by pass
+    // and runs as a device-resident one (CUDA graphs included).
     const uint16_t* q_targets = targets;
     if (async_ok && n && !on_dev) {
         TRY(ensure(ctx, ctx->tall, n * tlen * sizeof(uint16_t)));
-        CK(cudaMemcpyAsync(ctx->tall.p, targets, n * tlen * sizeof(uint16_t), cudaMemcpyHostToDevice, ctx->stream));
         q_targets = (const uint16_t*)ctx->tall.p;
     }
-    if (on_dev || (async_ok && n)) TRY(check_ops_device(ctx, q_targets, n * tlen));
+    if (on_dev && !async_ok) TRY(check_ops_device(ctx, q_targets, n * tlen));
     for (uint64_t b = async_ok ? n : 0; b < n; b += ctx->pass_targets) {   // passes one by one otherwise
         uint64_t nt = std::min<uint64_t>(ctx->pass_targets, n - b);
         const uint16_t* d_t;
@@ -3898,21 +3979,26 @@ int m6502_search(m6502_ctx* ctx, const m6502_search_cfg* cfg, const uint16_t* ta
             CK(cudaMemcpyAsync(ctx->targets.p, targets + b * tlen, nt * tlen * 2, cudaMemcpyHostToDevice, ctx->stream));
             d_t = (const uint16_t*)ctx->targets.p;
         }
-        TRY(run_pass(ctx, *cfg, d_t, nt, tlen, nullptr, b, &st));
+        TRY(run_pass(ctx, *cfg, d_t, nt, tlen, nullptr, b, sink, &st));
     }
-    bool delivered = false;
-    if (async_ok && n) TRY(search_async(ctx, *cfg, q_targets, n, tlen, &st, out, cap, &delivered));
+    if (async_ok && n) {
+        const int rc = search_async(ctx, *cfg, q_targets, on_dev ? nullptr : targets, n, tlen, &st, sink);
+        if (rc != M6502_OK) {   // no copy from the caller's memory outlives the call
+            cudaStreamSynchronize(ctx->copy);
+            return rc;
+        }
+    }
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     CK(cudaEventSynchronize(ctx->ev1));
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     st.ms_device = ms;
     if (stats) *stats = st;
-    if (delivered || (cfg->flags & M6502_COUNT_ONLY)) {
+    if (cfg->flags & M6502_COUNT_ONLY) {
         if (n_out) *n_out = st.rules;
         return M6502_OK;
     }
-    return finish(ctx, out, cap, n_out);
+    return finish_search(ctx, sink, n_out);
 }
 
 int m6502_enumerate(m6502_ctx* ctx, const m6502_search_cfg* cfg, uint32_t tlen, uint32_t first,
@@ -3928,6 +4014,7 @@ int m6502_enumerate(m6502_ctx* ctx, const m6502_search_cfg* cfg, uint32_t tlen, 
     std::memset(&st, 0, sizeof st);
     ctx->staging.clear();
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
+    RuleSink sink{out, cap, 0};
     const uint64_t per_first = tlen == 2 ? (uint64_t)kNumInsns : (uint64_t)kNumInsns * kNumInsns;
     // first-op slices sized so one slice holds at most ~pass_targets ids
     const uint64_t ops_per_slice = std::max<uint64_t>(1, ctx->pass_targets / per_first);
@@ -3949,7 +4036,7 @@ int m6502_enumerate(m6502_ctx* ctx, const m6502_search_cfg* cfg, uint32_t tlen, 
         for (uint64_t b = 0; b < nt; b += ctx->pass_targets) {
             uint64_t m = std::min<uint64_t>(ctx->pass_targets, nt - b);
             TRY(run_pass(ctx, *cfg, (const uint16_t*)ctx->targets.p + b * tlen, m, tlen,
-                         (const uint64_t*)ctx->ids.p + b, 0, &st));
+                         (const uint64_t*)ctx->ids.p + b, 0, sink, &st));
         }
     }
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
@@ -3962,7 +4049,7 @@ int m6502_enumerate(m6502_ctx* ctx, const m6502_search_cfg* cfg, uint32_t tlen, 
         if (n_out) *n_out = st.rules;
         return M6502_OK;
     }
-    return finish(ctx, out, cap, n_out);
+    return finish_search(ctx, sink, n_out);
 }
 
 int m6502_tune_get(m6502_ctx* ctx, m6502_tune* out) {

@@ -6,6 +6,7 @@ FlagDiff / Fingerprint / ShouldPrune keep the Go signatures and run on a
 shared default engine; the batch methods take many pairs at once.
 """
 import ctypes
+import itertools
 import sys
 import threading
 
@@ -18,15 +19,12 @@ _PINNED_MIN_RULES = 1 << 16   # rule buffers of at least 1 MiB are page-locked
 
 
 def _csr(seqs):
+    """Sequences as one instruction array and n + 1 offsets."""
     offs = np.zeros(len(seqs) + 1, dtype=np.uint32)
-    for i, s in enumerate(seqs):
-        offs[i + 1] = offs[i] + len(s)
-    flat = np.zeros(max(int(offs[-1]), 1), dtype=np.uint16)
-    k = 0
-    for s in seqs:
-        flat[k:k + len(s)] = s
-        k += len(s)
-    return flat, offs
+    np.cumsum(np.fromiter(map(len, seqs), dtype=np.uint32, count=len(seqs)), out=offs[1:])
+    n = int(offs[-1])
+    flat = np.fromiter(itertools.chain.from_iterable(seqs), dtype=np.uint16, count=n)
+    return (flat if n else np.zeros(1, dtype=np.uint16)), offs
 
 
 class Engine:
