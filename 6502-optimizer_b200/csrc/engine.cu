@@ -676,6 +676,78 @@ __device__ __noinline__ bool sweep_general(const PairView& pv, uint32_t cone, ui
     return sweep_states<4>(pv, make_fields(cone, swept, rep), om, s0, s1, stop, nstates, lane);
 }
 
+// A row's state: the values of the locations of `high` from its index `bits`,
+// the same in every byte; the others at the first value of their range.
+__device__ __forceinline__ St row_state(uint32_t bits, uint32_t high, uint32_t bs, bool rep) {
+    auto field = [&](uint32_t l, uint32_t fixed) -> uint32_t {
+        if (!(high & LB(l))) return fixed * kB1;
+        const uint32_t w = rep ? 5u : 8u, x = bits & ((1u << w) - 1u);
+        bits >>= w;
+        return (rep ? c_rep[x] : x) * kB1;
+    };
+    St in;
+    in.a = 0;
+    in.x = field(L_X, 0); in.y = field(L_Y, 0); in.s = field(L_S, bs); in.m = field(L_M, 0);
+    in.s0 = field(L_S0, 0); in.s1 = field(L_S1, 0);
+    in.p = (high & LB(L_C)) ? (bits & 1u) * kB1 : 0u;
+    return in;
+}
+__device__ __forceinline__ void put_reg(St& s, uint32_t loc, uint32_t v) {
+    if (loc == LB(L_A)) s.a = v;
+    else if (loc == LB(L_X)) s.x = v;
+    else if (loc == LB(L_Y)) s.y = v;
+    else if (loc == LB(L_S)) s.s = v;
+    else if (loc == LB(L_M)) s.m = v;
+    else if (loc == LB(L_S0)) s.s0 = v;
+    else s.s1 = v;
+}
+__device__ __forceinline__ OutMask out_mask4(uint64_t om) {
+    OutMask m = out_mask(om);
+    m.a *= kB1; m.x *= kB1; m.y *= kB1; m.p *= kB1; m.s *= kB1; m.m *= kB1; m.s0 *= kB1; m.s1 *= kB1;
+    return m;
+}
+// Target and candidate on two packed words: nonzero where they differ.
+__device__ __forceinline__ uint32_t words_differ(const PairView& pv, const St (&in)[2], const OutMask& m) {
+    St t[2] = {in[0], in[1]}, c[2] = {in[0], in[1]};
+    for (int i = 0; i < pv.tn; i++) exec_x4n(t, pv.t[i]);
+    for (int i = 0; i < pv.cn; i++) exec_x4n(c, pv.c[i]);
+    return out_diff(t[0], c[0], m) | out_diff(t[1], c[1], m);
+}
+
+// The reduced sweep of a cone without A: its registers have 32 values each (8
+// words).  Rows are the 1,024 states of the two lowest, in 4 steps of two
+// words; lane l holds the lowest one's word l % 8 for good and takes values
+// l / 8 + 4 j of the next.  Where the general sweep takes its place k_exhaustive
+// needs 1.8 ms for a STOKE run's proofs (256 targets of 4 to 8 instructions)
+// instead of 0.7.
+__device__ __noinline__ bool sweep_narrow(const PairView& pv, uint32_t cone, uint32_t low, uint32_t next, uint32_t bs,
+                                          uint64_t om, uint64_t s0, uint64_t s1, const volatile uint32_t* stop,
+                                          unsigned long long* nstates, int lane) {
+    const uint32_t i0 = 4u * ((uint32_t)lane & 7u);
+    const uint32_t v = c_rep[i0] | (c_rep[i0 + 1] << 8) | (c_rep[i0 + 2] << 16) | (c_rep[i0 + 3] << 24);
+    const OutMask m = out_mask4(om);
+    const uint32_t q1 = (uint32_t)(s1 >> 8);
+    for (uint32_t q = (uint32_t)(s0 >> 8); q < q1; q++) {   // steps of 256 states
+        const St row = row_state(q >> 2, cone & ~(low | next), bs, true);
+        St in[2] = {row, row};
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            put_reg(in[k], low, v);
+            put_reg(in[k], next, c_rep[((uint32_t)lane >> 3) + 4u * (2u * (q & 3u) + (uint32_t)k)] * kB1);
+        }
+        if (__any_sync(kFull, words_differ(pv, in, m) != 0)) {
+            if (lane == 0) *nstates += ((uint64_t)(q + 1) << 8) - s0;
+            return false;
+        }
+        if ((q & 31) == 31 && stop) {
+            const uint32_t sv = lane == 0 ? *stop : 0u;   // one read, broadcast: keeps the warp uniform
+            if (__shfl_sync(kFull, sv, 0)) break;
+        }
+    }
+    if (lane == 0) *nstates += s1 - s0;
+    return true;
+}
+
 // The same sweep by rows of 256 states when the cone's lowest field is a
 // whole register (A, or any register under the full sweep) and the range is
 // made of rows.  Lane l holds values 4 l .. 4 l + 3 and 4 l + 128 .. of that
@@ -689,45 +761,23 @@ __device__ __forceinline__ bool sweep_cone(const PairView& pv, uint32_t cone, ui
                                            unsigned long long* nstates, int lane) {
     const uint32_t regs = cone & ~LB(L_C);
     const uint32_t low = (cone & LB(L_A)) ? LB(L_A) : (regs & (0u - regs));   // A first, then X Y S M S0 S1
-    if (low == 0 || (rep && low != LB(L_A)) || ((s0 | s1) & 255))
+    const uint32_t bs = (swept & LB(L_S)) ? 0u : 0xFDu;   // S outside the cone: its first value
+    if (low == 0 || (rep && low != LB(L_A)) || ((s0 | s1) & 255)) {
+        const uint32_t rest = regs & ~low, next = rest & (0u - rest);
+        if (next && !((s0 | s1) & 1023)) return sweep_narrow(pv, cone, low, next, bs, om, s0, s1, stop, nstates, lane);
         return sweep_general(pv, cone, swept, rep, om, s0, s1, stop, nstates, lane);
-    const uint32_t high = cone & ~low, bs = (swept & LB(L_S)) ? 0u : 0xFDu;   // S outside the cone: its first value
+    }
+    const uint32_t high = cone & ~low;
     const uint32_t v0 = 4u * (uint32_t)lane * kB1 + 0x03020100u, v1 = v0 + 0x80808080u;
-    OutMask m = out_mask(om);
-    m.a *= kB1; m.x *= kB1; m.y *= kB1; m.p *= kB1; m.s *= kB1; m.m *= kB1; m.s0 *= kB1; m.s1 *= kB1;
+    const OutMask m = out_mask4(om);
     const uint32_t r1 = (uint32_t)(s1 >> 8);
     for (uint32_t row = (uint32_t)(s0 >> 8); row < r1; row++) {
-        uint32_t bits = row;
-        auto field = [&](uint32_t l, uint32_t fixed) -> uint32_t {   // the row's value of a location, in every byte
-            if (!(high & LB(l))) return fixed * kB1;
-            const uint32_t w = rep ? 5u : 8u, x = bits & ((1u << w) - 1u);
-            bits >>= w;
-            return (rep ? c_rep[x] : x) * kB1;
-        };
-        St in;
-        in.a = 0;
-        in.x = field(L_X, 0); in.y = field(L_Y, 0); in.s = field(L_S, bs); in.m = field(L_M, 0);
-        in.s0 = field(L_S0, 0); in.s1 = field(L_S1, 0);
-        in.p = (high & LB(L_C)) ? (bits & 1u) * kB1 : 0u;
-        St t[2], c[2];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const uint32_t v = k ? v1 : v0;
-            c[k] = in;
-            if (low == LB(L_A)) c[k].a = v;
-            else if (low == LB(L_X)) c[k].x = v;
-            else if (low == LB(L_Y)) c[k].y = v;
-            else if (low == LB(L_S)) c[k].s = v;
-            else if (low == LB(L_M)) c[k].m = v;
-            else if (low == LB(L_S0)) c[k].s0 = v;
-            else c[k].s1 = v;
-            t[k] = c[k];
-        }
-        for (int i = 0; i < pv.tn; i++) exec_x4n(t, pv.t[i]);
-        for (int i = 0; i < pv.cn; i++) exec_x4n(c, pv.c[i]);
-        const uint32_t d = out_diff(t[0], c[0], m) | out_diff(t[1], c[1], m);
-        if (__any_sync(kFull, d != 0)) {
-            if (lane == 0) *nstates += ((uint64_t)row << 8) + 256 - s0;
+        const St at = row_state(row, high, bs, rep);
+        St in[2] = {at, at};
+        put_reg(in[0], low, v0);
+        put_reg(in[1], low, v1);
+        if (__any_sync(kFull, words_differ(pv, in, m) != 0)) {
+            if (lane == 0) *nstates += ((uint64_t)(row + 1) << 8) - s0;
             return false;
         }
         if ((row & 31) == 31 && stop) {
