@@ -1437,8 +1437,8 @@ __global__ void __launch_bounds__(256, 4) k_expand(const Surv* __restrict__ matc
     const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;   // compared bits of a packed P word
     unsigned long long nqc = 0, nmid = 0, nrej = 0;
     const uint32_t nmatch = (uint32_t)cnt->matches;
-    int g = 4;   // lanes per match, log2
-    for (uint64_t warps = (uint64_t)gridDim.x * kWarpsPerBlock * 2; g > 0 && nmatch > warps; g--) warps <<= 1;
+    int g = 5;   // lanes per match, log2
+    for (uint64_t warps = (uint64_t)gridDim.x * kWarpsPerBlock; g > 0 && nmatch > warps; g--) warps <<= 1;
     const uint32_t sub = (uint32_t)lane & ((1u << g) - 1u), per = 32u >> g;
     for (uint64_t base = ((uint64_t)blockIdx.x * kWarpsPerBlock + w) * per; base < nmatch;
          base += (uint64_t)gridDim.x * kWarpsPerBlock * per) {
@@ -2754,7 +2754,7 @@ int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt
     CKL("k_qc_join");
     const uint16_t* mult = go ? nullptr : join_mult(ctx, dead);
     const uint32_t* lines = (const uint32_t*)ctx->join_lines[dead].p;
-    const uint32_t egrid = (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 4, (nt + 255) / 256);
+    const uint32_t egrid = (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 4, (nt + kWarpsPerBlock - 1) / kWarpsPerBlock);
     auto expand = [&](auto kernel) {
         kernel<<<egrid, 256, 0, ctx->stream>>>(match, d_t, tlen, cfp4, tab, dead, cfg.sweep, mult, lines, (Surv*)ctx->surv.p,
                                                scap, cnt, (Surv*)ctx->go_round.p, (uint32_t*)ctx->go_ord.p,
