@@ -3600,7 +3600,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 st->pairs += nt * (uint64_t)kNumInsns;
                 st->qc_hits += c.qc;
                 st->mid_hits += c.mid;
-                st->exh_checked += exh ? c.mid : 0;   // every MidCheck survivor, the join's probe included
+                st->exh_checked += exh ? c.mid : 0;   // every MidCheck survivor, the filtered ones included
                 st->exh_passed += c.exh_pass;
                 st->exh_states += c.states;
                 st->exh_items += c.v[0][0].items;

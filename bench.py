@@ -30,7 +30,6 @@ import sys
 import tempfile
 import time
 
-PROBE_STATES = 128   # random domain states k_exhaustive tries on every pair before its cone sweeps
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, os.path.join(ROOT, "6502-optimizer_b200"))
 
@@ -322,8 +321,7 @@ def run_engine(args):
         exh_ms = avg("ms_exhaustive") + avg("ms_exh_items")
         qc_ms = avg("ms_qc")
         exh_achieved = s0["exh_algo_ops"] / (exh_ms / 1e3) if exh_ms > 0 else 0.0
-        exh_exec = ((s0["exh_states"] + PROBE_STATES * s0["exh_checked"]) * (10 * 3 + 3) / (exh_ms / 1e3)
-                    if exh_ms > 0 else 0.0)
+        exh_exec = s0["exh_states"] * (10 * 3 + 3) / (exh_ms / 1e3) if exh_ms > 0 else 0.0
         qc_algo = 13 * s0["pairs"] + 13 * (7 + 24) * s0["qc_hits"]
         qc_achieved = qc_algo / (qc_ms / 1e3) if qc_ms > 0 else 0.0
         stages = {"fingerprint_ms": avg("ms_fingerprint"), "qc_mid_ms": qc_ms,
@@ -332,16 +330,16 @@ def run_engine(args):
         dominant = max(("k_exhaustive", avg("ms_exhaustive")), ("k_exh_items", avg("ms_exh_items")),
                        ("k_qc_join", qc_ms), key=lambda kv: kv[1])[0]
         figs, figs_source = load_profile_figures()
-        # the exhaustive stage's events bracket the probe kernel and k_exhaustive
-        exh_kernels = ("k_probe_pairs", "k_exhaustive", "k_exh_items")
+        # the QC stage's events bracket k_qc_join and k_expand, the exhaustive
+        # stage's k_small and k_exhaustive
+        exh_kernels = ("k_small", "k_exhaustive", "k_exh_items")
         if dominant == "k_qc_join":
             achieved, alg = qc_achieved, "13 ops/pair + 31x13 ops per QC hit (QC+MidCheck)"
-            kernels, ktime = ("k_qc_join",), qc_ms
+            kernels, ktime = ("k_qc_join", "k_expand"), qc_ms
         else:
-            # states the exhaustive stage's kernels evaluated (cone sweeps, work items
-            # and the 128-state random probes) at the convention's 10 ops per
-            # executed instruction + 3 per compare
-            achieved, alg = exh_exec, ("states evaluated (cone sweeps + items + 128-state probes) x "
+            # states the exhaustive stage's kernels evaluated (cone sweeps and work
+            # items) at the convention's 10 ops per executed instruction + 3 per compare
+            achieved, alg = exh_exec, ("states evaluated (cone sweeps + items) x "
                                        "(10 ops/instruction x 3 instructions + 3)")
             kernels, ktime = exh_kernels, exh_ms
         traffic = sum(figs[k]["traffic"] for k in kernels if k in figs) if all(k in figs for k in kernels) else None
@@ -387,10 +385,10 @@ def run_engine(args):
             "clocks": {"sm_mhz": clk["sm_mhz"], "sm_max_mhz": clk["sm_max_mhz"], "reasons": clk["reasons"]},
             "e2e": {"value": e2e_value, "unit": "pair-checks/s", "h2d_bytes_per_step": int(shard.nbytes),
                     "d2h_bytes_per_step": int(e2e_rules * 16 + 8 * 16 * s0["passes"])},
-            # per pass: QC join, exhaustive, work items, emit (the join computes the
-            # targets' outputs itself, so no fingerprint launch); per search: the
-            # opcode check of the targets
-            "gpu_launches": int((4 * s0["passes"] + 1) * args.steps),
+            # per pass: opcode check, QC join, expansion, small cones, exhaustive, work
+            # items, emit (the join computes the targets' outputs itself, so no
+            # fingerprint launch)
+            "gpu_launches": int(7 * s0["passes"] * args.steps),
         }
         line["config"]["tuning"] = dict(tuned, source=tune_source, calibration_ms=tune_ms,
                                         trace=m6502.Engine.tune_trace(tune_path) if args.tune != "default" else [])

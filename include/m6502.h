@@ -131,8 +131,8 @@ typedef struct m6502_stats {
     uint64_t exh_algo_ops; /* algorithmic ops of the accepted pairs: product-sweep
                               states x (10 per executed instruction + 3) */
     uint64_t passes;      /* device passes (blocks of targets) */
-    uint64_t exh_probe_rejects; /* pairs a random-state probe of the sweep domain
-                              rejected before the cone analysis */
+    uint64_t exh_probe_rejects; /* pairs rejected before the cone analysis by the line
+                              filter or a random-state probe of the sweep domain */
     double ms_device;     /* device time of the whole call, CUDA events */
     double ms_fingerprint, ms_qc, ms_exhaustive, ms_exh_items, ms_emit; /* per-stage
                               device time summed over passes, CUDA events */
