@@ -1901,6 +1901,23 @@ __global__ void __launch_bounds__(256) k_go_join2_items(Join2Args a) {
     join_counts(a.cnt, nqc, nqc);
 }
 
+// First ticket of a warp of a persistent grid: its own number, counted across
+// the blocks first, so that few pairs spread over the SMs.  Later tickets come
+// from a counter that starts behind those.  A launch with few pairs or none, as
+// in most rounds past the first, then costs neither an atomic per warp on one
+// address nor the tables of idle blocks (empty launches took 6.1 us in k_small
+// and 8.2 in k_exhaustive): one target 280 -> 227 us, 4,096 length-3 targets
+// 914 -> 832.  Not for k_exh_items, whose items outnumber its warps where they
+// count (0.6 % of the count at mask 0xFF slower): its idle blocks only leave.
+__device__ __forceinline__ unsigned long long first_ticket(unsigned long long batch) {
+    return ((unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * batch;
+}
+__device__ __forceinline__ unsigned long long later_ticket(unsigned long long* ctr, unsigned long long batch,
+                                                           unsigned long long n) {
+    const unsigned long long taken = (unsigned long long)gridDim.x * kWarpsPerBlock * batch;
+    return taken >= n ? n : taken + atomicAdd(ctr, batch);
+}
+
 // Exhaustive check, one pair per warp (persistent, device ticket).
 // MINB: resident 256-thread blocks per SM the register cap is set for (4:
 // 64 registers, 3: 80, 2: 128); the autotuner picks the variant.
@@ -1909,10 +1926,11 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
                                                         uint64_t n_cap, ExhArgs a) {
     __shared__ uint16_t s_t[kWarpsPerBlock][kMaxSeq], s_c[kWarpsPerBlock][kMaxSeq];
     __shared__ alignas(16) uint16_t s_dep[NUM_OPS][16];
-    for (int i = threadIdx.x; i < (int)NUM_OPS * 2; i += blockDim.x) reinterpret_cast<uint4*>(&s_dep[0][0])[i] = g_dep16[i];
-    __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t n = min((uint64_t)*n_pairs_ptr, n_cap);
+    if (blockIdx.x >= n) return;   // no warp of this block has a pair
+    for (int i = threadIdx.x; i < (int)NUM_OPS * 2; i += blockDim.x) reinterpret_cast<uint4*>(&s_dep[0][0])[i] = g_dep16[i];
+    __syncthreads();
     unsigned long long nstates = 0, probe_rej = 0;
     __shared__ TargetCache s_tc[kWarpsPerBlock];   // the warp's last target: probe outputs, composition
     TargetCache& tc = s_tc[threadIdx.x >> 5];
@@ -1928,12 +1946,12 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
     // Lane 0 claims the following batch while the warp works on the current
     // one, so the atomic's latency is hidden behind a batch of pairs.
     unsigned long long ahead = 0;
-    if (lane == 0) ahead = atomicAdd(&a.v->exh_ticket, tbatch);
+    if (lane == 0) ahead = first_ticket(tbatch);
     for (;;) {
         if (next >= lim) {
             next = __shfl_sync(kFull, ahead, 0);
             lim = next + tbatch;
-            if (lane == 0 && next < n) ahead = atomicAdd(&a.v->exh_ticket, tbatch);
+            if (lane == 0 && next < n) ahead = later_ticket(&a.v->exh_ticket, tbatch, n);
         }
         const unsigned long long q = next++;
         if (q >= n) break;
@@ -2052,10 +2070,11 @@ __global__ void __launch_bounds__(256) k_small(Src src, const unsigned long long
                                                ExhArgs a, uint32_t* __restrict__ order) {
     __shared__ uint16_t s_ins[Src::kMaxT + Src::kMaxC][256];
     __shared__ alignas(16) uint16_t s_dep[NUM_OPS][16];
-    for (int i = threadIdx.x; i < (int)NUM_OPS * 2; i += blockDim.x) reinterpret_cast<uint4*>(&s_dep[0][0])[i] = g_dep16[i];
-    __syncthreads();
     const int lane = threadIdx.x & 31;
     const uint64_t n = min((uint64_t)*n_pairs_ptr, n_cap);
+    if (blockIdx.x >= n) return;   // no warp of this block has a pair
+    for (int i = threadIdx.x; i < (int)NUM_OPS * 2; i += blockDim.x) reinterpret_cast<uint4*>(&s_dep[0][0])[i] = g_dep16[i];
+    __syncthreads();
     // Lanes per pair (log2): a warp while that fills the chip, then fewer.
     int g = 5;
     for (uint64_t warps = (uint64_t)gridDim.x * kWarpsPerBlock; g > kSmallLanesLog2 && n > warps; g--) warps <<= 1;
@@ -2069,14 +2088,14 @@ __global__ void __launch_bounds__(256) k_small(Src src, const unsigned long long
     // the pair's sequences: one column of the staging array for its lanes
     uint16_t *st = &s_ins[0][(threadIdx.x & ~31u) + lead], *sc = st + Src::kMaxT * 256;
     unsigned long long nstates = 0, next = 0;
-    if (lane == 0) next = atomicAdd(&a.v->small_ticket, batch);
+    if (lane == 0) next = first_ticket(batch);
     uint64_t first = 0, upto = 0;
     for (;; first += per) {
         if (first >= upto) {
             first = __shfl_sync(kFull, next, 0);
             if (first >= n) break;
             upto = first + batch;
-            if (lane == 0) next = atomicAdd(&a.v->small_ticket, batch);
+            if (lane == 0) next = later_ticket(&a.v->small_ticket, batch, n);
         }
         const uint64_t p = first + (uint32_t)(lane >> g);
         int tn = 0, cn = 0;
@@ -2160,6 +2179,7 @@ __global__ void __launch_bounds__(256) k_exh_items(Src src, ExhArgs a) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t n = min((uint64_t)a.v->items, a.item_cap);
     unsigned long long nstates = 0;
+    if (blockIdx.x >= n) return;   // the block's warps would find nothing
     for (;;) {
         unsigned long long q = 0;
         if (lane == 0) q = atomicAdd(&a.v->item_ticket, 1ull);
@@ -2733,15 +2753,18 @@ int launch_exh(m6502_ctx* ctx, const SurvSource& src, const unsigned long long* 
 // the value at n_ptr, at most cap.
 template <class Src>
 int launch_verify(m6502_ctx* ctx, const Src& src, const unsigned long long* n_ptr, uint64_t cap, ExhArgs ea) {
+    // A block per pair while that leaves blocks idle, then every resident one: a
+    // thread per pair as the size filled half the chip at 20,011 pairs and one
+    // SM at 48 (335 -> 278 and 135 -> 116 us, with the tickets above).
+    const uint64_t blocks = std::max<uint64_t>(cap, 1);
     if (!ea.brute) {
-        const uint64_t need = (cap + 255) / 256;
-        k_small<Src, true><<<(unsigned)std::min<uint64_t>(ctx->sms * 4, std::max<uint64_t>(need, 1)), 256, 0, ctx->stream>>>(
+        k_small<Src, true><<<(unsigned)std::min<uint64_t>(ctx->small_blocks, blocks), 256, 0, ctx->stream>>>(
             src, n_ptr, cap, ea, (uint32_t*)ctx->order.p);
         CKL("k_small");
         ea.order = (const uint32_t*)ctx->order.p;
         n_ptr = &ea.v->small_left;
     }
-    k_exhaustive<Src><<<ctx->exh_blocks, 256, 0, ctx->stream>>>(src, n_ptr, cap, ea);
+    k_exhaustive<Src><<<(unsigned)std::min<uint64_t>(ctx->exh_blocks, blocks), 256, 0, ctx->stream>>>(src, n_ptr, cap, ea);
     CKL("k_exhaustive");
     k_exh_items<Src><<<ctx->exh_item_blocks, 256, 0, ctx->stream>>>(src, ea);
     CKL("k_exh_items");
