@@ -489,7 +489,8 @@ enum : uint32_t { X4C_IMM = 1u << 9, X4C_DUP = 1u << 10, X4C_ADD = 1u << 11, X4C
 struct X4Row {
     uint32_t ctl;       // slots of a (bits 0-2), m (3-5) and the result (6-8), X4C_*, kind of the branching ones (13-15)
     uint32_t konst;     // added to the operand word (INC, DEC)
-    uint32_t pad[2];
+    uint32_t imm;       // the operand word is the instruction's byte times this: kB1, or 0 where it has none (INC, DEC)
+    uint32_t pad;
     uint32_t keep, upd, set;   // P: bits kept, taken from the new flags, set
     uint32_t inv;       // operand inverted
     uint32_t ka, k1, k2;       // logic unit: ((a & ka) & m & k1) | (((a & ka) ^ m) & k2)
@@ -499,7 +500,7 @@ struct X4Row {
 M6502_HD X4Row x4_row(uint32_t op) {
     const uint32_t d = x4_desc(op), src = (d >> 4) & 7u, dst = (d >> 7) & 7u, sub = (d >> 10) & 3u;
     const uint32_t all = 0xFFFFFFFFu, nz = (kFlagN | kFlagZ) * kB1, nzc = nz | kFlagC * kB1;
-    X4Row r{X4S_NONE << 6, 0, {0, 0}, all, 0, 0, 0, 0, 0, 0, 0};
+    X4Row r{X4S_NONE << 6, 0, kB1, 0, all, 0, 0, 0, 0, 0, 0, 0};
     // The register numbers of x4_desc (A X Y S M, 7 = immediate) are the slots'.
     auto ctl = [&](uint32_t a, uint32_t m, uint32_t out) {
         r.ctl = a | (m == X4R_IMM ? X4C_IMM : m << 3) | out << 6;
@@ -508,7 +509,7 @@ M6502_HD X4Row x4_row(uint32_t op) {
     switch (d & 15u) {
     case X4_MOVE_NZ: ctl(0, src, dst); r.k2 = all; flags(nz); break;
     case X4_MOVE: ctl(0, src, dst); r.k2 = all; break;
-    case X4_INCDEC: ctl(dst, X4R_IMM, dst); r.ctl |= X4C_ADD; r.konst = sub ? all : kB1; flags(nz); break;
+    case X4_INCDEC: ctl(dst, X4R_IMM, dst); r.ctl |= X4C_ADD; r.konst = sub ? all : kB1; r.imm = 0; flags(nz); break;
     case X4_SHIFT:
         ctl(dst, 0, dst);
         r.ctl |= (sub & 1u) ? X4C_RIGHT : X4C_ADD | X4C_DUP;   // left: a + a
@@ -533,7 +534,7 @@ M6502_HD X4Row x4_row(uint32_t op) {
 // in st and p.
 M6502_HD void exec_x4r(uint32_t* st, int stride, uint32_t& p, const X4Row& q, uint32_t insn) {
     const uint32_t a = st[(q.ctl & 7u) * stride], mr = st[((q.ctl >> 3) & 7u) * stride];
-    const uint32_t m = (q.ctl & X4C_IMM) ? (insn >> 8) * kB1 + q.konst : mr;
+    const uint32_t m = (q.ctl & X4C_IMM) ? (insn >> 8) * q.imm + q.konst : mr;
     const uint32_t b = (q.ctl & X4C_DUP) ? a : m ^ q.inv;
     uint32_t co;
     const uint32_t sum = x4_add(a, b, (p & q.carry & kB1) | ((q.carry >> 1) & kB1), co);
