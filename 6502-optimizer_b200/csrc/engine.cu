@@ -2666,6 +2666,8 @@ struct m6502_ctx {
     DevBuf join_tab[2][256];                      // JoinTable by semantics and dead-flags mask
     DevBuf join_groups[256];                      // CandGroups of the CUDA-semantics tables
     DevBuf join_lines[256];                       // line hashes of the candidates, [64 register sets][2863]
+    bool join_built[2][256] = {};                 // tables and groups are filled, or their copies are on the stream
+    bool lines_built[256] = {};
     struct Cand2Table {            // sorted (key, entry) of all length-2 sequences for one mask
         uint32_t dead = 0xFFFFFFFFu;
         uint32_t longest = 0;      // longest range of one key
@@ -2851,8 +2853,8 @@ int init_ctx(m6502_ctx* ctx) {
     uint32_t vec4[8][8];
     for (int g = 0; g < 8; g++)
         for (int f = 0; f < 8; f++) vec4[g][f] = pack4(vec + 4 * g, f);
-    CK(cudaMemcpyToSymbol(c_vec, vec, sizeof vec));
-    CK(cudaMemcpyToSymbol(c_vec4, vec4, sizeof vec4));
+    CK(cudaMemcpyToSymbolAsync(c_vec, vec, sizeof vec, 0, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyToSymbolAsync(c_vec4, vec4, sizeof vec4, 0, cudaMemcpyHostToDevice, ctx->stream));
     // Line states: A = i, the other registers a permutation of it each, the
     // carry the parity of i.
     uint32_t line[64][8];
@@ -2867,28 +2869,28 @@ int init_ctx(m6502_ctx* ctx) {
         }
         for (int f = 0; f < 8; f++) line[j][f] = pack4(st, f);
     }
-    CK(cudaMemcpyToSymbol(c_line, line, sizeof line));
-    CK(cudaMemcpyToSymbol(c_dep, dep, sizeof dep));
-    CK(cudaMemcpyToSymbol(c_wr, wr, sizeof wr));
+    CK(cudaMemcpyToSymbolAsync(c_line, line, sizeof line, 0, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyToSymbolAsync(c_dep, dep, sizeof dep, 0, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyToSymbolAsync(c_wr, wr, sizeof wr, 0, cudaMemcpyHostToDevice, ctx->stream));
     uint16_t dep16[NUM_OPS][16] = {};
     for (uint32_t op = 0; op < NUM_OPS; op++)
         for (uint32_t l = 0; l < NUM_LOCS; l++) dep16[op][l] = dep[op][l];
-    CK(cudaMemcpyToSymbol(g_dep16, dep16, sizeof dep16));
-    CK(cudaMemcpyToSymbol(c_sweep, sw, sizeof sw));
+    CK(cudaMemcpyToSymbolAsync(g_dep16, dep16, sizeof dep16, 0, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyToSymbolAsync(c_sweep, sw, sizeof sw, 0, cudaMemcpyHostToDevice, ctx->stream));
     uint32_t x4[NUM_OPS];
     for (uint32_t op = 0; op < NUM_OPS; op++) x4[op] = x4_desc(op);
-    CK(cudaMemcpyToSymbol(c_x4d, x4, sizeof x4));
+    CK(cudaMemcpyToSymbolAsync(c_x4d, x4, sizeof x4, 0, cudaMemcpyHostToDevice, ctx->stream));
     X4Row rows[NUM_OPS];
     static_assert(sizeof(X4Row) == 3 * sizeof(uint4), "three words of 16 bytes");
     for (uint32_t op = 0; op < NUM_OPS; op++) rows[op] = x4_row(op);
-    CK(cudaMemcpyToSymbol(g_x4row, rows, sizeof rows));
-    CK(cudaMemcpyToSymbol(c_tab, tab, sizeof tab));
-    CK(cudaMemcpyToSymbol(c_gotab, gotab, sizeof gotab));
-    CK(cudaMemcpyToSymbol(c_gorank, gorank, sizeof gorank));
+    CK(cudaMemcpyToSymbolAsync(g_x4row, rows, sizeof rows, 0, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyToSymbolAsync(c_tab, tab, sizeof tab, 0, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyToSymbolAsync(c_gotab, gotab, sizeof gotab, 0, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyToSymbolAsync(c_gorank, gorank, sizeof gorank, 0, cudaMemcpyHostToDevice, ctx->stream));
     static uint16_t goidx[kNumInsns];
     for (int i = 0; i < kNumInsns; i++) goidx[gorank[i]] = (uint16_t)i;
-    CK(cudaMemcpyToSymbol(c_goidx, goidx, sizeof goidx));
-    CK(cudaMemcpyToSymbol(c_rep, rep, sizeof rep));
+    CK(cudaMemcpyToSymbolAsync(c_goidx, goidx, sizeof goidx, 0, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyToSymbolAsync(c_rep, rep, sizeof rep, 0, cudaMemcpyHostToDevice, ctx->stream));
 
     int occ = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_exhaustive<SurvSource>, 256, 0));
@@ -2963,7 +2965,7 @@ int cand_group(uint32_t op, uint32_t dead) {
 // one entry per group of candidates; Go semantics: every candidate (its
 // passes and ranks tell the members of a group apart).
 int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
-    if (ctx->join_tab[go][dead].p) return M6502_OK;
+    if (ctx->join_built[go][dead]) return M6502_OK;
     const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;
     struct Entry {
         uint64_t key;
@@ -3017,11 +3019,13 @@ int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
     for (; bucket <= (1u << kDirBits); bucket++) t.dir[bucket] = (uint16_t)nu;
     for (uint32_t u = 0; go && u < nu; u++)
         ctx->join_longest[dead] = std::max<uint32_t>(ctx->join_longest[dead], t.start[t.sub[u + 1]] - t.start[t.sub[u]]);
-    if (!ctx->join_lines[dead].p) {
+    if (!ctx->lines_built[dead]) {
         TRY(ensure(ctx, ctx->join_lines[dead], 64 * kNumInsns * sizeof(uint32_t)));
         k_line_hash<<<(64 * kNumInsns + 255) / 256, 256, 0, ctx->stream>>>(dead, (uint32_t*)ctx->join_lines[dead].p);
         CKL("k_line_hash");
+        ctx->lines_built[dead] = true;
     }
+    // The copies go on the stream of the kernels that read them.
     if (!go) {
         uint16_t at = 0;
         for (const auto& e : groups) {
@@ -3033,10 +3037,11 @@ int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
             for (uint32_t i = t.start[t.sub[u]]; i < t.start[t.sub[u + 1]]; i++)
                 for (uint32_t b = t.cand[i] >> 12; b <= 2; b++) t.weight[u][b - 1] += gr.mult[t.cand[i] & 0xFFFu];
         TRY(ensure(ctx, ctx->join_groups[dead], sizeof gr));
-        CK(cudaMemcpy(ctx->join_groups[dead].p, &gr, sizeof gr, cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->join_groups[dead].p, &gr, sizeof gr, cudaMemcpyHostToDevice, ctx->stream));
     }
     TRY(ensure(ctx, ctx->join_tab[go][dead], sizeof t));
-    CK(cudaMemcpy(ctx->join_tab[go][dead].p, &t, sizeof t, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->join_tab[go][dead].p, &t, sizeof t, cudaMemcpyHostToDevice, ctx->stream));
+    ctx->join_built[go][dead] = true;
     return M6502_OK;
 }
 
@@ -4288,7 +4293,8 @@ int static_setup(int dev, StaticDevice** out) {
             cudaMemcpyToSymbol(c_wr, wr, sizeof wr) != cudaSuccess ||
             cudaMemcpyToSymbol(c_sweep, sw, sizeof sw) != cudaSuccess ||
             cudaMemcpyToSymbol(c_x4d, x4, sizeof x4) != cudaSuccess ||
-            cudaMemcpyToSymbol(c_rep, rep, sizeof rep) != cudaSuccess)
+            cudaMemcpyToSymbol(c_rep, rep, sizeof rep) != cudaSuccess ||
+            cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)   // the caller's stream does not wait for that one
             return M6502_E_CUDA;
         void* ptr = nullptr;
         if (cudaGetSymbolAddress(&ptr, g_static_scratch) != cudaSuccess || !ptr) return M6502_E_CUDA;
