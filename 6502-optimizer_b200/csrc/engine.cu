@@ -2643,6 +2643,7 @@ struct m6502_ctx {
     void* h_io = nullptr;                         // page-locked side of it
     size_t h_io_bytes = 0;
     std::string err;
+    bool failed = false;                          // this call reported an error (see Call)
     std::mutex mu;
     int sms = 148;
     int exh_blocks = 0, exh_item_blocks = 0, qc_blocks = 0, fp_blocks = 0, small_blocks = 0;
@@ -2687,8 +2688,26 @@ namespace {
 
 int set_err(m6502_ctx* ctx, int code, const std::string& msg) {
     ctx->err = msg;
+    ctx->failed = ctx->failed || code != M6502_OK;
     return code;
 }
+
+// A call into the context: holds its lock, and when the call failed ends what
+// it queued before it returns.  Copies from and to the caller's memory (which
+// the device reads and writes by itself where it is page-locked) do not
+// outlive the call, the next one does not overwrite buffers that kernels still
+// read, and its launch checks do not meet this call's error.
+struct Call {
+    m6502_ctx* ctx;
+    std::lock_guard<std::mutex> lk;
+    explicit Call(m6502_ctx* c) : ctx(c), lk(c->mu) { ctx->failed = false; }
+    ~Call() {
+        if (!ctx->failed) return;
+        cudaStreamSynchronize(ctx->copy);
+        cudaStreamSynchronize(ctx->stream);
+        cudaGetLastError();
+    }
+};
 
 #define CK(call)                                                                            \
     do {                                                                                    \
@@ -3893,7 +3912,7 @@ int m6502_check_pairs(m6502_ctx* ctx, uint64_t n, const uint16_t* t_insns, const
                       uint32_t checks, uint32_t sweep, uint32_t exh_mode, uint8_t* out,
                       uint8_t* flagdiff) {
     if (!ctx) return M6502_E_INVAL;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    Call call(ctx);
     if (n == 0) return M6502_OK;
     if (!t_insns || !t_offs || !c_insns || !c_offs || !out) return set_err(ctx, M6502_E_INVAL, "NULL buffer");
     if (sweep > M6502_SWEEP_FULL || exh_mode > M6502_EXH_BRUTE) return set_err(ctx, M6502_E_INVAL, "bad sweep mode");
@@ -3979,7 +3998,7 @@ int m6502_check_pairs(m6502_ctx* ctx, uint64_t n, const uint16_t* t_insns, const
 
 int m6502_fingerprint(m6502_ctx* ctx, uint64_t n, const uint16_t* insns, const uint32_t* offs, uint8_t* out) {
     if (!ctx) return M6502_E_INVAL;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    Call call(ctx);
     if (n == 0) return M6502_OK;
     if (!insns || !offs || !out) return set_err(ctx, M6502_E_INVAL, "NULL buffer");
     for (uint64_t i = 0; i < n; i++) {
@@ -4008,7 +4027,7 @@ int m6502_fingerprint(m6502_ctx* ctx, uint64_t n, const uint16_t* insns, const u
 int m6502_exec_batch(m6502_ctx* ctx, uint64_t n, const uint16_t* insns, const uint32_t* offs,
                      const uint64_t* states_in, uint64_t* states_out) {
     if (!ctx) return M6502_E_INVAL;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    Call call(ctx);
     if (n == 0) return M6502_OK;
     if (!insns || !offs || !states_in || !states_out) return set_err(ctx, M6502_E_INVAL, "NULL buffer");
     for (uint64_t i = 0; i < n; i++)
@@ -4034,7 +4053,7 @@ int m6502_exec_batch(m6502_ctx* ctx, uint64_t n, const uint16_t* insns, const ui
 
 int m6502_fetch_rules(m6502_ctx* ctx, m6502_rule* out, uint64_t cap, uint64_t* n_out) {
     if (!ctx) return M6502_E_INVAL;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    Call call(ctx);
     if (cap && !out) return set_err(ctx, M6502_E_INVAL, "NULL out");
     return finish(ctx, out, cap, n_out);
 }
@@ -4042,7 +4061,7 @@ int m6502_fetch_rules(m6502_ctx* ctx, m6502_rule* out, uint64_t cap, uint64_t* n
 int m6502_search(m6502_ctx* ctx, const m6502_search_cfg* cfg, const uint16_t* targets, uint64_t n,
                  uint32_t tlen, m6502_rule* out, uint64_t cap, uint64_t* n_out, m6502_stats* stats) {
     if (!ctx) return M6502_E_INVAL;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    Call call(ctx);
     TRY(check_cfg(ctx, cfg));
     if (tlen < 1 || tlen > 3) return set_err(ctx, M6502_E_INVAL, "target length must be 1..3");
     if (n > 0xFFFFFFFFull) return set_err(ctx, M6502_E_INVAL, "too many targets for one call");
@@ -4081,11 +4100,7 @@ int m6502_search(m6502_ctx* ctx, const m6502_search_cfg* cfg, const uint16_t* ta
         TRY(run_pass(ctx, *cfg, d_t, nt, tlen, nullptr, b, sink, &st));
     }
     if (async_ok && n) {
-        const int rc = search_async(ctx, *cfg, q_targets, on_dev ? nullptr : targets, n, tlen, &st, sink);
-        if (rc != M6502_OK) {   // no copy from the caller's memory outlives the call
-            cudaStreamSynchronize(ctx->copy);
-            return rc;
-        }
+        TRY(search_async(ctx, *cfg, q_targets, on_dev ? nullptr : targets, n, tlen, &st, sink));
     }
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     CK(cudaEventSynchronize(ctx->ev1));
@@ -4103,7 +4118,7 @@ int m6502_search(m6502_ctx* ctx, const m6502_search_cfg* cfg, const uint16_t* ta
 int m6502_enumerate(m6502_ctx* ctx, const m6502_search_cfg* cfg, uint32_t tlen, uint32_t first,
                     uint32_t last, m6502_rule* out, uint64_t cap, uint64_t* n_out, m6502_stats* stats) {
     if (!ctx) return M6502_E_INVAL;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    Call call(ctx);
     TRY(check_cfg(ctx, cfg));
     if (tlen < 2 || tlen > 3) return set_err(ctx, M6502_E_INVAL, "enumeration length must be 2 or 3");
     if (last > (uint32_t)kNumInsns) last = kNumInsns;
@@ -4153,14 +4168,14 @@ int m6502_enumerate(m6502_ctx* ctx, const m6502_search_cfg* cfg, uint32_t tlen, 
 
 int m6502_tune_get(m6502_ctx* ctx, m6502_tune* out) {
     if (!ctx || !out) return M6502_E_INVAL;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    Call call(ctx);
     *out = ctx->tune;
     return M6502_OK;
 }
 
 int m6502_tune_set(m6502_ctx* ctx, const m6502_tune* t) {
     if (!ctx || !t) return M6502_E_INVAL;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    Call call(ctx);
     if (!tune_valid(*t)) return set_err(ctx, M6502_E_INVAL, "tuning knob out of range");
     ctx->tune = *t;
     return M6502_OK;
@@ -4183,7 +4198,7 @@ int m6502_autotune(m6502_ctx* ctx, const char* cache_path, uint32_t flags, m6502
     const uint64_t span = (uint64_t)kNumInsns * kNumInsns;
     unsigned long long nt = 0;
     {
-        std::lock_guard<std::mutex> lk(ctx->mu);
+        Call call(ctx);
         CK(cudaSetDevice(ctx->device));
         TRY(ensure(ctx, tg, span * 2 * sizeof(uint16_t)));
         TRY(ensure(ctx, ids, span * sizeof(uint64_t)));

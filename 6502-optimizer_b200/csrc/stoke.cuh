@@ -646,7 +646,7 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
                     uint32_t n_targets, m6502_stoke_result* results, m6502_stoke_proof* proofs, uint64_t cap,
                     uint64_t* n_proofs, m6502_stoke_stats* stats) {
     if (!ctx) return M6502_E_INVAL;
-    std::lock_guard<std::mutex> lk(ctx->mu);
+    Call call(ctx);
     if (!cfg || !t_insns || !t_offs || (n_targets && !results)) return set_err(ctx, M6502_E_INVAL, "NULL argument");
     if (cfg->cost > M6502_COST_HAMMING || cfg->sweep > M6502_SWEEP_FULL || cfg->max_len > (uint32_t)kMaxSeq)
         return set_err(ctx, M6502_E_INVAL, "bad STOKE configuration");

@@ -150,19 +150,6 @@ int main(int argc, char** argv) {
             m6502_destroy(ctx);
             cudaGetLastError();
         }
-        if (!errors || s.kind || s.semantics != M6502_SEM_CUDA) continue;
-        // The caller's own work on the engine's stream writes the targets.
-        ctx = create(s);
-        fake::main_stream = (cudaStream_t)m6502_stream(ctx);
-        std::vector<uint16_t>* t = &b.t;
-        fake::enqueue(fake::main_stream, [t] { for (uint16_t& w : *t) w = 0x061A; });
-        want_target = 0x061A;
-        wrong = false;
-        expect(call(ctx, s, b) == M6502_OK, "fails", s.name, 0);
-        expect(!wrong, "targets were read before the stream's earlier work", s.name, 0);
-        want_target = 0;
-        fake::main_stream = nullptr;
-        m6502_destroy(ctx);
     }
     std::printf("%ld failures\n", bad);
     return bad ? 1 : 0;
