@@ -3612,6 +3612,9 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 const uint64_t b = p * P, nt = std::min(P, n - b);
                 // a single pass has nothing to run beside: its copy goes on the same stream
                 const cudaStream_t cs = npass > 1 ? ctx->copy : ctx->stream;
+                // not before what was on the context's stream when the call began: the caller's
+                // own work there may write the targets
+                if (npass > 1 && p == 0) CK(cudaStreamWaitEvent(ctx->copy, ctx->ev0, 0));
                 CK(cudaMemcpyAsync((void*)(targets + b * tlen), host + b * tlen, nt * tlen * sizeof(uint16_t),
                                    cudaMemcpyHostToDevice, cs));
                 if (npass > 1) {

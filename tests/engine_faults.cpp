@@ -11,6 +11,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <set>
+#include <string>
 #include <vector>
 
 #include "fake_cuda.h"
@@ -99,8 +100,25 @@ static m6502_ctx* create(const Scenario& s) {
     return ctx;
 }
 
+// The caller's own work on the engine's stream writes the targets: they are
+// read after it.
+static void read_in_order(const Scenario& s, Buffers& b) {
+    m6502_ctx* ctx = create(s);
+    fake::main_stream = (cudaStream_t)m6502_stream(ctx);
+    std::vector<uint16_t>* t = &b.t;
+    fake::enqueue(fake::main_stream, [t] { for (uint16_t& w : *t) w = 0x061A; });
+    want_target = 0x061A;
+    wrong = false;
+    expect(call(ctx, s, b) == M6502_OK, "fails", s.name, 0);
+    expect(!wrong, "targets were read before the stream's earlier work", s.name, 0);
+    want_target = 0;
+    fake::main_stream = nullptr;
+    m6502_destroy(ctx);
+}
+
 int main(int argc, char** argv) {
-    const bool errors = argc > 1 && !std::strcmp(argv[1], "errors");   // else: tables
+    const std::string mode = argc > 1 ? argv[1] : "";   // tables, errors or order
+    const bool errors = mode == "errors";
     const Scenario all[] = {
         {"search", 0, M6502_SEM_CUDA, 1, 0, 0, 20},
         {"search in three passes", 0, M6502_SEM_CUDA, 1, 0, 8, 20},
@@ -115,6 +133,7 @@ int main(int argc, char** argv) {
     fake::on_kernel = hook;
     for (const Scenario& s : all) {
         if (s.kind == 2 && !errors) continue;
+        if (mode == "order" && (s.kind || s.semantics != M6502_SEM_CUDA)) continue;
         Buffers b(s.n);
         // What the tables hold, from a call that everything before it has ended for.
         learn = true;
@@ -124,6 +143,10 @@ int main(int argc, char** argv) {
         expect(call(ctx, s, b) == M6502_OK, "fails when repeated", s.name, 0);
         m6502_destroy(ctx);
         learn = wrong = false;
+        if (mode == "order") {
+            read_in_order(s, b);
+            continue;
+        }
         // A first call without a failure.
         ctx = create(s);
         fake::calls = 0;
