@@ -44,7 +44,6 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <tuple>
 #include <vector>
 
 #include "internal.h"
@@ -204,7 +203,7 @@ __host__ __device__ __forceinline__ uint64_t join_key(const uint32_t (&w)[16]) {
 // The length-1 join's table for one dead-flags mask.  The non-pruned
 // candidates fall into classes of equal QuickCheck outputs (1,883 at mask
 // 0x00) and those into subclasses of equal MidCheck outputs (2,032): a class
-// is an entry, by ascending key (two entries may share one), and a target's
+// is an entry, by the directory's buckets (two entries may share a key), and a target's
 // outputs are compared once per class and subclass, not once per candidate
 // (runs of up to 43 compare operands share a class).  `key` and `dir`, a
 // directory of the keys' top bits, are copied into shared memory; the rest
@@ -2664,11 +2663,13 @@ struct m6502_ctx {
     DevBuf jitems;                                             // chunks of long length-2 equal ranges
     DevBuf order;                                              // k_small: the pairs it left
     DevBuf match;                                              // k_qc_join: the targets that match
-    DevBuf join_tab[2][256];                      // JoinTable by semantics and dead-flags mask
-    DevBuf join_groups[256];                      // CandGroups of the CUDA-semantics tables
-    DevBuf join_lines[256];                       // line hashes of the candidates, [64 register sets][2863]
+    JoinTable* join_tab[2][256] = {};             // by semantics and dead-flags mask
+    CandGroups* join_groups[256] = {};            // of the CUDA-semantics tables
+    uint32_t* join_lines[256] = {};               // line hashes of the candidates, [64 register sets][2863]
     bool join_built[2][256] = {};                 // tables and groups are filled, or their copies are on the stream
     bool lines_built[256] = {};
+    std::vector<void*> table_blocks;              // the memory of these tables (see table_mem)
+    size_t table_used = 0;                        // of the last block
     struct Cand2Table {            // sorted (key, entry) of all length-2 sequences for one mask
         uint32_t dead = 0xFFFFFFFFu;
         uint32_t longest = 0;      // longest range of one key
@@ -2793,7 +2794,7 @@ int launch_verify(m6502_ctx* ctx, const Src& src, const unsigned long long* n_pt
 }
 
 const uint16_t* join_mult(const m6502_ctx* ctx, uint32_t dead) {
-    const CandGroups* g = (const CandGroups*)ctx->join_groups[dead].p;
+    const CandGroups* g = ctx->join_groups[dead];
     return g ? g->mult : nullptr;
 }
 
@@ -2809,7 +2810,7 @@ int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt
     const uint32_t chunk = (uint32_t)std::min<uint64_t>(32, (nt + warps - 1) / warps);
     const uint64_t blocks = (nt + (uint64_t)chunk * kWarpsPerBlock - 1) / ((uint64_t)chunk * kWarpsPerBlock);
     const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->sms * 4, blocks));
-    const JoinTable* tab = (const JoinTable*)ctx->join_tab[go][dead].p;
+    const JoinTable* tab = ctx->join_tab[go][dead];
     const uint4* cfp4 = (const uint4*)ctx->cfp4.p;
     Surv* match = (Surv*)ctx->match.p;
     if (go)
@@ -2818,7 +2819,7 @@ int launch_join1(m6502_ctx* ctx, const uint16_t* d_t, uint32_t tlen, uint64_t nt
         k_qc_join<false><<<grid, 256, 0, ctx->stream>>>(d_t, tlen, (uint32_t)nt, chunk, cfp4, tab, dead, stages, match, cnt, bad);
     CKL("k_qc_join");
     const uint16_t* mult = go ? nullptr : join_mult(ctx, dead);
-    const uint32_t* lines = (const uint32_t*)ctx->join_lines[dead].p;
+    const uint32_t* lines = ctx->join_lines[dead];
     const uint32_t egrid = (uint32_t)std::min<uint64_t>((uint64_t)ctx->sms * 4, (nt + kWarpsPerBlock - 1) / kWarpsPerBlock);
     auto expand = [&](auto kernel) {
         kernel<<<egrid, 256, 0, ctx->stream>>>(match, d_t, tlen, cfp4, tab, dead, cfg.sweep, mult, lines, (Surv*)ctx->surv.p,
@@ -2979,87 +2980,150 @@ int cand_group(uint32_t op, uint32_t dead) {
     return (int)(sweep_locs_of_reads(op_reads(op)) << 4 | bytes_cuda(op));
 }
 
-// Sorted (QuickCheck key, candidate) table of the non-pruned length-1
-// candidates for one dead-flags mask, built once per mask.  CUDA semantics:
+// Memory for the tables of a mask, which live as long as the context: pieces
+// of 8 MB blocks (a mask of both semantics takes 0.87 MB; an allocation of its
+// own for each piece took 0.3 ms on every second or third new mask).
+constexpr size_t kTableBlock = 8u << 20;
+template <class T>
+int table_mem(m6502_ctx* ctx, size_t n, T** out) {
+    if (*out) return M6502_OK;   // kept from a call that failed later on
+    const size_t bytes = (n * sizeof(T) + 255) & ~(size_t)255;
+    if (ctx->table_blocks.empty() || ctx->table_used + bytes > kTableBlock) {
+        void* p = nullptr;
+        CK(cudaMalloc(&p, kTableBlock));
+        ctx->table_blocks.push_back(p);
+        ctx->table_used = 0;
+    }
+    *out = reinterpret_cast<T*>((char*)ctx->table_blocks.back() + ctx->table_used);
+    ctx->table_used += bytes;
+    return M6502_OK;
+}
+
+// JoinTable of the non-pruned length-1 candidates for one dead-flags mask,
+// built once per mask.  CUDA semantics:
 // one entry per group of candidates; Go semantics: every candidate (its
 // passes and ranks tell the members of a group apart).
+// It is part of a mask's first search: candidates go to the directory's buckets
+// in enumeration order and are compared with the first members of the
+// subclasses there (a vector of words per candidate and one sort over all of
+// them took 0.7 ms).
 int join_table(m6502_ctx* ctx, uint32_t dead, bool go) {
     if (ctx->join_built[go][dead]) return M6502_OK;
-    const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;
-    struct Entry {
-        uint64_t key;
-        std::vector<uint32_t> words;   // Go semantics has no MidCheck: QuickCheck's 16 only
-        uint32_t rank;                 // order among equals: CUDA or Go enumeration
-        uint16_t cand;
-    };
-    std::vector<Entry> v;
-    CandGroups gr;
-    std::memset(&gr, 0, sizeof gr);
-    std::vector<std::vector<uint16_t>> groups;   // members; a lone candidate is a group of its own
-    std::map<int, size_t> group_of;
-    for (int c = 0; c < kNumInsns; c++) {
-        if (ctx->h_cmeta[c] & 0x10) continue;
-        const int g = go ? -1 : cand_group(ctx->h_tab[c] & 0xFFu, dead);
-        if (g >= 0) {
-            const auto at = group_of.emplace(g, groups.size());
-            if (!at.second) { groups[at.first->second].push_back((uint16_t)c); continue; }
-        }
-        groups.push_back({(uint16_t)c});
-        std::vector<uint32_t> words(ctx->h_cfp4.begin() + (long)c * 64, ctx->h_cfp4.begin() + (long)(c + 1) * 64);
-        for (int g = 0; g < 8; g++) words[8 * g + 3] &= pm;
-        uint32_t qc[16];
-        std::copy(words.begin(), words.begin() + 16, qc);
-        if (go) words.resize(16);
-        v.push_back({join_key(qc), std::move(words), go ? ctx->h_gorank[c] : (uint32_t)c, (uint16_t)c});
-    }
-    std::sort(v.begin(), v.end(), [](const Entry& a, const Entry& b) {
-        return std::tie(a.key, a.words, a.rank) < std::tie(b.key, b.words, b.rank);
-    });
-    std::vector<JoinTable> tab(1);
-    JoinTable& t = tab[0];
-    std::memset(&t, 0, sizeof t);
-    uint32_t nu = 0, nj = 0, bucket = 0;
-    for (size_t i = 0; i < v.size(); i++) {
-        const Entry& e = v[i];
-        const uint32_t op = ctx->h_tab[e.cand] & 0xFFu, bytes = go ? bytes_go(op) : bytes_cuda(op);
-        const bool entry = i == 0 || e.key != v[i - 1].key ||
-                           !std::equal(e.words.begin(), e.words.begin() + 16, v[i - 1].words.begin());
-        if (entry) {
-            t.key[nu] = e.key;
-            t.sub[nu] = (uint16_t)nj;
-            for (const uint32_t b = (uint32_t)(e.key >> (64 - kDirBits)); bucket <= b; bucket++) t.dir[bucket] = (uint16_t)nu;
-            nu++;
-        }
-        if (entry || e.words != v[i - 1].words) t.start[nj++] = (uint16_t)i;
-        t.cand[i] = (uint16_t)(e.cand | bytes << 12);
-    }
-    t.sub[nu] = (uint16_t)nj;
-    t.start[nj] = (uint16_t)v.size();
-    for (; bucket <= (1u << kDirBits); bucket++) t.dir[bucket] = (uint16_t)nu;
-    for (uint32_t u = 0; go && u < nu; u++)
-        ctx->join_longest[dead] = std::max<uint32_t>(ctx->join_longest[dead], t.start[t.sub[u + 1]] - t.start[t.sub[u]]);
-    if (!ctx->lines_built[dead]) {
-        TRY(ensure(ctx, ctx->join_lines[dead], 64 * kNumInsns * sizeof(uint32_t)));
-        k_line_hash<<<(64 * kNumInsns + 255) / 256, 256, 0, ctx->stream>>>(dead, (uint32_t*)ctx->join_lines[dead].p);
+    if (!ctx->lines_built[dead]) {   // on the device meanwhile
+        TRY(table_mem(ctx, (size_t)64 * kNumInsns, &ctx->join_lines[dead]));
+        k_line_hash<<<(64 * kNumInsns + 255) / 256, 256, 0, ctx->stream>>>(dead, ctx->join_lines[dead]);
         CKL("k_line_hash");
         ctx->lines_built[dead] = true;
     }
+    // A candidate's outputs, the dead flags masked: two groups of 8 packed words
+    // (A X Y P S M S0 S1) of QuickCheck, then six of MidCheck, which Go semantics
+    // does not have.
+    const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1, all = 0xFFFFFFFFu;
+    const uint32_t mask[8] = {all, all, all, pm, all, all, all, all};
+    auto same = [&](uint32_t a, uint32_t b, int g0, int g1) {
+        const uint32_t *x = &ctx->h_cfp4[(size_t)a * 64], *y = &ctx->h_cfp4[(size_t)b * 64];
+        uint32_t d = 0;
+        for (int g = g0; g < g1 && !d; g++)
+            for (int k = 0; k < 8; k++) d |= (x[8 * g + k] ^ y[8 * g + k]) & mask[k];
+        return d == 0;
+    };
+    // The candidates that go into the table, in enumeration order (CUDA or Go),
+    // and the groups.
+    int group[NUM_OPS];
+    for (uint32_t op = 0; op < NUM_OPS; op++) group[op] = go ? -1 : cand_group(op, dead);
+    CandGroups gr;
+    std::memset(&gr, 0, sizeof gr);
+    uint16_t lead[kNumInsns], order[kNumInsns];   // the candidate that stands for this one; the candidates in order
+    for (uint32_t c = 0; c < (uint32_t)kNumInsns; c++) order[go ? ctx->h_gorank[c] : c] = (uint16_t)c;
+    std::map<int, uint16_t> lead_of;   // by group
+    struct Entry {
+        uint64_t key;
+        uint16_t cand, next;           // next member of its subclass
+    };
+    constexpr uint32_t kBuckets = 1u << kDirBits;
+    constexpr uint16_t kNone = 0xFFFFu;
+    std::vector<Entry> in, v;
+    std::vector<uint16_t> at(kBuckets + 1), fill;   // first place of each bucket's entries
+    in.reserve(kNumInsns);
+    for (uint16_t c : order) {
+        lead[c] = kNone;
+        if (ctx->h_cmeta[c] & 0x10) continue;
+        const int g = group[ctx->h_tab[c] & 0xFFu];
+        lead[c] = g < 0 ? c : lead_of.emplace(g, c).first->second;
+        gr.mult[lead[c]]++;
+        if (lead[c] != c) continue;
+        uint32_t qc[16];
+        for (int w = 0; w < 16; w++) qc[w] = ctx->h_cfp4[(size_t)c * 64 + w] & mask[w % 8];
+        in.push_back({join_key(qc), c, kNone});
+        at[(in.back().key >> (64 - kDirBits)) + 1]++;
+    }
+    for (uint32_t b = 0; b < kBuckets; b++) at[b + 1] = (uint16_t)(at[b + 1] + at[b]);
+    v.resize(in.size());
+    fill = at;
+    for (const Entry& e : in) v[fill[e.key >> (64 - kDirBits)]++] = e;
+    // Bucket by bucket: the subclasses in the order of their first members, those
+    // of one entry next to each other.
+    std::vector<JoinTable> tab(1);
+    JoinTable& t = tab[0];
+    std::memset(&t, 0, sizeof t);
+    struct Sub {
+        uint16_t head, tail;           // places in v
+        bool entry;                    // the first of its entry
+    };
+    std::vector<Sub> subs;
+    uint32_t nu = 0, nj = 0, nc = 0;
+    for (uint32_t b = 0; b < kBuckets; b++) {
+        t.dir[b] = (uint16_t)nu;
+        subs.clear();
+        for (uint16_t i = at[b]; i < at[b + 1]; i++) {
+            size_t place = 0;          // behind the subclasses of its entry
+            bool member = false;
+            for (size_t s = 0; s < subs.size() && !member; s++) {
+                const Entry& e = v[subs[s].head];
+                if (e.key != v[i].key || !same(e.cand, v[i].cand, 0, 2)) continue;
+                place = s + 1;
+                if (!go && !same(e.cand, v[i].cand, 2, 8)) continue;
+                v[subs[s].tail].next = i;
+                subs[s].tail = i;
+                member = true;
+            }
+            if (!member) subs.insert(place ? subs.begin() + (long)place : subs.end(), Sub{i, i, place == 0});
+        }
+        for (const Sub& s : subs) {
+            if (s.entry) {
+                t.key[nu] = v[s.head].key;
+                t.sub[nu++] = (uint16_t)nj;
+            }
+            t.start[nj++] = (uint16_t)nc;
+            for (uint16_t i = s.head; i != kNone; i = v[i].next) {
+                const uint32_t op = ctx->h_tab[v[i].cand] & 0xFFu;
+                t.cand[nc++] = (uint16_t)(v[i].cand | (go ? bytes_go(op) : bytes_cuda(op)) << 12);
+            }
+        }
+    }
+    t.dir[kBuckets] = (uint16_t)nu;
+    t.sub[nu] = (uint16_t)nj;
+    t.start[nj] = (uint16_t)nc;
+    for (uint32_t u = 0; go && u < nu; u++)
+        ctx->join_longest[dead] = std::max<uint32_t>(ctx->join_longest[dead], t.start[t.sub[u + 1]] - t.start[t.sub[u]]);
     // The copies go on the stream of the kernels that read them.
     if (!go) {
-        uint16_t at = 0;
-        for (const auto& e : groups) {
-            gr.mult[e[0]] = (uint16_t)e.size();
-            gr.first[e[0]] = at;
-            for (uint16_t c : e) gr.member[at++] = c;
+        uint16_t next = 0, place[kNumInsns];
+        for (int c = 0; c < kNumInsns; c++) {
+            if (!gr.mult[c]) continue;
+            gr.first[c] = place[c] = next;
+            next = (uint16_t)(next + gr.mult[c]);
         }
+        for (int c = 0; c < kNumInsns; c++)
+            if (lead[c] != kNone) gr.member[place[lead[c]]++] = (uint16_t)c;
         for (uint32_t u = 0; u < nu; u++)
             for (uint32_t i = t.start[t.sub[u]]; i < t.start[t.sub[u + 1]]; i++)
                 for (uint32_t b = t.cand[i] >> 12; b <= 2; b++) t.weight[u][b - 1] += gr.mult[t.cand[i] & 0xFFFu];
-        TRY(ensure(ctx, ctx->join_groups[dead], sizeof gr));
-        CK(cudaMemcpyAsync(ctx->join_groups[dead].p, &gr, sizeof gr, cudaMemcpyHostToDevice, ctx->stream));
+        TRY(table_mem(ctx, 1, &ctx->join_groups[dead]));
+        CK(cudaMemcpyAsync(ctx->join_groups[dead], &gr, sizeof gr, cudaMemcpyHostToDevice, ctx->stream));
     }
-    TRY(ensure(ctx, ctx->join_tab[go][dead], sizeof t));
-    CK(cudaMemcpyAsync(ctx->join_tab[go][dead].p, &t, sizeof t, cudaMemcpyHostToDevice, ctx->stream));
+    TRY(table_mem(ctx, 1, &ctx->join_tab[go][dead]));
+    CK(cudaMemcpyAsync(ctx->join_tab[go][dead], &t, sizeof t, cudaMemcpyHostToDevice, ctx->stream));
     ctx->join_built[go][dead] = true;
     return M6502_OK;
 }
@@ -3162,7 +3226,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
     const bool phase2 = cfg.max_cand_len >= 2;
     if (!scan) TRY(join_table(ctx, dead, go));
     // the scan's survivors are single candidates; the join's may stand for a group
-    const CandGroups* groups = scan || go ? nullptr : (const CandGroups*)ctx->join_groups[dead].p;
+    const CandGroups* groups = scan || go ? nullptr : ctx->join_groups[dead];
     const uint16_t* mult = groups ? groups->mult : nullptr;
     for (int attempt = 0; attempt < 6; attempt++) {
         // Every buffer the pass uses is allocated here, so that the launches
@@ -3357,7 +3421,7 @@ int run_pass(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* d_targ
                 (uint64_t)(uintptr_t)ctx->go_keys.p, (uint64_t)(uintptr_t)ctx->go_keys2.p,
                 (uint64_t)(uintptr_t)ctx->go_ord.p, (uint64_t)(uintptr_t)ctx->go_round.p,
                 (uint64_t)(uintptr_t)ctx->go_sort_tmp.p, ctx->go_sort_tmp.bytes, (uint64_t)(uintptr_t)ctx->jitems.p,
-                (uint64_t)(uintptr_t)ctx->join_tab[go][dead].p, c2 ? (uint64_t)(uintptr_t)c2->keys.p : 0,
+                (uint64_t)(uintptr_t)ctx->join_tab[go][dead], c2 ? (uint64_t)(uintptr_t)c2->keys.p : 0,
                 c2e ? (uint64_t)(uintptr_t)c2e->keys.p : 0, ctx->tune.exh_minb, ctx->tune.ticket_batch,
                 ctx->tune.chunk_log2};
             m6502_ctx::PassGraph* pg = nullptr;
@@ -3492,7 +3556,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
         TRY(ensure(ctx, ctx->tmeta, pmax));
     }
     if (!scan) TRY(join_table(ctx, dead, false));
-    const CandGroups* groups = scan ? nullptr : (const CandGroups*)ctx->join_groups[dead].p;
+    const CandGroups* groups = scan ? nullptr : ctx->join_groups[dead];
     TRY(ensure(ctx, ctx->cnt_slots, npass * sizeof(Counters)));
     Counters* slots = (Counters*)ctx->cnt_slots.p;
     TRY(ensure(ctx, ctx->opflag, 2 * sizeof(uint32_t)));
@@ -3572,7 +3636,7 @@ int search_async(m6502_ctx* ctx, const m6502_search_cfg& cfg, const uint16_t* ta
                 (uint64_t)(uintptr_t)ctx->match.p,
                 (uint64_t)(uintptr_t)ctx->rules.p, (uint64_t)(uintptr_t)ctx->cnt_slots.p,
                 (uint64_t)(uintptr_t)ctx->tfp.p, (uint64_t)(uintptr_t)ctx->tmeta.p, (uint64_t)(uintptr_t)ctx->opflag.p,
-                (uint64_t)(uintptr_t)ctx->join_tab[0][dead].p, ctx->tune.exh_minb, ctx->tune.ticket_batch,
+                (uint64_t)(uintptr_t)ctx->join_tab[0][dead], ctx->tune.exh_minb, ctx->tune.ticket_batch,
                 ctx->tune.chunk_log2};
             replayed = ctx->graph.exec.size() == npass && ctx->graph.key == key;
             if (!replayed) {
@@ -3867,12 +3931,7 @@ void m6502_destroy(m6502_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (int i = 0; i < 256; i++) {
-        for (int g = 0; g < 2; g++)
-            if (ctx->join_tab[g][i].p) cudaFree(ctx->join_tab[g][i].p);
-        if (ctx->join_groups[i].p) cudaFree(ctx->join_groups[i].p);
-        if (ctx->join_lines[i].p) cudaFree(ctx->join_lines[i].p);
-    }
+    for (void* p : ctx->table_blocks) cudaFree(p);
     DevBuf* bufs[] = {&ctx->cfp4, &ctx->cfp1, &ctx->cmeta1, &ctx->targets, &ctx->ids, &ctx->tfp, &ctx->tmeta,
                       &ctx->surv, &ctx->fail, &ctx->items, &ctx->rules, &ctx->cnt, &ctx->best,
                       &ctx->pins, &ctx->poffs,

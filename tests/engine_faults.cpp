@@ -116,8 +116,32 @@ static void read_in_order(const Scenario& s, Buffers& b) {
     m6502_destroy(ctx);
 }
 
+// New masks share blocks of memory: an allocation for each of a mask's tables
+// takes longer than building them.
+static int masks() {
+    Scenario s{"new masks", 0, M6502_SEM_CUDA, 1, 0, 0, 20};
+    Buffers b(s.n);
+    m6502_ctx* ctx = create(s);
+    expect(call(ctx, s, b) == M6502_OK, "fails", s.name, 0);
+    const long before = fake::mallocs;
+    for (uint32_t mask = 0; mask < 64; mask++) {
+        m6502_search_cfg cfg;
+        std::memset(&cfg, 0, sizeof cfg);
+        cfg.semantics = mask & 1 ? M6502_SEM_GO : M6502_SEM_CUDA;
+        cfg.max_cand_len = 1;
+        cfg.dead_flags = (uint8_t)mask;
+        uint64_t n = 0;
+        expect(m6502_search(ctx, &cfg, b.t.data(), s.n, 2, b.rules.data(), b.rules.size(), &n, nullptr) == M6502_OK, "fails", s.name, mask);
+    }
+    expect(fake::mallocs - before <= 16, "more than a block of memory for every four masks", s.name, 0);
+    m6502_destroy(ctx);
+    std::printf("%ld allocations, %ld failures\n", fake::mallocs - before, bad);
+    return bad ? 1 : 0;
+}
+
 int main(int argc, char** argv) {
-    const std::string mode = argc > 1 ? argv[1] : "";   // tables, errors or order
+    const std::string mode = argc > 1 ? argv[1] : "";   // tables, errors, order or masks
+    if (mode == "masks") return masks();
     const bool errors = mode == "errors";
     const Scenario all[] = {
         {"search", 0, M6502_SEM_CUDA, 1, 0, 0, 20},

@@ -23,7 +23,7 @@ struct CUgraph_st { std::vector<Op> ops; };
 struct CUgraphExec_st { std::vector<Op> ops; };
 
 namespace fake {
-long calls = 0, fail_at = 0;
+long calls = 0, fail_at = 0, mallocs = 0;
 cudaError_t fail_code = cudaErrorUnknown;
 cudaStream_t main_stream = nullptr;
 std::function<void(const std::string&, void**)> on_kernel;
@@ -105,7 +105,7 @@ const char* cudaGetErrorString(cudaError_t e) { return e == cudaSuccess ? "no er
 cudaError_t cudaGetLastError() { cudaError_t e = last; last = cudaSuccess; return e; }
 cudaError_t cudaPeekAtLastError() { return last; }
 
-cudaError_t cudaMalloc(void** p, size_t n) { FAILS(); *p = std::calloc(1, n ? n : 1); return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { FAILS(); mallocs++; *p = std::calloc(1, n ? n : 1); return cudaSuccess; }
 cudaError_t cudaFree(void* p) { drain(); std::free(p); return cudaSuccess; }   // waits for the device
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { FAILS(); *p = std::calloc(1, n); host_blocks[(const char*)*p] = n; return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { drain(); host_blocks.erase((const char*)p); std::free(p); return cudaSuccess; }

@@ -15,6 +15,7 @@ namespace fake {
 // returns `fail_code`; `calls` counts them.
 extern long calls, fail_at;
 extern cudaError_t fail_code;
+extern long mallocs;                   // of device memory
 // Copies to the device on any other stream than `main_stream` start at once,
 // as far as their stream's earlier waits allow (null: every queue is lazy).
 extern cudaStream_t main_stream;

@@ -23,7 +23,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["tables", "errors", "order"])
+@pytest.mark.parametrize("what", ["tables", "errors", "order", "masks"])
 def test_engine_faults(program, what):
     run = subprocess.run([program, what], capture_output=True, text=True, timeout=600)
     assert run.returncode == 0, run.stdout
