@@ -1601,37 +1601,62 @@ __global__ void k_cand2_keys(uint32_t dead, uint64_t salt, uint64_t* __restrict_
     }
 }
 
-// The two packed words of QuickCheck outputs of a length-2 sequence.
-__device__ __forceinline__ void cand2_outputs(uint32_t c, St (&v)[2]) {
-#pragma unroll
-    for (int g = 0; g < 2; g++)
-        v[g] = St{c_vec4[g][0], c_vec4[g][1], c_vec4[g][2], c_vec4[g][3],
-                  c_vec4[g][4], c_vec4[g][5], c_vec4[g][6], c_vec4[g][7]};
-    exec_x4n(v, c_tab[c / kNumInsns]);
-    exec_x4n(v, c_tab[c % kNumInsns]);
+// X4Row of an opcode in shared memory (copied from g_x4row).
+__device__ __forceinline__ X4Row load_row(const uint4 (&q)[3]) {
+    const uint4 a = q[0], b = q[1], c = q[2];
+    return X4Row{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
 }
 
 // After the sort: P after the QuickCheck vectors of every entry (pw, for
 // FlagDiff); whether two different sets of outputs share a key (info[0]: the
 // table is then built again with another salt, so that one candidate of a
 // range decides QuickCheck for all); the longest range of one key (info[1]).
-__global__ void k_cand2_info(uint32_t dead, const uint64_t* __restrict__ keys, const uint32_t* __restrict__ idx,
-                             uint2* __restrict__ pw, uint32_t* __restrict__ info) {
+// Sorted by a hash, neighbours share no opcode: the per-opcode switch runs up
+// to 30 arms for a warp, and every entry was run a second time for its
+// successor's comparison.  The table-driven executor has one course for all
+// lanes, and a warp takes 31 entries behind one that it runs for comparison
+// only, whose outputs the next lane gets by a shuffle: 2.5 -> 0.37 ms for a
+// mask's 8.2 M entries.
+constexpr int kInfoThreads = 256;
+__global__ void __launch_bounds__(kInfoThreads) k_cand2_info(uint32_t dead, const uint64_t* __restrict__ keys,
+                                                             const uint32_t* __restrict__ idx, uint2* __restrict__ pw,
+                                                             uint32_t* __restrict__ info) {
+    __shared__ uint4 s_row[NUM_OPS][3];
+    __shared__ uint32_t s_st[X4S_COUNT][kInfoThreads];   // each lane's registers
+    for (int i = threadIdx.x; i < (int)NUM_OPS * 3; i += kInfoThreads) (&s_row[0][0])[i] = g_x4row[i];
+    __syncthreads();
     const uint32_t pm = (kPMask & ~dead & 0xFFu) * kB1;
     const uint32_t n = (uint32_t)kNumInsns * (uint32_t)kNumInsns;
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (kInfoThreads / 32);
+    uint32_t* st = &s_st[0][threadIdx.x];
     uint32_t longest = 0, clash = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        St v[2];
-        cand2_outputs(idx[i] & kEntryIndex, v);
-        pw[i] = make_uint2(v[0].p & (kPMask * kB1), v[1].p & (kPMask * kB1));
-        const uint64_t key = keys[i];
-        if (i > 0 && keys[i - 1] == key) {
-            St u[2];
-            cand2_outputs(idx[i - 1] & kEntryIndex, u);
+    for (uint32_t first = (blockIdx.x * (kInfoThreads / 32) + (threadIdx.x >> 5)) * 31u; first < n; first += warps * 31u) {
+        // lane 0: the entry before `first` (the very first one stands in for its own)
+        const uint32_t at = first + lane, i = min(at ? at - 1u : 0u, n - 1u);
+        const uint32_t c = idx[i] & kEntryIndex;
+        const uint64_t key = keys[i], before = __shfl_up_sync(kFull, key, 1);
+        const uint32_t insn[2] = {c_tab[c / kNumInsns], c_tab[c % kNumInsns]};
+        const X4Row row[2] = {load_row(s_row[insn[0] & 0xFFu]), load_row(s_row[insn[1] & 0xFFu])};
+        uint32_t differ = 0, p[2];
 #pragma unroll
-            for (int g = 0; g < 2; g++)
-                clash |= (v[g].a ^ u[g].a) | (v[g].x ^ u[g].x) | (v[g].y ^ u[g].y) | ((v[g].p ^ u[g].p) & pm) |
-                         (v[g].s ^ u[g].s) | (v[g].m ^ u[g].m) | (v[g].s0 ^ u[g].s0) | (v[g].s1 ^ u[g].s1);
+        for (int g = 0; g < 2; g++) {
+            st[X4S_A * kInfoThreads] = c_vec4[g][0]; st[X4S_X * kInfoThreads] = c_vec4[g][1]; st[X4S_Y * kInfoThreads] = c_vec4[g][2];
+            st[X4S_S * kInfoThreads] = c_vec4[g][4]; st[X4S_M * kInfoThreads] = c_vec4[g][5]; st[X4S_S0 * kInfoThreads] = c_vec4[g][6];
+            st[X4S_S1 * kInfoThreads] = c_vec4[g][7];
+            p[g] = c_vec4[g][3];
+            exec_x4r(st, kInfoThreads, p[g], row[0], insn[0]);
+            exec_x4r(st, kInfoThreads, p[g], row[1], insn[1]);
+#pragma unroll
+            for (int f = 0; f < (int)X4S_NONE; f++) {
+                const uint32_t v = st[f * kInfoThreads];
+                differ |= v ^ __shfl_up_sync(kFull, v, 1);
+            }
+            differ |= (p[g] ^ __shfl_up_sync(kFull, p[g], 1)) & pm;
+        }
+        if (lane == 0 || at > n) continue;
+        pw[i] = make_uint2(p[0] & (kPMask * kB1), p[1] & (kPMask * kB1));
+        if (i > 0 && before == key) {
+            clash |= differ;
         } else {   // first of its range: the range's end by doubling and halving
             uint32_t step = 1;
             while (i + step < n && keys[i + step] == key) step <<= 1;
@@ -1643,8 +1668,9 @@ __global__ void k_cand2_info(uint32_t dead, const uint64_t* __restrict__ keys, c
             longest = max(longest, hi - i);
         }
     }
-    if (clash) info[0] = 1u;
-    atomicMax(info + 1, longest);
+    if (__any_sync(kFull, clash != 0) && lane == 0) info[0] = 1u;
+    longest = __reduce_max_sync(kFull, longest);
+    if (lane == 0) atomicMax(info + 1, longest);
 }
 
 // Equal ranges are very uneven (a flags-only target under mask 0xFF matches
@@ -3161,7 +3187,7 @@ int cand2_table(m6502_ctx* ctx, uint32_t dead, m6502_ctx::Cand2Table** out) {
                                                (uint64_t*)slot->keys.p, (const uint32_t*)ctx->c2_idx_in.p,
                                                (uint32_t*)slot->idx.p, (int)n, 0, 64, ctx->stream));
             CK(cudaMemsetAsync(ctx->opflag.p, 0, 2 * sizeof(uint32_t), ctx->stream));
-            k_cand2_info<<<ctx->sms * 8, 256, 0, ctx->stream>>>(dead, (const uint64_t*)slot->keys.p,
+            k_cand2_info<<<ctx->sms * 8, kInfoThreads, 0, ctx->stream>>>(dead, (const uint64_t*)slot->keys.p,
                                                                 (const uint32_t*)slot->idx.p, (uint2*)slot->pw.p,
                                                                 (uint32_t*)ctx->opflag.p);
             CKL("k_cand2_info");

@@ -192,10 +192,6 @@ __global__ void k_stoke_live(StokeChain* __restrict__ chains, uint32_t n_chains,
     }
 }
 
-__device__ __forceinline__ X4Row load_row(const uint4 (&q)[3]) {
-    const uint4 a = q[0], b = q[1], c = q[2];
-    return X4Row{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
-}
 // One epoch of the listed chains: eight lanes per chain, up to four chains per
 // warp.  Lane `sub` of a chain runs the candidate on vectors 4 sub .. 4 sub +
 // 3, packed in one word per register; the chain's random numbers are drawn by
