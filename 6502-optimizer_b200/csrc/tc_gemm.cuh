@@ -312,9 +312,11 @@ __global__ void __launch_bounds__(kThreads) k_gemm(const __grid_constant__ CUten
                 const bool wide = epi.wide && n0 + c0 + 32 <= N;   // warp-uniform
                 const size_t row_o = (size_t)(r0 + lane) * epi.ldc + (size_t)(n0 + c0);
                 uint32_t act[16];
-                if (wide && epi.mode == EPI_RELU_GRAD && r0 + lane < M) {   // in flight while TMEM is read
-                    load32(act, epi.act + row_o);
-                    load32(act + 8, epi.act + row_o + 16);
+                if (wide && epi.mode == EPI_RELU_GRAD) {   // in flight while TMEM is read
+                    // lanes past M load the last row: the warp stays converged for tcgen05.ld
+                    const __nv_bfloat16* a = epi.act + (size_t)min(r0 + lane, M - 1) * epi.ldc + (size_t)(n0 + c0);
+                    load32(act, a);
+                    load32(act + 8, a + 16);
                 }
                 uint32_t v[32];
                 asm volatile(
