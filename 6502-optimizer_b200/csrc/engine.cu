@@ -259,6 +259,12 @@ constexpr uint32_t kSurvLen2 = 1u << 23, kSurvMasked = 1u << 24;
 constexpr uint64_t kNoTarget = ~0ull;
 __host__ __device__ __forceinline__ uint32_t fd_pack(uint32_t fd) { return (fd & 0x0Fu) | ((fd >> 2) & 0x30u); }
 
+// fail[] of a pair: 0 passed, 3 undecided, 4 deferred (STOKE), kFailLine
+// rejected by k_small's line states, anything else rejected.  The kernels that
+// read the verdicts count the line states' rejects: a counter in k_small made
+// its callers up to 1 % slower.
+constexpr uint32_t kFailLine = 5u;
+
 // Counters of one verification (k_small, k_exhaustive, k_exh_items over one
 // list of pairs); zero at its start.
 constexpr uint32_t kGoBlock = 64;    // survivors of a (target, pass) in the first Go-order round
@@ -2184,7 +2190,7 @@ __global__ void __launch_bounds__(256) k_small(Src src, const unsigned long long
             differ = differ || bad;
             open = open && !differ && q - 2 * sub + (2u << g) < total;   // the same for all lanes of the pair
         }
-        if (p < n && sub == 0 && (small || differ)) a.fail[p] = differ ? 1u : 0u;
+        if (p < n && sub == 0 && (small || differ)) a.fail[p] = !differ ? 0u : small ? 1u : kFailLine;
         const unsigned left = __ballot_sync(kFull, wide && !differ && sub == 0);
         if (left) {
             unsigned long long b = 0;
@@ -2242,6 +2248,11 @@ __device__ __forceinline__ unsigned long long algo_ops(const uint16_t* t, uint32
     return (1ull << bits) * (unsigned long long)(10 * (tn + cn) + 3);
 }
 
+__device__ __forceinline__ void count_failed(Counters* cnt, unsigned long long n) {
+    if ((uint32_t)n) atomicAdd(&cnt->undecided, n & 0xFFFFFFFFull);
+    if (n >> 32) atomicAdd(&cnt->probe_rejects, n >> 32);
+}
+
 // CUDA semantics: every pair of a passing record is a rule; its target is
 // ids[t], or tbase + t (the pass-local index made global) without ids.  The
 // rules of a record that stands for several candidates are written by the
@@ -2255,13 +2266,14 @@ __global__ void k_emit_all(const Surv* __restrict__ surv, const unsigned long lo
     const uint64_t n = min((uint64_t)*n_ptr, n_cap);
     const int lane = threadIdx.x & 31;
     const uint16_t* mult = groups ? groups->mult : nullptr;
-    unsigned long long npass = 0, algo = 0, nund = 0;
+    unsigned long long npass = 0, algo = 0, nund = 0;   // nund: undecided, and rejected by the line states << 32
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t p = base + threadIdx.x;
-        bool pass = p < n && (!check_exh || fail[p] == 0);
+        const uint32_t f = p < n && check_exh ? fail[p] : 0u;
+        bool pass = p < n && f == 0;
         const Surv s = p < n ? surv[p] : Surv{0, 0};
         const uint32_t w = p < n ? surv_weight(s.c, mult) : 0u;
-        nund += (p < n && check_exh && fail[p] == 3u) ? w : 0u;   // left undecided: counted, not a rule
+        nund += f == 3u ? w : f == kFailLine ? (unsigned long long)w << 32 : 0u;   // counted, not rules
         m6502_rule r;
         memset(&r, 0, sizeof r);
         const uint32_t idx = s.c & 0x7FFFFFu;
@@ -2308,7 +2320,7 @@ __global__ void k_emit_all(const Surv* __restrict__ surv, const unsigned long lo
     }
     if (lane == 0 && npass) atomicAdd(&cnt->exh_pass, npass);
     if (lane == 0 && algo) atomicAdd(&cnt->algo, algo);
-    if (lane == 0 && nund) atomicAdd(&cnt->undecided, nund);
+    if (lane == 0 && nund) count_failed(cnt, nund);
 }
 
 // Go-order rank of a survivor's candidate; length-2 candidates (bit 28)
@@ -2328,7 +2340,10 @@ __global__ void k_go_select(const Surv* __restrict__ surv, const unsigned long l
     const uint64_t n = min((uint64_t)*n_ptr, n_cap);
     unsigned long long npass = 0, algo = 0, nund = 0;
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (uint64_t)gridDim.x * blockDim.x) {
-        if (fail[p]) { nund += fail[p] == 3u; continue; }   // undecided pairs count as not passing
+        if (const uint32_t f = fail[p]) {   // undecided pairs count as not passing
+            nund += f == 3u ? 1ull : f == kFailLine ? 1ull << 32 : 0ull;
+            continue;
+        }
         npass++;
         Surv s = surv[p];
         const uint32_t idx = s.c & 0x7FFFFFu, key = go_rank_of(s.c);
@@ -2349,7 +2364,7 @@ __global__ void k_go_select(const Surv* __restrict__ surv, const unsigned long l
     if ((threadIdx.x & 31) == 0) {
         if (npass) atomicAdd(&cnt->exh_pass, npass);
         if (algo) atomicAdd(&cnt->algo, algo);
-        if (nund) atomicAdd(&cnt->undecided, nund);
+        if (nund) count_failed(cnt, nund);
     }
 }
 
