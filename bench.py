@@ -201,9 +201,10 @@ def run_reference(args):
 def load_profile_figures():
     """Per-kernel figures of the committed ncu summary profiles/traffic.txt:
     DRAM bytes per full-workload launch (dram__bytes_read.sum +
-    dram__bytes_write.sum) and, where captured, the issue-slot utilisation
-    (smsp__issue_active.avg.pct_of_peak_sustained_active) of the same
-    capture.  Lines: `kernel bytes [issue_active]`; `# source:` names the
+    dram__bytes_write.sum), the issue-slot utilisation
+    (smsp__issue_active.avg.pct_of_peak_sustained_active) and the lane
+    instructions executed per unit of work of the same capture.  Lines:
+    `kernel bytes issue_active lane_instructions`; `# source:` names the
     capture."""
     p = os.path.join(ROOT, "profiles", "traffic.txt")
     out, source = {}, None
@@ -215,8 +216,38 @@ def load_profile_figures():
             parts = line.split()
             if len(parts) >= 2 and not line.startswith("#") and parts[1].isdigit():
                 out[parts[0]] = {"traffic": int(parts[1]),
-                                 "issue_active": float(parts[2]) if len(parts) > 2 else None}
+                                 "issue_active": float(parts[2]) if len(parts) > 2 else None,
+                                 "lane_insts": float(parts[3]) if len(parts) > 3 else None}
     return out, source
+
+
+# The stages of a search as its events bracket them, each kernel with the
+# statistic that counts its units of work.
+STAGE_KERNELS = {
+    "qc": (("k_qc_join", "targets"), ("k_expand", "mid_hits")),
+    "exhaustive": (("k_small", "exh_passed"), ("k_exhaustive", "exh_passed"), ("k_exh_items", "exh_items")),
+}
+
+
+def stage_roofline(stats, stage_ms, figs, peak_lane_ops):
+    """The longest stage against the integer issue rate: lane instructions its
+    kernels executed (per unit of work from the profiles, times this run's
+    units) over its measured time."""
+    stage = max(STAGE_KERNELS, key=lambda k: stage_ms[k])
+    kernels = STAGE_KERNELS[stage]
+    known = all(k in figs and figs[k]["lane_insts"] is not None for k, _ in kernels)
+    done = sum(figs[k]["lane_insts"] * stats[unit] for k, unit in kernels) if known else None
+    achieved = done / (stage_ms[stage] / 1e3) if known and stage_ms[stage] > 0 else None
+    return {"bound": "int-issue", "kernel": "+".join(k for k, _ in kernels),
+            "achieved": achieved / 1e12 if achieved is not None else None, "peak": peak_lane_ops / 1e12, "unit": "Tlane-op/s",
+            "frac": achieved / peak_lane_ops if achieved is not None else None,
+            "kernel_ms_per_step": stage_ms[stage],
+            "traffic": sum(figs[k]["traffic"] for k, _ in kernels) if all(k in figs for k, _ in kernels) else None,
+            "traffic_unit": "DRAM bytes per launch (one 2^21-target pass), summed over the kernels named",
+            "algorithmic": "lane instructions executed: " + ", ".join(f"{k} per {u}" for k, u in kernels) +
+                           " from the profiles, times this run's counts",
+            "issue_active_from_profile": {k: figs[k]["issue_active"] for k, _ in kernels
+                                          if k in figs and figs[k]["issue_active"] is not None}}
 
 
 def run_engine(args):
@@ -321,28 +352,23 @@ def run_engine(args):
         exh_ms = avg("ms_exhaustive") + avg("ms_exh_items")
         qc_ms = avg("ms_qc")
         exh_achieved = s0["exh_algo_ops"] / (exh_ms / 1e3) if exh_ms > 0 else 0.0
-        exh_exec = s0["exh_states"] * (10 * 3 + 3) / (exh_ms / 1e3) if exh_ms > 0 else 0.0
         qc_algo = 13 * s0["pairs"] + 13 * (7 + 24) * s0["qc_hits"]
         qc_achieved = qc_algo / (qc_ms / 1e3) if qc_ms > 0 else 0.0
         stages = {"fingerprint_ms": avg("ms_fingerprint"), "qc_mid_ms": qc_ms,
                   "exhaustive_ms": avg("ms_exhaustive"), "exh_items_ms": avg("ms_exh_items"),
                   "emit_ms": avg("ms_emit")}
-        dominant = max(("k_exhaustive", avg("ms_exhaustive")), ("k_exh_items", avg("ms_exh_items")),
-                       ("k_qc_join", qc_ms), key=lambda kv: kv[1])[0]
         figs, figs_source = load_profile_figures()
-        # the QC stage's events bracket k_qc_join and k_expand, the exhaustive
-        # stage's k_small and k_exhaustive
-        exh_kernels = ("k_small", "k_exhaustive", "k_exh_items")
-        if dominant == "k_qc_join":
-            achieved, alg = qc_achieved, "13 ops/pair + 31x13 ops per QC hit (QC+MidCheck)"
-            kernels, ktime = ("k_qc_join", "k_expand"), qc_ms
-        else:
-            # states the exhaustive stage's kernels evaluated (cone sweeps and work
-            # items) at the convention's 10 ops per executed instruction + 3 per compare
-            achieved, alg = exh_exec, ("states evaluated (cone sweeps + items) x "
-                                       "(10 ops/instruction x 3 instructions + 3)")
-            kernels, ktime = exh_kernels, exh_ms
-        traffic = sum(figs[k]["traffic"] for k in kernels if k in figs) if all(k in figs for k in kernels) else None
+        roof = stage_roofline(s0, {"qc": qc_ms, "exhaustive": exh_ms}, figs, peak_lane_ops)
+        roof.update({
+            "peak_basis": f"{sms} SMs x 128 int32 lanes x {f_mhz:.0f} MHz (median SM clock sampled)",
+            # the fixed convention: every pair costs its QuickCheck, every accepted
+            # pair its whole product sweep; neither the join nor the cones do that
+            # work, so these figures exceed the peak and are not a utilisation
+            "convention": {"qc_achieved": qc_achieved / 1e12, "exhaustive_achieved": exh_achieved / 1e12,
+                           "qc_algorithmic": "13 ops/pair + 31x13 ops per QC hit (QC+MidCheck)",
+                           "exhaustive_algorithmic": "accepted pairs x 2^(9+8k) states x (10 ops/instruction + 3)",
+                           "note": "emulation-equivalent, not a utilisation"},
+            "profile_source": figs_source})
         line = {
             "metric": "pair-checks/s", "value": value, "unit": "pair-checks/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": total_ms / args.steps,
@@ -361,27 +387,7 @@ def run_engine(args):
             "stage_counts": {k: s0[k] for k in ("qc_hits", "mid_hits", "exh_checked", "exh_passed", "rules",
                                                   "exh_states", "exh_items", "exh_probe_rejects")},
             "stages_ms": stages,
-            "roofline": {"bound": "int-issue", "kernel": "+".join(kernels), "achieved": achieved / 1e12,
-                         "peak": peak_lane_ops / 1e12, "unit": "Tlane-op/s",
-                         "frac": achieved / peak_lane_ops if peak_lane_ops else None,
-                         "kernel_ms_per_step": ktime,
-                         "traffic": traffic, "traffic_unit": "DRAM bytes per launch (one 2^21-target pass), "
-                                                             "summed over the kernels named",
-                         "algorithmic": alg,
-                         "peak_basis": f"{sms} SMs x 128 int32 lanes x {f_mhz:.0f} MHz (median SM clock sampled)",
-                         # the fixed convention: every accepted pair costs its whole product
-                         # sweep; the cone decomposition evaluates far fewer states, so this
-                         # figure exceeds the peak and is not a utilisation
-                         "convention": {"achieved": exh_achieved / 1e12,
-                                        "frac": exh_achieved / peak_lane_ops if peak_lane_ops else None,
-                                        "algorithmic": "accepted pairs x 2^(9+8k) states x "
-                                                       "(10 ops/instruction + 3)",
-                                        "note": "emulation-equivalent, not a utilisation"},
-                         "issue_active_from_profile": {k: figs[k]["issue_active"] for k in kernels
-                                                       if k in figs and figs[k]["issue_active"] is not None},
-                         "profile_source": figs_source},
-            "roofline_qc": {"achieved": qc_achieved / 1e12, "unit": "Tlane-op/s",
-                            "frac": qc_achieved / peak_lane_ops},
+            "roofline": roof,
             "clocks": {"sm_mhz": clk["sm_mhz"], "sm_max_mhz": clk["sm_max_mhz"], "reasons": clk["reasons"]},
             "e2e": {"value": e2e_value, "unit": "pair-checks/s", "h2d_bytes_per_step": int(shard.nbytes),
                     "d2h_bytes_per_step": int(e2e_rules * 16 + 8 * 16 * s0["passes"])},
