@@ -3,7 +3,7 @@
 // Pipeline of a search (all on one stream; a CUDA-semantics search with
 // length-1 candidates queues every pass and syncs once at the end):
 //
-//   k_check_ops     every opcode of the targets, once per search.
+//   k_check_ops     every opcode of a pass's targets, before the rest of it.
 //   k_qc_join       (default) lane per target: its 8 masked QC outputs are
 //                   hashed and looked up among the candidates' distinct
 //                   outputs (keys and bucket directory in shared memory);
@@ -249,7 +249,7 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const uint64_t* __restrict_
 
 // Survivor record: target (index within the pass) and candidate code:
 // bits 0..22 candidate index, bit 23 length-2 candidate, bit 24 Go masked
-// pass, bits 25..30 FlagDiff (P bits 0-3, 6-7 compressed to 6 bits).
+// pass (k_go_emit computes the winner's FlagDiff).
 struct Surv {
     uint32_t t;
     uint32_t c;
@@ -257,7 +257,6 @@ struct Surv {
 constexpr uint32_t kSurvLen2 = 1u << 23, kSurvMasked = 1u << 24;
 // target_id of a pair source whose pairs do not share targets.
 constexpr uint64_t kNoTarget = ~0ull;
-__host__ __device__ __forceinline__ uint32_t fd_pack(uint32_t fd) { return (fd & 0x0Fu) | ((fd >> 2) & 0x30u); }
 
 // fail[] of a pair: 0 passed, 3 undecided, 4 deferred (STOKE), kFailLine
 // rejected by k_small's line states, anything else rejected.  The kernels that
@@ -314,7 +313,8 @@ struct PairView {
 // candidates that change none either (CMP, CPX and CPY with any operand, the
 // flag instructions); they fall into 8 records instead, and the full length-2
 // enumeration at that mask, which is bound by the records it verifies, takes
-// 21.4 ms instead of 441 (0.74 ns of it per record before, 482 M of them).
+// 21.4 ms instead of 441 by this alone (482 M records before, 8 M now), 6.2 ms
+// with the kernels that verify them.
 struct CandGroups {
     uint16_t mult[kNumInsns];    // members of the group that candidate c stands for (0: another stands for c)
     uint16_t first[kNumInsns];   // index of its first member in `member`
@@ -1126,7 +1126,7 @@ __device__ __forceinline__ bool qc_candidate(const uint64_t* __restrict__ trow, 
         for (int v = 0; v < 8; v++) fd |= (uint32_t)((trow[v] ^ cfp[(uint64_t)v * kNumInsns + c]) >> 24) & kPMask;
         if (fd) {
             nqc++; nmid++;
-            code = c | kSurvMasked | (fd_pack(fd) << 25);
+            code = c | kSurvMasked;
             return true;
         }
     }
@@ -1516,12 +1516,9 @@ __global__ void __launch_bounds__(256, 4) k_expand(const Surv* __restrict__ matc
                 const uint32_t p0 = __shfl_sync(kFull, tp0, (int)own), p1 = __shfl_sync(kFull, tp1, (int)own);
                 if (pass) {
                     const uint32_t* row = reinterpret_cast<const uint32_t*>(cfp4) + (size_t)c * 64;
-                    uint32_t fd = ((p0 ^ __ldg(row + 3)) | (p1 ^ __ldg(row + 11))) & (kPMask * kB1);
-                    fd |= fd >> 16;
-                    fd = (fd | (fd >> 8)) & 0xFFu;
-                    if (fd) {
+                    if (((p0 ^ __ldg(row + 3)) | (p1 ^ __ldg(row + 11))) & (kPMask * kB1)) {
                         pass = dead != 0;
-                        code = c | kSurvMasked | (fd_pack(fd) << 25);
+                        code = c | kSurvMasked;
                     }
                 }
                 nqc += pass;
@@ -2084,9 +2081,9 @@ __global__ void __launch_bounds__(256, MINB) k_exhaustive(Src src, const unsigne
 // packed words of states.  The line at 9 bits: a lane takes 64 dispatches per
 // instruction for 512 states; one more register would make it 16,384.
 // Several lanes share a pair (a warp while that fills the chip, else eight:
-// lanes whose pairs differ in opcode diverge.  Four, eight, sixteen lanes:
-// the count at 0xFF 7.77, 7.19, 7.54 ms, 20,011 checked pairs 495, 460, 453 us,
-// this enumeration alike).  The same enumeration:
+// lanes whose pairs differ in opcode diverge.  When the line was drawn, four,
+// eight, sixteen lanes gave 7.77, 7.19, 7.54 ms for the count at 0xFF, 495, 460,
+// 453 us for 20,011 checked pairs, and this enumeration alike).  The same enumeration:
 // 0.56 ms for 1.1 M pairs; k_exhaustive took 2.63 ms for 1.36 M.
 constexpr int kSmallLanesLog2 = 3;   // lanes per pair once the pairs alone fill the chip: 2^3
 __device__ __forceinline__ uint32_t backward(uint32_t locs, uint32_t op, const uint16_t (*dep)[16]) {
@@ -2347,7 +2344,6 @@ __global__ void k_go_select(const Surv* __restrict__ surv, const unsigned long l
         npass++;
         Surv s = surv[p];
         const uint32_t idx = s.c & 0x7FFFFFu, key = go_rank_of(s.c);
-        // keep FlagDiff beside the rank so the winner carries its own
         uint64_t pass = (s.c & kSurvMasked) ? 1 : 0;
         atomicMin(&best[pass * nt + s.t], key);
         uint16_t cand[2];
@@ -2675,7 +2671,7 @@ struct m6502_ctx {
     PassGraph pass_graphs[8];
     uint64_t pass_graph_clock = 0;
     DevBuf cnt_slots;          // Counters of the queued passes
-    DevBuf tall;               // host targets of a queued search, copied to the device at once
+    DevBuf tall;               // host targets of a queued search, copied to the device pass by pass
     DevBuf opflag;             // k_check_ops result
     cudaStream_t copy = nullptr;                  // host targets of the next pass, beside the kernels of this one
     cudaEvent_t cev[kMaxAsyncPasses] = {};        // its copies

@@ -3,10 +3,11 @@
 // The machine state is A, X, Y, P, S, M, S0, S1 (pkg/cpu/state.go:11-16).
 // Kernels keep it in eight 32-bit registers (one byte value each) and pack
 // it into one 64-bit word, byte i = field i, for comparisons and storage.
-// Every kernel arranges its work so that the instruction being executed is
-// the same across a warp (a warp sweeps one pair, or one lane per test
-// vector runs the same sequence), so the opcode switch below is a uniform
-// indirect branch with no divergence.
+// Where a warp sweeps one pair, or one lane per test vector runs the same
+// sequence, the opcode switch below is a uniform branch.  Lanes with pairs or
+// targets of their own (the join, the filter, k_small) diverge in it and run
+// several states per dispatch; the STOKE chains and k_cand2_info use the
+// table-driven executor, which has no switch.
 #pragma once
 #include <cstdint>
 

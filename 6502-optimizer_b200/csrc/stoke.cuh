@@ -81,8 +81,6 @@ struct StokeParams {
     uint64_t seed;
     float decay;            // per-step temperature factor
     float t_start;
-    const uint32_t* proven; // per target: 1 once proved (stop_on_proof)
-    uint32_t stop_on_proof;
     const float* cdf;       // PROPOSAL_MIXED: 330 cumulative probabilities (3 heads) per row
     const uint32_t* row;    // per chain: its row of cdf, or kNoRow (uniform moves only)
     float learned_frac;
@@ -718,8 +716,6 @@ int m6502_stoke_run(m6502_ctx* ctx, const m6502_stoke_cfg* cfg, const uint16_t* 
     prm.max_len = cfg->max_len;
     prm.chains_per_target = cpt;
     prm.seed = cfg->seed;
-    prm.stop_on_proof = cfg->stop_on_proof;
-    prm.proven = (const uint32_t*)ctx->st_proven.p;
     prm.cdf = nullptr;
     prm.row = nullptr;
     prm.learned_frac = cfg->learned_frac > 0 ? cfg->learned_frac : 0.5f;

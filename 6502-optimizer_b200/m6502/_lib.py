@@ -136,8 +136,7 @@ assert ctypes.sizeof(Tune) == 32
 TUNE_FORCE = 1
 TUNE_DEFAULT = {"exh_minb": 4, "ticket_batch": 4, "chunk_log2": 11, "join_probe": 1}
 # the candidate values m6502_autotune tries for each knob
-TUNE_CANDIDATES = {"join_probe": (0, 1), "exh_minb": (2, 3, 4), "ticket_batch": (2, 4, 8, 16),
-                   "chunk_log2": (10, 11, 12, 13)}
+TUNE_CANDIDATES = {"exh_minb": (2, 3, 4), "ticket_batch": (2, 4, 8, 16), "chunk_log2": (10, 11, 12, 13)}
 
 
 _lib = None

@@ -728,7 +728,7 @@ def run_len3(args):
         return out, start.elapsed_time(stop)
 
     # the first step builds each mask's sorted key table of the 8.2 M length-2
-    # candidates (98 MB each) and records the passes as CUDA graphs; later
+    # candidates (164 MB each) and records the passes as CUDA graphs; later
     # steps reuse both
     torch.cuda.synchronize()
     _, first_ms = timed_step()

@@ -156,9 +156,10 @@ typedef struct m6502_tune {
                                64 registers per thread) */
     uint32_t ticket_batch;  /* 1..32: pairs an exhaustive warp claims per ticket */
     uint32_t chunk_log2;    /* 9..16: states per work item of a large cone, log2 */
-    uint32_t join_probe;    /* 0 or 1, without effect: the random-state probe of MidCheck
-                               survivors always runs in a kernel of its own (inside the
-                               QuickCheck join it doubled the full length-2 search) */
+    uint32_t join_probe;    /* 0 or 1, without effect (kept for callers and cache files):
+                               the random-state probe always runs in the exhaustive kernel
+                               (inside the QuickCheck join it doubled the full length-2
+                               search) */
     uint32_t reserved[4];
 } m6502_tune;               /* 32 bytes */
 
