@@ -3785,6 +3785,16 @@ int check_cfg(m6502_ctx* ctx, const m6502_search_cfg* cfg) {
     return M6502_OK;
 }
 
+// Nothing is staged any more: a large block goes back, others stay for the next
+// search.  The C library may return a freed block of this size to the system,
+// which depends on what else the process allocated, and clearing fresh pages
+// then doubles the call (1.29 M rules, 20 MB: 5.5 ms with the block kept, 11 to
+// 12.8 where it went back).
+constexpr size_t kStagingKept = 64u << 20;
+void staging_done(m6502_ctx* ctx) {
+    if (ctx->staging.capacity() * sizeof(m6502_rule) > kStagingKept) ctx->staging.shrink_to_fit();
+}
+
 // Hands staged rules to the caller; what does not fit stays staged for the
 // next m6502_fetch_rules.
 int finish(m6502_ctx* ctx, m6502_rule* out, uint64_t cap, uint64_t* n_out) {
@@ -3794,7 +3804,7 @@ int finish(m6502_ctx* ctx, m6502_rule* out, uint64_t cap, uint64_t* n_out) {
     if (k) std::memcpy(out, ctx->staging.data(), k * sizeof(m6502_rule));
     ctx->staging.erase(ctx->staging.begin(), ctx->staging.begin() + (long)k);
     if (n > k) return set_err(ctx, M6502_E_OVERFLOW, "rule buffer too small: the rest stays staged");
-    ctx->staging.shrink_to_fit();
+    staging_done(ctx);
     return M6502_OK;
 }
 
@@ -3803,7 +3813,7 @@ int finish_search(m6502_ctx* ctx, const RuleSink& sink, uint64_t* n_out) {
     const uint64_t rest = ctx->staging.size();
     if (n_out) *n_out = sink.n + rest;
     if (rest) return set_err(ctx, M6502_E_OVERFLOW, "rule buffer too small: the rest stays staged");
-    ctx->staging.shrink_to_fit();
+    staging_done(ctx);
     return M6502_OK;
 }
 
