@@ -531,11 +531,14 @@ M6502_HD X4Row x4_row(uint32_t op) {
     return r;
 }
 
-// One instruction (insn = op | imm << 8, q = x4_row(op)) on the four states
-// in st and p.
-M6502_HD void exec_x4r(uint32_t* st, int stride, uint32_t& p, const X4Row& q, uint32_t insn) {
+// The immediate operand of an instruction (insn = op | imm << 8, q = x4_row(op)).
+M6502_HD uint32_t x4_operand(const X4Row& q, uint32_t insn) { return (insn >> 8) * q.imm + q.konst; }
+
+// One instruction (q = x4_row(op), its operand from x4_operand) on the four
+// states in st and p.
+M6502_HD void exec_x4o(uint32_t* st, int stride, uint32_t& p, const X4Row& q, uint32_t operand) {
     const uint32_t a = st[(q.ctl & 7u) * stride], mr = st[((q.ctl >> 3) & 7u) * stride];
-    const uint32_t m = (q.ctl & X4C_IMM) ? (insn >> 8) * q.imm + q.konst : mr;
+    const uint32_t m = (q.ctl & X4C_IMM) ? operand : mr;
     const uint32_t b = (q.ctl & X4C_DUP) ? a : m ^ q.inv;
     uint32_t co;
     const uint32_t sum = x4_add(a, b, (p & q.carry & kB1) | ((q.carry >> 1) & kB1), co);
@@ -568,6 +571,10 @@ M6502_HD void exec_x4r(uint32_t* st, int stride, uint32_t& p, const X4Row& q, ui
             p = (was & (0x3Du * kB1)) | (w & (0xC0u * kB1)) | (x4_zero(ra & w) >> 6);
         }
     }
+}
+
+M6502_HD void exec_x4r(uint32_t* st, int stride, uint32_t& p, const X4Row& q, uint32_t insn) {
+    exec_x4o(st, stride, p, q, x4_operand(q, insn));
 }
 
 M6502_HD uint64_t pack(const St& s) {

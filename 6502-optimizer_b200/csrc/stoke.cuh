@@ -255,12 +255,14 @@ __global__ void __launch_bounds__(64) k_stoke_epoch(StokeChain* __restrict__ cha
         st[X4S_M * 64] = vin.m; st[X4S_S0 * 64] = vin.s0; st[X4S_S1 * 64] = vin.s1;
         uint32_t p = vin.p, insn = seq[0];
         X4Row row = load_row(s_row[min(insn & 0xFFu, NUM_OPS - 1u)]);
+        uint32_t operand = x4_operand(row, insn);
         for (int i = 0; i < n; i++) {
-            const uint32_t next = seq[min(i + 1, kMaxSeq - 1)];   // it and its row in flight while this one runs
+            const uint32_t next = seq[min(i + 1, kMaxSeq - 1)];   // it, its row and operand in flight while this one runs
             const X4Row next_row = load_row(s_row[min(next & 0xFFu, NUM_OPS - 1u)]);
-            exec_x4r(st, 64, p, row, insn);
-            insn = next;
+            const uint32_t next_operand = x4_operand(next_row, next);
+            exec_x4o(st, 64, p, row, operand);
             row = next_row;
+            operand = next_operand;
         }
         const St s{st[X4S_A * 64], st[X4S_X * 64], st[X4S_Y * 64], p, st[X4S_S * 64], st[X4S_M * 64], st[X4S_S0 * 64],
                    st[X4S_S1 * 64]};
