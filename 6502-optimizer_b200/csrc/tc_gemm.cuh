@@ -139,6 +139,21 @@ __device__ __forceinline__ void load32(uint32_t* v, const void* p) {
                  "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "l"(p));
 }
 
+// 32 columns of this warp's TMEM lanes, a row per lane.
+__device__ __forceinline__ void load_slab(uint32_t (&v)[32], uint32_t addr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(addr));
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(addr + 16u));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 // The epilogue of one lane's 32 consecutive columns of one row, from TMEM
 // registers straight to global memory: every 32-byte store of a lane is one
 // whole sector, so nothing is gained by transposing through shared memory
@@ -310,33 +325,21 @@ __global__ void __launch_bounds__(kThreads) k_gemm(const __grid_constant__ CUten
             for (int c0 = 0; c0 < kBN; c0 += 32) {
                 if (n0 + c0 >= N) break;   // warp-uniform
                 const bool wide = epi.wide && n0 + c0 + 32 <= N;   // warp-uniform
-                const size_t row_o = (size_t)(r0 + lane) * epi.ldc + (size_t)(n0 + c0);
-                uint32_t act[16];
-                if (wide && epi.mode == EPI_RELU_GRAD) {   // in flight while TMEM is read
-                    // lanes past M load the last row: the warp stays converged for tcgen05.ld
-                    const __nv_bfloat16* a = epi.act + (size_t)min(r0 + lane, M - 1) * epi.ldc + (size_t)(n0 + c0);
-                    load32(act, a);
-                    load32(act + 8, a + 16);
-                }
                 uint32_t v[32];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                      "=r"(v[15])
-                    : "r"(tbase + (uint32_t)c0));
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                    : "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
-                      "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
-                      "=r"(v[30]), "=r"(v[31])
-                    : "r"(tbase + (uint32_t)c0 + 16u));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (wide) {
+                    const size_t row_o = (size_t)(r0 + lane) * epi.ldc + (size_t)(n0 + c0);
+                    uint32_t act[16];
+                    if (epi.mode == EPI_RELU_GRAD && r0 + lane < M) {   // in flight while TMEM is read
+                        load32(act, epi.act + row_o);
+                        load32(act + 8, epi.act + row_o + 16);
+                    }
+                    __syncwarp();   // lanes past M come back: tcgen05.ld takes the whole warp
+                    load_slab(v, tbase + (uint32_t)c0);
                     if (r0 + lane < M) row_epilogue(epi, out_f32, v, act, row_o, n0 + c0);
                     __syncwarp();
                     continue;
                 }
+                load_slab(v, tbase + (uint32_t)c0);
 #pragma unroll
                 for (int jj = 0; jj < 32; jj++) stage[lane * kEpiPitch + jj] = __uint_as_float(v[jj]);
                 __syncwarp();
