@@ -329,11 +329,12 @@ __global__ void __launch_bounds__(kThreads) k_gemm(const __grid_constant__ CUten
                 if (wide) {
                     const size_t row_o = (size_t)(r0 + lane) * epi.ldc + (size_t)(n0 + c0);
                     uint32_t act[16];
-                    if (epi.mode == EPI_RELU_GRAD && r0 + lane < M) {   // in flight while TMEM is read
-                        load32(act, epi.act + row_o);
-                        load32(act + 8, epi.act + row_o + 16);
+                    if (epi.mode == EPI_RELU_GRAD) {   // in flight while TMEM is read
+                        // lanes past M load the last row: the warp stays converged for tcgen05.ld
+                        const __nv_bfloat16* a = epi.act + (size_t)min(r0 + lane, M - 1) * epi.ldc + (size_t)(n0 + c0);
+                        load32(act, a);
+                        load32(act + 8, a + 16);
                     }
-                    __syncwarp();   // lanes past M come back: tcgen05.ld takes the whole warp
                     load_slab(v, tbase + (uint32_t)c0);
                     if (r0 + lane < M) row_epilogue(epi, out_f32, v, act, row_o, n0 + c0);
                     __syncwarp();
